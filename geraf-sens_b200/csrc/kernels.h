@@ -53,6 +53,7 @@ struct MfArgs {
   int64_t A, S, N;
   float fs, As;
   int dtype, mode;
+  bool direct_only = false;  // never the range cells (no room for their tables)
 };
 
 Tuning mf_forward_resolve(const MfArgs& a, const Tuning& req);
@@ -78,6 +79,17 @@ cudaError_t launch_finalize_partials(int dtype, const float2* partial, int split
 Tuning mf_backward_resolve(const MfArgs& a, const Tuning& req);
 size_t mf_backward_workspace(const MfArgs& a, const Tuning& t);
 cudaError_t mf_backward(const MfArgs& a, const Tuning& t, void* ws, cudaStream_t st);
+
+// MIXED matched filter through range cells (mf_cells.cu).  `applies` decides by
+// the sizes; the workspace then holds the cells' tables and, from
+// `partial_offset`, the partial sums (also those of the direct kernel that runs
+// in their place when *bad_flag is set on the device).
+bool mf_cells_forward_applies(const MfArgs& a);
+bool mf_cells_scale_ok(const MfArgs& a);
+size_t mf_cells_forward_workspace(const MfArgs& a, size_t direct_partial_bytes);
+size_t mf_cells_forward_partial_offset(const MfArgs& a);
+const int* mf_cells_bad_flag(void* ws);
+cudaError_t mf_cells_forward(const MfArgs& a, void* ws, cudaStream_t st);
 
 struct MfFftArgs {
   const void* real;  // forward: [A, bins] spectrum; backward: unused

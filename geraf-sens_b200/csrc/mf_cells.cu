@@ -1,0 +1,652 @@
+// MIXED matched filter through range cells (range_cells.cuh): the forward
+// evaluates each pair's sample sum as a polynomial of the path length in the
+// pair's cell, from a per-antenna table of cell coefficients.
+//
+// Launches of the forward:
+//   1. cell_prep_kernel: the voxels' bounding box (per-block partials) and the
+//      interpolation basis of every sample;
+//   2. mf_cell_table_kernel: per antenna, the cells its path lengths to the box
+//      can reach, and their coefficients;
+//   3. mf_cell_gather_kernel: the pairs;
+//   4. the direct kernel (mf_kernels.cu), which returns at once unless step 2
+//      found an antenna whose cells do not fit (more than kMaxCells, a leg beyond
+//      kMaxLeg, non-finite positions): its band is only known on the device.
+#include <algorithm>
+#include <cmath>
+
+#include "kernels.h"
+#include "range_cells.cuh"
+
+namespace geraf {
+namespace {
+
+constexpr int kMaxCells = 64;    // cells per antenna: 1.2 m of path at 4 GHz swept
+constexpr int kPrepBlocks = 256;
+constexpr int kTableThreads = 128;
+constexpr int kTableTile = 256;  // samples staged at a time by the table kernel
+
+struct CellHead {
+  int bad;  // set when some antenna's cells do not fit: the direct kernel runs instead
+  int pad[3];
+};
+
+struct AntMeta {
+  double t[4];  // -2 t, |t|^2 in units of 2^-20 m (biased, see leg_length)
+  double r[4];
+  int c0, cells;  // first cell (absolute) and number of cells
+  int same_tx;    // the transmitter equals the preceding antenna's
+  int pad;
+};
+static_assert(sizeof(AntMeta) == 80, "copied in 16-byte units");
+
+size_t up256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
+
+struct CellLayout {
+  size_t head, bbox, basis, meta, table, partial, total;
+};
+
+CellLayout cell_layout(int64_t A, int64_t S, int64_t partial_bytes) {
+  CellLayout l;
+  l.head = 0;
+  l.bbox = 256;
+  l.basis = up256(l.bbox + kPrepBlocks * 6 * sizeof(float));
+  l.meta = up256(l.basis + static_cast<size_t>(S) * GatherCells::Q * sizeof(float));
+  l.table = up256(l.meta + static_cast<size_t>(A) * sizeof(AntMeta));
+  l.partial = up256(l.table + static_cast<size_t>(A) * kMaxCells * GatherCells::Q * sizeof(float2));
+  l.total = l.partial + up256(static_cast<size_t>(partial_bytes));
+  return l;
+}
+
+// ---------------------------------------------------------------------------
+template <typename T>
+struct PrepP {
+  const T* voxel;  // [3, N]
+  int64_t N;
+  int S;
+  double theta_step;  // theta of one sample, 2 pi k1 / kappa
+  float* bbox;        // [blocks][6]
+  float* basis;       // [S][Q]
+  CellHead* head;
+};
+
+template <typename T, int Q>
+__global__ void __launch_bounds__(256) cell_prep_kernel(const PrepP<T> p) {
+  __shared__ float red[8][6];
+  const int64_t gid = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  if (gid == 0) p.head->bad = 0;
+  for (int64_t n = gid; n < p.S; n += step) {
+    float g[Q];
+    cell_basis<Q>(p.theta_step * (static_cast<double>(n) - 0.5 * (p.S - 1)), g);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) p.basis[n * Q + q] = g[q];
+  }
+  float b[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  for (int64_t v = gid; v < p.N; v += step) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float x = ld_f(p.voxel, c * p.N + v);  // fminf / fmaxf drop a NaN coordinate
+      b[c] = fminf(b[c], x);
+      b[3 + c] = fmaxf(b[3 + c], x);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float y = __shfl_xor_sync(0xffffffffu, b[c], o);
+      b[c] = c < 3 ? fminf(b[c], y) : fmaxf(b[c], y);
+    }
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][c] = b[c];
+  }
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    float r = red[0][threadIdx.x];
+    for (int w = 1; w < 8; ++w) r = threadIdx.x < 3 ? fminf(r, red[w][threadIdx.x]) : fmaxf(r, red[w][threadIdx.x]);
+    p.bbox[blockIdx.x * 6 + threadIdx.x] = r;
+  }
+}
+
+// The box over all partials, by one warp; lane c < 6 returns component c.
+__device__ __forceinline__ float warp_bbox(const float* partial, int blocks, int lane) {
+  float b[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  for (int i = lane; i < blocks; i += 32) {
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      const float y = partial[i * 6 + c];
+      b[c] = c < 3 ? fminf(b[c], y) : fmaxf(b[c], y);
+    }
+  }
+  float out = 0.0f;
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float y = __shfl_xor_sync(0xffffffffu, b[c], o);
+      b[c] = c < 3 ? fminf(b[c], y) : fmaxf(b[c], y);
+    }
+    if (lane == c) out = b[c];
+  }
+  return out;
+}
+
+// ---------------------------------------------------------------------------
+template <typename T>
+struct TableP {
+  const T* real;
+  const T* imag;
+  const T* tx;
+  const T* rx;
+  const float* bbox;
+  const float* basis;
+  AntMeta* meta;
+  float2* table;  // [A][kMaxCells][Q]
+  CellHead* head;
+  int S, blocks;
+  double k1, b1, kappa;  // kappa as rounded to FP32
+};
+
+// One block per antenna; thread (cell k, slice) sums its slice of the samples
+// into the cell's Q coefficients: the sample turned by the exact phase of the
+// cell's centre (FP64, reduced in cycles), times its basis.  About 45
+// instructions per (cell, sample): 0.6 ms for 49152 antennas x 256 samples x 40 cells.
+template <typename T>
+__global__ void __launch_bounds__(kTableThreads) mf_cell_table_kernel(const TableP<T> p) {
+  constexpr int Q = GatherCells::Q;
+  __shared__ float box_s[6];
+  __shared__ int band_s[2];
+  __shared__ float2 smp[kTableTile];
+  __shared__ float bas[kTableTile * Q];
+  __shared__ float2 red[kTableThreads * Q];
+  const int64_t a = blockIdx.x;
+  if (threadIdx.x < 32) {
+    const float b = warp_bbox(p.bbox, p.blocks, threadIdx.x);
+    if (threadIdx.x < 6) box_s[threadIdx.x] = b;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t[3], r[3], box[6];
+    AntMeta m;
+    m.t[3] = m.r[3] = 0.0;
+    double vv = 0.0;
+    bool same = a > 0;
+#pragma unroll
+    for (int c = 0; c < 6; ++c) box[c] = box_s[c];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      t[c] = ld_f(p.tx, a * 3 + c);
+      r[c] = ld_f(p.rx, a * 3 + c);
+      if (a > 0) same = same && t[c] == static_cast<double>(ld_f(p.tx, (a - 1) * 3 + c));
+      m.t[c] = -2.0 * t[c];
+      m.r[c] = -2.0 * r[c];
+      m.t[3] = fma(t[c], t[c], m.t[3]);
+      m.r[3] = fma(r[c], r[c], m.r[3]);
+      const double e = fmax(fabs(box[c]), fabs(box[3 + c]));
+      vv = fma(e, e, vv);
+    }
+    double tn, tf, rn, rf;
+    leg_range(t, box, tn, tf);
+    leg_range(r, box, rn, rf);
+    // keeps the expanded square positive; moves a leg by < 1e-14 m
+    m.t[3] += 4e-15 * (m.t[3] + vv) + 1e-18;
+    m.r[3] += 4e-15 * (m.r[3] + vv) + 1e-18;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const double u = c < 3 ? kUnit : kUnit * kUnit;
+      m.t[c] *= u;
+      m.r[c] *= u;
+    }
+    tn = sqrt(tn);
+    tf = sqrt(tf);
+    rn = sqrt(rn);
+    rf = sqrt(rf);
+    const double lo = floor((tn + rn) * p.kappa) - 2.0, hi = ceil((tf + rf) * p.kappa) + 2.0;
+    const bool fits = tf < kMaxLeg && rf < kMaxLeg && hi - lo + 1.0 <= kMaxCells;  // false for NaN
+    if (!fits) p.head->bad = 1;
+    m.c0 = fits ? static_cast<int>(lo) : 0;
+    m.cells = fits ? static_cast<int>(hi - lo) + 1 : 0;
+    m.same_tx = same ? 1 : 0;
+    m.pad = 0;
+    p.meta[a] = m;
+    band_s[0] = m.c0;
+    band_s[1] = m.cells;
+  }
+  __syncthreads();
+  const int c0 = band_s[0], nc = band_s[1];
+  if (nc == 0) return;
+  const int slices = kTableThreads / nc;  // >= 2
+  const int slice = threadIdx.x / nc;
+  const int k = threadIdx.x - slice * nc;
+  const bool on = slice < slices;
+  const double dk = fma(p.k1, static_cast<double>(c0 + k) / p.kappa, p.b1);
+  const double mid = 0.5 * (p.S - 1);
+  float2 acc[Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) acc[q] = make_float2(0.0f, 0.0f);
+  for (int n0 = 0; n0 < p.S; n0 += kTableTile) {
+    const int cnt = min(kTableTile, p.S - n0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < cnt; i += kTableThreads) {
+      smp[i] = make_float2(ld_f(p.real, a * p.S + n0 + i), ld_f(p.imag, a * p.S + n0 + i));
+    }
+    for (int i = threadIdx.x; i < cnt * Q; i += kTableThreads) bas[i] = p.basis[n0 * Q + i];
+    __syncthreads();
+    if (on) {
+      for (int i = slice; i < cnt; i += slices) {
+        const double c = (static_cast<double>(n0 + i) - mid) * dk;
+        const float2 e = cis_cycles(static_cast<float>(c - rint(c)));
+        const float2 x = smp[i];
+        // v = x e^{-j phase}; odd powers carry -j v
+        const float2 v = make_float2(fmaf(x.x, e.x, x.y * e.y), fmaf(x.y, e.x, -x.x * e.y));
+        const float2 w = make_float2(v.y, -v.x);
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          const float g = bas[i * Q + q];
+          acc[q] = ffma2(make_float2(g, g), (q & 1) ? w : v, acc[q]);
+        }
+      }
+    }
+  }
+  if (on) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) red[(slice * nc + k) * Q + q] = acc[q];
+  }
+  __syncthreads();
+  float2* out = p.table + a * kMaxCells * Q;
+  for (int i = threadIdx.x; i < nc * Q; i += kTableThreads) {
+    float2 s = red[i];
+    for (int sl = 1; sl < slices; ++sl) s = fadd2(s, red[sl * nc * Q + i]);
+    out[i] = s;
+  }
+}
+
+// ---------------------------------------------------------------------------
+template <typename T>
+struct GatherCellsP {
+  const T* voxel;
+  T* out_r;
+  T* out_i;
+  const AntMeta* meta;
+  const float2* table;
+  float2* partial;
+  const CellHead* head;
+  int* status;
+  int64_t A, N;
+  int splits;
+  int64_t ant_per_split;
+  float kappa;  // cells per metre
+  PairPhase ph;
+};
+
+constexpr int kCellBytes = GatherCells::Q * sizeof(float2);  // 48
+constexpr int kRowBytes = kMaxCells * kCellBytes;            // 3072
+// Launch shape of the gather.  Measured on 49152 antennas x 512000 voxels: 52.7 ms; 2 voxels
+// per thread with 5 blocks per SM 65.2, 6 voxels with 2 blocks 59.0; stages of 4 antennas 75.1,
+// of up to 16 antennas (8 KB pool) 53.9.
+constexpr int kGatherVpt = 4;         // voxels per thread
+constexpr int kGatherThreads = 128;   // consumer threads; one more warp copies
+constexpr int kGatherBlocks = 3;      // resident per SM (128 registers)
+constexpr int kGatherRows = 32;       // antennas per stage, at most
+constexpr int kGatherStages = 3;
+constexpr int kGatherPool = 16384;    // bytes of cells per stage
+static_assert(kGatherPool >= kRowBytes, "any one antenna's cells fit");
+
+struct GatherSmem {
+  uint64_t full[kGatherStages];
+  uint64_t empty[kGatherStages];
+  int base[kGatherStages][kGatherRows];  // byte offset of the row's absolute cell 0, magic bits subtracted
+  int count[kGatherStages];              // antennas in the stage
+  float box[8];
+  float red[4][8];
+  alignas(16) AntMeta meta[kGatherStages][kGatherRows];
+  alignas(16) unsigned char pool[kGatherStages][kGatherPool];
+};
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// VPT voxels per thread; stages of up to kGatherRows antennas stream through a ring filled
+// by a warp of its own.  Of each antenna's cells a stage holds those that the
+// block's voxels can reach (their own bounding box): one bulk copy per antenna
+// row.  A pair is two legs (the transmitter's only where it differs from the
+// preceding antenna's: the virtual channels of one transmitter follow one
+// another), the phase, one sincos, three 16-byte shared loads and five packed
+// multiply-adds.  Terms are summed plainly within a stage and compensated across
+// stages.
+//
+// About 61 instructions per 32 pairs, of which the FP64 ones take 21 issue cycles
+// of their pipe, the rsqrt, sine and cosine 26 of theirs and the 16-byte loads (four
+// wavefronts each whatever the addresses) 48 of a scheduler's 78 cycles per 32
+// pairs (ncu, 3072 x 110592 pairs): shared-memory bandwidth comes first, then the
+// latency of the FP64 chains, which is why 4 voxels per thread with few warps beat
+// more warps with fewer.  49152 antennas x 256 samples x 512000 voxels: 950 ms by
+// the direct kernel, 52.7 ms through the cells (478 G pairs/s); 3072 x 128 x
+// 110592: 7.53 ms against 0.79 ms.
+template <typename T>
+__global__ void __launch_bounds__(kGatherThreads + 32, kGatherBlocks) mf_cell_gather_kernel(const GatherCellsP<T> p) {
+  constexpr int VPT = kGatherVpt;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  GatherSmem& sm = *reinterpret_cast<GatherSmem*>(smem_raw);
+  if (p.head->bad) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool producer = warp == kGatherThreads / 32;
+  // split-major blocks: those resident together stream the same antennas' rows
+  const int64_t vtiles = gridDim.x / p.splits;
+  const int split = static_cast<int>(blockIdx.x / vtiles);
+  const int64_t vtile = blockIdx.x - static_cast<int64_t>(split) * vtiles;
+  const int64_t a_begin = static_cast<int64_t>(split) * p.ant_per_split;
+  const int64_t a_end = min(p.A, a_begin + p.ant_per_split);
+  const int num_ant = static_cast<int>(max(int64_t{0}, a_end - a_begin));
+
+  float fx[VPT], fy[VPT], fz[VPT];
+  int64_t vid[VPT];
+  unsigned nan_voxel = 0;  // bit j: a NaN coordinate, whose result is NaN
+  {
+    float b[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+      vid[j] = vtile * (kGatherThreads * VPT) + threadIdx.x + j * kGatherThreads;
+      const int64_t v = min(vid[j], p.N - 1);
+      fx[j] = fy[j] = fz[j] = 0.0f;
+      if (producer) continue;
+      fx[j] = ld_f(p.voxel, v);
+      fy[j] = ld_f(p.voxel, p.N + v);
+      fz[j] = ld_f(p.voxel, 2 * p.N + v);
+      if (fx[j] != fx[j] || fy[j] != fy[j] || fz[j] != fz[j]) {
+        nan_voxel |= 1u << j;
+      } else {
+        b[0] = fminf(b[0], fx[j]);
+        b[1] = fminf(b[1], fy[j]);
+        b[2] = fminf(b[2], fz[j]);
+        b[3] = fmaxf(b[3], fx[j]);
+        b[4] = fmaxf(b[4], fy[j]);
+        b[5] = fmaxf(b[5], fz[j]);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float y = __shfl_xor_sync(0xffffffffu, b[c], o);
+        b[c] = c < 3 ? fminf(b[c], y) : fmaxf(b[c], y);
+      }
+      if (lane == 0 && !producer) sm.red[warp][c] = b[c];
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+      float r = sm.red[0][threadIdx.x];
+#pragma unroll
+      for (int w = 1; w < kGatherThreads / 32; ++w) {
+        r = threadIdx.x < 3 ? fminf(r, sm.red[w][threadIdx.x]) : fmaxf(r, sm.red[w][threadIdx.x]);
+      }
+      sm.box[threadIdx.x] = r;
+    }
+    if (threadIdx.x == 32) {
+      for (int s = 0; s < kGatherStages; ++s) {
+        mbar_init(&sm.full[s], 32);  // every lane of the copying warp arrives, with its bytes
+        mbar_init(&sm.empty[s], kGatherThreads / 32);
+      }
+      fence_barrier_init();
+    }
+    __syncthreads();
+  }
+  const bool any_valid = sm.box[0] <= sm.box[3];  // else every voxel of the block is NaN
+
+  if (producer) {
+    if (!any_valid) return;
+    for (int t = 0, done = 0; done < num_ant; ++t) {
+      const int s = t % kGatherStages, use = t / kGatherStages;
+      const int64_t a0 = a_begin + done;
+      uint32_t bytes = 0;
+      int lo = 0, c0 = 0;
+      if (lane < kGatherRows && lane < num_ant - done) {
+        const AntMeta& m = p.meta[a0 + lane];
+        float tp[3], rp[3], tn, tf, rn, rf;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          tp[c] = static_cast<float>(-0.5 / kUnit * m.t[c]);
+          rp[c] = static_cast<float>(-0.5 / kUnit * m.r[c]);
+        }
+        c0 = m.c0;
+        leg_range(tp, sm.box, tn, tf);
+        leg_range(rp, sm.box, rn, rf);
+        // one cell of margin on either side covers the FP32 rounding (~1e-4 cells)
+        lo = static_cast<int>(floorf((sqrtf(tn) + sqrtf(rn)) * p.kappa)) - 1 - c0;
+        int hi = static_cast<int>(ceilf((sqrtf(tf) + sqrtf(rf)) * p.kappa)) + 1 - c0;
+        lo = min(max(lo, 0), m.cells - 1);
+        hi = min(max(hi, lo), m.cells - 1);
+        bytes = static_cast<uint32_t>(hi - lo + 1) * kCellBytes;
+      }
+      uint32_t end = bytes;  // of the antenna's cells in the stage's pool
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= o) end += y;
+      }
+      const bool in = bytes != 0 && end <= kGatherPool;
+      const int count = __popc(__ballot_sync(0xffffffffu, in));  // the first ones: `end` grows with the lane
+      if (use > 0 && !__all_sync(0xffffffffu, mbar_wait_bounded(&sm.empty[s], (use - 1) & 1, p.status))) {
+        // the consumers gave up: wait for the copies still in flight
+        for (int u = max(0, t - kGatherStages); u < t; ++u) {
+          mbar_wait_bounded(&sm.full[u % kGatherStages], (u / kGatherStages) & 1, p.status);
+        }
+        return;
+      }
+      if (in) {
+        // byte offset of absolute cell k: base + (bits of k + magic) * 48, modulo 2^32
+        sm.base[s][lane] = static_cast<int>(static_cast<uint32_t>(s * kGatherPool) + end - bytes -
+                                            (static_cast<uint32_t>(c0 + lo) + kRoundMagicBits) * kCellBytes);
+      }
+      if (lane == 0) sm.count[s] = count;
+      const uint32_t meta_bytes = lane == 0 ? count * static_cast<uint32_t>(sizeof(AntMeta)) : 0;
+      mbar_arrive_expect_tx(&sm.full[s], (in ? bytes : 0) + meta_bytes);  // releases sm.base and sm.count too
+      if (lane == 0) bulk_g2s(&sm.meta[s][0], p.meta + a0, meta_bytes, &sm.full[s]);
+      if (in) {
+        bulk_g2s(&sm.pool[s][end - bytes],
+                 reinterpret_cast<const unsigned char*>(p.table) + (a0 + lane) * kRowBytes + lo * kCellBytes, bytes,
+                 &sm.full[s]);
+      }
+      done += count;
+    }
+    return;
+  }
+
+  // NaN voxels take the corner of the box, so that their cells stay in the rows
+  double vx[VPT], vy[VPT], vz[VPT], vv[VPT];
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) {
+    const bool nan = (nan_voxel >> j) & 1u;
+    vx[j] = static_cast<double>(nan ? sm.box[0] : fx[j]) * kUnit;
+    vy[j] = static_cast<double>(nan ? sm.box[1] : fy[j]) * kUnit;
+    vz[j] = static_cast<double>(nan ? sm.box[2] : fz[j]) * kUnit;
+    vv[j] = fma(vx[j], vx[j], fma(vy[j], vy[j], vz[j] * vz[j]));
+  }
+  float yr[VPT], yi[VPT], cr[VPT], ci[VPT];
+  float dt[VPT], lt[VPT];  // the transmitter's legs
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) yr[j] = yi[j] = cr[j] = ci[j] = dt[j] = lt[j] = 0.0f;
+
+  for (int t = 0, done = 0; any_valid && done < num_ant; ++t) {
+    const int s = t % kGatherStages;
+    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&sm.full[s], (t / kGatherStages) & 1, p.status))) return;
+    const int rws = sm.count[s];
+    done += rws;
+    float tr[VPT], ti[VPT];
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) tr[j] = ti[j] = 0.0f;
+    for (int r = 0; r < rws; ++r) {
+      const AntMeta& m = sm.meta[s][r];
+      if (!m.same_tx || (t == 0 && r == 0)) {
+        const double2 t0 = *reinterpret_cast<const double2*>(&m.t[0]);
+        const double2 t1 = *reinterpret_cast<const double2*>(&m.t[2]);
+#pragma unroll
+        for (int j = 0; j < VPT; ++j) {
+          const Leg g = leg_length(t0.x, t0.y, t1.x, t1.y, vx[j], vy[j], vz[j], vv[j]);
+          dt[j] = g.d;
+          lt[j] = g.l;
+        }
+      }
+      const double2 r0 = *reinterpret_cast<const double2*>(&m.r[0]);
+      const double2 r1 = *reinterpret_cast<const double2*>(&m.r[2]);
+      const unsigned char* rows = &sm.pool[0][0];
+      const uint32_t base = static_cast<uint32_t>(sm.base[s][r]);
+#pragma unroll
+      for (int j = 0; j < VPT; ++j) {
+        const Leg g = leg_length(r0.x, r0.y, r1.x, r1.y, vx[j], vy[j], vz[j], vv[j]);
+        const float hi = dt[j] + g.d, lo = lt[j] + g.l;
+        const CellPos c = pair_cell(p.ph, hi, lo);
+        const float4* q = reinterpret_cast<const float4*>(
+            rows + static_cast<uint32_t>(__float_as_uint(c.m) * static_cast<uint32_t>(kCellBytes) + base));
+        const float4 q2 = q[2], q1 = q[1], q0 = q[0];
+        const float2 xx = make_float2(c.x, c.x);
+        float2 acc = ffma2(make_float2(q2.z, q2.w), xx, make_float2(q2.x, q2.y));
+        acc = ffma2(acc, xx, make_float2(q1.z, q1.w));
+        acc = ffma2(acc, xx, make_float2(q1.x, q1.y));
+        acc = ffma2(acc, xx, make_float2(q0.z, q0.w));
+        acc = ffma2(acc, xx, make_float2(q0.x, q0.y));
+        float sn, cs;
+        __sincosf(6.28318530717958647692f * pair_cycles(p.ph, hi, lo), &sn, &cs);
+        tr[j] = fmaf(cs, acc.x, fmaf(sn, acc.y, tr[j]));
+        ti[j] = fmaf(cs, acc.y, fmaf(-sn, acc.x, ti[j]));
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+      kahan_add(yr[j], cr[j], tr[j]);
+      kahan_add(yi[j], ci[j], ti[j]);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sm.empty[s]);
+  }
+
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) {
+    if (vid[j] >= p.N) continue;
+    if ((nan_voxel >> j) & 1u) yr[j] = yi[j] = NAN;
+    if (p.splits == 1) {
+      p.out_r[vid[j]] = from_f<T>(yr[j] / static_cast<float>(p.A));
+      p.out_i[vid[j]] = from_f<T>(yi[j] / static_cast<float>(p.A));
+    } else {
+      p.partial[split * p.N + vid[j]] = make_float2(yr[j], yi[j]);
+    }
+  }
+}
+
+double cells_per_metre(double k1, int64_t S, int over) {
+  return static_cast<double>(static_cast<float>(over * static_cast<double>(S) * std::fabs(k1)));
+}
+
+int gather_splits(int64_t A, int64_t N) {
+  const int64_t vtiles = (N + kGatherThreads * kGatherVpt - 1) / (kGatherThreads * kGatherVpt);
+  const int64_t stages = std::max<int64_t>(1, (A + kGatherRows - 1) / kGatherRows);
+  return std::max(1, std::min<int>(pick_splits(vtiles, kGatherBlocks, current_device_info().sm_count, stages),
+                                   static_cast<int>(std::min<int64_t>(stages, 256))));
+}
+
+template <typename T>
+cudaError_t launch_cells_forward(const MfArgs& a, unsigned char* ws, const CellLayout& l, int splits, cudaStream_t st) {
+  const PhaseConsts pc = phase_consts(kMfStartFrequency, a.As, a.fs);
+  const double kappa = cells_per_metre(pc.k1, a.S, GatherCells::kOver);
+  CellHead* head = reinterpret_cast<CellHead*>(ws + l.head);
+  float* bbox = reinterpret_cast<float*>(ws + l.bbox);
+  float* basis = reinterpret_cast<float*>(ws + l.basis);
+  AntMeta* meta = reinterpret_cast<AntMeta*>(ws + l.meta);
+  float2* table = reinterpret_cast<float2*>(ws + l.table);
+  const int pb = static_cast<int>(std::min<int64_t>(kPrepBlocks, (std::max<int64_t>(a.N, a.S) + 255) / 256));
+
+  PrepP<T> pp;
+  pp.voxel = static_cast<const T*>(a.voxel);
+  pp.N = a.N;
+  pp.S = static_cast<int>(a.S);
+  pp.theta_step = 2.0 * M_PI * pc.k1 / kappa;
+  pp.bbox = bbox;
+  pp.basis = basis;
+  pp.head = head;
+  cell_prep_kernel<T, GatherCells::Q><<<pb, 256, 0, st>>>(pp);
+
+  TableP<T> tp;
+  tp.real = static_cast<const T*>(a.real);
+  tp.imag = static_cast<const T*>(a.imag);
+  tp.tx = static_cast<const T*>(a.tx);
+  tp.rx = static_cast<const T*>(a.rx);
+  tp.bbox = bbox;
+  tp.basis = basis;
+  tp.meta = meta;
+  tp.table = table;
+  tp.head = head;
+  tp.S = pp.S;
+  tp.blocks = pb;
+  tp.k1 = pc.k1;
+  tp.b1 = pc.b1;
+  tp.kappa = kappa;
+  mf_cell_table_kernel<T><<<static_cast<unsigned>(a.A), kTableThreads, 0, st>>>(tp);
+  cudaError_t err = cudaGetLastError();
+  if (err != cudaSuccess) return err;
+
+  GatherCellsP<T> gp;
+  gp.voxel = pp.voxel;
+  gp.out_r = static_cast<T*>(a.out_real);
+  gp.out_i = static_cast<T*>(a.out_imag);
+  gp.meta = meta;
+  gp.table = table;
+  gp.partial = reinterpret_cast<float2*>(ws + l.partial);
+  gp.head = head;
+  gp.status = device_status_ptr();
+  gp.A = a.A;
+  gp.N = a.N;
+  gp.splits = splits;
+  const int64_t stages = (a.A + kGatherRows - 1) / kGatherRows;
+  gp.ant_per_split = ((stages + splits - 1) / splits) * kGatherRows;
+  gp.kappa = static_cast<float>(kappa);
+  gp.ph = pair_phase(pc.k0, pc.b0, pc.k1, pc.b1, a.S, kappa);
+  const void* fn = reinterpret_cast<const void*>(&mf_cell_gather_kernel<T>);
+  const int smem = static_cast<int>(sizeof(GatherSmem));
+  err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (err != cudaSuccess) return err;
+  const int64_t vtiles = (a.N + kGatherThreads * kGatherVpt - 1) / (kGatherThreads * kGatherVpt);
+  if (vtiles * splits > 0x7fffffff) return cudaErrorInvalidConfiguration;
+  void* args[] = {&gp};
+  err = cudaLaunchKernel(fn, dim3(static_cast<unsigned>(vtiles * splits)), dim3(kGatherThreads + 32), args, smem, st);
+  if (err != cudaSuccess || splits == 1) return err;
+  return launch_finalize_partials(a.dtype, gp.partial, splits, a.N, static_cast<float>(a.A), a.out_real, a.out_imag, st);
+}
+
+}  // namespace
+
+// The cells take over where the pairs outweigh the tables and the extra
+// launches: enough voxels per table row, and a direct call of more than ~20 us.
+// Calls of up to 128 antennas, the size of a training step's chunk, keep the
+// direct kernel: the gradient of |y| divides by |y|, which turns the ~2e-6 between
+// the two kernels (the direct one's error near theta = 0) into 3e-5 of the
+// gradients, more than a training run should move by from one release to the next.
+bool mf_cells_forward_applies(const MfArgs& a) {
+  return a.mode == kMixed && !a.direct_only && a.dtype != kF64 && a.S >= 32 && a.S <= 4096 && a.N >= 512 &&
+         a.A > 128 && static_cast<double>(a.A) * a.N * a.S >= 1.0e8;
+}
+
+size_t mf_cells_forward_workspace(const MfArgs& a, size_t direct_partial_bytes) {
+  const int splits = gather_splits(a.A, a.N);
+  const size_t partial = splits > 1 ? static_cast<size_t>(splits) * a.N * sizeof(float2) : 0;
+  return cell_layout(a.A, a.S, static_cast<int64_t>(std::max(partial, direct_partial_bytes))).total;
+}
+
+size_t mf_cells_forward_partial_offset(const MfArgs& a) { return cell_layout(a.A, a.S, 0).partial; }
+
+bool mf_cells_scale_ok(const MfArgs& a) {
+  const PhaseConsts pc = phase_consts(kMfStartFrequency, a.As, a.fs);
+  const double kappa = GatherCells::kOver * static_cast<double>(a.S) * std::fabs(pc.k1);
+  return std::isfinite(kappa) && kappa >= 1e-2 && kappa <= 1e5;
+}
+
+const int* mf_cells_bad_flag(void* ws) { return &static_cast<CellHead*>(ws)->bad; }
+
+cudaError_t mf_cells_forward(const MfArgs& a, void* ws, cudaStream_t st) {
+  const int splits = gather_splits(a.A, a.N);
+  const CellLayout l = cell_layout(a.A, a.S, 0);
+  unsigned char* base = static_cast<unsigned char*>(ws);
+  if (a.dtype == kF16) return launch_cells_forward<__half>(a, base, l, splits, st);
+  return launch_cells_forward<float>(a, base, l, splits, st);
+}
+
+}  // namespace geraf

@@ -71,6 +71,7 @@ struct MfFwdP {
   int rows, ld, splits, bulk;
   int64_t ant_per_split;
   size_t pos_off, kn_off, buf_off, dup_off;
+  const int* run_if;  // MIXED: when set, the kernel runs only if *run_if != 0
 };
 
 __device__ __forceinline__ float sq(float x) { return x * x; }
@@ -99,6 +100,7 @@ __global__ void __launch_bounds__(256) mf_fwd_mixed_kernel(const MfFwdP<T> p) {
   double* pos = reinterpret_cast<double*>(smem + p.pos_off);
   float2* dup = reinterpret_cast<float2*>(smem + p.dup_off);  // [rows][ld] interleaved (re, im)
   PairStager<T> stg{reinterpret_cast<T*>(smem + p.buf_off), bar, p.ld, p.rows, p.bulk != 0};
+  if (p.run_if != nullptr && *p.run_if == 0) return;
 
   // Split-major block order: the blocks resident at one time work on the same
   // antenna split, so the IF rows they stream (A/splits of them) stay in L2.
@@ -387,7 +389,9 @@ __global__ void __launch_bounds__(256) mf_fwd_plain_kernel(const MfFwdP<T> p) {
 // and divides by `divisor`.
 template <typename T>
 __global__ void finalize_partials_kernel(const float2* __restrict__ partial, int splits,
-                                         int64_t count, float divisor, T* out_r, T* out_i) {
+                                         int64_t count, float divisor, T* out_r, T* out_i,
+                                         const int* run_if = nullptr) {
+  if (run_if != nullptr && *run_if == 0) return;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < count;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     double sr = 0.0, si = 0.0;
@@ -738,8 +742,9 @@ FwdShape fwd_shape(const MfArgs& a, const Tuning& t) {
 }
 
 template <typename T>
-cudaError_t launch_fwd(const MfArgs& a, const FwdShape& s, void* ws, cudaStream_t st) {
+cudaError_t launch_fwd(const MfArgs& a, const FwdShape& s, void* ws, cudaStream_t st, const int* run_if) {
   MfFwdP<T> p;
+  p.run_if = run_if;
   p.real = static_cast<const T*>(a.real);
   p.imag = static_cast<const T*>(a.imag);
   p.tx = static_cast<const T*>(a.tx);
@@ -783,7 +788,7 @@ cudaError_t launch_fwd(const MfArgs& a, const FwdShape& s, void* ws, cudaStream_
   if (s.splits > 1) {
     const int fin_blocks = static_cast<int>(std::min<int64_t>((a.N + 255) / 256, 148 * 16));
     finalize_partials_kernel<T><<<std::max(fin_blocks, 1), 256, 0, st>>>(
-        p.partial, s.splits, a.N, static_cast<float>(a.A), p.out_r, p.out_i);
+        p.partial, s.splits, a.N, static_cast<float>(a.A), p.out_r, p.out_i, run_if);
     err = cudaGetLastError();
   }
   return err;
@@ -982,18 +987,25 @@ Tuning mf_forward_resolve(const MfArgs& a, const Tuning& req) {
 
 size_t mf_forward_workspace(const MfArgs& a, const Tuning& t) {
   if (a.mode == kNufft) return mf_nufft_forward_workspace(a, t);
-  if (t.splits <= 1 || a.N == 0) return 0;
-  return static_cast<size_t>(t.splits) * a.N * sizeof(float2);
+  const size_t partial = t.splits <= 1 || a.N == 0 ? 0 : static_cast<size_t>(t.splits) * a.N * sizeof(float2);
+  return mf_cells_forward_applies(a) ? mf_cells_forward_workspace(a, partial) : partial;
 }
 
 cudaError_t mf_forward(const MfArgs& a, const Tuning& t, void* ws, cudaStream_t st) {
   if (a.mode == kNufft) return mf_nufft_forward(a, t, ws, st);
   if (a.N == 0) return cudaSuccess;
+  const int* run_if = nullptr;
+  if (mf_cells_forward_applies(a) && mf_cells_scale_ok(a)) {
+    const cudaError_t err = mf_cells_forward(a, ws, st);
+    if (err != cudaSuccess) return err;
+    run_if = mf_cells_bad_flag(ws);
+    ws = static_cast<unsigned char*>(ws) + mf_cells_forward_partial_offset(a);
+  }
   const FwdShape s = fwd_shape(a, t);
   switch (a.dtype) {
-    case kF64: return launch_fwd<double>(a, s, ws, st);
-    case kF16: return launch_fwd<__half>(a, s, ws, st);
-    default: return launch_fwd<float>(a, s, ws, st);
+    case kF64: return launch_fwd<double>(a, s, ws, st, run_if);
+    case kF16: return launch_fwd<__half>(a, s, ws, st, run_if);
+    default: return launch_fwd<float>(a, s, ws, st, run_if);
   }
 }
 

@@ -113,6 +113,7 @@ GERAF_EXPORT int32_t geraf_mf_forward_noalloc(const void* real, const void* imag
   a.As = chirp_slope_scaled;
   a.dtype = kF32;
   a.mode = kMixed;
+  a.direct_only = true;
   Tuning t = mf_forward_resolve(a, Tuning{});
   // Always the split variant: at least two partial sums per voxel, as many as fit.
   const int64_t rows_total = std::max<int64_t>(1, (a.A + t.stage_rows - 1) / t.stage_rows);

@@ -1,0 +1,117 @@
+"""The MIXED matched filter through range cells, at sizes large enough to take it,
+against the FP64 oracle.
+
+Tolerance: the interpolation of the sample sums errs by at most 1.6e-7 per
+sample, the hardware sine and cosine by 4e-7, the phase by ~1e-7 cycles
+(6e-7 rad), the FP32 sums by a few 1e-7; 2e-6 covers their sum."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import rel_l2
+from benchkit import scenes
+from gpu_helpers import cu, mf_backward, mf_forward
+from oracle import rf_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+TOL = 2e-6
+
+
+def box_points(rng, n, lo=(-0.1, -0.1, 0.3), hi=(0.1, 0.1, 0.5)):
+    return np.ascontiguousarray(rng.uniform(lo, hi, (n, 3)).T.astype(np.float32))
+
+
+def signal(rng, tx, rx, ch, extent=1.0, snr=20.0):
+    pos = rng.uniform((-0.1, -0.1, 0.3), (0.1, 0.1, 0.5), (6, 3)) * extent
+    amp = rng.standard_normal(6) + 1j * rng.standard_normal(6)
+    return scenes.synthesize_if_numpy(tx, rx, pos.astype(np.float32), amp, ch, snr_db=snr, rng=rng)
+
+
+def case(seed, A, S, N, shuffle=False, box=None, bandwidth=4e9):
+    rng = np.random.default_rng(seed)
+    tx, rx = scenes.virtual_array(int(np.ceil(np.sqrt(A / 12))))
+    pick = rng.permutation(tx.shape[0])[:A] if shuffle else np.arange(A)
+    tx, rx = np.ascontiguousarray(tx[pick]), np.ascontiguousarray(rx[pick])
+    ch = scenes.chirp(S, bandwidth=bandwidth)
+    re, im = signal(rng, tx, rx, ch)
+    return dict(re=re, im=im, tx=tx, rx=rx, ch=ch, vox=box_points(rng, N, *(box or ())), rng=rng)
+
+
+def oracle(c):
+    ch = c["ch"]
+    r = orc.mf_forward(c["re"], c["im"], c["tx"], c["rx"], c["vox"], ch.adc_sample_rate, ch.As_sci)
+    return r[0] + 1j * r[1]
+
+
+def forward(c, **kw):
+    ch = c["ch"]
+    y = mf_forward(c["re"], c["im"], c["tx"], c["rx"], c["vox"], ch.adc_sample_rate, ch.As_sci, "mixed", **kw)
+    return y[0] + 1j * y[1]
+
+
+# (antennas, samples, voxels): remainders of the 8-antenna stages, of the 256-sample
+# table tiles, of the 512-voxel blocks; the smallest voxel count; long rows
+SHAPES = [(1000, 200, 512), (1001, 199, 513), (131, 33, 24000), (197, 256, 4097), (148, 257, 3000), (132, 1025, 800),
+          (130, 4096, 515), (129, 256, 40000)]
+
+
+@pytest.mark.parametrize("shuffle", [False, True], ids=["mimo_order", "shuffled"])
+@pytest.mark.parametrize("A,S,N", SHAPES)
+def test_forward_vs_fp64(cuda, A, S, N, shuffle):
+    c = case(A + S, A, S, N, shuffle)
+    assert rel_l2(forward(c), oracle(c)) < TOL
+
+
+@pytest.mark.parametrize("splits", [1, 5])
+def test_forward_takes_any_tuning(cuda, splits):
+    c = case(3, 144, 128, 9001)
+    assert rel_l2(forward(c, tuning={"threads": 256, "items_per_thread": 2, "splits": splits}), oracle(c)) < TOL
+
+
+@pytest.mark.parametrize("box,bandwidth", [(((-0.5, -0.5, 0.2), (0.5, 0.5, 1.6)), 4e9),   # more cells than fit
+                                           (((-0.1, -0.1, 8.2), (0.1, 0.1, 8.4)), 1e9),   # legs beyond 8 m
+                                           (((-0.1, -0.1, 3.9), (0.1, 0.1, 4.1)), 4e9)],  # long legs, narrow band
+                         ids=["wide_band", "long_legs", "far_scene"])
+def test_forward_bands_that_leave_the_cells(cuda, box, bandwidth):
+    """The band is known on the device only: scenes whose cells do not fit run the direct kernel."""
+    c = case(8, 140, 256, 4000, box=box, bandwidth=bandwidth)
+    pos = c["rng"].uniform(box[0], box[1], (6, 3)).astype(np.float32)
+    c["re"], c["im"] = scenes.synthesize_if_numpy(c["tx"], c["rx"], pos, np.ones(6) + 0.5j, c["ch"], snr_db=20.0,
+                                                  rng=c["rng"])
+    # the direct kernel's own error grows with the phase step: its bound is the MIXED form's
+    assert rel_l2(forward(c), oracle(c)) < 1e-5
+
+
+def test_forward_without_a_sweep_and_with_a_falling_one(cuda):
+    c = case(5, 140, 128, 6000)
+    for As in (0.0, -c["ch"].As_sci):
+        args = (c["re"], c["im"], c["tx"], c["rx"], c["vox"], c["ch"].adc_sample_rate, As)
+        y, r = mf_forward(*args, "mixed"), orc.mf_forward(*args)
+        assert rel_l2(y[0] + 1j * y[1], r[0] + 1j * r[1]) < 1e-5
+
+
+def test_forward_half_inputs(cuda):
+    c = case(6, 140, 128, 6001)
+    r = {k: c[k].astype(np.float16).astype(np.float32) for k in ("re", "im", "tx", "rx", "vox")}
+    ref = oracle({**c, **r})
+    assert rel_l2(forward(c, dtype=torch.float16), ref) < 2e-3  # half-precision outputs
+
+
+def test_forward_non_finite_inputs(cuda):
+    """A NaN voxel gives NaN there and leaves the others alone; a voxel or antenna at infinity
+    runs the direct kernel; a voxel on an antenna stays finite."""
+    c = case(7, 140, 128, 6002)
+    ref = oracle(c)
+    c["vox"][1, 77] = np.nan
+    c["vox"][:, 600] = c["tx"][5]
+    ref600 = oracle({**c, "vox": np.ascontiguousarray(c["vox"][:, 600:601] + np.float32(1e-7))})
+    y = forward(c)
+    assert np.isnan(y[77].real) and np.isnan(y[77].imag)
+    keep = np.setdiff1d(np.arange(y.size), [77, 600])
+    assert rel_l2(y[keep], ref[keep]) < TOL
+    assert np.isfinite(y[600]) and abs(y[600] - ref600[0]) < 1e-2 * np.abs(ref).max()
+    c["vox"][1, 77] = np.inf
+    y = forward(c)
+    keep = np.setdiff1d(np.arange(y.size), [77, 600])
+    assert rel_l2(y[keep], ref[keep]) < 1e-5 and not np.isfinite(y[77])
