@@ -90,6 +90,11 @@ size_t mf_cells_forward_workspace(const MfArgs& a, size_t direct_partial_bytes);
 size_t mf_cells_forward_partial_offset(const MfArgs& a);
 const int* mf_cells_bad_flag(void* ws);
 cudaError_t mf_cells_forward(const MfArgs& a, void* ws, cudaStream_t st);
+bool mf_cells_backward_applies(const MfArgs& a);
+size_t mf_cells_backward_workspace(const MfArgs& a, size_t direct_partial_bytes);
+size_t mf_cells_backward_partial_offset(const MfArgs& a);
+const int* mf_moments_bad_flag(void* ws);
+cudaError_t mf_cells_backward(const MfArgs& a, void* ws, cudaStream_t st);
 
 struct MfFftArgs {
   const void* real;  // forward: [A, bins] spectrum; backward: unused

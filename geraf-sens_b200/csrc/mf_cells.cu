@@ -20,7 +20,7 @@
 namespace geraf {
 namespace {
 
-constexpr int kMaxCells = 64;    // cells per antenna: 1.2 m of path at 4 GHz swept
+constexpr int kMaxCells = 96;    // cells per antenna: 1.8 m of path at 4 GHz swept
 constexpr int kPrepBlocks = 256;
 constexpr int kTableThreads = 128;
 constexpr int kTableTile = 256;  // samples staged at a time by the table kernel
@@ -167,7 +167,6 @@ __global__ void __launch_bounds__(kTableThreads) mf_cell_table_kernel(const Tabl
   if (threadIdx.x == 0) {
     double t[3], r[3], box[6];
     AntMeta m;
-    m.t[3] = m.r[3] = 0.0;
     double vv = 0.0;
     bool same = a > 0;
 #pragma unroll
@@ -177,25 +176,14 @@ __global__ void __launch_bounds__(kTableThreads) mf_cell_table_kernel(const Tabl
       t[c] = ld_f(p.tx, a * 3 + c);
       r[c] = ld_f(p.rx, a * 3 + c);
       if (a > 0) same = same && t[c] == static_cast<double>(ld_f(p.tx, (a - 1) * 3 + c));
-      m.t[c] = -2.0 * t[c];
-      m.r[c] = -2.0 * r[c];
-      m.t[3] = fma(t[c], t[c], m.t[3]);
-      m.r[3] = fma(r[c], r[c], m.r[3]);
       const double e = fmax(fabs(box[c]), fabs(box[3 + c]));
       vv = fma(e, e, vv);
     }
+    leg_antenna(t, vv, m.t);
+    leg_antenna(r, vv, m.r);
     double tn, tf, rn, rf;
     leg_range(t, box, tn, tf);
     leg_range(r, box, rn, rf);
-    // keeps the expanded square positive; moves a leg by < 1e-14 m
-    m.t[3] += 4e-15 * (m.t[3] + vv) + 1e-18;
-    m.r[3] += 4e-15 * (m.r[3] + vv) + 1e-18;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const double u = c < 3 ? kUnit : kUnit * kUnit;
-      m.t[c] *= u;
-      m.r[c] *= u;
-    }
     tn = sqrt(tn);
     tf = sqrt(tf);
     rn = sqrt(rn);
@@ -214,7 +202,7 @@ __global__ void __launch_bounds__(kTableThreads) mf_cell_table_kernel(const Tabl
   __syncthreads();
   const int c0 = band_s[0], nc = band_s[1];
   if (nc == 0) return;
-  const int slices = kTableThreads / nc;  // >= 2
+  const int slices = kTableThreads / nc;
   const int slice = threadIdx.x / nc;
   const int k = threadIdx.x - slice * nc;
   const bool on = slice < slices;
@@ -279,7 +267,7 @@ struct GatherCellsP {
 };
 
 constexpr int kCellBytes = GatherCells::Q * sizeof(float2);  // 48
-constexpr int kRowBytes = kMaxCells * kCellBytes;            // 3072
+constexpr int kRowBytes = kMaxCells * kCellBytes;            // 4608
 // Launch shape of the gather.  Measured on 49152 antennas x 512000 voxels: 52.7 ms; 2 voxels
 // per thread with 5 blocks per SM 65.2, 6 voxels with 2 blocks 59.0; stages of 4 antennas 75.1,
 // of up to 16 antennas (8 KB pool) 53.9.
@@ -533,10 +521,6 @@ __global__ void __launch_bounds__(kGatherThreads + 32, kGatherBlocks) mf_cell_ga
   }
 }
 
-double cells_per_metre(double k1, int64_t S, int over) {
-  return static_cast<double>(static_cast<float>(over * static_cast<double>(S) * std::fabs(k1)));
-}
-
 int gather_splits(int64_t A, int64_t N) {
   const int64_t vtiles = (N + kGatherThreads * kGatherVpt - 1) / (kGatherThreads * kGatherVpt);
   const int64_t stages = std::max<int64_t>(1, (A + kGatherRows - 1) / kGatherRows);
@@ -612,6 +596,451 @@ cudaError_t launch_cells_forward(const MfArgs& a, unsigned char* ws, const CellL
   return launch_finalize_partials(a.dtype, gp.partial, splits, a.N, static_cast<float>(a.A), a.out_real, a.out_imag, st);
 }
 
+// ---------------------------------------------------------------------------
+// Adjoint.  g[a, n] = (1/A) sum_v G_v e^{+j 2 pi (c0 + n d)}: with w_v = G_v e^{+j 2 pi c}, c the
+// phase of carrier and middle sample, the voxels of one cell enter every sample
+// through the moments M_q = sum_v w_v x_v^q alone,
+//   g[a, n] = (1/A) sum_cells e^{+j 2 pi n' d_k} (sum_q even g_q(n) M_q + j sum_q odd g_q(n) M_q).
+// Launches: the boxes of voxels and antennas (partials) and the basis; the common
+// band of cells; the moments; the samples from the moments; the direct kernel,
+// which returns at once unless the band did not fit.
+constexpr int kMomentCap = 24 * MomentCells::kOver;  // cells: 1.8 m of path at 4 GHz swept
+constexpr int kBoxFloats = 20;                       // voxels, tx, rx: lo xyz, hi xyz; a NaN count; pad
+
+struct MomentHead {
+  int bad;
+  int k0, cells;
+  int pad;
+  double bias;  // |v|^2 bound for leg_antenna
+};
+
+struct MomentLayout {
+  size_t head, box, basis, moments, partial, total;
+};
+
+MomentLayout moment_layout(int64_t A, int64_t S, int splits, size_t partial_bytes) {
+  const size_t apad = static_cast<size_t>((A + 31) / 32) * 32;
+  MomentLayout l;
+  l.head = 0;
+  l.box = 256;
+  l.basis = up256(l.box + kPrepBlocks * kBoxFloats * sizeof(float));
+  l.moments = up256(l.basis + static_cast<size_t>(S) * MomentCells::Q * sizeof(float));
+  l.partial = l.moments + up256(splits * static_cast<size_t>(kMomentCap) * MomentCells::Q * sizeof(float2) * apad);
+  l.total = l.partial + up256(partial_bytes);
+  return l;
+}
+
+template <typename T>
+struct BoxP {
+  const T* voxel;  // [3, N]
+  const T* tx;     // [A, 3]
+  const T* rx;
+  int64_t N, A;
+  int S;
+  double theta_step;
+  float* box;  // [blocks][kBoxFloats]
+  float* basis;
+};
+
+template <typename T, int Q>
+__global__ void __launch_bounds__(256) moment_prep_kernel(const BoxP<T> p) {
+  __shared__ float red[8][kBoxFloats];
+  const int64_t gid = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  for (int64_t n = gid; n < p.S; n += step) {
+    float g[Q];
+    cell_basis<Q>(p.theta_step * (static_cast<double>(n) - 0.5 * (p.S - 1)), g);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) p.basis[n * Q + q] = g[q];
+  }
+  float b[18], nan_antennas = 0.0f;
+#pragma unroll
+  for (int c = 0; c < 18; ++c) b[c] = (c % 6) < 3 ? INFINITY : -INFINITY;
+  auto add = [&](float* box, float x, int c) {
+    box[c] = fminf(box[c], x);
+    box[3 + c] = fmaxf(box[3 + c], x);
+  };
+  for (int64_t v = gid; v < p.N; v += step) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) add(b, ld_f(p.voxel, c * p.N + v), c);
+  }
+  for (int64_t a = gid; a < p.A; a += step) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float t = ld_f(p.tx, a * 3 + c), r = ld_f(p.rx, a * 3 + c);
+      if (t != t || r != r) nan_antennas = 1.0f;
+      add(b + 6, t, c);
+      add(b + 12, r, c);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 19; ++c) {
+    float x = c < 18 ? b[c < 18 ? c : 0] : nan_antennas;
+    const bool low = c < 18 && (c % 6) < 3;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float y = __shfl_xor_sync(0xffffffffu, x, o);
+      x = low ? fminf(x, y) : fmaxf(x, y);
+    }
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][c] = x;
+  }
+  __syncthreads();
+  const int c = threadIdx.x;
+  if (c < 19) {
+    float r = red[0][c];
+    for (int w = 1; w < 8; ++w) r = c < 18 && (c % 6) < 3 ? fminf(r, red[w][c]) : fmaxf(r, red[w][c]);
+    p.box[blockIdx.x * kBoxFloats + c] = r;
+  }
+}
+
+// The cells that any antenna's path to any voxel can reach, from the boxes.
+__global__ void __launch_bounds__(32 * 19) moment_band_kernel(const float* partial, int blocks, double kappa,
+                                                             MomentHead* head) {
+  __shared__ float s[19];
+  const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool low = c < 18 && (c % 6) < 3;
+  float x = low ? INFINITY : -INFINITY;
+  for (int i = lane; i < blocks; i += 32) {
+    const float y = partial[i * kBoxFloats + c];
+    x = low ? fminf(x, y) : fmaxf(x, y);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float y = __shfl_xor_sync(0xffffffffu, x, o);
+    x = low ? fminf(x, y) : fmaxf(x, y);
+  }
+  if (lane == 0) s[c] = x;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  double near[2] = {0.0, 0.0}, far[2] = {0.0, 0.0}, vv = 0.0;
+  for (int k = 0; k < 3; ++k) {
+    const double lo = s[k], hi = s[3 + k];
+    for (int e = 0; e < 2; ++e) {
+      const double alo = s[6 + 6 * e + k], ahi = s[9 + 6 * e + k];
+      const double gap = fmax(0.0, fmax(lo - ahi, alo - hi)), reach = fmax(hi - alo, ahi - lo);
+      near[e] += gap * gap;
+      far[e] += reach * reach;
+    }
+    const double m = fmax(fabs(lo), fabs(hi));
+    vv += m * m;
+  }
+  const double ft = sqrt(far[0]), fr = sqrt(far[1]);
+  const double lo = floor((sqrt(near[0]) + sqrt(near[1])) * kappa) - 1.0, hi = ceil((ft + fr) * kappa) + 1.0;
+  const bool fits = s[18] == 0.0f && ft < kMaxLeg && fr < kMaxLeg && hi - lo + 1.0 <= kMomentCap;  // false for NaN
+  head->bad = fits ? 0 : 1;
+  head->k0 = fits ? static_cast<int>(lo) : 0;
+  head->cells = fits ? static_cast<int>(hi - lo) + 1 : 0;
+  head->bias = fits ? vv : 0.0;
+}
+
+template <typename T>
+struct MomentP {
+  const T* voxel;
+  const T* gr;
+  const T* gi;
+  const T* tx;
+  const T* rx;
+  float4* moments;  // [splits][kMomentCap][Q/2][apad]: pairs of complex moments
+  const MomentHead* head;
+  int64_t A, N, apad, vox_per_split;
+  PairPhase ph;
+};
+
+__device__ __forceinline__ void red_add4(float4* dst, float2 a, float2 b) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(a.x), "f"(a.y), "f"(b.x),
+               "f"(b.y)
+               : "memory");
+}
+
+// One thread per antenna; the voxels of the block's split pass through shared
+// memory in tiles and every thread reads the same one (broadcast).  The moments
+// of the thread's current cell stay in registers; consecutive voxels mostly
+// share a cell, and when it changes the moments are added to the antenna's own
+// record in memory (vector reductions without a return value: nothing waits for
+// them, and no other thread touches the record, so the order of its sums, and the
+// result, is the same on every run).  About 100 instructions per 32 pairs at 66% of the
+// issue slots (ncu, 972 x 50653 pairs): 972 antennas x 201 samples x 50653 voxels
+// take 0.24 ms here, 2.37 ms by the recurrence of the direct kernel.
+constexpr int kMomentTile = 128;
+
+template <typename T>
+__global__ void __launch_bounds__(128, 4) mf_moment_kernel(const MomentP<T> p) {
+  constexpr int Q = MomentCells::Q;
+  __shared__ double2 sxy[kMomentTile], szv[kMomentTile];
+  __shared__ float2 sg[kMomentTile];
+  if (p.head->bad) return;
+  const int k0 = p.head->k0, cells = p.head->cells;
+  const int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const int64_t split = blockIdx.y;
+  const int64_t v_begin = split * p.vox_per_split;
+  const int64_t v_end = min(p.N, v_begin + p.vox_per_split);
+  double mt[4], mr[4];
+  {
+    double t[3], r[3];
+    const int64_t al = min(a, p.A - 1);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      t[c] = ld_f(p.tx, al * 3 + c);
+      r[c] = ld_f(p.rx, al * 3 + c);
+    }
+    leg_antenna(t, p.head->bias, mt);
+    leg_antenna(r, p.head->bias, mr);
+  }
+  const bool mine = a < p.apad;
+  float4* rec = p.moments + split * kMomentCap * (Q / 2) * p.apad + a;
+  if (mine) {
+    for (int i = 0; i < cells * (Q / 2); ++i) rec[i * p.apad] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  }
+  float2 M[Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) M[q] = make_float2(0.0f, 0.0f);
+  float cur = __uint_as_float(kRoundMagicBits + static_cast<uint32_t>(k0));
+  auto flush = [&]() {
+    const int k = static_cast<int>(__float_as_uint(cur) - kRoundMagicBits) - k0;
+    float4* dst = rec + static_cast<int64_t>(min(max(k, 0), cells - 1)) * (Q / 2) * p.apad;
+    if (mine) {
+#pragma unroll
+      for (int q = 0; q < Q; q += 2) red_add4(dst + (q / 2) * p.apad, M[q], M[q + 1]);
+    }
+  };
+  for (int64_t v0 = v_begin; v0 < v_end; v0 += kMomentTile) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < kMomentTile; i += blockDim.x) {
+      const int64_t v = v0 + i;
+      double x = 0.0, y = 0.0, z = 0.0;
+      float2 g = make_float2(0.0f, 0.0f);
+      if (v < v_end) {
+        const float fx = ld_f(p.voxel, v), fy = ld_f(p.voxel, p.N + v), fz = ld_f(p.voxel, 2 * p.N + v);
+        g = make_float2(ld_f(p.gr, v), ld_f(p.gi, v));
+        x = fx * kUnit;
+        y = fy * kUnit;
+        z = fz * kUnit;
+        if (fx != fx || fy != fy || fz != fz) g = make_float2(NAN, NAN);  // its every sample is NaN
+      }
+      if (v >= v_end || g.x != g.x) {
+        // somewhere in the box: the split's first voxel, or antenna 0's cell k0 when that is NaN too
+        const float fx = ld_f(p.voxel, v_begin), fy = ld_f(p.voxel, p.N + v_begin), fz = ld_f(p.voxel, 2 * p.N + v_begin);
+        const bool ok = fx == fx && fy == fy && fz == fz;
+        x = ok ? fx * kUnit : 0.0;
+        y = ok ? fy * kUnit : 0.0;
+        z = ok ? fz * kUnit : 0.0;
+      }
+      sxy[i] = make_double2(x, y);
+      szv[i] = make_double2(z, fma(x, x, fma(y, y, z * z)));
+      sg[i] = g;
+    }
+    __syncthreads();
+    const int count = static_cast<int>(min(static_cast<int64_t>(kMomentTile), v_end - v0));
+    for (int i = 0; i < count; i += 2) {
+      float x[2], m[2];
+      float2 w[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const double2 xy = sxy[i + u], zv = szv[i + u];
+        const float2 g = sg[i + u];
+        const Leg lt = leg_length(mt[0], mt[1], mt[2], mt[3], xy.x, xy.y, zv.x, zv.y);
+        const Leg lr = leg_length(mr[0], mr[1], mr[2], mr[3], xy.x, xy.y, zv.x, zv.y);
+        const float hi = lt.d + lr.d, lo = lt.l + lr.l;
+        const CellPos c = pair_cell(p.ph, hi, lo);
+        float sn, cs;
+        __sincosf(6.28318530717958647692f * pair_cycles(p.ph, hi, lo), &sn, &cs);
+        w[u] = make_float2(fmaf(g.x, cs, -g.y * sn), fmaf(g.x, sn, g.y * cs));
+        x[u] = c.x;
+        m[u] = c.m;
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (m[u] != cur) {
+          flush();
+          cur = m[u];
+#pragma unroll
+          for (int q = 0; q < Q; ++q) M[q] = make_float2(0.0f, 0.0f);
+        }
+        M[0] = fadd2(M[0], w[u]);
+        float xq = x[u];
+#pragma unroll
+        for (int q = 1; q < Q; ++q) {
+          M[q] = ffma2(make_float2(xq, xq), w[u], M[q]);
+          xq *= x[u];
+        }
+      }
+    }
+  }
+  flush();
+}
+
+// Sums the splits' records into the first one's: block (x: 32 antennas, y: a pair
+// of moments of one cell), 16 warps over the splits, in a fixed order.
+constexpr int kSumWarps = 16;
+
+__global__ void __launch_bounds__(32 * kSumWarps) mf_moment_sum_kernel(float4* moments, const MomentHead* head,
+                                                                       int64_t apad, int splits, int pairs) {
+  __shared__ float4 part[kSumWarps][32];
+  if (head->bad || static_cast<int>(blockIdx.y) >= head->cells * pairs) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t stride = static_cast<int64_t>(kMomentCap) * pairs * apad;
+  float4* src = moments + static_cast<int64_t>(blockIdx.y) * apad + blockIdx.x * 32 + lane;
+  float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+  for (int k = warp; k < splits; k += kSumWarps) {
+    const float4 y = src[k * stride];
+    s.x += y.x;
+    s.y += y.y;
+    s.z += y.z;
+    s.w += y.w;
+  }
+  part[warp][lane] = s;
+  __syncthreads();
+  if (warp != 0) return;
+  for (int w = 1; w < kSumWarps; ++w) {
+    const float4 y = part[w][lane];
+    s.x += y.x;
+    s.y += y.y;
+    s.z += y.z;
+    s.w += y.w;
+  }
+  *src = s;
+}
+
+template <typename T>
+struct SamplesP {
+  const float4* moments;
+  const float* basis;
+  const MomentHead* head;
+  T* out_r;
+  T* out_i;
+  int64_t A, apad;
+  int S;
+  double k1, b1, kappa;
+};
+
+// Samples from the moments: 4 antennas per block, which share the phasors of the cells.
+constexpr int kSampleAnts = 4;
+
+template <typename T>
+__global__ void __launch_bounds__(128) mf_moment_samples_kernel(const SamplesP<T> p) {
+  constexpr int Q = MomentCells::Q;
+  __shared__ float4 mom[kMomentCap][Q / 2][kSampleAnts];
+  if (p.head->bad) return;
+  const int k0 = p.head->k0, cells = p.head->cells;
+  const int64_t a0 = blockIdx.x * static_cast<int64_t>(kSampleAnts);
+  for (int i = threadIdx.x; i < cells * (Q / 2) * kSampleAnts; i += blockDim.x) {
+    (&mom[0][0][0])[i] = p.moments[static_cast<int64_t>(i / kSampleAnts) * p.apad + a0 + i % kSampleAnts];
+  }
+  __syncthreads();
+  const double mid = 0.5 * (p.S - 1);
+  const float inv = static_cast<float>(p.A);
+  for (int n = blockIdx.y * blockDim.x + threadIdx.x; n < p.S; n += gridDim.y * blockDim.x) {
+    float g[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) g[q] = p.basis[n * Q + q];
+    float2 acc[kSampleAnts];
+#pragma unroll
+    for (int u = 0; u < kSampleAnts; ++u) acc[u] = make_float2(0.0f, 0.0f);
+    for (int k = 0; k < cells; ++k) {
+      const double c = (n - mid) * fma(p.k1, static_cast<double>(k0 + k) / p.kappa, p.b1);
+      const float2 e = cis_cycles(static_cast<float>(c - rint(c)));
+#pragma unroll
+      for (int u = 0; u < kSampleAnts; ++u) {
+        float2 ev = make_float2(0.0f, 0.0f), od = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int q = 0; q < Q; q += 2) {
+          const float4 m = mom[k][q / 2][u];
+          ev = ffma2(make_float2(g[q], g[q]), make_float2(m.x, m.y), ev);
+          od = ffma2(make_float2(g[q + 1], g[q + 1]), make_float2(m.z, m.w), od);
+        }
+        const float2 z = cmul(e, make_float2(ev.x - od.y, ev.y + od.x));
+        acc[u] = fadd2(acc[u], z);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kSampleAnts; ++u) {
+      if (a0 + u >= p.A) continue;
+      p.out_r[(a0 + u) * p.S + n] = from_f<T>(acc[u].x / inv);
+      p.out_i[(a0 + u) * p.S + n] = from_f<T>(acc[u].y / inv);
+    }
+  }
+}
+
+struct MomentShape {
+  int threads, groups, splits;
+  int64_t vox_per_split;
+};
+
+// Blocks of up to 128 antennas; enough voxel splits for four 4-warp blocks per SM.
+MomentShape moment_shape(int64_t A, int64_t N) {
+  MomentShape s;
+  s.threads = static_cast<int>(std::min<int64_t>(128, (A + 31) / 32 * 32));
+  s.groups = static_cast<int>((A + s.threads - 1) / s.threads);
+  const int64_t slots = static_cast<int64_t>(current_device_info().sm_count) * 4 * 128 / s.threads;
+  const int64_t tiles = std::max<int64_t>(1, (N + kMomentTile - 1) / kMomentTile);
+  int64_t splits = std::max<int64_t>(1, slots / s.groups);
+  splits = std::min<int64_t>(std::min<int64_t>(splits, tiles), 2048);
+  s.vox_per_split = (((N + splits - 1) / splits + 1) / 2) * 2;  // whole pairs of voxels
+  s.splits = static_cast<int>((N + s.vox_per_split - 1) / s.vox_per_split);
+  return s;
+}
+
+template <typename T>
+cudaError_t launch_cells_backward(const MfArgs& a, unsigned char* ws, cudaStream_t st) {
+  const MomentShape sh = moment_shape(a.A, a.N);
+  const MomentLayout l = moment_layout(a.A, a.S, sh.splits, 0);
+  const PhaseConsts pc = phase_consts(kMfStartFrequency, a.As, a.fs);
+  const double kappa = cells_per_metre(pc.k1, a.S, MomentCells::kOver);
+  MomentHead* head = reinterpret_cast<MomentHead*>(ws + l.head);
+  const int pb = static_cast<int>(std::min<int64_t>(kPrepBlocks, (std::max({a.N, a.S, a.A}) + 255) / 256));
+
+  BoxP<T> bp;
+  bp.voxel = static_cast<const T*>(a.voxel);
+  bp.tx = static_cast<const T*>(a.tx);
+  bp.rx = static_cast<const T*>(a.rx);
+  bp.N = a.N;
+  bp.A = a.A;
+  bp.S = static_cast<int>(a.S);
+  bp.theta_step = 2.0 * M_PI * pc.k1 / kappa;
+  bp.box = reinterpret_cast<float*>(ws + l.box);
+  bp.basis = reinterpret_cast<float*>(ws + l.basis);
+  moment_prep_kernel<T, MomentCells::Q><<<pb, 256, 0, st>>>(bp);
+  moment_band_kernel<<<1, 32 * 19, 0, st>>>(bp.box, pb, kappa, head);
+
+  MomentP<T> mp;
+  mp.voxel = bp.voxel;
+  mp.gr = static_cast<const T*>(a.grad_real_out);
+  mp.gi = static_cast<const T*>(a.grad_imag_out);
+  mp.tx = bp.tx;
+  mp.rx = bp.rx;
+  mp.moments = reinterpret_cast<float4*>(ws + l.moments);
+  mp.head = head;
+  mp.A = a.A;
+  mp.N = a.N;
+  mp.apad = (a.A + 31) / 32 * 32;
+  mp.vox_per_split = sh.vox_per_split;
+  mp.ph = pair_phase(pc.k0, pc.b0, pc.k1, pc.b1, a.S, kappa);
+  mf_moment_kernel<T><<<dim3(sh.groups, sh.splits), sh.threads, 0, st>>>(mp);
+
+  if (sh.splits > 1) {
+    constexpr int pairs = MomentCells::Q / 2;
+    mf_moment_sum_kernel<<<dim3(static_cast<unsigned>(mp.apad / 32), kMomentCap * pairs), 32 * kSumWarps, 0, st>>>(
+        mp.moments, head, mp.apad, sh.splits, pairs);
+  }
+
+  SamplesP<T> sp;
+  sp.moments = mp.moments;
+  sp.basis = bp.basis;
+  sp.head = head;
+  sp.out_r = static_cast<T*>(a.out_real);
+  sp.out_i = static_cast<T*>(a.out_imag);
+  sp.A = a.A;
+  sp.apad = mp.apad;
+  sp.S = bp.S;
+  sp.k1 = pc.k1;
+  sp.b1 = pc.b1;
+  sp.kappa = kappa;
+  const dim3 grid(static_cast<unsigned>((a.A + kSampleAnts - 1) / kSampleAnts), static_cast<unsigned>((a.S + 127) / 128));
+  mf_moment_samples_kernel<T><<<grid, 128, 0, st>>>(sp);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 // The cells take over where the pairs outweigh the tables and the extra
@@ -647,6 +1076,28 @@ cudaError_t mf_cells_forward(const MfArgs& a, void* ws, cudaStream_t st) {
   unsigned char* base = static_cast<unsigned char*>(ws);
   if (a.dtype == kF16) return launch_cells_forward<__half>(a, base, l, splits, st);
   return launch_cells_forward<float>(a, base, l, splits, st);
+}
+
+// The adjoint's work is the pairs' too; a lane of its warps is an antenna.
+bool mf_cells_backward_applies(const MfArgs& a) {
+  return a.mode == kMixed && a.dtype != kF64 && a.S >= 32 && a.S <= 4096 && a.N >= 512 && a.A >= 24 &&
+         static_cast<double>(a.A) * a.N * a.S >= 1.0e8;
+}
+
+size_t mf_cells_backward_workspace(const MfArgs& a, size_t direct_partial_bytes) {
+  return moment_layout(a.A, a.S, moment_shape(a.A, a.N).splits, direct_partial_bytes).total;
+}
+
+size_t mf_cells_backward_partial_offset(const MfArgs& a) {
+  return moment_layout(a.A, a.S, moment_shape(a.A, a.N).splits, 0).partial;
+}
+
+const int* mf_moments_bad_flag(void* ws) { return &static_cast<MomentHead*>(ws)->bad; }
+
+cudaError_t mf_cells_backward(const MfArgs& a, void* ws, cudaStream_t st) {
+  unsigned char* base = static_cast<unsigned char*>(ws);
+  if (a.dtype == kF16) return launch_cells_backward<__half>(a, base, st);
+  return launch_cells_backward<float>(a, base, st);
 }
 
 }  // namespace geraf

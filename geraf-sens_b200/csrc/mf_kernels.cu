@@ -423,6 +423,7 @@ struct MfBwdP {
   int splits;
   int64_t vox_per_split;
   int groups;  // sample groups per block
+  const int* run_if;  // MIXED: when set, the kernel runs only if *run_if != 0
 };
 
 // MIXED adjoint.  Block = (antenna, voxel split, sample range).  Phase 1:
@@ -435,6 +436,7 @@ struct MfBwdP {
 template <typename T, int K>
 __global__ void __launch_bounds__(256) mf_bwd_mixed_kernel(const MfBwdP<T> p) {
   extern __shared__ __align__(128) unsigned char smem[];
+  if (p.run_if != nullptr && *p.run_if == 0) return;
   const int TILE = blockDim.x;
   const int G = p.groups;
   const int L = blockDim.x / G;
@@ -821,8 +823,9 @@ size_t bwd_mixed_smem(int threads, int groups, int chunk) {
 }
 
 template <typename T>
-cudaError_t launch_bwd(const MfArgs& a, const Tuning& t, void* ws, cudaStream_t st) {
+cudaError_t launch_bwd(const MfArgs& a, const Tuning& t, void* ws, cudaStream_t st, const int* run_if) {
   MfBwdP<T> p;
+  p.run_if = run_if;
   p.gr = static_cast<const T*>(a.grad_real_out);
   p.gi = static_cast<const T*>(a.grad_imag_out);
   p.tx = static_cast<const T*>(a.tx);
@@ -869,7 +872,7 @@ cudaError_t launch_bwd(const MfArgs& a, const Tuning& t, void* ws, cudaStream_t 
     const int64_t count = a.A * a.S;
     const int fin_blocks = static_cast<int>(std::min<int64_t>((count + 255) / 256, 148 * 16));
     finalize_partials_kernel<T><<<std::max(fin_blocks, 1), 256, 0, st>>>(
-        p.partial, t.splits, count, static_cast<float>(a.A), p.out_r, p.out_i);
+        p.partial, t.splits, count, static_cast<float>(a.A), p.out_r, p.out_i, run_if);
     err = cudaGetLastError();
   }
   return err;
@@ -1038,17 +1041,25 @@ Tuning mf_backward_resolve(const MfArgs& a, const Tuning& req) {
 
 size_t mf_backward_workspace(const MfArgs& a, const Tuning& t) {
   if (a.mode == kNufft) return mf_nufft_backward_workspace(a, t);
-  if (a.mode == kPlain || t.splits <= 1) return 0;
-  return static_cast<size_t>(t.splits) * a.A * a.S * sizeof(float2);
+  if (a.mode == kPlain) return 0;
+  const size_t partial = t.splits <= 1 ? 0 : static_cast<size_t>(t.splits) * a.A * a.S * sizeof(float2);
+  return mf_cells_backward_applies(a) ? mf_cells_backward_workspace(a, partial) : partial;
 }
 
 cudaError_t mf_backward(const MfArgs& a, const Tuning& t, void* ws, cudaStream_t st) {
   if (a.mode == kNufft) return mf_nufft_backward(a, t, ws, st);
   if (a.A == 0 || a.S == 0) return cudaSuccess;
+  const int* run_if = nullptr;
+  if (mf_cells_backward_applies(a) && mf_cells_scale_ok(a)) {
+    const cudaError_t err = mf_cells_backward(a, ws, st);
+    if (err != cudaSuccess) return err;
+    run_if = mf_moments_bad_flag(ws);
+    ws = static_cast<unsigned char*>(ws) + mf_cells_backward_partial_offset(a);
+  }
   switch (a.dtype) {
-    case kF64: return launch_bwd<double>(a, t, ws, st);
-    case kF16: return launch_bwd<__half>(a, t, ws, st);
-    default: return launch_bwd<float>(a, t, ws, st);
+    case kF64: return launch_bwd<double>(a, t, ws, st, run_if);
+    case kF16: return launch_bwd<__half>(a, t, ws, st, run_if);
+    default: return launch_bwd<float>(a, t, ws, st, run_if);
   }
 }
 

@@ -25,14 +25,18 @@ namespace geraf {
 
 // Cell width and coefficients.  Evaluation (gather): 4 S k1 cells per metre
 // (18.7 mm at 4 GHz of swept bandwidth) with 6 coefficients: theta <= pi/4, error
-// <= 1.6e-7 for the outermost sample, 3e-8 in the mean.  Accumulation (moments): S k1 cells
-// per metre (75 mm) with 10: theta <= pi, <= 4.9e-8; wider cells are left less often.
+// <= 1.6e-7 for the outermost sample, 3e-8 in the mean.  Accumulation (moments):
+// 2 S k1 cells per metre (37 mm) with 8: theta <= pi/2, error <= 2.8e-8; wider cells are
+// left less often but hold more moments (10 in 75 mm cells and 6 in 18.7 mm cells
+// took the same time on 972 antennas x 50653 voxels, 6 in 18.7 mm cells 8% more on points
+// along rays).
 template <int OVERSAMPLE, int Q_>
 struct CellParams {
   static constexpr int kOver = OVERSAMPLE;
   static constexpr int Q = Q_;
 };
 using GatherCells = CellParams<4, 6>;
+using MomentCells = CellParams<2, 8>;
 
 // Lengths of the pairs' legs are held in units of 2^-20 m (coordinates scaled by
 // 2^20, exactly): a leg below 8 m is a whole number below 2^23 plus a rest, and
@@ -93,6 +97,11 @@ struct PairPhase {
 };
 
 // kappa: cells per metre.
+// Cells per metre for S samples, as the kernels round it.
+inline double cells_per_metre(double k1, int64_t S, int over) {
+  return static_cast<double>(static_cast<float>(over * static_cast<double>(S) * (k1 < 0.0 ? -k1 : k1)));
+}
+
 inline PairPhase pair_phase(double k0, double b0, double k1, double b1, int64_t S, double kappa) {
   const double mid = 0.5 * static_cast<double>(S - 1);
   const double K = (k0 + mid * k1) / kUnit;
@@ -124,6 +133,14 @@ __device__ __forceinline__ CellPos pair_cell(const PairPhase& p, float hi, float
   const float k = c.m - kRoundMagic;
   c.x = fmaf(lo, p.kappa_rest, fmaf(hi, p.kappa, -k));
   return c;
+}
+
+// A point's or an antenna's coordinates for leg_length.
+__device__ __forceinline__ void leg_antenna(const double* t, double bias, double* m) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) m[c] = -2.0 * kUnit * t[c];
+  const double tt = fma(t[2], t[2], fma(t[1], t[1], t[0] * t[0]));
+  m[3] = (tt + (4e-15 * (tt + bias) + 1e-18)) * (kUnit * kUnit);
 }
 
 // Range of |t - x| + |r - x| over the box [lo, hi] (lo xyz, hi xyz), and its longest leg.

@@ -63,13 +63,50 @@ def test_forward_vs_fp64(cuda, A, S, N, shuffle):
     assert rel_l2(forward(c), oracle(c)) < TOL
 
 
+def backward(c, **kw):
+    ch, A, S = c["ch"], c["tx"].shape[0], c["re"].shape[1]
+    N = c["vox"].shape[1]
+    gr, gi = c["rng"].standard_normal((2, N)).astype(np.float32)
+    h = mf_backward(gr, gi, c["tx"], c["rx"], c["vox"], A, S, ch.adc_sample_rate, ch.As_sci, "mixed", **kw)
+    r = orc.mf_backward(gr, gi, c["tx"], c["rx"], c["vox"], A, S, ch.adc_sample_rate, ch.As_sci)
+    return h[0] + 1j * h[1], r[0] + 1j * r[1]
+
+
+# remainders of the 32-antenna warps, of the 128-voxel tiles and their pairs, of the samples' blocks
+@pytest.mark.parametrize("A,S,N", [(24, 256, 16385), (33, 128, 24001), (64, 200, 8192), (130, 33, 24000), (1000, 200, 512),
+                                   (257, 129, 3100), (40, 4096, 700)])
+@pytest.mark.parametrize("order", ["grid", "random"])
+def test_backward_vs_fp64(cuda, A, S, N, order):
+    c = case(A + S, A, S, N)
+    if order == "grid":  # neighbouring voxels share cells
+        c["vox"] = np.ascontiguousarray(c["vox"][:, np.lexsort(c["vox"].round(2))])
+    got, ref = backward(c)
+    assert rel_l2(got, ref) < TOL
+
+
+@pytest.mark.parametrize("box,bandwidth", [(((-0.6, -0.6, 0.2), (0.6, 0.6, 1.9)), 4e9),
+                                           (((-0.1, -0.1, 8.2), (0.1, 0.1, 8.4)), 1e9),
+                                           (((-0.1, -0.1, 3.9), (0.1, 0.1, 4.1)), 4e9)],
+                         ids=["wide_band", "long_legs", "far_scene"])
+def test_backward_bands_that_leave_the_cells(cuda, box, bandwidth):
+    got, ref = backward(case(8, 140, 256, 4000, box=box, bandwidth=bandwidth))
+    assert rel_l2(got, ref) < 1e-5
+
+
+def test_backward_nan_voxel_poisons_every_sample(cuda):
+    c = case(9, 140, 128, 6001)
+    c["vox"][0, 5] = np.nan
+    got, _ = backward(c)
+    assert np.isnan(got.real).all() and np.isnan(got.imag).all()
+
+
 @pytest.mark.parametrize("splits", [1, 5])
 def test_forward_takes_any_tuning(cuda, splits):
     c = case(3, 144, 128, 9001)
     assert rel_l2(forward(c, tuning={"threads": 256, "items_per_thread": 2, "splits": splits}), oracle(c)) < TOL
 
 
-@pytest.mark.parametrize("box,bandwidth", [(((-0.5, -0.5, 0.2), (0.5, 0.5, 1.6)), 4e9),   # more cells than fit
+@pytest.mark.parametrize("box,bandwidth", [(((-0.6, -0.6, 0.2), (0.6, 0.6, 1.9)), 4e9),   # more cells than fit
                                            (((-0.1, -0.1, 8.2), (0.1, 0.1, 8.4)), 1e9),   # legs beyond 8 m
                                            (((-0.1, -0.1, 3.9), (0.1, 0.1, 4.1)), 4e9)],  # long legs, narrow band
                          ids=["wide_band", "long_legs", "far_scene"])
