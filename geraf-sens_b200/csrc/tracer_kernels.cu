@@ -774,53 +774,80 @@ __global__ void __launch_bounds__(256) bilinear_fwd_kernel(const BiP<T> p) {
 // Adjoint, gather form: lane j of the ray's warp owns coarse sample j and adds
 // the contributions of the targets bracketing it in target order -- the same
 // per-element order as the reference's single-writer atomicAdd sequence --
-// onto the existing gradient value.
+// onto the existing gradient value.  The brackets and weights of the ray's targets
+// are found once, into shared memory; where the targets ascend (the usual case),
+// those of one coarse sample are a contiguous range, found by binary search, else every
+// sample scans them all.  Bound by the latency of a ray's chain, not by its bytes:
+// 4096 rays x 128 samples x 128 targets took 0.86 ms when every (sample, target)
+// pair searched the bracket again.
+constexpr int kTargetTile = 512;  // targets held at a time; longer rows take several passes
+
 template <typename T>
 __global__ void __launch_bounds__(256) bilinear_bwd_kernel(const BiP<T> p) {
-  const int64_t ray = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  extern __shared__ __align__(16) unsigned char bi_smem[];
+  constexpr int kOut = 1 << 30;  // set in a bracket index: the target lies outside
+  const int warps = blockDim.x >> 5;
+  const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  const int64_t ray = blockIdx.x * static_cast<int64_t>(warps) + warp;
   if (ray >= p.R) return;
   const int S = static_cast<int>(p.S);
+  const int tile = static_cast<int>(min(p.T_, static_cast<int64_t>(kTargetTile)));
+  T* weight = reinterpret_cast<T*>(bi_smem) + warp * tile;  // of the upper sample
+  int* lower = reinterpret_cast<int*>(reinterpret_cast<T*>(bi_smem) + warps * tile) + warp * tile;
   const T* z = p.z + ray * p.S;
-  // p.normals = grad_output_normals [R,T,3], p.sigmas = grad_output_sigmas [A,R,T]
-  for (int j = lane; j < S; j += 32) {
-    T gn[3] = {p.out_n[(ray * p.S + j) * 3 + 0], p.out_n[(ray * p.S + j) * 3 + 1],
-               p.out_n[(ray * p.S + j) * 3 + 2]};
-    for (int64_t t = 0; t < p.T_; ++t) {
-      const T target = p.tz[ray * p.T_ + t];
+  for (int64_t t0 = 0; t0 < p.T_; t0 += kTargetTile) {
+    const int nt = static_cast<int>(min(p.T_ - t0, static_cast<int64_t>(kTargetTile)));
+    __syncwarp();
+    for (int t = lane; t < nt; t += 32) {
+      const T target = p.tz[ray * p.T_ + t0 + t];
       const int lo = bracket_lower(z, S, target);
-      if (lo != j && lo + 1 != j) continue;
       const T z0 = z[lo];
       const T z1 = z[lo + 1];
-      if (target < z0 || target > z1) continue;
-      const T weight_upper = (target - z0) / tmax(z1 - z0, static_cast<T>(1.0e-6f));
-      const T weight_lower = static_cast<T>(1) - weight_upper;
-      const T* gno = p.normals + (ray * p.T_ + t) * 3;
-      for (int axis = 0; axis < 3; ++axis) {
-        if (lo == j) gn[axis] = add_product(gn[axis], weight_lower, gno[axis]);
-        if (lo + 1 == j) gn[axis] = add_product(gn[axis], weight_upper, gno[axis]);
-      }
+      const bool out = target < z0 || target > z1;
+      weight[t] = (target - z0) / tmax(z1 - z0, static_cast<T>(1.0e-6f));
+      lower[t] = lo | (out ? kOut : 0);
     }
-    for (int axis = 0; axis < 3; ++axis) p.out_n[(ray * p.S + j) * 3 + axis] = gn[axis];
-  }
-  for (int64_t a = 0; a < p.A; ++a) {
-    const T* gso = p.sigmas + (a * p.R + ray) * p.T_;
-    T* gs = p.out_s + (a * p.R + ray) * p.S;
-    for (int j = lane; j < S; j += 32) {
-      T acc = gs[j];
-      for (int64_t t = 0; t < p.T_; ++t) {
-        const T target = p.tz[ray * p.T_ + t];
-        const int lo = bracket_lower(z, S, target);
-        if (lo != j && lo + 1 != j) continue;
-        const T z0 = z[lo];
-        const T z1 = z[lo + 1];
-        if (target < z0 || target > z1) continue;
-        const T weight_upper = (target - z0) / tmax(z1 - z0, static_cast<T>(1.0e-6f));
-        const T weight_lower = static_cast<T>(1) - weight_upper;
-        if (lo == j) acc = add_product(acc, weight_lower, gso[t]);
-        if (lo + 1 == j) acc = add_product(acc, weight_upper, gso[t]);
+    __syncwarp();
+    bool ascending = true;
+    for (int t = lane; t + 1 < nt; t += 32) ascending = ascending && (lower[t] & ~kOut) <= (lower[t + 1] & ~kOut);
+    ascending = __all_sync(0xffffffffu, ascending);
+    auto first_from = [&](int j) {  // the first target whose bracket is j or higher
+      int lo = 0, hi = nt;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if ((lower[mid] & ~kOut) >= j) hi = mid;
+        else lo = mid + 1;
       }
-      gs[j] = acc;
+      return lo;
+    };
+    // p.normals = grad_output_normals [R,T,3], p.sigmas = grad_output_sigmas [A,R,T]
+    const T* gno = p.normals + (ray * p.T_ + t0) * 3;
+    for (int j = lane; j < S; j += 32) {
+      const int t_begin = ascending ? first_from(j - 1) : 0;
+      const int t_end = ascending ? first_from(j + 1) : nt;
+      T* gn = p.out_n + (ray * p.S + j) * 3;
+      T acc[3] = {gn[0], gn[1], gn[2]};
+      for (int t = t_begin; t < t_end; ++t) {
+        const int lo = lower[t];
+        if (lo != j && lo + 1 != j) continue;
+        const T w = lo == j ? static_cast<T>(1) - weight[t] : weight[t];
+#pragma unroll
+        for (int axis = 0; axis < 3; ++axis) acc[axis] = add_product(acc[axis], w, gno[t * 3 + axis]);
+      }
+#pragma unroll
+      for (int axis = 0; axis < 3; ++axis) gn[axis] = acc[axis];
+      for (int64_t a = 0; a < p.A; ++a) {
+        const T* gso = p.sigmas + (a * p.R + ray) * p.T_ + t0;
+        T* gs = p.out_s + (a * p.R + ray) * p.S + j;
+        T sum = *gs;
+        for (int t = t_begin; t < t_end; ++t) {
+          const int lo = lower[t];
+          if (lo != j && lo + 1 != j) continue;
+          sum = add_product(sum, lo == j ? static_cast<T>(1) - weight[t] : weight[t], gso[t]);
+        }
+        *gs = sum;
+      }
     }
   }
 }
@@ -1164,9 +1191,14 @@ cudaError_t bilinear_forward(const BilinearArgs& a, cudaStream_t st) {
 
 cudaError_t bilinear_backward(const BilinearArgs& a, cudaStream_t st) {
   if (a.R == 0 || a.S == 0) return cudaSuccess;
-  const int64_t blocks = (a.R * 32 + 255) / 256;
-  if (a.dtype == kF64) bilinear_bwd_kernel<double><<<static_cast<unsigned>(blocks), 256, 0, st>>>(make_bi<double>(a));
-  else bilinear_bwd_kernel<float><<<static_cast<unsigned>(blocks), 256, 0, st>>>(make_bi<float>(a));
+  constexpr int kRays = 8;  // per block
+  const int64_t blocks = (a.R + kRays - 1) / kRays;
+  const size_t tile = static_cast<size_t>(std::min<int64_t>(a.T, kTargetTile)) * kRays;
+  if (a.dtype == kF64) {
+    bilinear_bwd_kernel<double><<<static_cast<unsigned>(blocks), kRays * 32, tile * (sizeof(double) + sizeof(int)), st>>>(make_bi<double>(a));
+  } else {
+    bilinear_bwd_kernel<float><<<static_cast<unsigned>(blocks), kRays * 32, tile * (sizeof(float) + sizeof(int)), st>>>(make_bi<float>(a));
+  }
   return cudaGetLastError();
 }
 
