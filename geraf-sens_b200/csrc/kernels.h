@@ -74,23 +74,24 @@ cudaError_t mf_nufft_backward(const MfArgs& a, const Tuning& t, void* ws, cudaSt
 // Sums `splits` float2 partials per element in split order (FP64), divides by
 // `divisor` and stores in the element type.
 cudaError_t launch_finalize_partials(int dtype, const float2* partial, int splits, int64_t count,
-                                     float divisor, void* out_r, void* out_i, cudaStream_t st);
+                                     float divisor, void* out_r, void* out_i, cudaStream_t st,
+                                     const int* run_if = nullptr);
 
 Tuning mf_backward_resolve(const MfArgs& a, const Tuning& req);
 size_t mf_backward_workspace(const MfArgs& a, const Tuning& t);
 cudaError_t mf_backward(const MfArgs& a, const Tuning& t, void* ws, cudaStream_t st);
 
-// MIXED matched filter through range cells (mf_cells.cu).  `applies` decides by
-// the sizes; the workspace then holds the cells' tables and, from
+// MIXED and NUFFT matched filter through range cells (mf_cells.cu).  `applies` decides by
+// the sizes (and the NUFFT form's taps); the workspace then holds the cells' tables and, from
 // `partial_offset`, the partial sums (also those of the direct kernel that runs
 // in their place when *bad_flag is set on the device).
-bool mf_cells_forward_applies(const MfArgs& a);
+bool mf_cells_forward_applies(const MfArgs& a, int taps);
 bool mf_cells_scale_ok(const MfArgs& a);
 size_t mf_cells_forward_workspace(const MfArgs& a, size_t direct_partial_bytes);
 size_t mf_cells_forward_partial_offset(const MfArgs& a);
 const int* mf_cells_bad_flag(void* ws);
 cudaError_t mf_cells_forward(const MfArgs& a, void* ws, cudaStream_t st);
-bool mf_cells_backward_applies(const MfArgs& a);
+bool mf_cells_backward_applies(const MfArgs& a, int taps);
 size_t mf_cells_backward_workspace(const MfArgs& a, size_t direct_partial_bytes);
 size_t mf_cells_backward_partial_offset(const MfArgs& a);
 const int* mf_moments_bad_flag(void* ws);

@@ -311,7 +311,9 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // more warps with fewer.  49152 antennas x 256 samples x 512000 voxels: 950 ms by
 // the direct kernel, 52.7 ms through the cells (478 G pairs/s); 3072 x 128 x
 // 110592: 7.53 ms against 0.79 ms.
-template <typename T>
+// ACCURATE: the phasor of a pair by sincospif (the NUFFT form's, ~1 ulp) instead
+// of the hardware sine and cosine (4e-7).
+template <typename T, bool ACCURATE>
 __global__ void __launch_bounds__(kGatherThreads + 32, kGatherBlocks) mf_cell_gather_kernel(const GatherCellsP<T> p) {
   constexpr int VPT = kGatherVpt;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -493,10 +495,9 @@ __global__ void __launch_bounds__(kGatherThreads + 32, kGatherBlocks) mf_cell_ga
         acc = ffma2(acc, xx, make_float2(q1.x, q1.y));
         acc = ffma2(acc, xx, make_float2(q0.z, q0.w));
         acc = ffma2(acc, xx, make_float2(q0.x, q0.y));
-        float sn, cs;
-        __sincosf(6.28318530717958647692f * pair_cycles(p.ph, hi, lo), &sn, &cs);
-        tr[j] = fmaf(cs, acc.x, fmaf(sn, acc.y, tr[j]));
-        ti[j] = fmaf(cs, acc.y, fmaf(-sn, acc.x, ti[j]));
+        const float2 e = pair_phasor<ACCURATE>(pair_cycles(p.ph, hi, lo));
+        tr[j] = fmaf(e.x, acc.x, fmaf(e.y, acc.y, tr[j]));
+        ti[j] = fmaf(e.x, acc.y, fmaf(-e.y, acc.x, ti[j]));
       }
     }
 #pragma unroll
@@ -584,7 +585,8 @@ cudaError_t launch_cells_forward(const MfArgs& a, unsigned char* ws, const CellL
   gp.ant_per_split = ((stages + splits - 1) / splits) * kGatherRows;
   gp.kappa = static_cast<float>(kappa);
   gp.ph = pair_phase(pc.k0, pc.b0, pc.k1, pc.b1, a.S, kappa);
-  const void* fn = reinterpret_cast<const void*>(&mf_cell_gather_kernel<T>);
+  const void* fn = a.mode == kNufft ? reinterpret_cast<const void*>(&mf_cell_gather_kernel<T, true>)
+                                   : reinterpret_cast<const void*>(&mf_cell_gather_kernel<T, false>);
   const int smem = static_cast<int>(sizeof(GatherSmem));
   err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (err != cudaSuccess) return err;
@@ -763,7 +765,7 @@ __device__ __forceinline__ void red_add4(float4* dst, float2 a, float2 b) {
 // take 0.24 ms here, 2.37 ms by the recurrence of the direct kernel.
 constexpr int kMomentTile = 128;
 
-template <typename T>
+template <typename T, bool ACCURATE>
 __global__ void __launch_bounds__(128, 4) mf_moment_kernel(const MomentP<T> p) {
   constexpr int Q = MomentCells::Q;
   __shared__ double2 sxy[kMomentTile], szv[kMomentTile];
@@ -842,9 +844,7 @@ __global__ void __launch_bounds__(128, 4) mf_moment_kernel(const MomentP<T> p) {
         const Leg lr = leg_length(mr[0], mr[1], mr[2], mr[3], xy.x, xy.y, zv.x, zv.y);
         const float hi = lt.d + lr.d, lo = lt.l + lr.l;
         const CellPos c = pair_cell(p.ph, hi, lo);
-        float sn, cs;
-        __sincosf(6.28318530717958647692f * pair_cycles(p.ph, hi, lo), &sn, &cs);
-        w[u] = make_float2(fmaf(g.x, cs, -g.y * sn), fmaf(g.x, sn, g.y * cs));
+        w[u] = cmul(g, pair_phasor<ACCURATE>(pair_cycles(p.ph, hi, lo)));
         x[u] = c.x;
         m[u] = c.m;
       }
@@ -1016,7 +1016,8 @@ cudaError_t launch_cells_backward(const MfArgs& a, unsigned char* ws, cudaStream
   mp.apad = (a.A + 31) / 32 * 32;
   mp.vox_per_split = sh.vox_per_split;
   mp.ph = pair_phase(pc.k0, pc.b0, pc.k1, pc.b1, a.S, kappa);
-  mf_moment_kernel<T><<<dim3(sh.groups, sh.splits), sh.threads, 0, st>>>(mp);
+  if (a.mode == kNufft) mf_moment_kernel<T, true><<<dim3(sh.groups, sh.splits), sh.threads, 0, st>>>(mp);
+  else mf_moment_kernel<T, false><<<dim3(sh.groups, sh.splits), sh.threads, 0, st>>>(mp);
 
   if (sh.splits > 1) {
     constexpr int pairs = MomentCells::Q / 2;
@@ -1049,10 +1050,15 @@ cudaError_t launch_cells_backward(const MfArgs& a, unsigned char* ws, cudaStream
 // direct kernel: the gradient of |y| divides by |y|, which turns the ~2e-6 between
 // the two kernels (the direct one's error near theta = 0) into 3e-5 of the
 // gradients, more than a training run should move by from one release to the next.
-bool mf_cells_forward_applies(const MfArgs& a) {
-  return a.mode == kMixed && !a.direct_only && a.dtype != kF64 && a.S >= 32 && a.S <= 4096 && a.N >= 512 &&
-         a.A > 128 && static_cast<double>(a.A) * a.N * a.S >= 1.0e8;
+// The NUFFT form goes the same way from 8 taps on (fewer taps are a coarser form
+// of their own), with the accurate phasor.
+bool cells_apply(const MfArgs& a, int taps, int64_t min_antennas) {
+  if (a.mode == kPlain || (a.mode == kNufft && taps < 8)) return false;
+  return !a.direct_only && a.dtype != kF64 && a.S >= 32 && a.S <= 4096 && a.N >= 512 && a.A >= min_antennas &&
+         static_cast<double>(a.A) * a.N * a.S >= 1.0e8;
 }
+
+bool mf_cells_forward_applies(const MfArgs& a, int taps) { return cells_apply(a, taps, a.mode == kMixed ? 129 : 24); }
 
 size_t mf_cells_forward_workspace(const MfArgs& a, size_t direct_partial_bytes) {
   const int splits = gather_splits(a.A, a.N);
@@ -1079,10 +1085,7 @@ cudaError_t mf_cells_forward(const MfArgs& a, void* ws, cudaStream_t st) {
 }
 
 // The adjoint's work is the pairs' too; a lane of its warps is an antenna.
-bool mf_cells_backward_applies(const MfArgs& a) {
-  return a.mode == kMixed && a.dtype != kF64 && a.S >= 32 && a.S <= 4096 && a.N >= 512 && a.A >= 24 &&
-         static_cast<double>(a.A) * a.N * a.S >= 1.0e8;
-}
+bool mf_cells_backward_applies(const MfArgs& a, int taps) { return cells_apply(a, taps, 24); }
 
 size_t mf_cells_backward_workspace(const MfArgs& a, size_t direct_partial_bytes) {
   return moment_layout(a.A, a.S, moment_shape(a.A, a.N).splits, direct_partial_bytes).total;

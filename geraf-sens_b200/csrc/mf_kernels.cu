@@ -909,20 +909,20 @@ cudaError_t launch_fft(const MfFftArgs& a, bool backward, cudaStream_t st) {
 
 // ---------------------------------------------------------------------------
 cudaError_t launch_finalize_partials(int dtype, const float2* partial, int splits, int64_t count,
-                                     float divisor, void* out_r, void* out_i, cudaStream_t st) {
+                                     float divisor, void* out_r, void* out_i, cudaStream_t st, const int* run_if) {
   const int blocks = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((count + 255) / 256, 148 * 16)));
   switch (dtype) {
     case kF64:
       finalize_partials_kernel<double><<<blocks, 256, 0, st>>>(
-          partial, splits, count, divisor, static_cast<double*>(out_r), static_cast<double*>(out_i));
+          partial, splits, count, divisor, static_cast<double*>(out_r), static_cast<double*>(out_i), run_if);
       break;
     case kF16:
       finalize_partials_kernel<__half><<<blocks, 256, 0, st>>>(
-          partial, splits, count, divisor, static_cast<__half*>(out_r), static_cast<__half*>(out_i));
+          partial, splits, count, divisor, static_cast<__half*>(out_r), static_cast<__half*>(out_i), run_if);
       break;
     default:
       finalize_partials_kernel<float><<<blocks, 256, 0, st>>>(
-          partial, splits, count, divisor, static_cast<float*>(out_r), static_cast<float*>(out_i));
+          partial, splits, count, divisor, static_cast<float*>(out_r), static_cast<float*>(out_i), run_if);
   }
   return cudaGetLastError();
 }
@@ -991,14 +991,14 @@ Tuning mf_forward_resolve(const MfArgs& a, const Tuning& req) {
 size_t mf_forward_workspace(const MfArgs& a, const Tuning& t) {
   if (a.mode == kNufft) return mf_nufft_forward_workspace(a, t);
   const size_t partial = t.splits <= 1 || a.N == 0 ? 0 : static_cast<size_t>(t.splits) * a.N * sizeof(float2);
-  return mf_cells_forward_applies(a) ? mf_cells_forward_workspace(a, partial) : partial;
+  return mf_cells_forward_applies(a, t.taps) ? mf_cells_forward_workspace(a, partial) : partial;
 }
 
 cudaError_t mf_forward(const MfArgs& a, const Tuning& t, void* ws, cudaStream_t st) {
   if (a.mode == kNufft) return mf_nufft_forward(a, t, ws, st);
   if (a.N == 0) return cudaSuccess;
   const int* run_if = nullptr;
-  if (mf_cells_forward_applies(a) && mf_cells_scale_ok(a)) {
+  if (mf_cells_forward_applies(a, t.taps) && mf_cells_scale_ok(a)) {
     const cudaError_t err = mf_cells_forward(a, ws, st);
     if (err != cudaSuccess) return err;
     run_if = mf_cells_bad_flag(ws);
@@ -1043,14 +1043,14 @@ size_t mf_backward_workspace(const MfArgs& a, const Tuning& t) {
   if (a.mode == kNufft) return mf_nufft_backward_workspace(a, t);
   if (a.mode == kPlain) return 0;
   const size_t partial = t.splits <= 1 ? 0 : static_cast<size_t>(t.splits) * a.A * a.S * sizeof(float2);
-  return mf_cells_backward_applies(a) ? mf_cells_backward_workspace(a, partial) : partial;
+  return mf_cells_backward_applies(a, t.taps) ? mf_cells_backward_workspace(a, partial) : partial;
 }
 
 cudaError_t mf_backward(const MfArgs& a, const Tuning& t, void* ws, cudaStream_t st) {
   if (a.mode == kNufft) return mf_nufft_backward(a, t, ws, st);
   if (a.A == 0 || a.S == 0) return cudaSuccess;
   const int* run_if = nullptr;
-  if (mf_cells_backward_applies(a) && mf_cells_scale_ok(a)) {
+  if (mf_cells_backward_applies(a, t.taps) && mf_cells_scale_ok(a)) {
     const cudaError_t err = mf_cells_backward(a, ws, st);
     if (err != cudaSuccess) return err;
     run_if = mf_moments_bad_flag(ws);

@@ -151,6 +151,7 @@ int grid_points(int64_t S) {
 // ---------------------------------------------------------------------------
 // 1. Deconvolution factors 1 / Phi((n - h) / M), n in [0, S).
 struct DeconvP {
+  const int* run_if;  // when set, the kernel runs only if *run_if != 0 (so for the others)
   GlRule gl;
   float* deconv;
   int S, h, M, W;
@@ -158,17 +159,23 @@ struct DeconvP {
 };
 
 __global__ void nufft_deconv_kernel(const DeconvP p) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p.run_if != nullptr && *p.run_if == 0) return;
+  // one warp per sample, the quadrature nodes over its lanes (a thread per sample took
+  // 17 us of dependent FP64 exponentials)
+  const int n = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
   if (n >= p.S) return;
   const double xi = static_cast<double>(n - p.h) / p.M;
   const double inv_half = 2.0 / p.W;
   double acc = 0.0;
-  for (int q = 0; q < kGlNodes; ++q) {
+  for (int q = lane; q < kGlNodes; q += 32) {
     const double t = p.gl.x[q] * inv_half;
     const double phi = exp(p.beta * (sqrt(fmax(0.0, 1.0 - t * t)) - 1.0));
     acc += p.gl.w[q] * phi * cospi(2.0 * xi * p.gl.x[q]);
   }
-  p.deconv[n] = static_cast<float>(1.0 / (2.0 * acc));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0) p.deconv[n] = static_cast<float>(1.0 / (2.0 * acc));
 }
 
 // ---------------------------------------------------------------------------
@@ -183,6 +190,7 @@ struct GridP {
   int64_t A;
   int S, h, M, log2M;
   int index_weight;  // 1: grid of n * s[a, n] instead of s[a, n]
+  const int* run_if = nullptr;
 };
 
 __device__ __forceinline__ unsigned bit_reverse(unsigned x, int bits) {
@@ -213,6 +221,7 @@ __device__ __forceinline__ void fft_radix2(float2* fbuf, int M, float sign) {
 template <typename T>
 __global__ void __launch_bounds__(512) nufft_grid_kernel(const GridP<T> p) {
   extern __shared__ float2 fbuf[];  // [M]
+  if (p.run_if != nullptr && *p.run_if == 0) return;
   const int M = p.M;
   for (int64_t a = blockIdx.x; a < p.A; a += gridDim.x) {
     for (int idx = threadIdx.x; idx < M; idx += blockDim.x) {
@@ -289,8 +298,10 @@ struct RowStager {
   }
 };
 
-cudaError_t launch_deconv(float* deconv, int64_t S, int h, int M, int W, double beta, cudaStream_t st) {
+cudaError_t launch_deconv(float* deconv, int64_t S, int h, int M, int W, double beta, cudaStream_t st,
+                          const int* run_if = nullptr) {
   DeconvP dp;
+  dp.run_if = run_if;
   dp.gl = gauss_legendre(0.5 * W);
   dp.deconv = deconv;
   dp.S = static_cast<int>(S);
@@ -298,7 +309,7 @@ cudaError_t launch_deconv(float* deconv, int64_t S, int h, int M, int W, double 
   dp.M = M;
   dp.W = W;
   dp.beta = beta;
-  nufft_deconv_kernel<<<static_cast<unsigned>((S + 127) / 128), 128, 0, st>>>(dp);
+  nufft_deconv_kernel<<<static_cast<unsigned>((S + 3) / 4), 128, 0, st>>>(dp);
   return cudaGetLastError();
 }
 
@@ -316,11 +327,13 @@ struct BboxP {
   int64_t N, pstride, cstride;
   float* partial;  // [blocks][6]
   float* bbox;     // [6]: lo xyz, hi xyz
+  const int* run_if = nullptr;
 };
 
 template <typename T>
 __global__ void __launch_bounds__(256) voxel_bbox_partial_kernel(const BboxP<T> p) {
   __shared__ float red[6][256];
+  if (p.run_if != nullptr && *p.run_if == 0) return;
   float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
   for (int64_t v = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; v < p.N;
        v += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -350,12 +363,18 @@ __global__ void __launch_bounds__(256) voxel_bbox_partial_kernel(const BboxP<T> 
   if (threadIdx.x < 6) p.partial[blockIdx.x * 6 + threadIdx.x] = red[threadIdx.x][0];
 }
 
-__global__ void voxel_bbox_final_kernel(const float* partial, int blocks, float* bbox) {
-  const int c = threadIdx.x;
-  if (c >= 6) return;
+// One warp per component (192 threads).
+__global__ void voxel_bbox_final_kernel(const float* partial, int blocks, float* bbox, const int* run_if = nullptr) {
+  if (run_if != nullptr && *run_if == 0) return;
+  const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float r = c < 3 ? INFINITY : -INFINITY;
-  for (int b = 0; b < blocks; ++b) r = c < 3 ? fminf(r, partial[b * 6 + c]) : fmaxf(r, partial[b * 6 + c]);
-  bbox[c] = r;
+  for (int b = lane; b < blocks; b += 32) r = c < 3 ? fminf(r, partial[b * 6 + c]) : fmaxf(r, partial[b * 6 + c]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float y = __shfl_xor_sync(0xffffffffu, r, o);
+    r = c < 3 ? fminf(r, y) : fmaxf(r, y);
+  }
+  if (lane == 0) bbox[c] = r;
 }
 
 // Range of path lengths |t - x| + |r - x| over x in the box [lo, hi].
@@ -387,11 +406,13 @@ struct AdjFftP {
   int64_t A;
   int S, h, M, log2M, vsplits;
   float scale;  // 1/A (matched-filter adjoint) or 1/P (tracer forward)
+  const int* run_if = nullptr;
 };
 
 template <typename T>
 __global__ void __launch_bounds__(512) nufft_adjoint_fft_kernel(const AdjFftP<T> p) {
   extern __shared__ float2 fbuf[];  // [M]
+  if (p.run_if != nullptr && *p.run_if == 0) return;
   const int M = p.M;
   for (int64_t a = blockIdx.x; a < p.A; a += gridDim.x) {
     for (int l = threadIdx.x; l < M; l += blockDim.x) {

@@ -104,11 +104,13 @@ struct GatherP {
   int M, h, rows, splits;
   double k0, b0, k1, b1;
   size_t pos_off, buf_off;
+  const int* run_if;  // when set, the kernel runs only if *run_if != 0
 };
 
 template <typename T, int VPT, int W>
 __global__ void __launch_bounds__(256) nufft_gather_kernel(const GatherP<T> p) {
   extern __shared__ __align__(128) unsigned char smem[];
+  if (p.run_if != nullptr && *p.run_if == 0) return;
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
   double* pos = reinterpret_cast<double*>(smem + p.pos_off);
   const int Mp = p.M + kGridPad;
@@ -245,6 +247,7 @@ struct SpreadP {
   int64_t A, N, vox_per_split;
   int M, h, vsplits;
   double k0, b0, k1, b1;
+  const int* run_if;
 };
 
 struct SpreadVoxel {
@@ -271,6 +274,7 @@ __global__ void __launch_bounds__(kSpreadThreads) nufft_spread_kernel(const Spre
   __shared__ double pos[6];
   __shared__ int s_mode, s_w0;
   __shared__ float sums[2 * kWin];
+  if (p.run_if != nullptr && *p.run_if == 0) return;
   const int vs = blockIdx.x % p.vsplits;
   const int64_t a = blockIdx.x / p.vsplits;
   const int mask = p.M - 1;
@@ -413,14 +417,14 @@ AdjShape adj_shape(const MfArgs& a, const Tuning& t) {
 }
 
 template <typename T>
-cudaError_t launch_nufft_backward(const MfArgs& a, const Tuning& t, void* ws, cudaStream_t st) {
+cudaError_t launch_nufft_backward(const MfArgs& a, const Tuning& t, void* ws, cudaStream_t st, const int* run_if) {
   const AdjShape s = adj_shape(a, t);
   const NufftShape& b = s.base;
   unsigned char* base = static_cast<unsigned char*>(ws);
   float* deconv = reinterpret_cast<float*>(base + s.deconv_off);
   float2* grid = reinterpret_cast<float2*>(base + s.grid_off);
   const DeviceInfo dev = current_device_info();
-  cudaError_t err = launch_deconv(deconv, a.S, b.h, b.M, b.W, b.beta, st);
+  cudaError_t err = launch_deconv(deconv, a.S, b.h, b.M, b.W, b.beta, st, run_if);
   if (err != cudaSuccess) return err;
 
   float* bbox_partial = reinterpret_cast<float*>(base + s.bbox_off);
@@ -433,9 +437,10 @@ cudaError_t launch_nufft_backward(const MfArgs& a, const Tuning& t, void* ws, cu
     bp.cstride = a.N;
     bp.partial = bbox_partial;
     bp.bbox = bbox;
+    bp.run_if = run_if;
     const int nb = static_cast<int>(std::min<int64_t>(kBboxBlocks, (a.N + 255) / 256));
     voxel_bbox_partial_kernel<T><<<nb, 256, 0, st>>>(bp);
-    voxel_bbox_final_kernel<<<1, 32, 0, st>>>(bbox_partial, nb, bbox);
+    voxel_bbox_final_kernel<<<1, 192, 0, st>>>(bbox_partial, nb, bbox, run_if);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
   }
@@ -456,6 +461,7 @@ cudaError_t launch_nufft_backward(const MfArgs& a, const Tuning& t, void* ws, cu
   sp.M = b.M;
   sp.h = b.h;
   sp.vsplits = s.vsplits;
+  sp.run_if = run_if;
   const PhaseConsts pc = phase_consts(kMfStartFrequency, a.As, a.fs);
   sp.k0 = pc.k0;
   sp.b0 = pc.b0;
@@ -482,6 +488,7 @@ cudaError_t launch_nufft_backward(const MfArgs& a, const Tuning& t, void* ws, cu
   fp.M = b.M;
   fp.log2M = b.log2M;
   fp.vsplits = s.vsplits;
+  fp.run_if = run_if;
   fp.scale = 1.0f / static_cast<float>(a.A);
   const size_t fsmem = static_cast<size_t>(b.M) * sizeof(float2);
   err = cudaFuncSetAttribute(&nufft_adjoint_fft_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -494,14 +501,14 @@ cudaError_t launch_nufft_backward(const MfArgs& a, const Tuning& t, void* ws, cu
 }
 
 template <typename T>
-cudaError_t launch_nufft_forward(const MfArgs& a, const NufftShape& s, void* ws, cudaStream_t st) {
+cudaError_t launch_nufft_forward(const MfArgs& a, const NufftShape& s, void* ws, cudaStream_t st, const int* run_if) {
   unsigned char* base = static_cast<unsigned char*>(ws);
   float* deconv = reinterpret_cast<float*>(base + s.deconv_off);
   float2* grid = reinterpret_cast<float2*>(base + s.grid_off);
   const DeviceInfo dev = current_device_info();
 
   if (a.S > 0) {
-    cudaError_t err = launch_deconv(deconv, a.S, s.h, s.M, s.W, s.beta, st);
+    cudaError_t err = launch_deconv(deconv, a.S, s.h, s.M, s.W, s.beta, st, run_if);
     if (err != cudaSuccess) return err;
 
     GridP<T> gp;
@@ -515,6 +522,7 @@ cudaError_t launch_nufft_forward(const MfArgs& a, const NufftShape& s, void* ws,
     gp.M = s.M;
     gp.log2M = s.log2M;
     gp.index_weight = 0;
+    gp.run_if = run_if;
     const size_t fsmem = static_cast<size_t>(s.M) * sizeof(float2);
     err = cudaFuncSetAttribute(&nufft_grid_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(fsmem));
@@ -556,6 +564,7 @@ cudaError_t launch_nufft_forward(const MfArgs& a, const NufftShape& s, void* ws,
   p.b1 = pc.b1;
   p.pos_off = s.pos_off;
   p.buf_off = s.buf_off;
+  p.run_if = run_if;
 
   const void* fn = gather_kernel_ptr<T>(s.vpt, s.W);
   cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -570,7 +579,7 @@ cudaError_t launch_nufft_forward(const MfArgs& a, const NufftShape& s, void* ws,
   if (err != cudaSuccess) return err;
   if (s.splits > 1) {
     err = launch_finalize_partials(a.dtype, p.partial, s.splits, a.N, static_cast<float>(a.A),
-                                   a.out_real, a.out_imag, st);
+                                   a.out_real, a.out_imag, st, run_if);
   }
   return err;
 }
@@ -626,30 +635,46 @@ Tuning mf_nufft_backward_resolve(const MfArgs& a, const Tuning& req) {
 
 size_t mf_nufft_backward_workspace(const MfArgs& a, const Tuning& t) {
   if (a.A == 0 || a.S == 0) return 0;
-  return adj_shape(a, t).total;
+  const size_t cells = mf_cells_backward_applies(a, t.taps) ? mf_cells_backward_workspace(a, 0) : 0;
+  return cells + adj_shape(a, t).total;
 }
 
 cudaError_t mf_nufft_backward(const MfArgs& a, const Tuning& t, void* ws, cudaStream_t st) {
   if (a.A == 0 || a.S == 0) return cudaSuccess;
+  const int* run_if = nullptr;  // the range cells' flag: this form's kernels run where their bands do not fit
+  if (mf_cells_backward_applies(a, t.taps) && mf_cells_scale_ok(a)) {
+    const cudaError_t err = mf_cells_backward(a, ws, st);
+    if (err != cudaSuccess) return err;
+    run_if = mf_moments_bad_flag(ws);
+    ws = static_cast<unsigned char*>(ws) + mf_cells_backward_workspace(a, 0);
+  }
   switch (a.dtype) {
-    case kF64: return launch_nufft_backward<double>(a, t, ws, st);
-    case kF16: return launch_nufft_backward<__half>(a, t, ws, st);
-    default: return launch_nufft_backward<float>(a, t, ws, st);
+    case kF64: return launch_nufft_backward<double>(a, t, ws, st, run_if);
+    case kF16: return launch_nufft_backward<__half>(a, t, ws, st, run_if);
+    default: return launch_nufft_backward<float>(a, t, ws, st, run_if);
   }
 }
 
 size_t mf_nufft_forward_workspace(const MfArgs& a, const Tuning& t) {
   if (a.N == 0) return 0;
-  return nufft_shape(a, t).total;
+  const size_t cells = mf_cells_forward_applies(a, t.taps) ? mf_cells_forward_workspace(a, 0) : 0;
+  return cells + nufft_shape(a, t).total;
 }
 
 cudaError_t mf_nufft_forward(const MfArgs& a, const Tuning& t, void* ws, cudaStream_t st) {
   if (a.N == 0) return cudaSuccess;
+  const int* run_if = nullptr;
+  if (mf_cells_forward_applies(a, t.taps) && mf_cells_scale_ok(a)) {
+    const cudaError_t err = mf_cells_forward(a, ws, st);
+    if (err != cudaSuccess) return err;
+    run_if = mf_cells_bad_flag(ws);
+    ws = static_cast<unsigned char*>(ws) + mf_cells_forward_workspace(a, 0);
+  }
   const NufftShape s = nufft_shape(a, t);
   switch (a.dtype) {
-    case kF64: return launch_nufft_forward<double>(a, s, ws, st);
-    case kF16: return launch_nufft_forward<__half>(a, s, ws, st);
-    default: return launch_nufft_forward<float>(a, s, ws, st);
+    case kF64: return launch_nufft_forward<double>(a, s, ws, st, run_if);
+    case kF16: return launch_nufft_forward<__half>(a, s, ws, st, run_if);
+    default: return launch_nufft_forward<float>(a, s, ws, st, run_if);
   }
 }
 

@@ -492,7 +492,7 @@ cudaError_t launch_tracer_nufft_forward(const TracerArgs& a, const Tuning& t, vo
     bp.bbox = bbox;
     const int nb = static_cast<int>(std::min<int64_t>(kBboxBlocks, (a.P + 255) / 256));
     voxel_bbox_partial_kernel<T><<<nb, 256, 0, st>>>(bp);
-    voxel_bbox_final_kernel<<<1, 32, 0, st>>>(bbox_partial, nb, bbox);
+    voxel_bbox_final_kernel<<<1, 192, 0, st>>>(bbox_partial, nb, bbox);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
   }

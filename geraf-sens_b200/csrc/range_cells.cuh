@@ -123,6 +123,11 @@ __device__ __forceinline__ float pair_cycles(const PairPhase& p, float hi, float
   return fmaf(hi, p.kh, -k) + fmaf(lo, p.k_rest, fmaf(hi, p.kl, p.b));
 }
 
+template <bool ACCURATE>
+__device__ __forceinline__ float2 pair_phasor(float cycles) {
+  return ACCURATE ? cis_cycles(cycles) : cis_cycles_fast(cycles);
+}
+
 // Cell of the path and the offset x in it; m is the cell index plus the magic.
 struct CellPos {
   float m, x;

@@ -93,6 +93,23 @@ def test_backward_bands_that_leave_the_cells(cuda, box, bandwidth):
     assert rel_l2(got, ref) < 1e-5
 
 
+@pytest.mark.parametrize("box", [None, ((-0.6, -0.6, 0.2), (0.6, 0.6, 1.9))], ids=["cells", "wide_band"])
+@pytest.mark.parametrize("A,S,N", [(24, 256, 16385), (130, 33, 24001)])
+def test_nufft_form_vs_fp64(cuda, A, S, N, box):
+    """The NUFFT form takes the cells too (its own kernels where the band does not fit)."""
+    c = case(A + S, A, S, N, box=box)
+    ch = c["ch"]
+    args = (c["tx"], c["rx"], c["vox"])
+    y = mf_forward(c["re"], c["im"], *args, ch.adc_sample_rate, ch.As_sci, "nufft")
+    ref = oracle(c)
+    scale = np.linalg.norm(c["re"] + 1j * c["im"]) / np.sqrt(A)  # the wide scene's voxels see noise only
+    assert np.linalg.norm(y[0] + 1j * y[1] - ref) / np.sqrt(N) < 5e-6 * max(scale, np.linalg.norm(ref) / np.sqrt(N))
+    gr, gi = c["rng"].standard_normal((2, N)).astype(np.float32)
+    h = mf_backward(gr, gi, *args, A, S, ch.adc_sample_rate, ch.As_sci, "nufft")
+    r = orc.mf_backward(gr, gi, *args, A, S, ch.adc_sample_rate, ch.As_sci)
+    assert rel_l2(h[0] + 1j * h[1], r[0] + 1j * r[1]) < 5e-6
+
+
 def test_backward_nan_voxel_poisons_every_sample(cuda):
     c = case(9, 140, 128, 6001)
     c["vox"][0, 5] = np.nan
