@@ -158,7 +158,20 @@ struct PointList {
 bool tracer_point_list_applies(const TracerArgs& a);
 size_t tracer_point_list_bytes(int64_t P);
 PointList tracer_point_list_view(void* ws, int64_t P);
-cudaError_t tracer_point_list(const TracerArgs& a, void* ws, bool zero_grads, cudaStream_t st);
+// With `boxes`, the bounding boxes of each chunk's listed points (6 floats: lo xyz,
+// hi xyz) for tracer_point_chunks(P) chunks.
+int64_t tracer_point_chunks(int64_t P);
+cudaError_t tracer_point_list(const TracerArgs& a, void* ws, bool zero_grads, cudaStream_t st, float* boxes = nullptr);
+
+// MIXED tracer adjoint through range cells (tracer_adjoint_cells.cu), for calls with a point
+// list: its workspace comes first, then the partials and the list.  `partial` ([splits][P][6])
+// is summed by launch_tracer_bwd_finalize.  *bad is the device flag that sends a call to the
+// general kernel instead.
+bool tracer_adjoint_cells_apply(const TracerArgs& a);
+size_t tracer_adjoint_cells_workspace(const TracerArgs& a);
+float* tracer_adjoint_cells_boxes(void* ws);
+cudaError_t tracer_adjoint_cells(const TracerArgs& a, void* ws, PointList list, float* partial, int splits, cudaStream_t st,
+                                 const int** bad);
 
 // Fast approximate tracer (MODE_NUFFT, nufft_tracer_kernels.cu); the generic
 // tracer_* entry points dispatch here for that mode.

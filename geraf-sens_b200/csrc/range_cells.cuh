@@ -163,42 +163,49 @@ __device__ __forceinline__ void leg_range(const F* t, const F* box, F& near2, F&
   }
 }
 
+// Positive Chebyshev nodes on [-1/2, 1/2], cos((2 i + 1) pi / (2 Q)) / 2.
+template <int Q>
+__host__ __device__ constexpr double cell_node(int i) {
+  static_assert(Q == 6 || Q == 8, "the numbers of coefficients in use");
+  if (Q == 6) return i == 0 ? 0.48296291314453416 : i == 1 ? 0.3535533905932738 : 0.12940952255126037;
+  return i == 0 ? 0.4903926402016152 : i == 1 ? 0.4157348061512726 : i == 2 ? 0.27778511650980114 : 0.09754516100806417;
+}
+
 // Interpolation of cos(theta x) and sin(theta x) on [-1/2, 1/2]: coefficients
 // g[j] of x^j, even j for the cosine, odd j for the sine, from Newton's divided
-// differences in x^2 at the positive Chebyshev nodes (FP64).
+// differences in x^2 at the positive nodes (FP64; every divisor is a compile-time constant).
 template <int Q>
 __device__ __forceinline__ void cell_basis(double theta, float* g) {
-  static_assert(Q % 2 == 0, "even number of coefficients");
   constexpr int H = Q / 2;
-  double X[H], c[H], s[H];
+  double c[H], s[H];
 #pragma unroll
   for (int i = 0; i < H; ++i) {
-    const double x = 0.5 * cospi((2 * i + 1) / (2.0 * Q));
-    X[i] = x * x;
     double sn, cs;
-    sincos(theta * x, &sn, &cs);
+    sincos(theta * cell_node<Q>(i), &sn, &cs);
     c[i] = cs;
-    s[i] = sn / x;
+    s[i] = sn * (1.0 / cell_node<Q>(i));
   }
 #pragma unroll
   for (int o = 1; o < H; ++o) {
 #pragma unroll
     for (int i = H - 1; i >= o; --i) {
-      c[i] = (c[i] - c[i - 1]) / (X[i] - X[i - o]);
-      s[i] = (s[i] - s[i - 1]) / (X[i] - X[i - o]);
+      const double d = 1.0 / (cell_node<Q>(i) * cell_node<Q>(i) - cell_node<Q>(i - o) * cell_node<Q>(i - o));
+      c[i] = (c[i] - c[i - 1]) * d;
+      s[i] = (s[i] - s[i - 1]) * d;
     }
   }
-  // Newton form to monomials in X
+  // Newton form to monomials in x^2
   double mc[H] = {}, ms[H] = {};
 #pragma unroll
   for (int i = H - 1; i >= 0; --i) {
+    const double X = cell_node<Q>(i) * cell_node<Q>(i);
 #pragma unroll
     for (int q = H - 1; q >= 1; --q) {
-      mc[q] = mc[q - 1] - X[i] * mc[q];
-      ms[q] = ms[q - 1] - X[i] * ms[q];
+      mc[q] = mc[q - 1] - X * mc[q];
+      ms[q] = ms[q - 1] - X * ms[q];
     }
-    mc[0] = c[i] - X[i] * mc[0];
-    ms[0] = s[i] - X[i] * ms[0];
+    mc[0] = c[i] - X * mc[0];
+    ms[0] = s[i] - X * ms[0];
   }
 #pragma unroll
   for (int q = 0; q < H; ++q) {

@@ -1,0 +1,417 @@
+// MIXED tracer adjoint through range cells: per live (point, antenna) pair the sums over
+// the residual row g[a, :] that the gradients need,
+//   Q = sum_n conj(g_n) e^{+j 2 pi n' d},   Q1 = sum_n n' conj(g_n) e^{+j 2 pi n' d},
+// are the conjugates of a polynomial of the path length and (scaled) of its
+// derivative, whose coefficients per cell are formed once per antenna
+// (range_cells.cuh, the matched filter's table).  Samples are counted from their
+// middle, so Q1 carries only the sweep's share of the phase rate (a few percent of
+// the carrier's): the derivative's larger interpolation error stays below the
+// FP32 rounding of the result.
+//
+// Launches: the band of cells from the boxes of the listed points and of the
+// antennas, with the interpolation basis; the antennas' tables; the pairs.  Where the
+// band does not fit kAdjCells cells the pairs are left to the general kernel
+// (tracer_kernels.cu), which returns at once otherwise.
+#include <algorithm>
+#include <cmath>
+
+#include "kernels.h"
+#include "range_cells.cuh"
+#include "tracer_geometry.cuh"
+
+namespace geraf {
+namespace {
+
+using namespace tracer;
+
+constexpr int kQ = GatherCells::Q;
+constexpr int kAdjCells = 128;  // 2.4 m of path at 4 GHz swept
+constexpr int kBandThreads = 1024;
+constexpr int kTableThreads = 128;
+constexpr int kTableCells = 16;  // cells per block of the table kernel
+constexpr int kPairThreads = 128;
+constexpr int kPairAnts = 32;    // antennas staged at a time
+
+struct AdjHead {
+  int bad;
+  int k0, cells;
+  int pad;
+};
+
+struct AdjLayout {
+  size_t head, boxes, basis, table, total;
+};
+
+size_t up256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
+
+AdjLayout adj_layout(const TracerArgs& a) {
+  AdjLayout l;
+  l.head = 0;
+  l.boxes = 256;
+  l.basis = up256(l.boxes + static_cast<size_t>(tracer_point_chunks(a.P)) * 6 * sizeof(float));
+  l.table = up256(l.basis + static_cast<size_t>(a.S) * kQ * sizeof(float));
+  l.total = up256(l.table + static_cast<size_t>(a.A) * kAdjCells * kQ * sizeof(float2));
+  return l;
+}
+
+struct AdjConsts {
+  double K, b, k1, b1, kappa, theta_step;
+  int S;
+};
+
+template <typename T>
+struct BandP {
+  const float* boxes;
+  int64_t chunks, A;
+  const T* tx;
+  const T* rx;
+  AdjHead* head;
+  float* basis;
+  AdjConsts c;
+};
+
+// One block.  Lane groups of 32 x 18 box components would leave most of a block idle on
+// long chunk lists, so every thread reduces all components over its share.
+template <typename T>
+__global__ void __launch_bounds__(kBandThreads) adj_band_kernel(const BandP<T> p) {
+  __shared__ float red[kBandThreads / 32][18];
+  __shared__ float box[18];
+  for (int n = threadIdx.x; n < p.c.S; n += kBandThreads) {
+    float g[kQ];
+    cell_basis<kQ>(p.c.theta_step * (n - 0.5 * (p.c.S - 1)), g);
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) p.basis[static_cast<int64_t>(n) * kQ + q] = g[q];
+  }
+  float b[18];
+#pragma unroll
+  for (int c = 0; c < 18; ++c) b[c] = c % 6 < 3 ? INFINITY : -INFINITY;
+  for (int64_t i = threadIdx.x; i < p.chunks; i += kBandThreads) {
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      const float x = p.boxes[i * 6 + c];
+      b[c] = c < 3 ? fminf(b[c], x) : fmaxf(b[c], x);
+    }
+  }
+  for (int64_t a = threadIdx.x; a < p.A; a += kBandThreads) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float t = ld_f(p.tx, a * 3 + c), r = ld_f(p.rx, a * 3 + c);
+      // a NaN antenna widens its box to infinity
+      b[6 + c] = fminf(b[6 + c], t == t ? t : -INFINITY);
+      b[9 + c] = fmaxf(b[9 + c], t == t ? t : INFINITY);
+      b[12 + c] = fminf(b[12 + c], r == r ? r : -INFINITY);
+      b[15 + c] = fmaxf(b[15 + c], r == r ? r : INFINITY);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 18; ++c) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float y = __shfl_xor_sync(0xffffffffu, b[c], o);
+      b[c] = c % 6 < 3 ? fminf(b[c], y) : fmaxf(b[c], y);
+    }
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][c] = b[c];
+  }
+  __syncthreads();
+  if (threadIdx.x < 18) {
+    const int c = threadIdx.x;
+    float r = red[0][c];
+    for (int w = 1; w < kBandThreads / 32; ++w) r = c % 6 < 3 ? fminf(r, red[w][c]) : fmaxf(r, red[w][c]);
+    box[c] = r;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  double near[2] = {0.0, 0.0}, far[2] = {0.0, 0.0};
+  for (int k = 0; k < 3; ++k) {
+    const double lo = box[k], hi = box[3 + k];
+    for (int e = 0; e < 2; ++e) {
+      const double alo = box[6 + 6 * e + k], ahi = box[9 + 6 * e + k];
+      const double gap = fmax(0.0, fmax(lo - ahi, alo - hi)), reach = fmax(hi - alo, ahi - lo);
+      near[e] += gap * gap;
+      far[e] += reach * reach;
+    }
+  }
+  const double lo = floor((sqrt(near[0]) + sqrt(near[1])) * p.c.kappa) - 1.0;
+  const double hi = ceil((sqrt(far[0]) + sqrt(far[1])) * p.c.kappa) + 1.0;
+  const bool none = box[0] > box[3];  // no listed point: no pairs either
+  const bool fits = none || (hi - lo + 1.0 <= kAdjCells && hi < 1073741824.0);  // false for NaN
+  p.head->bad = fits ? 0 : 1;
+  p.head->k0 = fits && !none ? static_cast<int>(lo) : 0;
+  p.head->cells = fits && !none ? static_cast<int>(hi - lo) + 1 : 0;
+}
+
+template <typename T>
+struct AdjTableP {
+  const T* gr;
+  const T* gi;
+  const float* basis;
+  const AdjHead* head;
+  float2* table;  // [A][kAdjCells][kQ]
+  AdjConsts c;
+};
+
+// Block (antenna, 16 cells): thread (cell, slice of 8) as in the matched filter's table.
+template <typename T>
+__global__ void __launch_bounds__(kTableThreads) adj_table_kernel(const AdjTableP<T> p) {
+  constexpr int kSlices = kTableThreads / kTableCells;
+  __shared__ float2 red[kSlices][kTableCells][kQ];
+  const int cell = static_cast<int>(blockIdx.y) * kTableCells + threadIdx.x % kTableCells;
+  const int cells = p.head->cells;
+  if (static_cast<int>(blockIdx.y) * kTableCells >= cells) return;
+  const int64_t a = blockIdx.x;
+  const int slice = threadIdx.x / kTableCells;
+  const double dk = fma(p.c.k1, static_cast<double>(p.head->k0 + cell) / p.c.kappa, p.c.b1);
+  const double mid = 0.5 * (p.c.S - 1);
+  float2 acc[kQ];
+#pragma unroll
+  for (int q = 0; q < kQ; ++q) acc[q] = make_float2(0.0f, 0.0f);
+  for (int n = slice; n < p.c.S; n += kSlices) {
+    const double ph = (n - mid) * dk;
+    const float2 e = cis_cycles(static_cast<float>(ph - rint(ph)));
+    const float xr = ld_f(p.gr, a * p.c.S + n), xi = ld_f(p.gi, a * p.c.S + n);
+    const float2 v = make_float2(fmaf(xr, e.x, xi * e.y), fmaf(xi, e.x, -xr * e.y));
+    const float2 w = make_float2(v.y, -v.x);
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) {
+      const float g = p.basis[static_cast<int64_t>(n) * kQ + q];
+      acc[q] = ffma2(make_float2(g, g), (q & 1) ? w : v, acc[q]);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < kQ; ++q) red[slice][threadIdx.x % kTableCells][q] = acc[q];
+  __syncthreads();
+  float2* out = p.table + (a * kAdjCells + blockIdx.y * kTableCells) * kQ;
+  const int live = min(kTableCells, cells - static_cast<int>(blockIdx.y) * kTableCells);
+  for (int i = threadIdx.x; i < live * kQ; i += kTableThreads) {
+    float2 s = (&red[0][0][0])[i];
+    for (int k = 1; k < kSlices; ++k) s = fadd2(s, (&red[k][0][0])[i]);
+    out[i] = s;
+  }
+}
+
+template <typename T>
+struct AdjPairP {
+  const T* normals;
+  const T* sigmas;
+  const T* points;
+  const T* tx;
+  const T* rx;
+  T* g_normals;
+  T* g_sigmas;
+  T* g_points;
+  const int* plist;
+  const int* plist_count;
+  const float2* table;
+  const AdjHead* head;
+  float* partial;  // [splits][P][6]
+  int64_t A, P, per_split;
+  int splits;
+  float w_mid, kappa_c;  // phase rate of carrier and middle sample, cells per unit delay
+  AdjConsts c;
+};
+
+// One thread per listed point, the antennas of the block's split in order; nothing is
+// shared but the antennas' positions, so the warps run free of barriers.  About 260
+// instructions per live pair, independent of the sample count.
+template <typename T, bool WITH_POINTS>
+__global__ void __launch_bounds__(kPairThreads, 5) adj_pair_kernel(const AdjPairP<T> p) {
+  __shared__ float ant[kPairAnts][6];
+  if (p.head->bad) return;
+  const int split = blockIdx.x % p.splits;
+  const int64_t base = static_cast<int64_t>(blockIdx.x / p.splits) * kPairThreads;
+  const int64_t count = *p.plist_count;
+  if (base >= count) return;
+  const bool inside = base + threadIdx.x < count;
+  const int64_t q = p.plist[min(base + threadIdx.x, count - 1)];
+  const int k0 = p.head->k0, cells = p.head->cells;
+  float nrm[3], pt[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    nrm[c] = ld_f(p.normals, q * 3 + c);
+    pt[c] = ld_f(p.points, q * 3 + c);
+  }
+  float gn[3] = {0.0f, 0.0f, 0.0f}, gp[3] = {0.0f, 0.0f, 0.0f};
+  const int64_t a_begin = split * p.per_split, a_end = min(p.A, a_begin + p.per_split);
+  const float inv_p = static_cast<float>(p.P);
+  for (int64_t a0 = a_begin; a0 < a_end; a0 += kPairAnts) {
+    const int rows = static_cast<int>(min(static_cast<int64_t>(kPairAnts), a_end - a0));
+    __syncthreads();
+    for (int i = threadIdx.x; i < rows * 6; i += kPairThreads) {
+      const int r = i / 6, c = i % 6;
+      ant[r][c] = c < 3 ? ld_f(p.tx, (a0 + r) * 3 + c) : ld_f(p.rx, (a0 + r) * 3 + c - 3);
+    }
+    __syncthreads();
+    if (!inside) continue;
+    float sigma = ld_f(p.sigmas, a0 * p.P + q);
+    for (int r = 0; r < rows; ++r) {
+      const int64_t a = a0 + r;
+      const float sigma_value = sigma;
+      if (r + 1 < rows) sigma = ld_f(p.sigmas, (a + 1) * p.P + q);
+      float txp[3], rxp[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        txp[c] = ant[r][c];
+        rxp[c] = ant[r][3 + c];
+      }
+      PairGeom g;
+      if (!pair_geometry(txp, rxp, nrm, pt, g)) {
+        p.g_sigmas[a * p.P + q] = from_f<T>(0.0f);
+        continue;
+      }
+      double st = 0.0, sr = 0.0;
+#pragma unroll
+      for (int c = 2; c >= 0; --c) {
+        const double dt = static_cast<double>(txp[c]) - static_cast<double>(pt[c]);
+        const double dr = static_cast<double>(rxp[c]) - static_cast<double>(pt[c]);
+        st = fma(dt, dt, st);
+        sr = fma(dr, dr, sr);
+      }
+      const double d = sqrt_f64_fast(st) + sqrt_f64_fast(sr);
+      const double u = d * p.c.kappa, ku = rint(u);
+      const double ph = fma(d, p.c.K, p.c.b);
+      const float x = static_cast<float>(u - ku);
+      const int k = min(max(static_cast<int>(ku) - k0, 0), cells - 1);
+      const float4* row = reinterpret_cast<const float4*>(p.table + (a * kAdjCells + k) * kQ);
+      const float4 c2 = __ldg(row + 2), c1 = __ldg(row + 1), c0 = __ldg(row);
+      const float2 xx = make_float2(x, x);
+      // the polynomial and its derivative by Horner
+      float2 pv = make_float2(c2.z, c2.w), dv = pv;
+      pv = ffma2(pv, xx, make_float2(c2.x, c2.y));
+      dv = ffma2(dv, xx, pv);
+      pv = ffma2(pv, xx, make_float2(c1.z, c1.w));
+      dv = ffma2(dv, xx, pv);
+      pv = ffma2(pv, xx, make_float2(c1.x, c1.y));
+      dv = ffma2(dv, xx, pv);
+      pv = ffma2(pv, xx, make_float2(c0.z, c0.w));
+      dv = ffma2(dv, xx, pv);
+      pv = ffma2(pv, xx, make_float2(c0.x, c0.y));
+      const float2 e = cis_cycles_fast(static_cast<float>(ph - rint(ph)));
+      // sum_n (g_r cos + g_i sin) = Re(e conj(P))
+      const float sum_re = fmaf(e.x, pv.x, e.y * pv.y);
+      const float atten = 1.0f / sq(g.dist);
+      p.g_sigmas[a * p.P + q] = from_f<T>(atten * g.align * sum_re / inv_p);
+      const float scale = sigma_value * atten;
+      const float nu = dot3(nrm, g.u);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) gn[c] = fmaf(-2.0f * scale * sum_re, fmaf(nu, g.inc[c], g.idn * g.u[c]), gn[c]);
+      if (WITH_POINTS) {
+        // sum_n w_n (g_i cos - g_r sin) = -Im(e (w_mid conj(P) - j kappa c conj(P')))
+        const float f = p.w_mid * fmaf(e.y, pv.x, -e.x * pv.y) - p.kappa_c * fmaf(e.x, dv.x, e.y * dv.y);
+        const float amp = scale * g.align;
+        const float d_tau = -amp * f / kSpeedOfLight;
+        const float d_dist = -2.0f * amp / g.dist * sum_re + d_tau;
+        float v[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[c] = fmaf(-2.0f * nu, nrm[c], g.u[c]);
+        const float iv = dot3(g.inc, v);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          // d rho / d p, and the change of the path length
+          const float drho = (v[c] - g.inc[c] * iv) * g.inv_t - (g.refl[c] - g.ret[c] * g.align) * g.inv_r;
+          gp[c] += fmaf(scale * sum_re, drho, d_dist * (g.inc[c] - g.ret[c]));
+        }
+      }
+    }
+  }
+  if (!inside) return;
+  if (p.splits == 1) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      p.g_normals[q * 3 + c] = from_f<T>(gn[c] / inv_p);
+      if (WITH_POINTS) p.g_points[q * 3 + c] = from_f<T>(gp[c] / inv_p);
+    }
+  } else {
+    float* dst = p.partial + (split * p.P + q) * 6;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      dst[c] = gn[c];
+      dst[3 + c] = gp[c];
+    }
+  }
+}
+
+template <typename T>
+cudaError_t launch_adjoint(const TracerArgs& a, unsigned char* ws, PointList list, float* partial, int splits,
+                           cudaStream_t st) {
+  const AdjLayout l = adj_layout(a);
+  const PhaseConsts pc = phase_consts(a.f0, a.As, a.fs);
+  const double mid = 0.5 * static_cast<double>(a.S - 1);
+  AdjConsts c;
+  c.K = pc.k0 + mid * pc.k1;
+  c.b = pc.b0 + mid * pc.b1;
+  c.k1 = pc.k1;
+  c.b1 = pc.b1;
+  // without a sweep every path is in one cell
+  c.kappa = std::max(1e-6, GatherCells::kOver * static_cast<double>(a.S) * std::fabs(pc.k1));
+  c.theta_step = 2.0 * M_PI * pc.k1 / c.kappa;
+  c.S = static_cast<int>(a.S);
+  AdjHead* head = reinterpret_cast<AdjHead*>(ws + l.head);
+
+  BandP<T> bp;
+  bp.boxes = reinterpret_cast<const float*>(ws + l.boxes);
+  bp.chunks = tracer_point_chunks(a.P);
+  bp.A = a.A;
+  bp.tx = static_cast<const T*>(a.tx);
+  bp.rx = static_cast<const T*>(a.rx);
+  bp.head = head;
+  bp.basis = reinterpret_cast<float*>(ws + l.basis);
+  bp.c = c;
+  adj_band_kernel<T><<<1, kBandThreads, 0, st>>>(bp);
+
+  AdjTableP<T> tp;
+  tp.gr = static_cast<const T*>(a.grad_real_out);
+  tp.gi = static_cast<const T*>(a.grad_imag_out);
+  tp.basis = bp.basis;
+  tp.head = head;
+  tp.table = reinterpret_cast<float2*>(ws + l.table);
+  tp.c = c;
+  adj_table_kernel<T><<<dim3(static_cast<unsigned>(a.A), kAdjCells / kTableCells), kTableThreads, 0, st>>>(tp);
+
+  AdjPairP<T> pp;
+  pp.normals = static_cast<const T*>(a.normals);
+  pp.sigmas = static_cast<const T*>(a.sigmas);
+  pp.points = static_cast<const T*>(a.points);
+  pp.tx = bp.tx;
+  pp.rx = bp.rx;
+  pp.g_normals = static_cast<T*>(a.grad_normals);
+  pp.g_sigmas = static_cast<T*>(a.grad_sigmas);
+  pp.g_points = static_cast<T*>(a.grad_points);
+  pp.plist = list.list;
+  pp.plist_count = list.count;
+  pp.table = tp.table;
+  pp.head = head;
+  pp.partial = partial;
+  pp.A = a.A;
+  pp.P = a.P;
+  pp.splits = splits;
+  pp.per_split = (a.A + splits - 1) / splits;
+  pp.w_mid = static_cast<float>(2.0 * static_cast<double>(kPiF) * (static_cast<double>(a.f0) + static_cast<double>(a.As) / a.fs * mid));
+  pp.kappa_c = static_cast<float>(c.kappa * static_cast<double>(kSpeedOfLight));
+  pp.c = c;
+  // the grid covers all P points; blocks past the listed ones return at once
+  const int64_t blocks = (a.P + kPairThreads - 1) / kPairThreads * splits;
+  if (blocks > 0x7fffffff) return cudaErrorInvalidConfiguration;
+  if (a.grad_points != nullptr) adj_pair_kernel<T, true><<<static_cast<unsigned>(blocks), kPairThreads, 0, st>>>(pp);
+  else adj_pair_kernel<T, false><<<static_cast<unsigned>(blocks), kPairThreads, 0, st>>>(pp);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+bool tracer_adjoint_cells_apply(const TracerArgs& a) {
+  return a.mode == kMixed && tracer_point_list_applies(a) && a.A > 0 && a.S >= 32 && a.S <= 4096;
+}
+
+size_t tracer_adjoint_cells_workspace(const TracerArgs& a) { return adj_layout(a).total; }
+
+float* tracer_adjoint_cells_boxes(void* ws) { return reinterpret_cast<float*>(static_cast<unsigned char*>(ws) + 256); }
+
+cudaError_t tracer_adjoint_cells(const TracerArgs& a, void* ws, PointList list, float* partial, int splits, cudaStream_t st,
+                                 const int** bad) {
+  unsigned char* base = static_cast<unsigned char*>(ws);
+  *bad = &reinterpret_cast<AdjHead*>(base)->bad;
+  if (a.dtype == kF64) return launch_adjoint<double>(a, base, list, partial, splits, st);
+  return launch_adjoint<float>(a, base, list, partial, splits, st);
+}
+
+}  // namespace geraf

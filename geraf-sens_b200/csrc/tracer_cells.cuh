@@ -1,0 +1,402 @@
+// MIXED tracer forward through range cells: the live points of one antenna enter
+// its samples through the moments of their cells (range_cells.cuh, the adjoint of
+// the matched filter),
+//   x[a, n] = (1/P) sum_cells e^{+j 2 pi n' d_k} (sum_q even g_q(n) M_q + j sum_q odd g_q(n) M_q),
+//   M_q = sum_p amp_p e^{+j 2 pi c_p} x_p^q,
+// so a live point costs eight multiply-adds instead of S phasors.
+//
+// A block takes runs of one antenna's points.  Points are screened with the
+// conservative early test as they stream in; those it cannot cull are listed, and
+// 128 at a time get the exact geometry, one per thread, so no lane sits out the
+// expensive part (on a typical scene one point in ten is live).  The 128 points'
+// contributions are then sorted by cell in shared memory and added up by groups
+// of eight lanes, one per moment, in list order: no floating-point atomics, the
+// same bits on every run.
+//
+// Cells are kept in kTraceSlots slots, cell k in slot k mod kTraceSlots.  Two
+// cells of one run that fall in the same slot (2.4 m of path apart at 4 GHz swept)
+// are kept apart: the later ones wait until the slot's moments were turned into
+// samples and added to the run's row of samples.
+#pragma once
+
+#include "range_cells.cuh"
+#include "tracer_geometry.cuh"
+
+namespace geraf {
+namespace tracer {
+
+constexpr int kTraceThreads = 128;
+constexpr int kTraceWarps = kTraceThreads / 32;
+constexpr int kTracePer = 4;  // points per thread and screening pass
+constexpr int kTraceQ = MomentCells::Q;
+constexpr int kTraceSlots = 64;
+constexpr int kTraceEmpty = INT32_MIN + 1;  // no finite path has this cell
+constexpr int kTraceRow = kTraceQ + 2;      // float2 per contribution row: 80 bytes, conflict-free
+
+struct TraceConsts {
+  double K, b;       // phase of carrier and middle sample, cycles per metre and bias
+  double k1, b1;     // phase step per sample
+  double kappa;      // cells per metre
+  double theta_step;
+  int S;
+};
+
+inline TraceConsts trace_consts(double k0, double b0, double k1, double b1, int64_t S) {
+  TraceConsts t;
+  const double mid = 0.5 * static_cast<double>(S - 1);
+  t.K = k0 + mid * k1;
+  t.b = b0 + mid * b1;
+  t.k1 = k1;
+  t.b1 = b1;
+  // without a sweep every path is in cell 0
+  const double kappa = MomentCells::kOver * static_cast<double>(S) * (k1 < 0.0 ? -k1 : k1);
+  t.kappa = kappa > 1e-6 ? kappa : 1e-6;
+  t.theta_step = 2.0 * 3.14159265358979323846 * k1 / t.kappa;
+  t.S = static_cast<int>(S);
+  return t;
+}
+
+// A run's result: moments of the cells in its slots (tag kTraceEmpty: unused), and a
+// row of S samples when `rows` says that cells were evicted.
+struct TraceRecord {
+  float2 moments[kTraceSlots][kTraceQ];
+  int tag[kTraceSlots];
+  int has_row;
+  int pad[15];
+};
+
+struct TraceSmem {
+  float2 rows[kTraceThreads][kTraceRow];
+  float2 moments[kTraceSlots][kTraceQ];
+  int4 hist[kTraceSlots];  // per warp
+  int start[kTraceSlots + 1];
+  int tag[kTraceSlots];
+  int list[kTraceThreads * (kTracePer + 1)];
+  int counts[kTracePer * kTraceWarps];
+  int evict[kTraceSlots];
+  int has_row;
+};
+
+// Adds a cell's moments, seen by sample n, to acc.
+__device__ __forceinline__ void add_cell(const TraceConsts& c, int k, const float2* m, const float* g, int n, float2& acc) {
+  const double ph = (n - 0.5 * (c.S - 1)) * fma(c.k1, static_cast<double>(k) / c.kappa, c.b1);
+  const float2 e = cis_cycles(static_cast<float>(ph - rint(ph)));
+  float2 ev = make_float2(0.0f, 0.0f), od = make_float2(0.0f, 0.0f);
+#pragma unroll
+  for (int q = 0; q < kTraceQ; q += 2) {
+    ev = ffma2(make_float2(g[q], g[q]), m[q], ev);
+    od = ffma2(make_float2(g[q + 1], g[q + 1]), m[q + 1], od);
+  }
+  const float2 z = cmul(e, make_float2(ev.x - od.y, ev.y + od.x));
+  acc = fadd2(acc, z);
+}
+
+__device__ __forceinline__ void trace_begin(TraceSmem& sm) {
+  for (int i = threadIdx.x; i < kTraceSlots * kTraceQ; i += kTraceThreads) {
+    (&sm.moments[0][0])[i] = make_float2(0.0f, 0.0f);
+  }
+  for (int i = threadIdx.x; i < kTraceSlots; i += kTraceThreads) {
+    sm.tag[i] = kTraceEmpty;
+    sm.hist[i] = make_int4(0, 0, 0, 0);
+    sm.evict[i] = 0;
+  }
+  if (threadIdx.x == 0) sm.has_row = 0;
+  __syncthreads();
+}
+
+// The slots marked for eviction go to the run's row of samples (in device memory,
+// touched by this block only) and are emptied.
+static __device__ __noinline__ void trace_evict(TraceSmem& sm, const TraceConsts c, float2* row) {
+  const bool first = sm.has_row == 0;
+  for (int n = threadIdx.x; n < c.S; n += kTraceThreads) {
+    float g[kTraceQ];
+    cell_basis<kTraceQ>(c.theta_step * (n - 0.5 * (c.S - 1)), g);
+    float2 acc = first ? make_float2(0.0f, 0.0f) : row[n];
+    for (int s = 0; s < kTraceSlots; ++s) {
+      if (sm.evict[s]) add_cell(c, sm.tag[s], sm.moments[s], g, n, acc);
+    }
+    row[n] = acc;
+  }
+  __syncthreads();
+  for (int s = threadIdx.x; s < kTraceSlots; s += kTraceThreads) {
+    if (!sm.evict[s]) continue;
+    sm.evict[s] = 0;
+    sm.tag[s] = kTraceEmpty;
+    for (int q = 0; q < kTraceQ; ++q) sm.moments[s][q] = make_float2(0.0f, 0.0f);
+  }
+  if (threadIdx.x == 0) sm.has_row = 1;
+  __syncthreads();
+}
+
+// One batch: thread t holds a live contribution w at cell k, offset x (or none).
+__device__ __forceinline__ void trace_batch(TraceSmem& sm, const TraceConsts& c, float2* row, bool live, float2 w, int k,
+                                            float x) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int slot = k & (kTraceSlots - 1);
+  bool pending = live;
+  for (;;) {
+    bool in = false;
+    if (pending) {
+      const int old = sm.tag[slot] == k ? k : atomicCAS(&sm.tag[slot], kTraceEmpty, k);
+      in = old == kTraceEmpty || old == k;
+      if (!in) sm.evict[slot] = 1;
+    }
+    const unsigned same = __match_any_sync(0xffffffffu, in ? slot : kTraceSlots);
+    const int rank = __popc(same & ((1u << lane) - 1u));
+    if (in && rank == 0) reinterpret_cast<int*>(&sm.hist[slot])[warp] = __popc(same);
+    __syncthreads();
+    if (warp == 0) {  // exclusive prefix over (slot, warp), two slots per lane
+      const int4 a = sm.hist[2 * lane], b = sm.hist[2 * lane + 1];
+      const int sa = a.x + a.y + a.z + a.w, sb = b.x + b.y + b.z + b.w;
+      int run = sa + sb;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += y;
+      }
+      const int e = run - sa - sb;
+      sm.start[2 * lane] = e;
+      sm.start[2 * lane + 1] = e + sa;
+      sm.hist[2 * lane] = make_int4(e, e + a.x, e + a.x + a.y, e + a.x + a.y + a.z);
+      const int f = e + sa;
+      sm.hist[2 * lane + 1] = make_int4(f, f + b.x, f + b.x + b.y, f + b.x + b.y + b.z);
+      if (lane == 31) sm.start[kTraceSlots] = run;
+    }
+    __syncthreads();
+    if (in) {  // the contribution row w x^q, at its place in cell order
+      const int place = reinterpret_cast<const int*>(&sm.hist[slot])[warp] + rank;
+      float4* dst = reinterpret_cast<float4*>(&sm.rows[place][0]);
+      float2 v = w;
+#pragma unroll
+      for (int q = 0; q < kTraceQ; q += 2) {
+        const float2 u = make_float2(v.x * x, v.y * x);
+        dst[q / 2] = make_float4(v.x, v.y, u.x, u.y);
+        v = make_float2(u.x * x, u.y * x);
+      }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kTraceSlots; i += kTraceThreads) sm.hist[i] = make_int4(0, 0, 0, 0);
+    const int q = threadIdx.x & (kTraceQ - 1);
+    for (int s = threadIdx.x / kTraceQ; s < kTraceSlots; s += kTraceThreads / kTraceQ) {
+      const int i0 = sm.start[s], i1 = sm.start[s + 1];
+      if (i0 == i1) continue;
+      float2 acc = sm.moments[s][q];
+#pragma unroll 4
+      for (int i = i0; i < i1; ++i) acc = fadd2(acc, sm.rows[i][q]);
+      sm.moments[s][q] = acc;
+    }
+    pending = pending && !in;
+    if (!__syncthreads_or(pending)) break;
+    trace_evict(sm, c, row);
+  }
+}
+
+// A point and its contribution.
+struct TracePoint {
+  float nrm[3], pt[3], sigma;
+};
+
+template <typename T>
+__device__ __forceinline__ void load_point(const T* normals, const T* points, int64_t q, float* nrm, float* pt) {
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    nrm[a] = ld_f(normals, q * 3 + a);
+    pt[a] = ld_f(points, q * 3 + a);
+  }
+}
+
+__device__ __forceinline__ bool trace_point(const TraceConsts& c, const float* txp, const float* rxp, const TracePoint& t,
+                                            float2& w, int& cell, float& x) {
+  PairGeom g;
+  if (!pair_geometry(txp, rxp, t.nrm, t.pt, g)) return false;
+  const float amp = t.sigma * g.align / sq(g.dist);
+  double st = 0.0, sr = 0.0;
+#pragma unroll
+  for (int a = 2; a >= 0; --a) {
+    const double dt = static_cast<double>(txp[a]) - static_cast<double>(t.pt[a]);
+    const double dr = static_cast<double>(rxp[a]) - static_cast<double>(t.pt[a]);
+    st = fma(dt, dt, st);
+    sr = fma(dr, dr, sr);
+  }
+  const double d = sqrt_f64_fast(st) + sqrt_f64_fast(sr);
+  const double ph = fma(d, c.K, c.b);
+  const double u = d * c.kappa, ku = rint(u);
+  cell = fabs(ku) < 1073741824.0 ? static_cast<int>(ku) : 0;  // a non-finite path: w is NaN
+  x = static_cast<float>(u - ku);
+  const float2 e = cis_cycles_fast(static_cast<float>(ph - rint(ph)));
+  w = make_float2(amp * e.x, amp * e.y);
+  return true;
+}
+
+// All points of positions [begin, end) in batches of consecutive ones: for points
+// of which most are live (the pre-cull's list).  The next batch's points are loaded
+// while one is summed.
+template <typename T, typename IndexOf, typename SigmaOf>
+__device__ __forceinline__ void trace_all(TraceSmem& sm, const TraceConsts& c, float2* row, const T* normals,
+                                          const T* points, const float* txp, const float* rxp, int64_t begin,
+                                          int64_t end, IndexOf index_of, SigmaOf sigma_of) {
+  TracePoint next;
+  int64_t next_q = -1;
+  auto load = [&](int64_t k) {
+    next_q = k < end ? index_of(k) : -1;
+    if (next_q >= 0) {
+      load_point(normals, points, next_q, next.nrm, next.pt);
+      next.sigma = sigma_of(next_q);
+    }
+  };
+  load(begin + threadIdx.x);
+  for (int64_t p0 = begin; p0 < end; p0 += kTraceThreads) {
+    float2 w = make_float2(0.0f, 0.0f);
+    float x = 0.0f;
+    int cell = 0;
+    const bool live = next_q >= 0 && trace_point(c, txp, rxp, next, w, cell, x);
+    load(p0 + kTraceThreads + threadIdx.x);
+    trace_batch(sm, c, row, live, w, cell, x);
+  }
+}
+
+// All points of positions [begin, end), screened first: index_of(k) is the point at
+// position k, or -1 when it is out of bounds; sigma_of(q) its amplitude weight.
+template <typename T, typename IndexOf, typename SigmaOf>
+__device__ __forceinline__ void trace_screened(TraceSmem& sm, const TraceConsts& c, float2* row, const T* normals,
+                                               const T* points, const float* txp, const float* rxp, int64_t begin,
+                                               int64_t end, IndexOf index_of, SigmaOf sigma_of) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int listed = 0;
+  float nrm[kTracePer][3], pt[kTracePer][3];
+  int idx[kTracePer];
+  auto load = [&](int64_t p0) {  // of the next pass, in flight while batches are summed
+#pragma unroll
+    for (int j = 0; j < kTracePer; ++j) {
+      const int64_t k = p0 + j * kTraceThreads + threadIdx.x;
+      idx[j] = k < end ? index_of(k) : -1;
+      if (idx[j] >= 0) load_point(normals, points, idx[j], nrm[j], pt[j]);
+    }
+  };
+  load(begin);
+  for (int64_t p0 = begin; p0 < end; p0 += kTraceThreads * kTracePer) {
+    unsigned mask[kTracePer];
+#pragma unroll
+    for (int j = 0; j < kTracePer; ++j) {
+      const bool keep = idx[j] >= 0 && !surely_culled(txp, rxp, nrm[j], pt[j]);
+      mask[j] = __ballot_sync(0xffffffffu, keep);
+      if (lane == 0) sm.counts[j * kTraceWarps + warp] = __popc(mask[j]);
+    }
+    __syncthreads();
+    int before = listed;
+#pragma unroll
+    for (int j = 0; j < kTracePer; ++j) {
+#pragma unroll
+      for (int w = 0; w < kTraceWarps; ++w) {
+        if (w == warp && ((mask[j] >> lane) & 1u)) sm.list[before + __popc(mask[j] & ((1u << lane) - 1u))] = idx[j];
+        before += sm.counts[j * kTraceWarps + w];
+      }
+    }
+    listed = before;
+    load(p0 + kTraceThreads * kTracePer);
+    __syncthreads();
+    const bool last = p0 + kTraceThreads * kTracePer >= end;
+    while (listed >= kTraceThreads || (last && listed > 0)) {
+      const int cnt = min(listed, kTraceThreads);
+      listed -= cnt;
+      bool live = false;
+      float2 w = make_float2(0.0f, 0.0f);
+      float x = 0.0f;
+      int cell = 0;
+      if (threadIdx.x < cnt) {
+        const int64_t q = sm.list[listed + threadIdx.x];
+        TracePoint t;
+        load_point(normals, points, q, t.nrm, t.pt);
+        t.sigma = sigma_of(q);
+        live = trace_point(c, txp, rxp, t, w, cell, x);
+      }
+      trace_batch(sm, c, row, live, w, cell, x);
+    }
+  }
+}
+
+__device__ __forceinline__ void trace_store(const TraceSmem& sm, TraceRecord* rec) {
+  __syncthreads();
+  for (int i = threadIdx.x; i < kTraceSlots * kTraceQ; i += kTraceThreads) {
+    if (sm.tag[i / kTraceQ] != kTraceEmpty) (&rec->moments[0][0])[i] = (&sm.moments[0][0])[i];
+  }
+  for (int i = threadIdx.x; i < kTraceSlots; i += kTraceThreads) rec->tag[i] = sm.tag[i];
+  if (threadIdx.x == 0) rec->has_row = sm.has_row;
+  __syncthreads();
+}
+
+// Samples of one antenna from its runs' records, 256 threads.  Per slot the cells
+// are taken in ascending order, one per round (one round, unless runs of the
+// antenna lie more than kTraceSlots cells apart); the runs' moments are added in run order.
+constexpr int kFinishThreads = 256;
+
+template <typename T>
+__device__ __forceinline__ void trace_finish(const TraceConsts& c, const TraceRecord* rec, const float2* rows,
+                                             int64_t runs, float divisor, int n_begin, int n_end, T* out_r, T* out_i) {
+  __shared__ float2 mom[kTraceSlots][kTraceQ];
+  __shared__ int tag[kTraceSlots];
+  static_assert(kFinishThreads == kTraceSlots * kTraceQ / 2, "a thread per slot and pair of moments");
+  const int slot = threadIdx.x / (kTraceQ / 2), pair = threadIdx.x % (kTraceQ / 2);
+  const int n = n_begin + threadIdx.x;
+  const bool mine = n < n_end;
+  float2 acc = make_float2(0.0f, 0.0f);
+  float g[kTraceQ];
+  bool rowed = false;
+  for (int64_t r = threadIdx.x; r < runs; r += kFinishThreads) rowed = rowed || rec[r].has_row != 0;
+  if (__syncthreads_or(rowed) && mine) {
+    for (int64_t r = 0; r < runs; ++r) {
+      if (rec[r].has_row) acc = fadd2(acc, rows[r * c.S + n]);
+    }
+  }
+  if (mine) cell_basis<kTraceQ>(c.theta_step * (n - 0.5 * (c.S - 1)), g);
+  int done = INT32_MIN;
+  for (;;) {
+    // the slot's lowest cell above the one done, and whether higher ones follow
+    int next = INT32_MAX, top = INT32_MIN;
+#pragma unroll 4
+    for (int64_t r = pair; r < runs; r += kTraceQ / 2) {
+      const int t = rec[r].tag[slot];
+      if (t != kTraceEmpty && t > done) {
+        next = min(next, t);
+        top = max(top, t);
+      }
+    }
+#pragma unroll
+    for (int o = 1; o < kTraceQ / 2; o <<= 1) {
+      next = min(next, __shfl_xor_sync(0xffffffffu, next, o));
+      top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+    }
+    float4 m = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (next != INT32_MAX) {
+#pragma unroll 8
+      for (int64_t r = 0; r < runs; ++r) {
+        const int t = rec[r].tag[slot];
+        const float4 y = reinterpret_cast<const float4*>(&rec[r].moments[slot][0])[pair];
+        const bool take = t == next;  // unused slots hold no moments
+        m.x += take ? y.x : 0.0f;
+        m.y += take ? y.y : 0.0f;
+        m.z += take ? y.z : 0.0f;
+        m.w += take ? y.w : 0.0f;
+      }
+    }
+    reinterpret_cast<float4*>(&mom[slot][0])[pair] = m;
+    if (pair == 0) tag[slot] = next;  // INT32_MAX: none
+    const bool more = next != INT32_MAX && top > next;
+    done = next;
+    const bool again = __syncthreads_or(more) != 0;
+    if (mine) {
+      for (int k = 0; k < kTraceSlots; ++k) {
+        if (tag[k] != INT32_MAX) add_cell(c, tag[k], mom[k], g, n, acc);
+      }
+    }
+    if (!again) break;
+    __syncthreads();
+  }
+  if (mine) {
+    out_r[n] = from_f<T>(acc.x / divisor);
+    out_i[n] = from_f<T>(acc.y / divisor);
+  }
+}
+
+}  // namespace tracer
+}  // namespace geraf

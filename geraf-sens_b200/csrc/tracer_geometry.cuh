@@ -100,6 +100,85 @@ __device__ __forceinline__ float path_distance(const float* tx, const float* rx,
          sqrtf(sq(rx[0] - pt[0]) + sq(rx[1] - pt[1]) + sq(rx[2] - pt[2]));
 }
 
+// 1 / sqrt(s) to ~1 ulp: the hardware seed and one Newton step.
+__device__ __forceinline__ float rsqrt_newton(float s) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(s));
+  const float h = 0.5f * s * r;
+  return r * fmaf(-h, r, 1.5f);
+}
+
+// The geometry of a pair that its amplitude and its gradients need.
+struct PairGeom {
+  float inc[3];   // normalize(p - tx)
+  float ret[3];   // normalize(rx - p)
+  float refl[3];  // normalize(reflection)
+  float u[3];     // d rho / d (reflection): (ret - refl rho) / |reflection|
+  float idn, align, dist;
+  float inv_t, inv_r;  // 1 / |p - tx|, 1 / |rx - p|
+};
+
+// A pair's geometry without divisions and square roots (about 70 operations
+// against ~190 of specular_geometry and path_distance), with the reference's
+// epsilon in the norms.  Culling stays the reference's to the bit: the signs of i.n
+// and of o.r (r the reflection of the normalised incident ray) decide it only where
+// they are clear, |i.n| > 1e-5 |n| and |o.r| > 1e-5 |o| m with m = 1 + 2 |n|^2,
+// against errors of ~1e-6 in either evaluation; and rho is then above 1e-5, clear of
+// the reference's 1e-6.  Everything else, non-finite values included (they fail the
+// comparisons), takes the exact form.  Returns whether the pair is live; g is then set.
+__device__ __forceinline__ bool pair_geometry(const float* tx, const float* rx, const float* nrm, const float* pt,
+                                              PairGeom& g) {
+  float i[3], o[3], r[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    i[k] = pt[k] - tx[k];
+    o[k] = rx[k] - pt[k];
+  }
+  const float ii = dot3(i, i), oo = dot3(o, o), nn = dot3(nrm, nrm);
+  g.inv_t = rsqrt_newton(ii);
+  g.inv_r = rsqrt_newton(oo);
+  const float ei = fmaf(-kNormEps * g.inv_t, g.inv_t, g.inv_t), eo = fmaf(-kNormEps * g.inv_r, g.inv_r, g.inv_r);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    g.inc[k] = i[k] * ei;  // 1 / (norm + eps)
+    g.ret[k] = o[k] * eo;
+  }
+  g.idn = dot3(g.inc, nrm);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) r[k] = fmaf(-2.0f * g.idn, nrm[k], g.inc[k]);
+  const float orr = dot3(g.ret, r);
+  const float m = fmaf(2.0f, nn, 1.0f);
+  float er;
+  if (g.idn * g.idn > 1.0e-10f * nn && orr * orr > 1.0e-10f * (m * m)) {
+    if (g.idn > 0.0f || orr < 0.0f) return false;
+    const float ir = rsqrt_newton(dot3(r, r));
+    er = fmaf(-kNormEps * ir, ir, ir);
+    g.align = orr * er;
+    g.dist = fmaf(ii, g.inv_t, oo * g.inv_r);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) g.refl[k] = r[k] * er;
+  } else {
+    SpecGeom s;
+    specular_geometry(tx, rx, nrm, pt, s);
+    if (culled(s)) return false;
+    g.align = s.align;
+    g.dist = path_distance(tx, rx, pt);
+    g.idn = s.idn;
+    er = 1.0f / (sqrtf(dot3(s.refl_raw, s.refl_raw)) + kNormEps);
+    g.inv_t = 1.0f / sqrtf(ii);
+    g.inv_r = 1.0f / sqrtf(oo);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      g.inc[k] = s.inc[k];
+      g.ret[k] = s.ret[k];
+      g.refl[k] = s.refl[k];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) g.u[k] = (g.ret[k] - g.refl[k] * g.align) * er;
+  return true;
+}
+
 // d rho / d n through the reflection and its normalisation, in the reference's
 // order (SignalTracer_cuda_kernel.cu:91-170, 531-542).
 __device__ __forceinline__ void align_normal_gradient(const SpecGeom& g, const float* nrm,

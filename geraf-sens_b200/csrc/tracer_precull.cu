@@ -154,15 +154,17 @@ __device__ __forceinline__ bool culled_for_all(const Aperture& ap, const float* 
 }
 
 // Flag word w of chunk c covers points c*1024 + w*32 + lane; counts[c] is the
-// number of listed points of the chunk.  With a null `aperture` each block
+// number of listed points of the chunk and boxes[c] (when given) their bounding box.  With a null `aperture` each block
 // bounds the antennas itself.
 template <typename T>
 __global__ void __launch_bounds__(kChunkThreads) point_flags_kernel(const T* normals, const T* points,
                                                                     const uint8_t* inb, int64_t P,
                                                                     const Aperture* aperture, const T* tx,
                                                                     const T* rx, int64_t A, uint32_t* words,
-                                                                    int* counts) {
+                                                                    int* counts, float* boxes) {
   __shared__ int warp_count[kChunkThreads / 32];
+  __shared__ float box_s[kChunkThreads / 32][6];
+  float box[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
   __shared__ Aperture ap_s;
   if (aperture == nullptr) block_aperture(tx, rx, A, &ap_s);
   const Aperture ap = aperture != nullptr ? *aperture : ap_s;
@@ -182,6 +184,14 @@ __global__ void __launch_bounds__(kChunkThreads) point_flags_kernel(const T* nor
         pt[j] = ld_f(points, q * 3 + j);
       }
       listed = !culled_for_all(ap, n, pt);
+      if (listed) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          // a NaN coordinate widens the box to infinity: nothing is bounded then
+          box[j] = fminf(box[j], pt[j] == pt[j] ? pt[j] : -INFINITY);
+          box[3 + j] = fmaxf(box[3 + j], pt[j] == pt[j] ? pt[j] : INFINITY);
+        }
+      }
     }
     const unsigned b = __ballot_sync(0xffffffffu, listed);
     if (lane == 0) {
@@ -190,7 +200,25 @@ __global__ void __launch_bounds__(kChunkThreads) point_flags_kernel(const T* nor
     }
   }
   if (lane == 0) warp_count[warp] = c;
+  if (boxes != nullptr) {
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float y = __shfl_xor_sync(0xffffffffu, box[j], o);
+        box[j] = j < 3 ? fminf(box[j], y) : fmaxf(box[j], y);
+      }
+      if (lane == 0) box_s[warp][j] = box[j];
+    }
+  }
   __syncthreads();
+  if (boxes != nullptr && threadIdx.x < 6) {
+    float r = box_s[0][threadIdx.x];
+    for (int w = 1; w < kChunkThreads / 32; ++w) {
+      r = threadIdx.x < 3 ? fminf(r, box_s[w][threadIdx.x]) : fmaxf(r, box_s[w][threadIdx.x]);
+    }
+    boxes[static_cast<int64_t>(blockIdx.x) * 6 + threadIdx.x] = r;
+  }
   if (threadIdx.x == 0) {
     int total = 0;
     for (int w = 0; w < kChunkThreads / 32; ++w) total += warp_count[w];
@@ -329,7 +357,7 @@ ListLayout list_layout(int64_t P) {
 }
 
 template <typename T>
-cudaError_t launch_point_list(const TracerArgs& a, void* ws, bool zero_grads, cudaStream_t st) {
+cudaError_t launch_point_list(const TracerArgs& a, void* ws, bool zero_grads, float* boxes, cudaStream_t st) {
   const ListLayout l = list_layout(a.P);
   unsigned char* base = static_cast<unsigned char*>(ws);
   Aperture* ap = reinterpret_cast<Aperture*>(base + l.aperture);
@@ -346,7 +374,7 @@ cudaError_t launch_point_list(const TracerArgs& a, void* ws, bool zero_grads, cu
   if (!inline_aperture) aperture_kernel<T><<<1, 256, 0, st>>>(tx, rx, a.A, ap);
   point_flags_kernel<T><<<static_cast<unsigned>(chunks), kChunkThreads, 0, st>>>(
       static_cast<const T*>(a.normals), static_cast<const T*>(a.points), a.inbounds, a.P,
-      inline_aperture ? nullptr : ap, tx, rx, a.A, words, counts);
+      inline_aperture ? nullptr : ap, tx, rx, a.A, words, counts, boxes);
   if (!inline_scan) chunk_scan_kernel<<<1, 1024, 0, st>>>(counts, chunks, offsets, total);
   point_scatter_kernel<T><<<static_cast<unsigned>(chunks), kChunkThreads, 0, st>>>(
       words, inline_scan ? nullptr : offsets, counts, chunks, total, a.P, list, a.A,
@@ -370,9 +398,11 @@ PointList tracer_point_list_view(void* ws, int64_t P) {
   return PointList{reinterpret_cast<const int*>(base + l.list), reinterpret_cast<const int*>(base + l.total)};
 }
 
-cudaError_t tracer_point_list(const TracerArgs& a, void* ws, bool zero_grads, cudaStream_t st) {
-  if (a.dtype == kF64) return launch_point_list<double>(a, ws, zero_grads, st);
-  return launch_point_list<float>(a, ws, zero_grads, st);
+int64_t tracer_point_chunks(int64_t P) { return (P + kChunk - 1) / kChunk; }
+
+cudaError_t tracer_point_list(const TracerArgs& a, void* ws, bool zero_grads, cudaStream_t st, float* boxes) {
+  if (a.dtype == kF64) return launch_point_list<double>(a, ws, zero_grads, boxes, st);
+  return launch_point_list<float>(a, ws, zero_grads, boxes, st);
 }
 
 }  // namespace geraf
