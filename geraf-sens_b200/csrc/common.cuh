@@ -418,6 +418,18 @@ __device__ __forceinline__ void stage_positions(PosT* pos, int stage, int rows_m
   }
 }
 
+// Zeros for elements [begin, end) of an array, by the whole block; 16 bytes at a time
+// where the address allows it.
+template <typename T>
+__device__ __forceinline__ void zero_range(T* base, int64_t begin, int64_t end) {
+  constexpr int kVec = 16 / sizeof(T);
+  T* p = base + begin;
+  const int64_t n = end - begin;
+  const int64_t vecs = (reinterpret_cast<uintptr_t>(p) & 15u) == 0 ? n / kVec : 0;
+  for (int64_t i = threadIdx.x; i < vecs; i += blockDim.x) reinterpret_cast<uint4*>(p)[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int64_t i = vecs * kVec + threadIdx.x; i < n; i += blockDim.x) p[i] = from_f<T>(0.0f);
+}
+
 // Kahan-compensated accumulation of one component.
 __device__ __forceinline__ void kahan_add(float& sum, float& comp, float x) {
   const float y = x - comp;

@@ -911,7 +911,7 @@ struct SamplesP {
   T* out_i;
   int64_t A, apad;
   int S;
-  double k1, b1, kappa;
+  double k1, b1, inv_kappa;
 };
 
 // Samples from the moments: 4 antennas per block, which share the phasors of the cells.
@@ -938,7 +938,7 @@ __global__ void __launch_bounds__(128) mf_moment_samples_kernel(const SamplesP<T
 #pragma unroll
     for (int u = 0; u < kSampleAnts; ++u) acc[u] = make_float2(0.0f, 0.0f);
     for (int k = 0; k < cells; ++k) {
-      const double c = (n - mid) * fma(p.k1, static_cast<double>(k0 + k) / p.kappa, p.b1);
+      const double c = (n - mid) * fma(p.k1, (k0 + k) * p.inv_kappa, p.b1);
       const float2 e = cis_cycles(static_cast<float>(c - rint(c)));
 #pragma unroll
       for (int u = 0; u < kSampleAnts; ++u) {
@@ -1036,7 +1036,7 @@ cudaError_t launch_cells_backward(const MfArgs& a, unsigned char* ws, cudaStream
   sp.S = bp.S;
   sp.k1 = pc.k1;
   sp.b1 = pc.b1;
-  sp.kappa = kappa;
+  sp.inv_kappa = 1.0 / kappa;
   const dim3 grid(static_cast<unsigned>((a.A + kSampleAnts - 1) / kSampleAnts), static_cast<unsigned>((a.S + 127) / 128));
   mf_moment_samples_kernel<T><<<grid, 128, 0, st>>>(sp);
   return cudaGetLastError();

@@ -15,7 +15,7 @@
 // antennas with 512 rays and antennas with 8192 rays load-balance; a finish
 // pass sums each antenna's item partials in item order (deterministic).
 // Adjoint: a point belongs to one antenna, so its gradients need no reduction
-// across antennas; blocks screen tiles of points and deal the live ones out
+// across antennas; blocks screen runs of points and deal the live ones out
 // over their threads.
 #include <algorithm>
 
@@ -23,6 +23,7 @@
 #include "kernels.h"
 #include "tracer_cells.cuh"
 #include "tracer_geometry.cuh"
+#include "tracer_gradients.cuh"
 
 namespace geraf {
 namespace {
@@ -133,10 +134,10 @@ __device__ __forceinline__ int64_t item_antenna(const int64_t* item_offsets, int
 }
 
 // Each work item's points go into the moments of their cells (tracer_cells.cuh).
-// 64 antennas x 295000 points each (10% live) x 256 samples: FWD_US against 590 us with
+// 64 antennas x 295000 points each (10% live) x 256 samples: 173 us against 590 us with
 // a recurrence over the samples of every live point and a compaction per 128 points.
 template <typename T>
-__global__ void __launch_bounds__(kTraceThreads, 5) ragged_fwd_kernel(const RgP<T> p) {
+__global__ void __launch_bounds__(kTraceThreads, 6) ragged_fwd_kernel(const RgP<T> p) {
   __shared__ TraceSmem sm;
   __shared__ long long s_item;
   const int64_t total = p.item_offsets[p.A];
@@ -152,10 +153,8 @@ __global__ void __launch_bounds__(kTraceThreads, 5) ragged_fwd_kernel(const RgP<
     ld3(p.tx, a, txp);
     ld3(p.rx, a, rxp);
     trace_begin(sm);
-    trace_screened<T>(
-        sm, p.c, p.rows + item * p.c.S, p.normals + first * 3, p.points + first * 3, txp, rxp, 0, count,
-        [&](int64_t k) { return p.inb == nullptr || p.inb[first + k] ? static_cast<int>(k) : -1; },
-        [&](int64_t q) { return ld_f(p.sigmas, first + q); });
+    trace_screened<T>(sm, p.c, p.rows + item * p.c.S, p.normals + first * 3, p.points + first * 3, p.sigmas + first,
+                      p.inb != nullptr ? p.inb + first : nullptr, txp, rxp, static_cast<int>(count));
     trace_store(sm, p.records + item);
   }
 }
@@ -185,189 +184,165 @@ __device__ __forceinline__ int64_t point_antenna(const int64_t* offsets, int64_t
   return lo;
 }
 
-// Gradients of one in-bounds point pi of antenna a that the early test cannot
-// cull (zeros when its exact geometry culls it).  The residual row comes from
-// shared memory (rr, ri: ld floats each) or, when rr is null, from global
-// memory.
-template <typename T, bool WITH_POINTS>
-__device__ __forceinline__ void ragged_point_grads(const RgP<T>& p, int64_t pi, int64_t a, const float* rr,
-                                                   const float* ri, int ld) {
-  float nrm[3], pt[3], txp[3], rxp[3];
-  ld3(p.normals, pi, nrm);
-  ld3(p.points, pi, pt);
-  ld3(p.tx, a, txp);
-  ld3(p.rx, a, rxp);
-  SpecGeom geo;
-  specular_geometry(txp, rxp, nrm, pt, geo);
-  if (culled(geo)) {  // a candidate the exact geometry culls
-    p.g_sigmas[pi] = from_f<T>(0.0f);
+// Adjoint.  A point belongs to one antenna, so its gradients depend on nothing else.  A
+// block takes a run of consecutive points, kBwdTile at a time: it writes zeros for
+// all of them (whole lines), screens them with the early test while the next tile's
+// points are on their way, lists those the test cannot cull and, a full block of
+// them at a time, gives them the exact geometry and the residual sums (packed
+// even/odd Horner over the antenna's row in shared memory).
+// The sums stay a recurrence over the samples here: the cell polynomials of
+// tracer_gradients.cuh would need tables, for which a call has no workspace (formed per
+// block in shared memory they took 309 us against 365 us here, on 64 antennas x 295000
+// points, 10% live, x 256 samples, and moved the largest gradients by up to 1e-3 of
+// their norm, the recurrence's own error).  404 us with 1024-point blocks that each
+// looked their antenna up first and stored zeros point by point.
+constexpr int kBwdThreads = 128;
+constexpr int kBwdPer = 4;
+constexpr int kBwdTile = kBwdThreads * kBwdPer;
+
+// Zeros for kBwdTile consecutive points' `width` elements each, 16-byte aligned.
+template <typename T, int WIDTH>
+__device__ __forceinline__ void zero_tile(T* p) {
+  constexpr int kVecs = kBwdTile * WIDTH * sizeof(T) / 16;
 #pragma unroll
-    for (int q = 0; q < 3; ++q) p.g_normals[pi * 3 + q] = from_f<T>(0.0f);
-    if (WITH_POINTS) {
-#pragma unroll
-      for (int q = 0; q < 3; ++q) p.g_points[pi * 3 + q] = from_f<T>(0.0f);
-    }
-    return;
-  }
-  const double px = pt[0], py = pt[1], pz = pt[2];
-  const PhaseCycles pc = path_cycles(txp[0] - px, txp[1] - py, txp[2] - pz, rxp[0] - px, rxp[1] - py,
-                                     rxp[2] - pz, p.k0, p.b0, p.k1, p.b1);
-  const float2 zt = cis_cycles(pc.dcyc);
-  float qr = 0.0f, qi = 0.0f, dr = 0.0f, di = 0.0f;
-  float2 q1 = make_float2(0.0f, 0.0f);
-  auto step = [&](float cr, float ci) {
-    if (WITH_POINTS) {
-      const float ndr = fmaf(dr, zt.x, fmaf(-di, zt.y, qr));
-      const float ndi = fmaf(dr, zt.y, fmaf(di, zt.x, qi));
-      dr = ndr;
-      di = ndi;
-    }
-    const float nqr = fmaf(qr, zt.x, fmaf(-qi, zt.y, cr));
-    const float nqi = fmaf(qr, zt.y, fmaf(qi, zt.x, -ci));
-    qr = nqr;
-    qi = nqi;
-  };
-  if (rr != nullptr) {
-    // staged row: packed even/odd Horner in zeta^2
-    float2 qv;
-    residual_sums<WITH_POINTS>(rr, ri, ld, zt, qv, q1);
-    qr = qv.x;
-    qi = qv.y;
-  } else {
-    // row read from global memory: scalar Horner, Q1 = zeta Q'(zeta) from its derivative chain
-    for (int64_t n = p.S - 1; n >= 0; --n) step(ld_f(p.gr, a * p.S + n), ld_f(p.gi, a * p.S + n));
-    q1 = cmul(zt, make_float2(dr, di));
-  }
-  const float inv_pa = 1.0f / static_cast<float>(p.offsets[a + 1] - p.offsets[a]);
-  const float2 e0 = cis_cycles(pc.frac0);
-  const float sum_re = cmul(e0, make_float2(qr, qi)).x;
-  const float propagation_distance = path_distance(txp, rxp, pt);
-  const float atten = 1.0f / sq(propagation_distance);
-  const float sigma_value = ld_f(p.sigmas, pi);
-  p.g_sigmas[pi] = from_f<T>(atten * geo.align * sum_re * inv_pa);
-  float gsa[3];
-  align_normal_gradient(geo, nrm, gsa);
-  const float normal_scale = sigma_value * atten;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) p.g_normals[pi * 3 + k] = from_f<T>(normal_scale * gsa[k] * sum_re * inv_pa);
-  if (WITH_POINTS) {
-    const float w0 = static_cast<float>(2.0 * static_cast<double>(kPiF) * p.f0);
-    const float w1s = static_cast<float>(2.0 * static_cast<double>(kPiF) * p.As / p.fs);
-    const float2 f = cmul(e0, make_float2(w0 * qr + w1s * q1.x, w0 * qi + w1s * q1.y));
-    const float amp = sigma_value * geo.align * atten;
-    const float d_tau = -amp * f.y;
-    const float dist_t = sqrtf(sq(txp[0] - pt[0]) + sq(txp[1] - pt[1]) + sq(txp[2] - pt[2]));
-    const float dist_r = sqrtf(sq(rxp[0] - pt[0]) + sq(rxp[1] - pt[1]) + sq(rxp[2] - pt[2]));
-    float drho[3];
-    align_point_gradient(geo, nrm, dist_t, dist_r, drho);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const float dD = geo.inc[k] - geo.ret[k];
-      const float damp_dp = normal_scale * drho[k] - 2.0f * amp / propagation_distance * dD;
-      p.g_points[pi * 3 + k] = from_f<T>((sum_re * damp_dp + d_tau * dD / kSpeedOfLight) * inv_pa);
-    }
-  }
+  for (int i = 0; i < kVecs; i += kBwdThreads) reinterpret_cast<uint4*>(p)[i + threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// Adjoint.  A block screens kBwdTile consecutive points, kBwdCand per thread:
-// it finds each point's antenna, applies the early cull test, and writes zero
-// gradients for culled, out-of-bounds and unowned points; the other points are
-// listed in shared memory and then dealt out over the block, so every lane forms
-// a listed point's exact geometry and, unless that culls it, runs its full
-// sample recurrence (packed even/odd Horner, residual_sums).  (About 60% of a typical
-// step's points are live; with one point per thread 40% of the lanes would sit
-// out the recurrence.)  A point's gradients depend on that point only, so the
-// results do not depend on the list order.  Residual rows of the antennas the
-// tile spans are staged in shared memory when there are few of them (points
-// are grouped by antenna, so a tile usually lies within one antenna).
-constexpr int kBwdThreads = 128;
-constexpr int kBwdCand = 8;
-constexpr int kBwdTile = kBwdThreads * kBwdCand;
-
 template <typename T, bool WITH_POINTS>
-__global__ void __launch_bounds__(kBwdThreads) ragged_bwd_kernel(const RgP<T> p, int ld, int max_rows) {
-  extern __shared__ __align__(16) float srow[];  // [max_rows][2][ld]
-  __shared__ int s_live[kBwdTile];
-  __shared__ int s_nlive;
-  __shared__ long long s_a0, s_a1;
-  __shared__ int s_single;
-  const int64_t base = blockIdx.x * static_cast<int64_t>(kBwdTile);
+__global__ void __launch_bounds__(kBwdThreads, 6) ragged_bwd_kernel(const RgP<T> p, int64_t run, int ld, int aligned) {
+  extern __shared__ __align__(16) float srow[];  // [2][ld]
+  __shared__ int list[kBwdTile + kBwdThreads];   // offsets in the run
+  __shared__ int s_listed;
   const int lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
-    bool owned0, owned1;
-    s_nlive = 0;
-    s_a0 = point_antenna(p.offsets, p.A, base, &owned0);
-    s_a1 = point_antenna(p.offsets, p.A, min(p.P, base + kBwdTile) - 1, &owned1);
-    // Both ends owned by one antenna: with offsets[a] <= first <= pi <= last <
-    // offsets[a + 1], that antenna owns every point between, no search needed.
-    s_single = owned0 && owned1 && s_a0 == s_a1;
-  }
-  __syncthreads();
-  const bool single = s_single != 0;
-  const int64_t a_single = s_a0;
-  for (int k = 0; k < kBwdCand; ++k) {
-    const int c = threadIdx.x + k * kBwdThreads;
-    const int64_t pi = base + c;
-    bool live = false;
-    if (pi < p.P) {
-      bool owned = true;
-      const int64_t a = single ? a_single : point_antenna(p.offsets, p.A, pi, &owned);
-      if (!owned && p.status != nullptr) atomicExch(p.status, kStatusBadOffsets);
-      if (owned && (p.inb == nullptr || p.inb[pi])) {
-        float nrm[3], pt[3], txp[3], rxp[3];
-        ld3(p.normals, pi, nrm);
-        ld3(p.points, pi, pt);
-        ld3(p.tx, a, txp);
-        ld3(p.rx, a, rxp);
-        // a candidate: the exact geometry, formed once when its gradients are, decides it
-        live = !surely_culled(txp, rxp, nrm, pt);
-      }
-      if (!live) {
-        p.g_sigmas[pi] = from_f<T>(0.0f);
+  const int64_t begin = blockIdx.x * run;
+  const int64_t end = min(p.P, begin + run);
+  float* rowr = srow;
+  float* rowi = srow + ld;
+  if (threadIdx.x == 0) s_listed = 0;
+
+  int64_t a = 0, seg_end = begin;  // the current antenna's points end at seg_end
+  float txp[3] = {0.0f, 0.0f, 0.0f}, rxp[3] = {0.0f, 0.0f, 0.0f};
+  float inv_pa = 0.0f;
+
+  // Gradients of listed points [from, from + cnt) of the current antenna.
+  auto batch = [&](int cnt, int from) {
+    if (threadIdx.x >= cnt) return;
+    const int64_t pi = begin + list[from + threadIdx.x];
+    float nrm[3], pt[3];
+    ld3(p.normals, pi, nrm);
+    ld3(p.points, pi, pt);
+    const float sigma = ld_f(p.sigmas, pi);
+    PairGeom g;
+    if (!pair_geometry(txp, rxp, nrm, pt, g)) return;  // keeps its zeros
+    const PhaseCycles pc =
+        path_cycles(static_cast<double>(txp[0]) - pt[0], static_cast<double>(txp[1]) - pt[1],
+                    static_cast<double>(txp[2]) - pt[2], static_cast<double>(rxp[0]) - pt[0],
+                    static_cast<double>(rxp[1]) - pt[1], static_cast<double>(rxp[2]) - pt[2], p.k0, p.b0, p.k1, p.b1);
+    float2 q, q1;
+    residual_sums<WITH_POINTS>(rowr, rowi, ld, cis_cycles(pc.dcyc), q, q1);
+    float gs, gn[3] = {0.0f, 0.0f, 0.0f}, gp[3] = {0.0f, 0.0f, 0.0f};
+    const float2 e0 = cis_cycles_fast(pc.frac0);
+    // sum_n w_n (g_i cos - g_r sin) = -Im(exp(j phi0) (w0 Q + w1 Q1))
+    const float w0 = static_cast<float>(2.0 * static_cast<double>(kPiF) * p.f0);
+    const float w1s = static_cast<float>(2.0 * static_cast<double>(kPiF) * p.As / p.fs);
+    const float f = cmul(e0, make_float2(w0 * q.x + w1s * q1.x, w0 * q.y + w1s * q1.y)).y;
+    pair_gradients<WITH_POINTS>(g, cmul(e0, q).x, f, sigma, nrm, &gs, gn, gp);
+    p.g_sigmas[pi] = from_f<T>(gs * inv_pa);
 #pragma unroll
-        for (int q = 0; q < 3; ++q) p.g_normals[pi * 3 + q] = from_f<T>(0.0f);
-        if (WITH_POINTS) {
+    for (int c = 0; c < 3; ++c) {
+      p.g_normals[pi * 3 + c] = from_f<T>(gn[c] * inv_pa);
+      if (WITH_POINTS) p.g_points[pi * 3 + c] = from_f<T>(gp[c] * inv_pa);
+    }
+  };
+  // The full batches that the list holds; all of it when `drain`.  Between two barriers.
+  auto serve = [&](bool drain) {
+    __syncthreads();
+    int listed = s_listed;
+    while (listed >= kBwdThreads || (drain && listed > 0)) {
+      const int cnt = min(listed, kBwdThreads);
+      listed -= cnt;
+      batch(cnt, listed);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) s_listed = listed;
+  };
+
+  float nrm[kBwdPer][3], pt[kBwdPer][3];
+  unsigned inb = 0;  // bit j: point j of the thread is in bounds
+  auto load = [&](int64_t t0) {
+    inb = 0;
+    if (t0 >= end) return;
+    const int rest = static_cast<int>(min(end - t0, static_cast<int64_t>(kBwdTile))) - static_cast<int>(threadIdx.x);
+    const T* pn = p.normals + (t0 + threadIdx.x) * 3;
+    const T* pp = p.points + (t0 + threadIdx.x) * 3;
+    const uint8_t* pb = p.inb != nullptr ? p.inb + t0 + threadIdx.x : nullptr;
 #pragma unroll
-          for (int q = 0; q < 3; ++q) p.g_points[pi * 3 + q] = from_f<T>(0.0f);
+    for (int j = 0; j < kBwdPer; ++j) {
+      if (j * kBwdThreads < rest && (pb == nullptr || pb[j * kBwdThreads])) {
+        inb |= 1u << j;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          nrm[j][c] = ld_f(pn, j * kBwdThreads * 3 + c);
+          pt[j][c] = ld_f(pp, j * kBwdThreads * 3 + c);
         }
       }
     }
-    const unsigned ballot = __ballot_sync(0xffffffffu, live);
-    if (ballot != 0u) {
-      int wbase = 0;
-      if (lane == 0) wbase = atomicAdd(&s_nlive, __popc(ballot));
-      wbase = __shfl_sync(0xffffffffu, wbase, 0);
-      if (live) s_live[wbase + __popc(ballot & ((1u << lane) - 1u))] = c;
+  };
+  load(begin);
+  for (int64_t t0 = begin; t0 < end; t0 += kBwdTile) {
+    const int64_t t1 = min(end, t0 + kBwdTile);
+    if (aligned && t1 - t0 == kBwdTile) {
+      zero_tile<T, 1>(p.g_sigmas + t0);
+      zero_tile<T, 3>(p.g_normals + t0 * 3);
+      if (WITH_POINTS) zero_tile<T, 3>(p.g_points + t0 * 3);
+    } else {
+      zero_range(p.g_sigmas, t0, t1);
+      zero_range(p.g_normals, t0 * 3, t1 * 3);
+      if (WITH_POINTS) zero_range(p.g_points, t0 * 3, t1 * 3);
     }
-  }
-  const int64_t a0 = s_a0;
-  const int64_t a1 = max(s_a0, s_a1);
-  const bool staged = p.A > 0 && (a1 - a0 + 1) <= max_rows;
-  if (staged) {
-    const int rows = static_cast<int>(a1 - a0 + 1);
-    for (int i = threadIdx.x; i < rows * ld; i += kBwdThreads) {
-      const int r = i / ld, c = i - r * ld;
-      float vr = 0.0f, vi = 0.0f;
-      if (c < p.S) {
-        vr = ld_f(p.gr, (a0 + r) * p.S + c);
-        vi = ld_f(p.gi, (a0 + r) * p.S + c);
+    // the antennas of the tile, usually one
+    for (int64_t cur = t0; cur < t1;) {
+      if (cur >= seg_end) {
+        serve(true);  // the preceding antenna's points
+        bool owned;
+        a = point_antenna(p.offsets, p.A, cur, &owned);
+        if (!owned) {  // malformed offsets: the point keeps its zeros
+          if (threadIdx.x == 0 && p.status != nullptr) atomicExch(p.status, kStatusBadOffsets);
+          ++cur;
+          continue;
+        }
+        seg_end = p.offsets[a + 1];
+        inv_pa = 1.0f / static_cast<float>(seg_end - p.offsets[a]);
+        ld3(p.tx, a, txp);
+        ld3(p.rx, a, rxp);
+        for (int n = threadIdx.x; n < ld; n += kBwdThreads) {
+          rowr[n] = n < p.S ? ld_f(p.gr, a * p.S + n) : 0.0f;
+          rowi[n] = n < p.S ? ld_f(p.gi, a * p.S + n) : 0.0f;
+        }
+        __syncthreads();
       }
-      srow[(r * 2 + 0) * ld + c] = vr;
-      srow[(r * 2 + 1) * ld + c] = vi;
+      const int64_t stop = min(t1, seg_end);
+      const int lo = static_cast<int>(cur - t0) - static_cast<int>(threadIdx.x);
+      const int hi = static_cast<int>(stop - t0) - static_cast<int>(threadIdx.x);
+      const int at0 = static_cast<int>(t0 - begin) + static_cast<int>(threadIdx.x);
+#pragma unroll
+      for (int j = 0; j < kBwdPer; ++j) {
+        const bool keep = ((inb >> j) & 1u) && j * kBwdThreads >= lo && j * kBwdThreads < hi &&
+                          !surely_culled(txp, rxp, nrm[j], pt[j]);
+        const unsigned mask = __ballot_sync(0xffffffffu, keep);
+        if (mask == 0u) continue;
+        int at = 0;
+        if (lane == 0) at = atomicAdd(&s_listed, __popc(mask));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (keep) list[at + __popc(mask & ((1u << lane) - 1u))] = at0 + j * kBwdThreads;
+      }
+      cur = stop;
     }
+    load(t0 + kBwdTile);
+    serve(false);
+    __syncthreads();
   }
-  __syncthreads();
-  const int nlive = s_nlive;
-  for (int i = threadIdx.x; i < nlive; i += kBwdThreads) {
-    const int64_t pi = base + s_live[i];
-    bool owned;
-    const int64_t a = single ? a_single : point_antenna(p.offsets, p.A, pi, &owned);
-    // A row outside the staged span (possible only with non-monotonic offsets) is read from global memory.
-    const bool row_staged = staged && a >= a0 && a <= a1;
-    const float* rr = row_staged ? srow + ((a - a0) * 2 + 0) * ld : nullptr;
-    const float* ri = row_staged ? srow + ((a - a0) * 2 + 1) * ld : nullptr;
-    ragged_point_grads<T, WITH_POINTS>(p, pi, a, rr, ri, ld);
-  }
+  serve(true);
 }
 
 // ---------------------------------------------------------------------------
@@ -467,16 +442,19 @@ template <typename T>
 cudaError_t launch_ragged_bwd(const RaggedArgs& a, const Tuning& t, cudaStream_t st) {
   RgP<T> p = make_rg<T>(a, t, nullptr);
   const int ld = static_cast<int>(((std::max<int64_t>(a.S, 1) + 3) / 4) * 4);
-  const int max_rows = t.stage_rows;
-  const size_t smem = static_cast<size_t>(max_rows) * 2 * ld * sizeof(float);
+  const size_t smem = static_cast<size_t>(2 * ld) * sizeof(float);
   const bool with_points = a.grad_points != nullptr;
   const void* fn = with_points ? reinterpret_cast<const void*>(&ragged_bwd_kernel<T, true>)
                                : reinterpret_cast<const void*>(&ragged_bwd_kernel<T, false>);
-  cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (err != cudaSuccess) return err;
-  const int64_t blocks = (a.P + kBwdTile - 1) / kBwdTile;
+  auto aligned16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
+  int aligned = aligned16(a.grad_sigmas) && aligned16(a.grad_normals) && aligned16(a.grad_points) ? 1 : 0;
+  // Runs of consecutive points: a few per resident block, so that the last ones end together.
+  const int64_t slots = static_cast<int64_t>(current_device_info().sm_count) * 6;
+  int64_t run = (a.P + 4 * slots - 1) / (4 * slots);
+  run = std::max<int64_t>(1, std::min<int64_t>((run + kBwdTile - 1) / kBwdTile, 64)) * kBwdTile;
+  const int64_t blocks = (a.P + run - 1) / run;
   if (blocks > 0x7fffffff) return cudaErrorInvalidConfiguration;
-  void* args[] = {&p, const_cast<int*>(&ld), const_cast<int*>(&max_rows)};
+  void* args[] = {&p, &run, const_cast<int*>(&ld), &aligned};
   return cudaLaunchKernel(fn, dim3(static_cast<unsigned>(blocks)), dim3(kBwdThreads), args, smem, st);
 }
 

@@ -1,12 +1,7 @@
-// MIXED tracer adjoint through range cells: per live (point, antenna) pair the sums over
-// the residual row g[a, :] that the gradients need,
-//   Q = sum_n conj(g_n) e^{+j 2 pi n' d},   Q1 = sum_n n' conj(g_n) e^{+j 2 pi n' d},
-// are the conjugates of a polynomial of the path length and (scaled) of its
-// derivative, whose coefficients per cell are formed once per antenna
-// (range_cells.cuh, the matched filter's table).  Samples are counted from their
-// middle, so Q1 carries only the sweep's share of the phase rate (a few percent of
-// the carrier's): the derivative's larger interpolation error stays below the
-// FP32 rounding of the result.
+// MIXED tracer adjoint through range cells: per live (point, antenna) pair the sums
+// over the residual row g[a, :] that the gradients need come from a polynomial of the
+// path length and its derivative (tracer_gradients.cuh), whose coefficients per cell
+// are formed once per antenna (range_cells.cuh, the matched filter's table).
 //
 // Launches: the band of cells from the boxes of the listed points and of the
 // antennas, with the interpolation basis; the antennas' tables; the pairs.  Where the
@@ -16,8 +11,7 @@
 #include <cmath>
 
 #include "kernels.h"
-#include "range_cells.cuh"
-#include "tracer_geometry.cuh"
+#include "tracer_gradients.cuh"
 
 namespace geraf {
 namespace {
@@ -53,11 +47,6 @@ AdjLayout adj_layout(const TracerArgs& a) {
   l.total = up256(l.table + static_cast<size_t>(a.A) * kAdjCells * kQ * sizeof(float2));
   return l;
 }
-
-struct AdjConsts {
-  double K, b, k1, b1, kappa, theta_step;
-  int S;
-};
 
 template <typename T>
 struct BandP {
@@ -206,126 +195,83 @@ struct AdjPairP {
   float* partial;  // [splits][P][6]
   int64_t A, P, per_split;
   int splits;
-  float w_mid, kappa_c;  // phase rate of carrier and middle sample, cells per unit delay
   AdjConsts c;
 };
 
 // One thread per listed point, the antennas of the block's split in order; nothing is
 // shared but the antennas' positions, so the warps run free of barriers.  About 260
-// instructions per live pair, independent of the sample count.
+// instructions per live pair, independent of the sample count: 64 antennas x 52000 listed
+// points take 77 us, 282 us with two recurrences over 128 samples per live pair.
 template <typename T, bool WITH_POINTS>
 __global__ void __launch_bounds__(kPairThreads, 5) adj_pair_kernel(const AdjPairP<T> p) {
   __shared__ float ant[kPairAnts][6];
   if (p.head->bad) return;
-  const int split = blockIdx.x % p.splits;
-  const int64_t base = static_cast<int64_t>(blockIdx.x / p.splits) * kPairThreads;
   const int64_t count = *p.plist_count;
-  if (base >= count) return;
-  const bool inside = base + threadIdx.x < count;
-  const int64_t q = p.plist[min(base + threadIdx.x, count - 1)];
-  const int k0 = p.head->k0, cells = p.head->cells;
-  float nrm[3], pt[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    nrm[c] = ld_f(p.normals, q * 3 + c);
-    pt[c] = ld_f(p.points, q * 3 + c);
-  }
-  float gn[3] = {0.0f, 0.0f, 0.0f}, gp[3] = {0.0f, 0.0f, 0.0f};
-  const int64_t a_begin = split * p.per_split, a_end = min(p.A, a_begin + p.per_split);
-  const float inv_p = static_cast<float>(p.P);
-  for (int64_t a0 = a_begin; a0 < a_end; a0 += kPairAnts) {
-    const int rows = static_cast<int>(min(static_cast<int64_t>(kPairAnts), a_end - a0));
-    __syncthreads();
-    for (int i = threadIdx.x; i < rows * 6; i += kPairThreads) {
-      const int r = i / 6, c = i % 6;
-      ant[r][c] = c < 3 ? ld_f(p.tx, (a0 + r) * 3 + c) : ld_f(p.rx, (a0 + r) * 3 + c - 3);
+  const int64_t tiles = (count + kPairThreads - 1) / kPairThreads * p.splits;
+  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int split = static_cast<int>(tile % p.splits);
+    const int64_t base = tile / p.splits * kPairThreads;
+    const bool inside = base + threadIdx.x < count;
+    const int64_t q = p.plist[min(base + threadIdx.x, count - 1)];
+    const int k0 = p.head->k0, cells = p.head->cells;
+    float nrm[3], pt[3];
+  #pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      nrm[c] = ld_f(p.normals, q * 3 + c);
+      pt[c] = ld_f(p.points, q * 3 + c);
     }
-    __syncthreads();
-    if (!inside) continue;
-    float sigma = ld_f(p.sigmas, a0 * p.P + q);
-    for (int r = 0; r < rows; ++r) {
-      const int64_t a = a0 + r;
-      const float sigma_value = sigma;
-      if (r + 1 < rows) sigma = ld_f(p.sigmas, (a + 1) * p.P + q);
-      float txp[3], rxp[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        txp[c] = ant[r][c];
-        rxp[c] = ant[r][3 + c];
+    float gn[3] = {0.0f, 0.0f, 0.0f}, gp[3] = {0.0f, 0.0f, 0.0f};
+    const int64_t a_begin = split * p.per_split, a_end = min(p.A, a_begin + p.per_split);
+    const float num_points = static_cast<float>(p.P);
+    for (int64_t a0 = a_begin; a0 < a_end; a0 += kPairAnts) {
+      const int rows = static_cast<int>(min(static_cast<int64_t>(kPairAnts), a_end - a0));
+      __syncthreads();
+      for (int i = threadIdx.x; i < rows * 6; i += kPairThreads) {
+        const int r = i / 6, c = i % 6;
+        ant[r][c] = c < 3 ? ld_f(p.tx, (a0 + r) * 3 + c) : ld_f(p.rx, (a0 + r) * 3 + c - 3);
       }
-      PairGeom g;
-      if (!pair_geometry(txp, rxp, nrm, pt, g)) {
-        p.g_sigmas[a * p.P + q] = from_f<T>(0.0f);
-        continue;
-      }
-      double st = 0.0, sr = 0.0;
-#pragma unroll
-      for (int c = 2; c >= 0; --c) {
-        const double dt = static_cast<double>(txp[c]) - static_cast<double>(pt[c]);
-        const double dr = static_cast<double>(rxp[c]) - static_cast<double>(pt[c]);
-        st = fma(dt, dt, st);
-        sr = fma(dr, dr, sr);
-      }
-      const double d = sqrt_f64_fast(st) + sqrt_f64_fast(sr);
-      const double u = d * p.c.kappa, ku = rint(u);
-      const double ph = fma(d, p.c.K, p.c.b);
-      const float x = static_cast<float>(u - ku);
-      const int k = min(max(static_cast<int>(ku) - k0, 0), cells - 1);
-      const float4* row = reinterpret_cast<const float4*>(p.table + (a * kAdjCells + k) * kQ);
-      const float4 c2 = __ldg(row + 2), c1 = __ldg(row + 1), c0 = __ldg(row);
-      const float2 xx = make_float2(x, x);
-      // the polynomial and its derivative by Horner
-      float2 pv = make_float2(c2.z, c2.w), dv = pv;
-      pv = ffma2(pv, xx, make_float2(c2.x, c2.y));
-      dv = ffma2(dv, xx, pv);
-      pv = ffma2(pv, xx, make_float2(c1.z, c1.w));
-      dv = ffma2(dv, xx, pv);
-      pv = ffma2(pv, xx, make_float2(c1.x, c1.y));
-      dv = ffma2(dv, xx, pv);
-      pv = ffma2(pv, xx, make_float2(c0.z, c0.w));
-      dv = ffma2(dv, xx, pv);
-      pv = ffma2(pv, xx, make_float2(c0.x, c0.y));
-      const float2 e = cis_cycles_fast(static_cast<float>(ph - rint(ph)));
-      // sum_n (g_r cos + g_i sin) = Re(e conj(P))
-      const float sum_re = fmaf(e.x, pv.x, e.y * pv.y);
-      const float atten = 1.0f / sq(g.dist);
-      p.g_sigmas[a * p.P + q] = from_f<T>(atten * g.align * sum_re / inv_p);
-      const float scale = sigma_value * atten;
-      const float nu = dot3(nrm, g.u);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) gn[c] = fmaf(-2.0f * scale * sum_re, fmaf(nu, g.inc[c], g.idn * g.u[c]), gn[c]);
-      if (WITH_POINTS) {
-        // sum_n w_n (g_i cos - g_r sin) = -Im(e (w_mid conj(P) - j kappa c conj(P')))
-        const float f = p.w_mid * fmaf(e.y, pv.x, -e.x * pv.y) - p.kappa_c * fmaf(e.x, dv.x, e.y * dv.y);
-        const float amp = scale * g.align;
-        const float d_tau = -amp * f / kSpeedOfLight;
-        const float d_dist = -2.0f * amp / g.dist * sum_re + d_tau;
-        float v[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) v[c] = fmaf(-2.0f * nu, nrm[c], g.u[c]);
-        const float iv = dot3(g.inc, v);
-#pragma unroll
+      __syncthreads();
+      if (!inside) continue;
+      float sigma = ld_f(p.sigmas, a0 * p.P + q);
+      for (int r = 0; r < rows; ++r) {
+        const int64_t a = a0 + r;
+        const float sigma_value = sigma;
+        if (r + 1 < rows) sigma = ld_f(p.sigmas, (a + 1) * p.P + q);
+        float txp[3], rxp[3];
+  #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          // d rho / d p, and the change of the path length
-          const float drho = (v[c] - g.inc[c] * iv) * g.inv_t - (g.refl[c] - g.ret[c] * g.align) * g.inv_r;
-          gp[c] += fmaf(scale * sum_re, drho, d_dist * (g.inc[c] - g.ret[c]));
+          txp[c] = ant[r][c];
+          rxp[c] = ant[r][3 + c];
         }
+        PairGeom g;
+        if (!pair_geometry(txp, rxp, nrm, pt, g)) {
+          p.g_sigmas[a * p.P + q] = from_f<T>(0.0f);
+          continue;
+        }
+        const PairPath path = pair_path(p.c, txp, rxp, pt);
+        const int k = min(max(static_cast<int>(path.cell) - k0, 0), cells - 1);
+        const float4* row = reinterpret_cast<const float4*>(p.table + (a * kAdjCells + k) * kQ);
+        const float4 c2 = __ldg(row + 2), c1 = __ldg(row + 1), c0 = __ldg(row);
+        float gs;
+        const float2 sums = cell_sums(p.c, path, c0, c1, c2);
+        pair_gradients<WITH_POINTS>(g, sums.x, sums.y, sigma_value, nrm, &gs, gn, gp);
+        p.g_sigmas[a * p.P + q] = from_f<T>(gs / num_points);
       }
     }
-  }
-  if (!inside) return;
-  if (p.splits == 1) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      p.g_normals[q * 3 + c] = from_f<T>(gn[c] / inv_p);
-      if (WITH_POINTS) p.g_points[q * 3 + c] = from_f<T>(gp[c] / inv_p);
-    }
-  } else {
-    float* dst = p.partial + (split * p.P + q) * 6;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      dst[c] = gn[c];
-      dst[3 + c] = gp[c];
+    if (!inside) continue;
+    if (p.splits == 1) {
+  #pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        p.g_normals[q * 3 + c] = from_f<T>(gn[c] / num_points);
+        if (WITH_POINTS) p.g_points[q * 3 + c] = from_f<T>(gp[c] / num_points);
+      }
+    } else {
+      float* dst = p.partial + (split * p.P + q) * 6;
+  #pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        dst[c] = gn[c];
+        dst[3 + c] = gp[c];
+      }
     }
   }
 }
@@ -335,16 +281,7 @@ cudaError_t launch_adjoint(const TracerArgs& a, unsigned char* ws, PointList lis
                            cudaStream_t st) {
   const AdjLayout l = adj_layout(a);
   const PhaseConsts pc = phase_consts(a.f0, a.As, a.fs);
-  const double mid = 0.5 * static_cast<double>(a.S - 1);
-  AdjConsts c;
-  c.K = pc.k0 + mid * pc.k1;
-  c.b = pc.b0 + mid * pc.b1;
-  c.k1 = pc.k1;
-  c.b1 = pc.b1;
-  // without a sweep every path is in one cell
-  c.kappa = std::max(1e-6, GatherCells::kOver * static_cast<double>(a.S) * std::fabs(pc.k1));
-  c.theta_step = 2.0 * M_PI * pc.k1 / c.kappa;
-  c.S = static_cast<int>(a.S);
+  const AdjConsts c = adj_consts(pc.k0, pc.b0, pc.k1, pc.b1, a.f0, a.As, a.fs, a.S);
   AdjHead* head = reinterpret_cast<AdjHead*>(ws + l.head);
 
   BandP<T> bp;
@@ -385,12 +322,10 @@ cudaError_t launch_adjoint(const TracerArgs& a, unsigned char* ws, PointList lis
   pp.P = a.P;
   pp.splits = splits;
   pp.per_split = (a.A + splits - 1) / splits;
-  pp.w_mid = static_cast<float>(2.0 * static_cast<double>(kPiF) * (static_cast<double>(a.f0) + static_cast<double>(a.As) / a.fs * mid));
-  pp.kappa_c = static_cast<float>(c.kappa * static_cast<double>(kSpeedOfLight));
   pp.c = c;
-  // the grid covers all P points; blocks past the listed ones return at once
-  const int64_t blocks = (a.P + kPairThreads - 1) / kPairThreads * splits;
-  if (blocks > 0x7fffffff) return cudaErrorInvalidConfiguration;
+  // the number of listed points is on the device only: a few waves of blocks take its tiles in turn
+  const int64_t blocks = std::min<int64_t>((a.P + kPairThreads - 1) / kPairThreads * splits,
+                                           static_cast<int64_t>(current_device_info().sm_count) * 40);
   if (a.grad_points != nullptr) adj_pair_kernel<T, true><<<static_cast<unsigned>(blocks), kPairThreads, 0, st>>>(pp);
   else adj_pair_kernel<T, false><<<static_cast<unsigned>(blocks), kPairThreads, 0, st>>>(pp);
   return cudaGetLastError();

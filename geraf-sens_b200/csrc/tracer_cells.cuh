@@ -36,7 +36,7 @@ constexpr int kTraceRow = kTraceQ + 2;      // float2 per contribution row: 80 b
 struct TraceConsts {
   double K, b;       // phase of carrier and middle sample, cycles per metre and bias
   double k1, b1;     // phase step per sample
-  double kappa;      // cells per metre
+  double kappa, inv_kappa;  // cells per metre
   double theta_step;
   int S;
 };
@@ -51,6 +51,7 @@ inline TraceConsts trace_consts(double k0, double b0, double k1, double b1, int6
   // without a sweep every path is in cell 0
   const double kappa = MomentCells::kOver * static_cast<double>(S) * (k1 < 0.0 ? -k1 : k1);
   t.kappa = kappa > 1e-6 ? kappa : 1e-6;
+  t.inv_kappa = 1.0 / t.kappa;
   t.theta_step = 2.0 * 3.14159265358979323846 * k1 / t.kappa;
   t.S = static_cast<int>(S);
   return t;
@@ -72,14 +73,14 @@ struct TraceSmem {
   int start[kTraceSlots + 1];
   int tag[kTraceSlots];
   int list[kTraceThreads * (kTracePer + 1)];
-  int counts[kTracePer * kTraceWarps];
+  alignas(16) int counts[kTracePer * kTraceWarps];
   int evict[kTraceSlots];
   int has_row;
 };
 
 // Adds a cell's moments, seen by sample n, to acc.
 __device__ __forceinline__ void add_cell(const TraceConsts& c, int k, const float2* m, const float* g, int n, float2& acc) {
-  const double ph = (n - 0.5 * (c.S - 1)) * fma(c.k1, static_cast<double>(k) / c.kappa, c.b1);
+  const double ph = (n - 0.5 * (c.S - 1)) * fma(c.k1, k * c.inv_kappa, c.b1);
   const float2 e = cis_cycles(static_cast<float>(ph - rint(ph)));
   float2 ev = make_float2(0.0f, 0.0f), od = make_float2(0.0f, 0.0f);
 #pragma unroll
@@ -255,47 +256,61 @@ __device__ __forceinline__ void trace_all(TraceSmem& sm, const TraceConsts& c, f
   }
 }
 
-// All points of positions [begin, end), screened first: index_of(k) is the point at
-// position k, or -1 when it is out of bounds; sigma_of(q) its amplitude weight.
-template <typename T, typename IndexOf, typename SigmaOf>
+// `count` consecutive points (their arrays from the first one on; inb may be null),
+// screened first.
+template <typename T>
 __device__ __forceinline__ void trace_screened(TraceSmem& sm, const TraceConsts& c, float2* row, const T* normals,
-                                               const T* points, const float* txp, const float* rxp, int64_t begin,
-                                               int64_t end, IndexOf index_of, SigmaOf sigma_of) {
+                                               const T* points, const T* sigmas, const uint8_t* inb, const float* txp,
+                                               const float* rxp, int count) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int listed = 0;
   float nrm[kTracePer][3], pt[kTracePer][3];
-  int idx[kTracePer];
-  auto load = [&](int64_t p0) {  // of the next pass, in flight while batches are summed
+  unsigned in = 0;  // bit j: point j of the thread is in bounds
+  auto load = [&](int p0) {  // of the next pass, in flight while batches are summed
+    in = 0;
+    const int rest = count - p0 - static_cast<int>(threadIdx.x);
+    const T* pn = normals + (static_cast<int64_t>(p0) + threadIdx.x) * 3;
+    const T* pp = points + (static_cast<int64_t>(p0) + threadIdx.x) * 3;
+    const uint8_t* pb = inb != nullptr ? inb + p0 + threadIdx.x : nullptr;
 #pragma unroll
     for (int j = 0; j < kTracePer; ++j) {
-      const int64_t k = p0 + j * kTraceThreads + threadIdx.x;
-      idx[j] = k < end ? index_of(k) : -1;
-      if (idx[j] >= 0) load_point(normals, points, idx[j], nrm[j], pt[j]);
+      if (j * kTraceThreads < rest && (pb == nullptr || pb[j * kTraceThreads])) {
+        in |= 1u << j;
+        load_point(pn, pp, j * kTraceThreads, nrm[j], pt[j]);
+      }
     }
   };
-  load(begin);
-  for (int64_t p0 = begin; p0 < end; p0 += kTraceThreads * kTracePer) {
+  load(0);
+  for (int p0 = 0; p0 < count; p0 += kTraceThreads * kTracePer) {
     unsigned mask[kTracePer];
 #pragma unroll
     for (int j = 0; j < kTracePer; ++j) {
-      const bool keep = idx[j] >= 0 && !surely_culled(txp, rxp, nrm[j], pt[j]);
+      const bool keep = ((in >> j) & 1u) && !surely_culled(txp, rxp, nrm[j], pt[j]);
       mask[j] = __ballot_sync(0xffffffffu, keep);
-      if (lane == 0) sm.counts[j * kTraceWarps + warp] = __popc(mask[j]);
+      if (lane == 0) sm.counts[warp * kTracePer + j] = __popc(mask[j]);
     }
     __syncthreads();
+    // the list's order is that of (warp, pass, lane): the same on every run
     int before = listed;
 #pragma unroll
-    for (int j = 0; j < kTracePer; ++j) {
+    for (int w = 0; w < kTraceWarps; ++w) {
+      static_assert(kTracePer == 4, "one 16-byte load per warp's counts");
+      const int4 n = *reinterpret_cast<const int4*>(&sm.counts[w * kTracePer]);
+      if (w == warp) {
+        const int at[kTracePer] = {before, before + n.x, before + n.x + n.y, before + n.x + n.y + n.z};
 #pragma unroll
-      for (int w = 0; w < kTraceWarps; ++w) {
-        if (w == warp && ((mask[j] >> lane) & 1u)) sm.list[before + __popc(mask[j] & ((1u << lane) - 1u))] = idx[j];
-        before += sm.counts[j * kTraceWarps + w];
+        for (int j = 0; j < kTracePer; ++j) {
+          if ((mask[j] >> lane) & 1u) {
+            sm.list[at[j] + __popc(mask[j] & ((1u << lane) - 1u))] = p0 + j * kTraceThreads + static_cast<int>(threadIdx.x);
+          }
+        }
       }
+      before += n.x + n.y + n.z + n.w;
     }
     listed = before;
     load(p0 + kTraceThreads * kTracePer);
     __syncthreads();
-    const bool last = p0 + kTraceThreads * kTracePer >= end;
+    const bool last = p0 + kTraceThreads * kTracePer >= count;
     while (listed >= kTraceThreads || (last && listed > 0)) {
       const int cnt = min(listed, kTraceThreads);
       listed -= cnt;
@@ -307,7 +322,7 @@ __device__ __forceinline__ void trace_screened(TraceSmem& sm, const TraceConsts&
         const int64_t q = sm.list[listed + threadIdx.x];
         TracePoint t;
         load_point(normals, points, q, t.nrm, t.pt);
-        t.sigma = sigma_of(q);
+        t.sigma = ld_f(sigmas, q);
         live = trace_point(c, txp, rxp, t, w, cell, x);
       }
       trace_batch(sm, c, row, live, w, cell, x);

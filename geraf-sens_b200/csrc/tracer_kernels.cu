@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(128) tracer_fwd_plain_kernel(const TrP<T> p) {
 
 // MIXED forward.  Block = (antenna, point split): the points of the split (of the
 // pre-cull's list) into the moments of their cells (tracer_cells.cuh).  64 antennas x
-// 524288 points (10% listed, 8% of the pairs live) x 128 samples: FWD_US against 181 us
+// 524288 points (10% listed, 8% of the pairs live) x 128 samples: 119 us against 181 us
 // with a recurrence over the samples of every live pair.
 template <typename T>
 struct TrCellP {
@@ -414,163 +414,165 @@ __global__ void __launch_bounds__(128, 6) tracer_bwd_mixed_kernel(const TrP<T> p
   PairStager<T> stg{reinterpret_cast<T*>(smem + p.buf_off), bar, p.ld, p.rows, p.bulk != 0};
 
   const int TILE = blockDim.x;
-  const int split = blockIdx.x % p.splits;
-  const int64_t ptile = blockIdx.x / p.splits;
-  // Thread t owns point position k = ptile * TILE + t: listed point list[k],
-  // or point k when every point is visited.  The grid covers all P points;
-  // blocks past the listed ones have nothing to do.
+  // The number of listed points is on the device only: the blocks take the tiles of
+  // points (times splits) in turn.  Thread t owns point position k = ptile * TILE + t:
+  // listed point list[k], or point k when every point is visited.
   const int64_t npts = p.plist != nullptr ? static_cast<int64_t>(*p.plist_count) : p.P;
-  const int64_t p_base = ptile * TILE;
-  if (p_base >= npts) return;
-  const int64_t k_own = p_base + threadIdx.x;
-  const bool inside = k_own < npts;
-  const int64_t pi = !inside ? 0 : p.plist != nullptr ? static_cast<int64_t>(p.plist[k_own]) : k_own;
-  const int64_t a_begin = static_cast<int64_t>(split) * p.per_split;
-  const int64_t a_end = min(p.A, a_begin + p.per_split);
-  const int ntiles = a_end > a_begin ? ceil_div(a_end - a_begin, p.rows) : 0;
-  const bool active = inside && (p.plist != nullptr || p.inb[pi]);
-
+  const int64_t tiles = (npts + TILE - 1) / TILE * p.splits;
   if (p.bulk && threadIdx.x == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
     fence_barrier_init();
   }
   __syncthreads();
+  int used = 0;  // stages the ring has carried: the phases of its barriers go on from tile to tile
+  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int split = static_cast<int>(tile % p.splits);
+    const int64_t p_base = tile / p.splits * TILE;
+    const int64_t k_own = p_base + threadIdx.x;
+    const bool inside = k_own < npts;
+    const int64_t pi = !inside ? 0 : p.plist != nullptr ? static_cast<int64_t>(p.plist[k_own]) : k_own;
+    const int64_t a_begin = static_cast<int64_t>(split) * p.per_split;
+    const int64_t a_end = min(p.A, a_begin + p.per_split);
+    const int ntiles = a_end > a_begin ? ceil_div(a_end - a_begin, p.rows) : 0;
+    const bool active = inside && (p.plist != nullptr || p.inb[pi]);
 
-  float own_nrm[3] = {0.0f, 0.0f, 1.0f}, own_pt[3] = {0.0f, 0.0f, 0.0f};
-  if (active) {
-    load3(p.normals, pi, own_nrm);
-    load3(p.points, pi, own_pt);
-  }
-  // w0 and w1/fs in rad per unit delay, as exact FP64 products of the FP32 constants.
-  const float w0 = static_cast<float>(2.0 * static_cast<double>(kPiF) * p.f0);
-  const float w1s = static_cast<float>(2.0 * static_cast<double>(kPiF) * p.As / p.fs);
-  float gnorm[3] = {0.0f, 0.0f, 0.0f};
-  float gpt[3] = {0.0f, 0.0f, 0.0f};
-
-  auto issue = [&](int tile, int stage) {
-    const int64_t a0 = a_begin + static_cast<int64_t>(tile) * p.rows;
-    const int rws = static_cast<int>(min(static_cast<int64_t>(p.rows), a_end - a0));
-    stg.issue(stage, p.gr, p.gi, a0, rws, static_cast<int>(p.S));
-    stage_positions_f<T>(pos, stage, p.rows, p.tx, p.rx, a0, rws);
-  };
-  if (ntiles > 0) issue(0, 0);
-  if (ntiles > 1) issue(1, 1);
-
-  for (int t = 0; t < ntiles; ++t) {
-    const int s = t & 1;
-    for (int r = threadIdx.x; r < p.rows; r += TILE) cnt[r] = 0;
-    if (!stg.wait(s, (t >> 1) & 1, p.status)) {  // (its barrier also publishes cnt)
-      if (t + 1 < ntiles) stg.drain(s ^ 1, ((t + 1) >> 1) & 1, p.status);
-      return;
+    float own_nrm[3] = {0.0f, 0.0f, 1.0f}, own_pt[3] = {0.0f, 0.0f, 0.0f};
+    if (active) {
+      load3(p.normals, pi, own_nrm);
+      load3(p.points, pi, own_pt);
     }
-    const int64_t a0 = a_begin + static_cast<int64_t>(t) * p.rows;
-    const int rws = static_cast<int>(min(static_cast<int64_t>(p.rows), a_end - a0));
+    // w0 and w1/fs in rad per unit delay, as exact FP64 products of the FP32 constants.
+    const float w0 = static_cast<float>(2.0 * static_cast<double>(kPiF) * p.f0);
+    const float w1s = static_cast<float>(2.0 * static_cast<double>(kPiF) * p.As / p.fs);
+    float gnorm[3] = {0.0f, 0.0f, 0.0f};
+    float gpt[3] = {0.0f, 0.0f, 0.0f};
 
-    // 1. list the stage's candidate pairs, those the early test cannot cull (the
-    //    exact geometry, formed once in step 2, decides them); the other pairs get
-    //    zero gradients here
-    for (int r = 0; r < rws; ++r) {
-      if (!inside) break;
-      const float* ps = pos + (s * p.rows + r) * 6;
-      const float txp[3] = {ps[0], ps[1], ps[2]};
-      const float rxp[3] = {ps[3], ps[4], ps[5]};
-      const bool live = active && !surely_culled(txp, rxp, own_nrm, own_pt);
-      if (live) {
-        list[r * TILE + atomicAdd(&cnt[r], 1)] = threadIdx.x;
-      } else {
-        p.g_sigmas[(a0 + r) * p.P + pi] = from_f<T>(0.0f);
-#pragma unroll
-        for (int k = 0; k < NC; ++k) contrib[(r * NC + k) * TILE + threadIdx.x] = 0.0f;
-      }
-    }
-    __syncthreads();
+    auto issue = [&](int tile, int stage) {
+      const int64_t a0 = a_begin + static_cast<int64_t>(tile) * p.rows;
+      const int rws = static_cast<int>(min(static_cast<int64_t>(p.rows), a_end - a0));
+      stg.issue(stage, p.gr, p.gi, a0, rws, static_cast<int>(p.S));
+      stage_positions_f<T>(pos, stage, p.rows, p.tx, p.rx, a0, rws);
+    };
+    if (ntiles > 0) issue(0, used & 1);
+    if (ntiles > 1) issue(1, (used + 1) & 1);
 
-    // 2. every thread takes candidate pairs k = tid, tid + TILE, ... in (row, list) order
-    int total = 0;
-    for (int r = 0; r < rws; ++r) total += cnt[r];
-    int r_cur = 0, r_start = 0;
-    for (int k = threadIdx.x; k < total; k += TILE) {
-      while (k >= r_start + cnt[r_cur]) {
-        r_start += cnt[r_cur];
-        ++r_cur;
+    for (int t = 0; t < ntiles; ++t) {
+      const int s = (used + t) & 1;
+      for (int r = threadIdx.x; r < p.rows; r += TILE) cnt[r] = 0;
+      if (!stg.wait(s, ((used + t) >> 1) & 1, p.status)) {  // (its barrier also publishes cnt)
+        if (t + 1 < ntiles) stg.drain(s ^ 1, ((used + t + 1) >> 1) & 1, p.status);
+        return;
       }
-      const int r = r_cur;
-      const int slot = list[r * TILE + (k - r_start)];
-      const int64_t pj = p.plist != nullptr ? static_cast<int64_t>(p.plist[p_base + slot]) : p_base + slot;
-      const int64_t a = a0 + r;
-      float nrm[3], pt[3];
-      load3(p.normals, pj, nrm);
-      load3(p.points, pj, pt);
-      const float* ps = pos + (s * p.rows + r) * 6;
-      const float txp[3] = {ps[0], ps[1], ps[2]};
-      const float rxp[3] = {ps[3], ps[4], ps[5]};
-      SpecGeom geo;
-      specular_geometry(txp, rxp, nrm, pt, geo);
-      if (culled(geo)) {
-        p.g_sigmas[a * p.P + pj] = from_f<T>(0.0f);
-#pragma unroll
-        for (int c = 0; c < NC; ++c) contrib[(r * NC + c) * TILE + slot] = 0.0f;
-        continue;
-      }
-      const double px = pt[0], py = pt[1], pz = pt[2];
-      const PhaseCycles pc = path_cycles(ps[0] - px, ps[1] - py, ps[2] - pz, ps[3] - px,
-                                         ps[4] - py, ps[5] - pz, p.k0, p.b0, p.k1, p.b1);
-      const float2 zt = cis_cycles(pc.dcyc);
-      const T* rowr = stg.stage_ptr(s, 0) + r * p.ld;
-      const T* rowi = stg.stage_ptr(s, 1) + r * p.ld;
-      float2 qv, q1;  // Q and Q1 = zeta Q'(zeta): packed even/odd Horner in zeta^2
-      residual_sums<WITH_POINTS>(rowr, rowi, p.ld, zt, qv, q1);
-      const float qr = qv.x, qi = qv.y;
-      const float2 e0 = cis_cycles_fast(pc.frac0);
-      const float2 eq = cmul(e0, make_float2(qr, qi));
-      // sum_n (g_r cos + g_i sin) = Re(exp(j phi0) Q)
-      const float sum_re = eq.x;
-      const float propagation_distance = path_distance(txp, rxp, pt);
-      const float propagation_attenuation = 1.0f / sq(propagation_distance);
-      const float sigma_value = ld_f(p.sigmas, a * p.P + pj);
-      p.g_sigmas[a * p.P + pj] =
-          from_f<T>(propagation_attenuation * geo.align * sum_re / static_cast<float>(p.P));
-      float gsa[3];
-      align_normal_gradient(geo, nrm, gsa);
-      const float normal_scale = sigma_value * propagation_attenuation;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) contrib[(r * NC + c) * TILE + slot] = normal_scale * gsa[c] * sum_re;
-      if (WITH_POINTS) {
-        // sum_n w_n (g_i cos - g_r sin) = -Im(exp(j phi0) (w0 Q + w1s Q1))
-        const float2 f = cmul(e0, make_float2(w0 * qr + w1s * q1.x, w0 * qi + w1s * q1.y));
-        const float amp = sigma_value * geo.align * propagation_attenuation;
-        const float d_tau = -amp * f.y;
-        const float dist_t = sqrtf(sq(txp[0] - pt[0]) + sq(txp[1] - pt[1]) + sq(txp[2] - pt[2]));
-        const float dist_r = sqrtf(sq(rxp[0] - pt[0]) + sq(rxp[1] - pt[1]) + sq(rxp[2] - pt[2]));
-        float drho[3];
-        align_point_gradient(geo, nrm, dist_t, dist_r, drho);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const float dD = geo.inc[c] - geo.ret[c];
-          const float damp_dp =
-              normal_scale * drho[c] - 2.0f * amp / propagation_distance * dD;
-          contrib[(r * NC + 3 + c) * TILE + slot] = sum_re * damp_dp + d_tau * dD / kSpeedOfLight;
-        }
-      }
-    }
-    __syncthreads();
+      const int64_t a0 = a_begin + static_cast<int64_t>(t) * p.rows;
+      const int rws = static_cast<int>(min(static_cast<int64_t>(p.rows), a_end - a0));
 
-    // 3. each owner adds its point's contributions in antenna order
-    if (inside) {
+      // 1. list the stage's candidate pairs, those the early test cannot cull (the
+      //    exact geometry, formed once in step 2, decides them); the other pairs get
+      //    zero gradients here
       for (int r = 0; r < rws; ++r) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) gnorm[c] += contrib[(r * NC + c) * TILE + threadIdx.x];
-        if (WITH_POINTS) {
-#pragma unroll
-          for (int c = 0; c < 3; ++c) gpt[c] += contrib[(r * NC + 3 + c) * TILE + threadIdx.x];
+        if (!inside) break;
+        const float* ps = pos + (s * p.rows + r) * 6;
+        const float txp[3] = {ps[0], ps[1], ps[2]};
+        const float rxp[3] = {ps[3], ps[4], ps[5]};
+        const bool live = active && !surely_culled(txp, rxp, own_nrm, own_pt);
+        if (live) {
+          list[r * TILE + atomicAdd(&cnt[r], 1)] = threadIdx.x;
+        } else {
+          p.g_sigmas[(a0 + r) * p.P + pi] = from_f<T>(0.0f);
+  #pragma unroll
+          for (int k = 0; k < NC; ++k) contrib[(r * NC + k) * TILE + threadIdx.x] = 0.0f;
         }
       }
+      __syncthreads();
+
+      // 2. every thread takes candidate pairs k = tid, tid + TILE, ... in (row, list) order
+      int total = 0;
+      for (int r = 0; r < rws; ++r) total += cnt[r];
+      int r_cur = 0, r_start = 0;
+      for (int k = threadIdx.x; k < total; k += TILE) {
+        while (k >= r_start + cnt[r_cur]) {
+          r_start += cnt[r_cur];
+          ++r_cur;
+        }
+        const int r = r_cur;
+        const int slot = list[r * TILE + (k - r_start)];
+        const int64_t pj = p.plist != nullptr ? static_cast<int64_t>(p.plist[p_base + slot]) : p_base + slot;
+        const int64_t a = a0 + r;
+        float nrm[3], pt[3];
+        load3(p.normals, pj, nrm);
+        load3(p.points, pj, pt);
+        const float* ps = pos + (s * p.rows + r) * 6;
+        const float txp[3] = {ps[0], ps[1], ps[2]};
+        const float rxp[3] = {ps[3], ps[4], ps[5]};
+        SpecGeom geo;
+        specular_geometry(txp, rxp, nrm, pt, geo);
+        if (culled(geo)) {
+          p.g_sigmas[a * p.P + pj] = from_f<T>(0.0f);
+  #pragma unroll
+          for (int c = 0; c < NC; ++c) contrib[(r * NC + c) * TILE + slot] = 0.0f;
+          continue;
+        }
+        const double px = pt[0], py = pt[1], pz = pt[2];
+        const PhaseCycles pc = path_cycles(ps[0] - px, ps[1] - py, ps[2] - pz, ps[3] - px,
+                                           ps[4] - py, ps[5] - pz, p.k0, p.b0, p.k1, p.b1);
+        const float2 zt = cis_cycles(pc.dcyc);
+        const T* rowr = stg.stage_ptr(s, 0) + r * p.ld;
+        const T* rowi = stg.stage_ptr(s, 1) + r * p.ld;
+        float2 qv, q1;  // Q and Q1 = zeta Q'(zeta): packed even/odd Horner in zeta^2
+        residual_sums<WITH_POINTS>(rowr, rowi, p.ld, zt, qv, q1);
+        const float qr = qv.x, qi = qv.y;
+        const float2 e0 = cis_cycles_fast(pc.frac0);
+        const float2 eq = cmul(e0, make_float2(qr, qi));
+        // sum_n (g_r cos + g_i sin) = Re(exp(j phi0) Q)
+        const float sum_re = eq.x;
+        const float propagation_distance = path_distance(txp, rxp, pt);
+        const float propagation_attenuation = 1.0f / sq(propagation_distance);
+        const float sigma_value = ld_f(p.sigmas, a * p.P + pj);
+        p.g_sigmas[a * p.P + pj] =
+            from_f<T>(propagation_attenuation * geo.align * sum_re / static_cast<float>(p.P));
+        float gsa[3];
+        align_normal_gradient(geo, nrm, gsa);
+        const float normal_scale = sigma_value * propagation_attenuation;
+  #pragma unroll
+        for (int c = 0; c < 3; ++c) contrib[(r * NC + c) * TILE + slot] = normal_scale * gsa[c] * sum_re;
+        if (WITH_POINTS) {
+          // sum_n w_n (g_i cos - g_r sin) = -Im(exp(j phi0) (w0 Q + w1s Q1))
+          const float2 f = cmul(e0, make_float2(w0 * qr + w1s * q1.x, w0 * qi + w1s * q1.y));
+          const float amp = sigma_value * geo.align * propagation_attenuation;
+          const float d_tau = -amp * f.y;
+          const float dist_t = sqrtf(sq(txp[0] - pt[0]) + sq(txp[1] - pt[1]) + sq(txp[2] - pt[2]));
+          const float dist_r = sqrtf(sq(rxp[0] - pt[0]) + sq(rxp[1] - pt[1]) + sq(rxp[2] - pt[2]));
+          float drho[3];
+          align_point_gradient(geo, nrm, dist_t, dist_r, drho);
+  #pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const float dD = geo.inc[c] - geo.ret[c];
+            const float damp_dp =
+                normal_scale * drho[c] - 2.0f * amp / propagation_distance * dD;
+            contrib[(r * NC + 3 + c) * TILE + slot] = sum_re * damp_dp + d_tau * dD / kSpeedOfLight;
+          }
+        }
+      }
+      __syncthreads();
+
+      // 3. each owner adds its point's contributions in antenna order
+      if (inside) {
+        for (int r = 0; r < rws; ++r) {
+  #pragma unroll
+          for (int c = 0; c < 3; ++c) gnorm[c] += contrib[(r * NC + c) * TILE + threadIdx.x];
+          if (WITH_POINTS) {
+  #pragma unroll
+            for (int c = 0; c < 3; ++c) gpt[c] += contrib[(r * NC + 3 + c) * TILE + threadIdx.x];
+          }
+        }
+      }
+      __syncthreads();
+      if (t + 2 < ntiles) issue(t + 2, s);
     }
-    __syncthreads();
-    if (t + 2 < ntiles) issue(t + 2, s);
+    used += ntiles;
+    if (inside) store_point_grads(p, split, pi, gnorm, gpt, WITH_POINTS);
   }
-  if (inside) store_point_grads(p, split, pi, gnorm, gpt, WITH_POINTS);
 }
 
 // With a point list, only the listed points' partials are summed (the others'
@@ -907,7 +909,9 @@ cudaError_t launch_tracer_bwd(const TracerArgs& a, const Tuning& t, void* ws, cu
                                          static_cast<int>(lay.total));
   if (err != cudaSuccess) return err;
   const int64_t ptiles = (a.P + threads - 1) / threads;
-  const int64_t blocks = ptiles * t.splits;
+  int64_t blocks = ptiles * t.splits;
+  // MIXED blocks take tiles in turn; a few waves of them
+  if (a.mode == kMixed) blocks = std::min<int64_t>(blocks, static_cast<int64_t>(dev.sm_count) * 24);
   if (blocks > 0x7fffffff) return cudaErrorInvalidConfiguration;
   if (a.mode == kMixed && tracer_point_list_applies(a)) {
     // lists the points and zeroes the gradients of every point it leaves out

@@ -15,9 +15,8 @@
 // every pair of the point meets i.n > 1e-4 |i||n| or o.r < -1e-4 |o||i| m, the
 // margins under which the reference's FP32 geometry culls a pair
 // (surely_culled() in tracer_geometry.cuh derives them); the per-pair kernels
-// would discard all of the point's pairs.  The test runs in FP64 on the FP32
-// values the kernels use; its rounding (~1e-16 relative) is far inside the
-// 1e-4 margin.  Non-finite values fail both comparisons, so such points are
+// would discard all of the point's pairs.  The test runs on the FP32 values the
+// kernels use, with twice the margin for its own rounding (culled_for_all).  Non-finite values fail both comparisons, so such points are
 // listed and decided by the exact form.  Out-of-bounds points are never listed.
 //
 // Launches: per-point flags with a count per 1024-point chunk, and the ordered
@@ -52,9 +51,9 @@ struct Aperture {
 // is written by thread 0 and published by the closing barrier.
 template <typename T>
 __device__ void block_aperture(const T* tx, const T* rx, int64_t A, Aperture* out) {
-  __shared__ double red[6][256];
+  __shared__ double red[8][6];
   __shared__ double cen[6];
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   double s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   for (int64_t a = tid; a < A; a += 256) {
 #pragma unroll
@@ -63,19 +62,25 @@ __device__ void block_aperture(const T* tx, const T* rx, int64_t A, Aperture* ou
       s[3 + k] += static_cast<double>(ld_f(rx, a * 3 + k));
     }
   }
+  if (warp * 32 < A) {
 #pragma unroll
-  for (int k = 0; k < 6; ++k) red[k][tid] = s[k];
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (tid < w) {
+    for (int k = 0; k < 6; ++k) {
 #pragma unroll
-      for (int k = 0; k < 6; ++k) red[k][tid] += red[k][tid + w];
+      for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
     }
-    __syncthreads();
   }
-  if (tid < 6) cen[tid] = A > 0 ? red[tid][0] / static_cast<double>(A) : NAN;
+  if (lane == 0) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) red[warp][k] = s[k];
+  }
   __syncthreads();
-  double mt = 0.0, mr = 0.0;
+  if (tid < 6) {
+    double t = red[0][tid];
+    for (int w = 1; w < 8; ++w) t += red[w][tid];
+    cen[tid] = A > 0 ? t / static_cast<double>(A) : NAN;
+  }
+  __syncthreads();
+  double m[2] = {0.0, 0.0};  // largest squared distances
   for (int64_t a = tid; a < A; a += 256) {
     double dt = 0.0, dr = 0.0;
 #pragma unroll
@@ -87,21 +92,29 @@ __device__ void block_aperture(const T* tx, const T* rx, int64_t A, Aperture* ou
     }
     // fmax drops a NaN operand; a non-finite antenna makes its centre (and so
     // every test) non-finite instead
-    mt = fmax(mt, sqrt(dt));
-    mr = fmax(mr, sqrt(dr));
+    m[0] = fmax(m[0], dt);
+    m[1] = fmax(m[1], dr);
   }
-  __syncthreads();  // red is reused
-  red[0][tid] = mt;
-  red[1][tid] = mr;
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (tid < w) {
-      red[0][tid] = fmax(red[0][tid], red[0][tid + w]);
-      red[1][tid] = fmax(red[1][tid], red[1][tid + w]);
+  if (warp * 32 < A) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m[k] = fmax(m[k], __shfl_xor_sync(0xffffffffu, m[k], o));
     }
-    __syncthreads();
   }
+  if (lane == 0) {
+    red[warp][0] = m[0];
+    red[warp][1] = m[1];
+  }
+  __syncthreads();
   if (tid == 0) {
+    double rt = red[0][0], rr = red[0][1];
+    for (int w = 1; w < 8; ++w) {
+      rt = fmax(rt, red[w][0]);
+      rr = fmax(rr, red[w][1]);
+    }
+    rt = sqrt(rt);
+    rr = sqrt(rr);
     // widen the radii by far more than the FP64 rounding of the distances
     const double st = fabs(cen[0]) + fabs(cen[1]) + fabs(cen[2]);
     const double sr = fabs(cen[3]) + fabs(cen[4]) + fabs(cen[5]);
@@ -110,8 +123,8 @@ __device__ void block_aperture(const T* tx, const T* rx, int64_t A, Aperture* ou
       out->ct[k] = cen[k];
       out->cr[k] = cen[3 + k];
     }
-    out->rt = red[0][0] + 1e-12 * (red[0][0] + st);
-    out->rr = red[1][0] + 1e-12 * (red[1][0] + sr);
+    out->rt = rt + 1e-12 * (rt + st);
+    out->rr = rr + 1e-12 * (rr + sr);
   }
   __syncthreads();
 }
@@ -121,36 +134,47 @@ __global__ void __launch_bounds__(256) aperture_kernel(const T* tx, const T* rx,
   block_aperture(tx, rx, A, out);
 }
 
-__device__ __forceinline__ double dot3d(const double* a, const double* b) {
-  return fma(a[2], b[2], fma(a[1], b[1], a[0] * b[0]));
+// Square root within ~1e-6, zero at zero.
+__device__ __forceinline__ float sqrt_rough(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 }
 
-// True when every pair of the point is culled with the margin above.
-__device__ __forceinline__ bool culled_for_all(const Aperture& ap, const float* nf, const float* pf) {
-  double n[3], ic[3], oc[3];
+__device__ __forceinline__ float dot3f(const float* a, const float* b) {
+  return fmaf(a[2], b[2], fmaf(a[1], b[1], a[0] * b[0]));
+}
+
+// True when every pair of the point is culled with the margin above.  The offsets
+// from the centres are formed in FP64 (exact to ~1e-16 of the coordinates), the rest in
+// FP32 with the margin doubled: its rounding, below 3e-6 of the terms compared, leaves
+// every culled point well inside the 1e-4 that the argument needs.  (In FP64 throughout,
+// the four square roots and ~60 operations took 12 us for 524288 points.)
+__device__ __forceinline__ bool culled_for_all(const Aperture& ap, const float* n, const float* pf) {
+  constexpr float kMargin = 2e-4f;
+  float ic[3], oc[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    n[k] = nf[k];
-    ic[k] = static_cast<double>(pf[k]) - ap.ct[k];
-    oc[k] = ap.cr[k] - static_cast<double>(pf[k]);
+    ic[k] = static_cast<float>(static_cast<double>(pf[k]) - ap.ct[k]);
+    oc[k] = static_cast<float>(ap.cr[k] - static_cast<double>(pf[k]));
   }
-  const double nn = dot3d(n, n);
-  const double nrm = sqrt(nn);
-  const double m = 1.0 + 2.0 * nn;
-  const double icn = dot3d(ic, n);
-  const double ni = sqrt(dot3d(ic, ic));
-  const double no = sqrt(dot3d(oc, oc));
-  if (icn - ap.rt * nrm > 1e-4 * (ni + ap.rt) * nrm) return true;
-  const double ocn = dot3d(oc, n);
-  double hi[3], ho[3];
+  const float rt = static_cast<float>(ap.rt), rr = static_cast<float>(ap.rr);
+  const float nn = dot3f(n, n);
+  const float nrm = sqrt_rough(nn);
+  const float m = 1.0f + 2.0f * nn;
+  const float icn = dot3f(ic, n);
+  const float ni = sqrt_rough(dot3f(ic, ic)) + rt;
+  if (icn - rt * nrm > kMargin * ni * nrm) return true;
+  const float no = sqrt_rough(dot3f(oc, oc)) + rr;
+  const float ocn = dot3f(oc, n);
+  float hi[3], ho[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    hi[k] = ic[k] - 2.0 * icn * n[k];
-    ho[k] = oc[k] - 2.0 * ocn * n[k];
+    hi[k] = ic[k] - 2.0f * icn * n[k];
+    ho[k] = oc[k] - 2.0f * ocn * n[k];
   }
-  const double bound = dot3d(oc, hi) + ap.rr * sqrt(dot3d(hi, hi)) + ap.rt * sqrt(dot3d(ho, ho)) +
-                       m * ap.rr * ap.rt;
-  return bound < -1e-4 * (no + ap.rr) * (ni + ap.rt) * m;
+  const float bound = dot3f(oc, hi) + rr * sqrt_rough(dot3f(hi, hi)) + rt * sqrt_rough(dot3f(ho, ho)) + m * rr * rt;
+  return bound < -kMargin * no * ni * m;
 }
 
 // Flag word w of chunk c covers points c*1024 + w*32 + lane; counts[c] is the
@@ -262,8 +286,9 @@ __global__ void __launch_bounds__(1024) chunk_scan_kernel(const int* counts, int
 }
 
 // Writes the listed point indices of each chunk in ascending order; with
-// gradient outputs, every unlisted point gets zero gradients (all antennas'
-// grad_sigmas, grad_normals and grad_points).  With a null `offsets` each block
+// gradient outputs, the chunk's gradients (all antennas' grad_sigmas, grad_normals and
+// grad_points) are zeroed, whole lines at a time: the kernels that follow write the
+// listed points'.  With a null `offsets` each block
 // sums the counts of the chunks before its own, and the last block writes the
 // total.
 template <typename T>
@@ -309,7 +334,6 @@ __global__ void __launch_bounds__(kChunkThreads) point_scatter_kernel(const uint
   }
   __syncthreads();
   const int off = off_s;
-  const T zero = from_f<T>(0.0f);
 #pragma unroll
   for (int k = 0; k < kChunk / kChunkThreads; ++k) {
     const int wi = k * (kChunkThreads / 32) + warp;
@@ -318,15 +342,13 @@ __global__ void __launch_bounds__(kChunkThreads) point_scatter_kernel(const uint
     const uint32_t w = w_s[wi];
     if ((w >> lane) & 1u) {
       list[off + pre_s[wi] + __popc(w & ((1u << lane) - 1u))] = static_cast<int>(q);
-    } else if (g_normals != nullptr) {
-#pragma unroll
-      for (int j = 0; j < 3; ++j) g_normals[q * 3 + j] = zero;
-      if (g_points != nullptr) {
-#pragma unroll
-        for (int j = 0; j < 3; ++j) g_points[q * 3 + j] = zero;
-      }
-      for (int64_t a = 0; a < A; ++a) g_sigmas[a * P + q] = zero;
     }
+  }
+  if (g_normals != nullptr) {
+    const int64_t q0 = chunk * kChunk, q1 = min(P, q0 + kChunk);
+    zero_range(g_normals, q0 * 3, q1 * 3);
+    if (g_points != nullptr) zero_range(g_points, q0 * 3, q1 * 3);
+    for (int64_t a = 0; a < A; ++a) zero_range(g_sigmas, a * P + q0, a * P + q1);
   }
 }
 
