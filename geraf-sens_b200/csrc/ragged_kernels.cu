@@ -153,8 +153,11 @@ __global__ void __launch_bounds__(kTraceThreads, 6) ragged_fwd_kernel(const RgP<
     ld3(p.tx, a, txp);
     ld3(p.rx, a, rxp);
     trace_begin(sm);
-    trace_screened<T>(sm, p.c, p.rows + item * p.c.S, p.normals + first * 3, p.points + first * 3, p.sigmas + first,
-                      p.inb != nullptr ? p.inb + first : nullptr, txp, rxp, static_cast<int>(count));
+    for (int64_t at = first; at < first + count; at += kTraceRun) {
+      trace_screened<T>(sm, p.c, p.rows + item * p.c.S, p.normals + at * 3, p.points + at * 3, p.sigmas + at,
+                        p.inb != nullptr ? p.inb + at : nullptr, txp, rxp,
+                        static_cast<int>(min(first + count - at, static_cast<int64_t>(kTraceRun))));
+    }
     trace_store(sm, p.records + item);
   }
 }

@@ -5,7 +5,7 @@
 //
 // Launches: the band of cells from the boxes of the listed points and of the
 // antennas, with the interpolation basis; the antennas' tables; the pairs.  Where the
-// band does not fit kAdjCells cells the pairs are left to the general kernel
+// band does not fit adj_cells() cells the pairs are left to the general kernel
 // (tracer_kernels.cu), which returns at once otherwise.
 #include <algorithm>
 #include <cmath>
@@ -19,7 +19,9 @@ namespace {
 using namespace tracer;
 
 constexpr int kQ = GatherCells::Q;
-constexpr int kAdjCells = 128;  // 2.4 m of path at 4 GHz swept
+// Cells per antenna: 9.6 m of path at 4 GHz swept; 2.4 m for large arrays, whose tables
+// would outgrow the rest of the call's memory.
+int64_t adj_cells(int64_t A) { return A <= 2048 ? 512 : 128; }
 constexpr int kBandThreads = 1024;
 constexpr int kTableThreads = 128;
 constexpr int kTableCells = 16;  // cells per block of the table kernel
@@ -44,7 +46,7 @@ AdjLayout adj_layout(const TracerArgs& a) {
   l.boxes = 256;
   l.basis = up256(l.boxes + static_cast<size_t>(tracer_point_chunks(a.P)) * 6 * sizeof(float));
   l.table = up256(l.basis + static_cast<size_t>(a.S) * kQ * sizeof(float));
-  l.total = up256(l.table + static_cast<size_t>(a.A) * kAdjCells * kQ * sizeof(float2));
+  l.total = up256(l.table + static_cast<size_t>(a.A) * adj_cells(a.A) * kQ * sizeof(float2));
   return l;
 }
 
@@ -56,6 +58,7 @@ struct BandP {
   const T* rx;
   AdjHead* head;
   float* basis;
+  int max_cells;
   AdjConsts c;
 };
 
@@ -123,7 +126,7 @@ __global__ void __launch_bounds__(kBandThreads) adj_band_kernel(const BandP<T> p
   const double lo = floor((sqrt(near[0]) + sqrt(near[1])) * p.c.kappa) - 1.0;
   const double hi = ceil((sqrt(far[0]) + sqrt(far[1])) * p.c.kappa) + 1.0;
   const bool none = box[0] > box[3];  // no listed point: no pairs either
-  const bool fits = none || (hi - lo + 1.0 <= kAdjCells && hi < 1073741824.0);  // false for NaN
+  const bool fits = none || (hi - lo + 1.0 <= p.max_cells && hi < 1073741824.0);  // false for NaN
   p.head->bad = fits ? 0 : 1;
   p.head->k0 = fits && !none ? static_cast<int>(lo) : 0;
   p.head->cells = fits && !none ? static_cast<int>(hi - lo) + 1 : 0;
@@ -135,7 +138,8 @@ struct AdjTableP {
   const T* gi;
   const float* basis;
   const AdjHead* head;
-  float2* table;  // [A][kAdjCells][kQ]
+  float2* table;  // [A][max_cells][kQ]
+  int max_cells;
   AdjConsts c;
 };
 
@@ -169,7 +173,7 @@ __global__ void __launch_bounds__(kTableThreads) adj_table_kernel(const AdjTable
 #pragma unroll
   for (int q = 0; q < kQ; ++q) red[slice][threadIdx.x % kTableCells][q] = acc[q];
   __syncthreads();
-  float2* out = p.table + (a * kAdjCells + blockIdx.y * kTableCells) * kQ;
+  float2* out = p.table + (a * p.max_cells + blockIdx.y * kTableCells) * kQ;
   const int live = min(kTableCells, cells - static_cast<int>(blockIdx.y) * kTableCells);
   for (int i = threadIdx.x; i < live * kQ; i += kTableThreads) {
     float2 s = (&red[0][0][0])[i];
@@ -194,7 +198,7 @@ struct AdjPairP {
   const AdjHead* head;
   float* partial;  // [splits][P][6]
   int64_t A, P, per_split;
-  int splits;
+  int splits, max_cells;
   AdjConsts c;
 };
 
@@ -250,7 +254,7 @@ __global__ void __launch_bounds__(kPairThreads, 5) adj_pair_kernel(const AdjPair
         }
         const PairPath path = pair_path(p.c, txp, rxp, pt);
         const int k = min(max(static_cast<int>(path.cell) - k0, 0), cells - 1);
-        const float4* row = reinterpret_cast<const float4*>(p.table + (a * kAdjCells + k) * kQ);
+        const float4* row = reinterpret_cast<const float4*>(p.table + (a * p.max_cells + k) * kQ);
         const float4 c2 = __ldg(row + 2), c1 = __ldg(row + 1), c0 = __ldg(row);
         float gs;
         const float2 sums = cell_sums(p.c, path, c0, c1, c2);
@@ -292,6 +296,7 @@ cudaError_t launch_adjoint(const TracerArgs& a, unsigned char* ws, PointList lis
   bp.rx = static_cast<const T*>(a.rx);
   bp.head = head;
   bp.basis = reinterpret_cast<float*>(ws + l.basis);
+  bp.max_cells = static_cast<int>(adj_cells(a.A));
   bp.c = c;
   adj_band_kernel<T><<<1, kBandThreads, 0, st>>>(bp);
 
@@ -301,8 +306,9 @@ cudaError_t launch_adjoint(const TracerArgs& a, unsigned char* ws, PointList lis
   tp.basis = bp.basis;
   tp.head = head;
   tp.table = reinterpret_cast<float2*>(ws + l.table);
+  tp.max_cells = bp.max_cells;
   tp.c = c;
-  adj_table_kernel<T><<<dim3(static_cast<unsigned>(a.A), kAdjCells / kTableCells), kTableThreads, 0, st>>>(tp);
+  adj_table_kernel<T><<<dim3(static_cast<unsigned>(a.A), static_cast<unsigned>(bp.max_cells / kTableCells)), kTableThreads, 0, st>>>(tp);
 
   AdjPairP<T> pp;
   pp.normals = static_cast<const T*>(a.normals);
@@ -322,6 +328,7 @@ cudaError_t launch_adjoint(const TracerArgs& a, unsigned char* ws, PointList lis
   pp.P = a.P;
   pp.splits = splits;
   pp.per_split = (a.A + splits - 1) / splits;
+  pp.max_cells = bp.max_cells;
   pp.c = c;
   // the number of listed points is on the device only: a few waves of blocks take its tiles in turn
   const int64_t blocks = std::min<int64_t>((a.P + kPairThreads - 1) / kPairThreads * splits,

@@ -13,10 +13,13 @@
 // of eight lanes, one per moment, in list order: no floating-point atomics, the
 // same bits on every run.
 //
-// Cells are kept in kTraceSlots slots, cell k in slot k mod kTraceSlots.  Two
-// cells of one run that fall in the same slot (2.4 m of path apart at 4 GHz swept)
-// are kept apart: the later ones wait until the slot's moments were turned into
-// samples and added to the run's row of samples.
+// Cells are kept in kTraceSlots slots, cell k in slot k mod kTraceSlots.  Points whose
+// slot another cell of the run holds (2.4 m of path away at 4 GHz swept) are
+// deferred: when the run's other points are done, the moments so far are turned into
+// samples, added to the run's row of samples, and the deferred points have the slots
+// to themselves.  A wide scene thus takes a few passes over its live points, not one
+// conversion per conflict.  (128 slots took 10 to 13% longer on scenes that need a
+// dozen cells.)
 #pragma once
 
 #include "range_cells.cuh"
@@ -31,6 +34,7 @@ constexpr int kTracePer = 4;  // points per thread and screening pass
 constexpr int kTraceQ = MomentCells::Q;
 constexpr int kTraceSlots = 64;
 constexpr int kTraceEmpty = INT32_MIN + 1;  // no finite path has this cell
+constexpr int kTraceRun = 16384;            // positions per run, at most (the deferral mask's size)
 constexpr int kTraceRow = kTraceQ + 2;      // float2 per contribution row: 80 bytes, conflict-free
 
 struct TraceConsts {
@@ -74,7 +78,7 @@ struct TraceSmem {
   int tag[kTraceSlots];
   int list[kTraceThreads * (kTracePer + 1)];
   alignas(16) int counts[kTracePer * kTraceWarps];
-  int evict[kTraceSlots];
+  uint32_t defer[kTraceRun / 32];
   int has_row;
 };
 
@@ -99,14 +103,14 @@ __device__ __forceinline__ void trace_begin(TraceSmem& sm) {
   for (int i = threadIdx.x; i < kTraceSlots; i += kTraceThreads) {
     sm.tag[i] = kTraceEmpty;
     sm.hist[i] = make_int4(0, 0, 0, 0);
-    sm.evict[i] = 0;
   }
+  for (int i = threadIdx.x; i < kTraceRun / 32; i += kTraceThreads) sm.defer[i] = 0u;
   if (threadIdx.x == 0) sm.has_row = 0;
   __syncthreads();
 }
 
-// The slots marked for eviction go to the run's row of samples (in device memory,
-// touched by this block only) and are emptied.
+// The moments of all slots go to the run's row of samples (in device memory, touched
+// by this block only) and the slots are emptied.
 static __device__ __noinline__ void trace_evict(TraceSmem& sm, const TraceConsts c, float2* row) {
   const bool first = sm.has_row == 0;
   for (int n = threadIdx.x; n < c.S; n += kTraceThreads) {
@@ -114,82 +118,75 @@ static __device__ __noinline__ void trace_evict(TraceSmem& sm, const TraceConsts
     cell_basis<kTraceQ>(c.theta_step * (n - 0.5 * (c.S - 1)), g);
     float2 acc = first ? make_float2(0.0f, 0.0f) : row[n];
     for (int s = 0; s < kTraceSlots; ++s) {
-      if (sm.evict[s]) add_cell(c, sm.tag[s], sm.moments[s], g, n, acc);
+      if (sm.tag[s] != kTraceEmpty) add_cell(c, sm.tag[s], sm.moments[s], g, n, acc);
     }
     row[n] = acc;
   }
   __syncthreads();
-  for (int s = threadIdx.x; s < kTraceSlots; s += kTraceThreads) {
-    if (!sm.evict[s]) continue;
-    sm.evict[s] = 0;
-    sm.tag[s] = kTraceEmpty;
-    for (int q = 0; q < kTraceQ; ++q) sm.moments[s][q] = make_float2(0.0f, 0.0f);
+  for (int i = threadIdx.x; i < kTraceSlots * kTraceQ; i += kTraceThreads) {
+    (&sm.moments[0][0])[i] = make_float2(0.0f, 0.0f);
   }
+  for (int s = threadIdx.x; s < kTraceSlots; s += kTraceThreads) sm.tag[s] = kTraceEmpty;
   if (threadIdx.x == 0) sm.has_row = 1;
   __syncthreads();
 }
 
-// One batch: thread t holds a live contribution w at cell k, offset x (or none).
-__device__ __forceinline__ void trace_batch(TraceSmem& sm, const TraceConsts& c, float2* row, bool live, float2 w, int k,
-                                            float x) {
+// One batch: thread t holds a live contribution w at cell k, offset x, of the run's
+// position `pos` (or none).  Returns, on every thread, whether any was deferred.
+__device__ __forceinline__ bool trace_batch(TraceSmem& sm, bool live, float2 w, int k, float x, int pos) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int slot = k & (kTraceSlots - 1);
-  bool pending = live;
-  for (;;) {
-    bool in = false;
-    if (pending) {
-      const int old = sm.tag[slot] == k ? k : atomicCAS(&sm.tag[slot], kTraceEmpty, k);
-      in = old == kTraceEmpty || old == k;
-      if (!in) sm.evict[slot] = 1;
-    }
-    const unsigned same = __match_any_sync(0xffffffffu, in ? slot : kTraceSlots);
-    const int rank = __popc(same & ((1u << lane) - 1u));
-    if (in && rank == 0) reinterpret_cast<int*>(&sm.hist[slot])[warp] = __popc(same);
-    __syncthreads();
-    if (warp == 0) {  // exclusive prefix over (slot, warp), two slots per lane
-      const int4 a = sm.hist[2 * lane], b = sm.hist[2 * lane + 1];
-      const int sa = a.x + a.y + a.z + a.w, sb = b.x + b.y + b.z + b.w;
-      int run = sa + sb;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, run, o);
-        if (lane >= o) run += y;
-      }
-      const int e = run - sa - sb;
-      sm.start[2 * lane] = e;
-      sm.start[2 * lane + 1] = e + sa;
-      sm.hist[2 * lane] = make_int4(e, e + a.x, e + a.x + a.y, e + a.x + a.y + a.z);
-      const int f = e + sa;
-      sm.hist[2 * lane + 1] = make_int4(f, f + b.x, f + b.x + b.y, f + b.x + b.y + b.z);
-      if (lane == 31) sm.start[kTraceSlots] = run;
-    }
-    __syncthreads();
-    if (in) {  // the contribution row w x^q, at its place in cell order
-      const int place = reinterpret_cast<const int*>(&sm.hist[slot])[warp] + rank;
-      float4* dst = reinterpret_cast<float4*>(&sm.rows[place][0]);
-      float2 v = w;
-#pragma unroll
-      for (int q = 0; q < kTraceQ; q += 2) {
-        const float2 u = make_float2(v.x * x, v.y * x);
-        dst[q / 2] = make_float4(v.x, v.y, u.x, u.y);
-        v = make_float2(u.x * x, u.y * x);
-      }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kTraceSlots; i += kTraceThreads) sm.hist[i] = make_int4(0, 0, 0, 0);
-    const int q = threadIdx.x & (kTraceQ - 1);
-    for (int s = threadIdx.x / kTraceQ; s < kTraceSlots; s += kTraceThreads / kTraceQ) {
-      const int i0 = sm.start[s], i1 = sm.start[s + 1];
-      if (i0 == i1) continue;
-      float2 acc = sm.moments[s][q];
-#pragma unroll 4
-      for (int i = i0; i < i1; ++i) acc = fadd2(acc, sm.rows[i][q]);
-      sm.moments[s][q] = acc;
-    }
-    pending = pending && !in;
-    if (!__syncthreads_or(pending)) break;
-    trace_evict(sm, c, row);
+  bool in = false;
+  if (live) {
+    const int old = sm.tag[slot] == k ? k : atomicCAS(&sm.tag[slot], kTraceEmpty, k);
+    in = old == kTraceEmpty || old == k;
+    if (!in) atomicOr(&sm.defer[pos >> 5], 1u << (pos & 31));
   }
+  const unsigned same = __match_any_sync(0xffffffffu, in ? slot : kTraceSlots);
+  const int rank = __popc(same & ((1u << lane) - 1u));
+  if (in && rank == 0) reinterpret_cast<int*>(&sm.hist[slot])[warp] = __popc(same);
+  __syncthreads();
+  if (warp == 0) {  // exclusive prefix over (slot, warp), two slots per lane
+    const int4 a = sm.hist[2 * lane], b = sm.hist[2 * lane + 1];
+    const int sa = a.x + a.y + a.z + a.w, sb = b.x + b.y + b.z + b.w;
+    int run = sa + sb;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, run, o);
+      if (lane >= o) run += y;
+    }
+    const int e = run - sa - sb;
+    sm.start[2 * lane] = e;
+    sm.start[2 * lane + 1] = e + sa;
+    sm.hist[2 * lane] = make_int4(e, e + a.x, e + a.x + a.y, e + a.x + a.y + a.z);
+    const int f = e + sa;
+    sm.hist[2 * lane + 1] = make_int4(f, f + b.x, f + b.x + b.y, f + b.x + b.y + b.z);
+    if (lane == 31) sm.start[kTraceSlots] = run;
+  }
+  __syncthreads();
+  if (in) {  // the contribution row w x^q, at its place in cell order
+    const int place = reinterpret_cast<const int*>(&sm.hist[slot])[warp] + rank;
+    float4* dst = reinterpret_cast<float4*>(&sm.rows[place][0]);
+    float2 v = w;
+#pragma unroll
+    for (int q = 0; q < kTraceQ; q += 2) {
+      const float2 u = make_float2(v.x * x, v.y * x);
+      dst[q / 2] = make_float4(v.x, v.y, u.x, u.y);
+      v = make_float2(u.x * x, u.y * x);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kTraceSlots; i += kTraceThreads) sm.hist[i] = make_int4(0, 0, 0, 0);
+  const int q = threadIdx.x & (kTraceQ - 1);
+  for (int s = threadIdx.x / kTraceQ; s < kTraceSlots; s += kTraceThreads / kTraceQ) {
+    const int i0 = sm.start[s], i1 = sm.start[s + 1];
+    if (i0 == i1) continue;
+    float2 acc = sm.moments[s][q];
+#pragma unroll 4
+    for (int i = i0; i < i1; ++i) acc = fadd2(acc, sm.rows[i][q]);
+    sm.moments[s][q] = acc;
+  }
+  return __syncthreads_or(live && !in) != 0;
 }
 
 // A point and its contribution.
@@ -229,41 +226,136 @@ __device__ __forceinline__ bool trace_point(const TraceConsts& c, const float* t
   return true;
 }
 
-// All points of positions [begin, end) in batches of consecutive ones: for points
-// of which most are live (the pre-cull's list).  The next batch's points are loaded
+// A run's list of positions, filled 512 positions at a time and served in batches of 128.
+template <typename T, typename IndexOf, typename SigmaOf>
+struct TraceList {
+  TraceSmem& sm;
+  const TraceConsts& c;
+  const T* normals;
+  const T* points;
+  const float* txp;
+  const float* rxp;
+  IndexOf index_of;  // the point at a position, or -1 when it is out of bounds
+  SigmaOf sigma_of;
+  int listed = 0;
+  bool deferred = false;
+
+  // Lane l of warp w keeps position p0 + 128 j + 32 w + l where bit l of its mask[j] is set.
+  // The list's order is that of (warp, j, lane): the same on every run.
+  __device__ __forceinline__ void append(int p0, const unsigned (&mask)[kTracePer]) {
+    static_assert(kTracePer == 4, "one 16-byte load per warp's counts");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) {
+      *reinterpret_cast<int4*>(&sm.counts[warp * kTracePer]) =
+          make_int4(__popc(mask[0]), __popc(mask[1]), __popc(mask[2]), __popc(mask[3]));
+    }
+    __syncthreads();
+    int before = listed;
+#pragma unroll
+    for (int w = 0; w < kTraceWarps; ++w) {
+      const int4 n = *reinterpret_cast<const int4*>(&sm.counts[w * kTracePer]);
+      if (w == warp) {
+        const int at[kTracePer] = {before, before + n.x, before + n.x + n.y, before + n.x + n.y + n.z};
+#pragma unroll
+        for (int j = 0; j < kTracePer; ++j) {
+          if ((mask[j] >> lane) & 1u) {
+            sm.list[at[j] + __popc(mask[j] & ((1u << lane) - 1u))] = p0 + j * kTraceThreads + static_cast<int>(threadIdx.x);
+          }
+        }
+      }
+      before += n.x + n.y + n.z + n.w;
+    }
+    listed = before;
+  }
+
+  // The full batches, or all of the list (after a barrier that follows append).
+  __device__ __forceinline__ void serve(bool drain) {
+    while (listed >= kTraceThreads || (drain && listed > 0)) {
+      const int cnt = min(listed, kTraceThreads);
+      listed -= cnt;
+      bool live = false;
+      float2 w = make_float2(0.0f, 0.0f);
+      float x = 0.0f;
+      int cell = 0, pos = 0;
+      if (threadIdx.x < cnt) {
+        pos = sm.list[listed + threadIdx.x];
+        const int64_t q = index_of(pos);
+        TracePoint t;
+        load_point(normals, points, q, t.nrm, t.pt);
+        t.sigma = sigma_of(q);
+        live = trace_point(c, txp, rxp, t, w, cell, x);
+      }
+      if (trace_batch(sm, live, w, cell, x, pos)) deferred = true;
+    }
+  }
+
+  // Passes over the deferred positions until none is left.
+  __device__ __forceinline__ void serve_deferred(int count, float2* row) {
+    while (deferred) {
+      deferred = false;
+      trace_evict(sm, c, row);
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+      for (int p0 = 0; p0 < count; p0 += kTraceThreads * kTracePer) {
+        unsigned mask[kTracePer];
+#pragma unroll
+        for (int j = 0; j < kTracePer; ++j) {
+          const int word = (p0 >> 5) + j * kTraceWarps + warp;
+          mask[j] = word < kTraceRun / 32 ? sm.defer[word] : 0u;
+          __syncwarp();
+          if (lane == 0 && mask[j] != 0u) sm.defer[word] = 0u;
+        }
+        append(p0, mask);
+        __syncthreads();
+        serve(p0 + kTraceThreads * kTracePer >= count);
+      }
+    }
+  }
+};
+
+template <typename T, typename IndexOf, typename SigmaOf>
+__device__ __forceinline__ TraceList<T, IndexOf, SigmaOf> trace_list(TraceSmem& sm, const TraceConsts& c, const T* normals,
+                                                                     const T* points, const float* txp, const float* rxp,
+                                                                     IndexOf index_of, SigmaOf sigma_of) {
+  return TraceList<T, IndexOf, SigmaOf>{sm, c, normals, points, txp, rxp, index_of, sigma_of};
+}
+
+// `count` positions, at most kTraceRun, in batches of consecutive ones: for points of
+// which most are live (the pre-cull's list).  The next batch's points are loaded
 // while one is summed.
 template <typename T, typename IndexOf, typename SigmaOf>
 __device__ __forceinline__ void trace_all(TraceSmem& sm, const TraceConsts& c, float2* row, const T* normals,
-                                          const T* points, const float* txp, const float* rxp, int64_t begin,
-                                          int64_t end, IndexOf index_of, SigmaOf sigma_of) {
+                                          const T* points, const float* txp, const float* rxp, int count,
+                                          IndexOf index_of, SigmaOf sigma_of) {
+  auto list = trace_list<T>(sm, c, normals, points, txp, rxp, index_of, sigma_of);
   TracePoint next;
   int64_t next_q = -1;
-  auto load = [&](int64_t k) {
-    next_q = k < end ? index_of(k) : -1;
+  auto load = [&](int pos) {
+    next_q = pos < count ? index_of(pos) : -1;
     if (next_q >= 0) {
       load_point(normals, points, next_q, next.nrm, next.pt);
       next.sigma = sigma_of(next_q);
     }
   };
-  load(begin + threadIdx.x);
-  for (int64_t p0 = begin; p0 < end; p0 += kTraceThreads) {
+  load(threadIdx.x);
+  for (int p0 = 0; p0 < count; p0 += kTraceThreads) {
     float2 w = make_float2(0.0f, 0.0f);
     float x = 0.0f;
     int cell = 0;
     const bool live = next_q >= 0 && trace_point(c, txp, rxp, next, w, cell, x);
     load(p0 + kTraceThreads + threadIdx.x);
-    trace_batch(sm, c, row, live, w, cell, x);
+    if (trace_batch(sm, live, w, cell, x, p0 + threadIdx.x)) list.deferred = true;
   }
+  list.serve_deferred(count, row);
 }
 
-// `count` consecutive points (their arrays from the first one on; inb may be null),
-// screened first.
+// `count` consecutive points, at most kTraceRun (their arrays from the first one on;
+// inb may be null), screened first.
 template <typename T>
 __device__ __forceinline__ void trace_screened(TraceSmem& sm, const TraceConsts& c, float2* row, const T* normals,
                                                const T* points, const T* sigmas, const uint8_t* inb, const float* txp,
                                                const float* rxp, int count) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int listed = 0;
+  auto list = trace_list<T>(sm, c, normals, points, txp, rxp, [](int pos) { return pos; },
+                            [=](int64_t q) { return ld_f(sigmas, q); });
   float nrm[kTracePer][3], pt[kTracePer][3];
   unsigned in = 0;  // bit j: point j of the thread is in bounds
   auto load = [&](int p0) {  // of the next pass, in flight while batches are summed
@@ -285,49 +377,14 @@ __device__ __forceinline__ void trace_screened(TraceSmem& sm, const TraceConsts&
     unsigned mask[kTracePer];
 #pragma unroll
     for (int j = 0; j < kTracePer; ++j) {
-      const bool keep = ((in >> j) & 1u) && !surely_culled(txp, rxp, nrm[j], pt[j]);
-      mask[j] = __ballot_sync(0xffffffffu, keep);
-      if (lane == 0) sm.counts[warp * kTracePer + j] = __popc(mask[j]);
+      mask[j] = __ballot_sync(0xffffffffu, ((in >> j) & 1u) && !surely_culled(txp, rxp, nrm[j], pt[j]));
     }
-    __syncthreads();
-    // the list's order is that of (warp, pass, lane): the same on every run
-    int before = listed;
-#pragma unroll
-    for (int w = 0; w < kTraceWarps; ++w) {
-      static_assert(kTracePer == 4, "one 16-byte load per warp's counts");
-      const int4 n = *reinterpret_cast<const int4*>(&sm.counts[w * kTracePer]);
-      if (w == warp) {
-        const int at[kTracePer] = {before, before + n.x, before + n.x + n.y, before + n.x + n.y + n.z};
-#pragma unroll
-        for (int j = 0; j < kTracePer; ++j) {
-          if ((mask[j] >> lane) & 1u) {
-            sm.list[at[j] + __popc(mask[j] & ((1u << lane) - 1u))] = p0 + j * kTraceThreads + static_cast<int>(threadIdx.x);
-          }
-        }
-      }
-      before += n.x + n.y + n.z + n.w;
-    }
-    listed = before;
+    list.append(p0, mask);
     load(p0 + kTraceThreads * kTracePer);
     __syncthreads();
-    const bool last = p0 + kTraceThreads * kTracePer >= count;
-    while (listed >= kTraceThreads || (last && listed > 0)) {
-      const int cnt = min(listed, kTraceThreads);
-      listed -= cnt;
-      bool live = false;
-      float2 w = make_float2(0.0f, 0.0f);
-      float x = 0.0f;
-      int cell = 0;
-      if (threadIdx.x < cnt) {
-        const int64_t q = sm.list[listed + threadIdx.x];
-        TracePoint t;
-        load_point(normals, points, q, t.nrm, t.pt);
-        t.sigma = ld_f(sigmas, q);
-        live = trace_point(c, txp, rxp, t, w, cell, x);
-      }
-      trace_batch(sm, c, row, live, w, cell, x);
-    }
+    list.serve(p0 + kTraceThreads * kTracePer >= count);
   }
+  list.serve_deferred(count, row);
 }
 
 __device__ __forceinline__ void trace_store(const TraceSmem& sm, TraceRecord* rec) {
@@ -340,7 +397,7 @@ __device__ __forceinline__ void trace_store(const TraceSmem& sm, TraceRecord* re
   __syncthreads();
 }
 
-// Samples of one antenna from its runs' records, 256 threads.  Per slot the cells
+// Samples of one antenna from its runs' records, kFinishThreads threads.  Per slot the cells
 // are taken in ascending order, one per round (one round, unless runs of the
 // antenna lie more than kTraceSlots cells apart); the runs' moments are added in run order.
 constexpr int kFinishThreads = 256;

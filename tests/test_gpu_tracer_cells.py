@@ -1,0 +1,98 @@
+"""The MIXED and NUFFT tracers through range cells against the FP64 oracle, where
+their special paths are: scenes whose cells share slots (deferred points), bands
+that leave the adjoint's tables, runs of points longer than a pass, remainders.
+
+Tolerance: FP32 geometry (~5e-7), phases good to 1e-7 cycles, hardware sine and
+cosine (4e-7) and FP32 sums, with the positions' gradient a difference of terms ten
+times its size: 2e-5."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import rel_l2
+from benchkit import scenes
+from gpu_helpers import cu, tracer_backward, tracer_forward
+from oracle import rf_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+TOL = 2e-5
+
+
+def case(seed, A, P, S, depth=(0.3, 0.5), bandwidth=4e9):
+    """Points of a slab facing the array, most of the pairs live."""
+    rng = np.random.default_rng(seed)
+    tx, rx = scenes.virtual_array(4)
+    tx, rx = tx[:A], rx[:A]
+    pts = np.stack([rng.uniform(-0.2, 0.2, P), rng.uniform(-0.2, 0.2, P), rng.uniform(*depth, P)], 1)
+    nrm = -pts / np.linalg.norm(pts, axis=1, keepdims=True) + rng.normal(0, 0.15, (P, 3))
+    nrm /= np.linalg.norm(nrm, axis=1, keepdims=True)
+    ch = scenes.chirp(S, bandwidth=bandwidth)
+    f = np.float32
+    return dict(normals=nrm.astype(f), sigmas=rng.uniform(0, 1, (A, P)).astype(f), points=pts.astype(f),
+                tx=tx.astype(f), rx=rx.astype(f), inbounds=rng.uniform(0, 1, P) < 0.9, fs=f(ch.adc_sample_rate),
+                f0=f(770.0), As=f(ch.As_sci), S=S, rng=rng)
+
+
+def check(c, precision, tuning=None):
+    scal = float(c["fs"]), float(c["f0"]), float(c["As"])
+    geo = (c["normals"], c["sigmas"], c["points"], c["tx"], c["rx"], c["inbounds"])
+    x = tracer_forward(c, c["S"], precision, tuning=tuning)
+    r = orc.tracer_forward(*geo, c["S"], *scal, "f64")
+    assert rel_l2(x[0] + 1j * x[1], r[0] + 1j * r[1]) < TOL
+    A = c["tx"].shape[0]
+    gr, gi = c["rng"].standard_normal((2, A, c["S"])).astype(np.float32)
+    got = tracer_backward(c, gr, gi, precision, tuning=tuning)
+    ref = orc.tracer_backward(gr, gi, *geo, *scal)
+    for g, w in zip(got, ref):
+        assert rel_l2(g, w) < TOL
+
+
+@pytest.mark.parametrize("precision", ["mixed", "nufft"])
+@pytest.mark.parametrize("A,P,S", [(1, 129, 32), (33, 1024, 33), (12, 5003, 101), (70, 700, 256), (3, 40001, 64)])
+def test_shapes(cuda, A, P, S, precision):
+    check(case(A + S, A, P, S), precision)
+
+
+@pytest.mark.parametrize("depth,bandwidth", [((0.3, 3.3), 4e9),   # cells up to 160 apart: several passes over a run
+                                             ((0.3, 6.0), 4e9),   # and a band outside the adjoint's tables
+                                             ((0.3, 0.5), 60e9)], # the same by a wide sweep
+                         ids=["deep", "deeper", "wide_sweep"])
+@pytest.mark.parametrize("splits", [0, 1])
+def test_cells_that_share_slots(cuda, depth, bandwidth, splits):
+    check(case(4, 7, 3000, 128, depth, bandwidth), "mixed", {"splits": splits})
+
+
+def test_runs_longer_than_a_pass(cuda):
+    check(case(5, 2, 40001, 48), "mixed", {"splits": 1})
+
+
+@pytest.mark.parametrize("depth", [(0.3, 0.5), (0.3, 3.3)], ids=["near", "deep"])
+def test_ragged_runs(cuda, depth):
+    """Long work items (several passes each), antennas of 1 to 33000 points, against the tracer
+    over each antenna's points alone."""
+    from geraf_b200.ops.RFSignalTracer.ragged import signal_tracer_ragged
+
+    c = case(6, 4, 36000, 64, depth)
+    counts = [1, 33000, 511, 2488]
+    off = np.concatenate([[0], np.cumsum(counts)])
+    sig = c["sigmas"][0]
+    t = {k: cu(v).requires_grad_(True) for k, v in (("normals", c["normals"]), ("points", c["points"]), ("sigmas", sig))}
+    xr, xi = signal_tracer_ragged(t["normals"], t["sigmas"], t["points"], torch.tensor(off, device="cuda"), cu(c["tx"]),
+                                  cu(c["rx"]), c["S"], float(c["fs"]), float(c["f0"]), float(c["As"]),
+                                  inbounds=torch.tensor(c["inbounds"], device="cuda"), tuning={"items_per_thread": 512})
+    gr, gi = c["rng"].standard_normal((2, 4, c["S"])).astype(np.float32)
+    gn, gs, gp = torch.autograd.grad((xr, xi), (t["normals"], t["sigmas"], t["points"]), (cu(gr), cu(gi)))
+    x = xr.detach().cpu().numpy() + 1j * xi.detach().cpu().numpy()
+    pairs = [], [], []  # every pair's gradients, without its antenna's 1 / points: (got, reference)
+    for a in range(4):
+        e = slice(off[a], off[a + 1])
+        args = (c["normals"][e], sig[None, e], c["points"][e], c["tx"][a:a + 1], c["rx"][a:a + 1], c["inbounds"][e])
+        scal = float(c["fs"]), float(c["f0"]), float(c["As"])
+        r = orc.tracer_forward(*args, c["S"], *scal, "f64")
+        assert rel_l2(x[a], (r[0] + 1j * r[1])[0]) < TOL
+        rn, rs, rp = orc.tracer_backward(gr[a:a + 1], gi[a:a + 1], *args, *scal)
+        for k, (got, ref) in enumerate(((gn, rn), (gs, rs[0]), (gp, rp))):
+            pairs[k].append((counts[a] * got[e].double().cpu().numpy(), counts[a] * ref))
+    for p in pairs:
+        assert rel_l2(np.concatenate([g for g, _ in p]), np.concatenate([r for _, r in p])) < TOL
