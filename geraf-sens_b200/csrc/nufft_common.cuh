@@ -50,6 +50,13 @@ GlRule gauss_legendre(double b) {
   return r;
 }
 
+// The rule on [0, W/2], formed once per width (W even, at most 12).
+const GlRule& gauss_legendre_cached(int W) {
+  static const GlRule rules[5] = {gauss_legendre(2.0), gauss_legendre(3.0), gauss_legendre(4.0), gauss_legendre(5.0),
+                                  gauss_legendre(6.0)};
+  return rules[std::min(std::max(W / 2 - 2, 0), 4)];
+}
+
 // Interpolation weights.  For a point at grid coordinate u = base + W/2 - 1 + f
 // (f in [0, 1)), grid point base + k gets phi((f + W/2 - 1 - k) 2 / W).  Each
 // tap's weight is a polynomial of degree P in z = 2f - 1: the Chebyshev
@@ -108,6 +115,13 @@ EsPoly es_poly(int W, double beta) {
     for (int q = 0; q <= P; ++q) e.c[k][q] = static_cast<float>(mono[q]);
   }
   return e;
+}
+
+// The weights for beta = 2.30 W, formed once per width (W even, 4 to 12).
+const EsPoly& es_poly_cached(int W) {
+  static const EsPoly polys[5] = {es_poly(4, 2.30 * 4), es_poly(6, 2.30 * 6), es_poly(8, 2.30 * 8), es_poly(10, 2.30 * 10),
+                                  es_poly(12, 2.30 * 12)};
+  return polys[std::min(std::max(W / 2 - 2, 0), 4)];
 }
 
 template <int W>
@@ -302,7 +316,7 @@ cudaError_t launch_deconv(float* deconv, int64_t S, int h, int M, int W, double 
                           const int* run_if = nullptr) {
   DeconvP dp;
   dp.run_if = run_if;
-  dp.gl = gauss_legendre(0.5 * W);
+  dp.gl = gauss_legendre_cached(W);
   dp.deconv = deconv;
   dp.S = static_cast<int>(S);
   dp.h = h;

@@ -446,7 +446,7 @@ cudaError_t launch_nufft_backward(const MfArgs& a, const Tuning& t, void* ws, cu
   }
 
   SpreadP<T> sp;
-  sp.poly = es_poly(b.W, b.beta);
+  sp.poly = es_poly_cached(b.W);
   sp.tx = static_cast<const T*>(a.tx);
   sp.rx = static_cast<const T*>(a.rx);
   sp.voxel = static_cast<const T*>(a.voxel);
@@ -541,7 +541,7 @@ cudaError_t launch_nufft_forward(const MfArgs& a, const NufftShape& s, void* ws,
   }
 
   GatherP<T> p;
-  p.poly = es_poly(s.W, s.beta);
+  p.poly = es_poly_cached(s.W);
   p.g = grid;
   p.tx = static_cast<const T*>(a.tx);
   p.rx = static_cast<const T*>(a.rx);

@@ -497,7 +497,7 @@ cudaError_t launch_tracer_nufft_forward(const TracerArgs& a, const Tuning& t, vo
     if (err != cudaSuccess) return err;
   }
   TrSpreadP<T> sp;
-  sp.poly = es_poly(s.W, s.beta);
+  sp.poly = es_poly_cached(s.W);
   sp.normals = static_cast<const T*>(a.normals);
   sp.sigmas = static_cast<const T*>(a.sigmas);
   sp.points = static_cast<const T*>(a.points);
@@ -600,7 +600,7 @@ cudaError_t launch_tracer_nufft_backward(const TracerArgs& a, const Tuning& t, v
     }
   }
   TrGatherP<T> p;
-  p.poly = es_poly(s.W, s.beta);
+  p.poly = es_poly_cached(s.W);
   p.g1 = g1;
   p.g2 = with_points ? g2 : g1;  // without position gradients the second grid is never read
   p.normals = static_cast<const T*>(a.normals);

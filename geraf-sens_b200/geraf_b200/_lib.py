@@ -180,7 +180,9 @@ def check(rc: int, what: str) -> None:
 
 def call(name: str, *args) -> None:
     """Calls a status-returning entry point; raises GerafError on failure."""
-    check(getattr(load(), name)(*args), name)
+    rc = getattr(_lib or load(), name)(*args)
+    if rc != GERAF_OK:
+        check(rc, name)
 
 
 def workspace_bytes(name: str, *args) -> int:

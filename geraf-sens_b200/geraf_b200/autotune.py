@@ -48,6 +48,8 @@ def _maybe_load() -> None:
 
 
 def lookup(op: str, sizes: tuple, mode: int) -> dict | None:
+    if not _cache and _cache_file() is None:
+        return None
     with _lock:
         _maybe_load()
         return _cache.get(_key(op, sizes, mode))

@@ -20,6 +20,7 @@ from ... import _lib
 from ...runtime import (
     check_cuda_contig,
     check_same_dtype,
+    cuda_arrays,
     device_guard,
     dtype_code,
     mode_code,
@@ -50,6 +51,10 @@ def _check_common(real, imag, tx_pos, rx_pos, voxel):
 
 def _check_forward(real, imag, tx_pos, rx_pos, output_real, output_imag, voxel, A, S, N):
     # MatchedFilter_cuda.cu:39-69
+    if (cuda_arrays(real.dtype, real, imag, tx_pos, rx_pos, output_real, output_imag, voxel)
+            and real.shape == (A, S) == imag.shape and tx_pos.shape == (A, 3) == rx_pos.shape
+            and output_real.shape == (N,) == output_imag.shape and voxel.shape == (3, N)):
+        return
     _check_common(real, imag, tx_pos, rx_pos, voxel)
     torch_check(output_real.is_cuda, "`output_real` must be a CUDA tensor.")
     torch_check(output_imag.is_cuda, "`output_imag` must be a CUDA tensor.")
@@ -73,6 +78,11 @@ def _check_forward(real, imag, tx_pos, rx_pos, output_real, output_imag, voxel, 
 
 def _check_backward(gr, gi, real, imag, tx_pos, rx_pos, grad_real, grad_imag, voxel, A, S, N):
     # MatchedFilter_cuda.cu:71-107
+    if (cuda_arrays(real.dtype, real, imag, tx_pos, rx_pos, gr, gi, grad_real, grad_imag)
+            and real.shape == imag.shape and grad_real.shape == (A, S) == grad_imag.shape
+            and tx_pos.shape == (A, 3) == rx_pos.shape and gr.shape == (N,) == gi.shape and real.dim() == 2
+            and voxel.is_cuda and voxel.is_contiguous() and voxel.shape == (3, N) and voxel.dtype is real.dtype):
+        return
     _check_common(real, imag, tx_pos, rx_pos, voxel)
     for t, n in ((gr, "grad_output_real"), (gi, "grad_output_imag"), (grad_real, "grad_real"),
                  (grad_imag, "grad_imag")):

@@ -21,6 +21,7 @@ from ... import _lib
 from ...runtime import (
     check_cuda_contig,
     check_same_dtype,
+    cuda_arrays,
     device_guard,
     dtype_code,
     mode_code,
@@ -36,6 +37,11 @@ from ...runtime import (
 def _check_tracer(normals, sigmas, points, tx_pos, rx_pos, inbounds, output_real, output_imag,
                   S, A, P):
     # SignalTracer_cuda.cu:100-140
+    if (cuda_arrays(normals.dtype, normals, sigmas, points, tx_pos, rx_pos, output_real, output_imag)
+            and inbounds.dtype is torch.bool and inbounds.is_cuda and inbounds.is_contiguous()
+            and inbounds.shape == (P,) and normals.shape == (P, 3) == points.shape and sigmas.shape == (A, P)
+            and tx_pos.shape == (A, 3) == rx_pos.shape and output_real.shape == (A, S) == output_imag.shape):
+        return
     for t, n in ((normals, "normals"), (sigmas, "sigmas"), (points, "points"), (tx_pos, "tx_pos"),
                  (rx_pos, "rx_pos"), (inbounds, "inbounds"), (output_real, "output_real"),
                  (output_imag, "output_imag")):
@@ -82,17 +88,12 @@ def SignalTracer_forward(normals, sigmas, points, tx_pos, rx_pos, inbounds, outp
                   dt, mode, tuning_ref(tun), ptr(ws), nbytes, stream_ptr(normals.device))
 
 
-def SignalTracer_backward_normal_sigma(grad_output_real, grad_output_imag, normals, sigmas, points,
-                                       tx_pos, rx_pos, inbounds, grad_normals, grad_sigmas,
-                                       num_adc_samples, adc_sample_rate, start_frequency,
-                                       chirp_slope_scaled, total_ant_size, total_point_size, *,
-                                       grad_points=None, precision=None, tuning=None):
-    """Adjoint of :func:`SignalTracer_forward` into ``grad_normals`` [P,3], ``grad_sigmas``
-    [A,P] and, if given, ``grad_points`` [P,3]."""
-    S, A, P = int(num_adc_samples), int(total_ant_size), int(total_point_size)
-    # SignalTracer_cuda.cu:142-178: the forward checks with grad_output in the output slots.
-    _check_tracer(normals, sigmas, points, tx_pos, rx_pos, inbounds, grad_output_real,
-                  grad_output_imag, S, A, P)
+def _check_tracer_grads(normals, grad_normals, grad_sigmas, grad_points, A, P):
+    # SignalTracer_cuda.cu:142-178
+    if (cuda_arrays(normals.dtype, grad_normals, grad_sigmas, *(() if grad_points is None else (grad_points,)))
+            and grad_normals.shape == (P, 3) and grad_sigmas.shape == (A, P)
+            and (grad_points is None or grad_points.shape == (P, 3))):
+        return
     check_cuda_contig(grad_normals, "grad_normals")
     check_cuda_contig(grad_sigmas, "grad_sigmas")
     torch_check(grad_normals.dim() == 2 and grad_normals.size(1) == 3,
@@ -106,6 +107,20 @@ def SignalTracer_backward_normal_sigma(grad_output_real, grad_output_imag, norma
         torch_check(grad_points.dim() == 2 and grad_points.size(0) == P and grad_points.size(1) == 3,
                     "`grad_points` must have shape [P, 3].")
         check_same_dtype(normals, (grad_points, "grad_points"))
+
+
+def SignalTracer_backward_normal_sigma(grad_output_real, grad_output_imag, normals, sigmas, points,
+                                       tx_pos, rx_pos, inbounds, grad_normals, grad_sigmas,
+                                       num_adc_samples, adc_sample_rate, start_frequency,
+                                       chirp_slope_scaled, total_ant_size, total_point_size, *,
+                                       grad_points=None, precision=None, tuning=None):
+    """Adjoint of :func:`SignalTracer_forward` into ``grad_normals`` [P,3], ``grad_sigmas``
+    [A,P] and, if given, ``grad_points`` [P,3]."""
+    S, A, P = int(num_adc_samples), int(total_ant_size), int(total_point_size)
+    # SignalTracer_cuda.cu:142-178: the forward checks with grad_output in the output slots.
+    _check_tracer(normals, sigmas, points, tx_pos, rx_pos, inbounds, grad_output_real,
+                  grad_output_imag, S, A, P)
+    _check_tracer_grads(normals, grad_normals, grad_sigmas, grad_points, A, P)
     dt = dtype_code(grad_output_real, "signal_tracer_backward_normal_sigma_cuda", allow_half=False)
     mode = mode_code(precision, allow_nufft=True)
     tun = tuning_struct("tracer_backward", (A, S, P), mode, tuning)
@@ -123,6 +138,11 @@ def SignalTracer_backward_normal_sigma(grad_output_real, grad_output_imag, norma
 
 def _check_bilinear_fwd(normals, sigmas, z_vals, tz, out_n, out_s, out_inb, A, R, S, T):
     # SignalTracer_cuda.cu:15-57
+    if (cuda_arrays(normals.dtype, normals, sigmas, z_vals, tz, out_n, out_s) and out_inb.dtype is torch.bool
+            and out_inb.is_cuda and out_inb.is_contiguous() and normals.shape == (R, S, 3)
+            and sigmas.shape == (A, R, S) and z_vals.shape == (R, S) and tz.shape == (R, T) == out_inb.shape
+            and out_n.shape == (R, T, 3) and out_s.shape == (A, R, T)):
+        return
     for t, n in ((normals, "normals"), (sigmas, "sigmas"), (z_vals, "z_vals"), (tz, "target_z_vals"),
                  (out_n, "output_normals"), (out_s, "output_sigmas"), (out_inb, "output_inbounds")):
         check_cuda_contig(t, n)
@@ -159,12 +179,15 @@ def BilinearRaysample_forward(normals, sigmas, z_vals, target_z_vals, output_nor
                   ptr(output_inbounds), A, R, S, T, dt, stream_ptr(normals.device))
 
 
-def BilinearRaysample_backward(grad_output_normals, grad_output_sigmas, z_vals, target_z_vals,
-                               grad_normals, grad_sigmas, num_antennas, num_rays, num_samples,
-                               num_target_samples):
-    """Adjoint of the resampler; ADDS into ``grad_normals`` [R,S,3] and ``grad_sigmas`` [A,R,S]."""
-    A, R, S, T = int(num_antennas), int(num_rays), int(num_samples), int(num_target_samples)
+def _check_bilinear_bwd(grad_output_normals, grad_output_sigmas, z_vals, target_z_vals, grad_normals, grad_sigmas,
+                        A, R, S, T):
     # SignalTracer_cuda.cu:59-98
+    if (cuda_arrays(grad_output_normals.dtype, grad_output_normals, grad_output_sigmas, z_vals, target_z_vals,
+                    grad_normals, grad_sigmas)
+            and grad_output_normals.shape == (R, T, 3) and grad_output_sigmas.shape == (A, R, T)
+            and z_vals.shape == (R, S) and target_z_vals.shape == (R, T) and grad_normals.shape == (R, S, 3)
+            and grad_sigmas.shape == (A, R, S)):
+        return
     for t, n in ((grad_output_normals, "grad_output_normals"),
                  (grad_output_sigmas, "grad_output_sigmas"), (z_vals, "z_vals"),
                  (target_z_vals, "target_z_vals"), (grad_normals, "grad_normals"),
@@ -183,6 +206,15 @@ def BilinearRaysample_backward(grad_output_normals, grad_output_sigmas, z_vals, 
     check_same_dtype(grad_output_normals, (grad_output_sigmas, "grad_output_sigmas"),
                      (z_vals, "z_vals"), (target_z_vals, "target_z_vals"),
                      (grad_normals, "grad_normals"), (grad_sigmas, "grad_sigmas"))
+
+
+def BilinearRaysample_backward(grad_output_normals, grad_output_sigmas, z_vals, target_z_vals,
+                               grad_normals, grad_sigmas, num_antennas, num_rays, num_samples,
+                               num_target_samples):
+    """Adjoint of the resampler; ADDS into ``grad_normals`` [R,S,3] and ``grad_sigmas`` [A,R,S]."""
+    A, R, S, T = int(num_antennas), int(num_rays), int(num_samples), int(num_target_samples)
+    _check_bilinear_bwd(grad_output_normals, grad_output_sigmas, z_vals, target_z_vals, grad_normals, grad_sigmas,
+                        A, R, S, T)
     dt = dtype_code(grad_output_normals, "bilinear_raysample_backward_cuda", allow_half=False)
     with device_guard(grad_output_normals.device):
         _lib.call("geraf_bilinear_backward", ptr(grad_output_normals), ptr(grad_output_sigmas),

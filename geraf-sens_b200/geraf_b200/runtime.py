@@ -100,13 +100,28 @@ def check_same_dtype(ref: torch.Tensor, *named: tuple[torch.Tensor, str]) -> Non
         torch_check(t.dtype == ref.dtype, f"`{name}` must have dtype {ref.dtype}, got {t.dtype}.")
 
 
+def cuda_arrays(dtype: torch.dtype, *tensors: torch.Tensor) -> bool:
+    """True when every tensor is a contiguous CUDA tensor of ``dtype``: the common case, found
+    without naming the argument that fails (the checks above do that when it is False)."""
+    for t in tensors:
+        if t.dtype is not dtype or not t.is_cuda or not t.is_contiguous():
+            return False
+    return True
+
+
 def ptr(t: torch.Tensor | None) -> int | None:
     if t is None or t.numel() == 0:
         return None
     return t.data_ptr()
 
 
+# The current stream's handle without a Stream object, where this torch offers it.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream_ptr(device: torch.device) -> int:
+    if _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)
     return torch.cuda.current_stream(device).cuda_stream
 
 
@@ -135,12 +150,16 @@ def tuning_ref(t: _lib.Tuning | None):
 class device_guard:
     """Makes ``device`` current for the call (the reference's CUDAGuard)."""
 
+    __slots__ = ("_ctx",)
+
     def __init__(self, device: torch.device):
-        self._ctx = torch.cuda.device(device)
+        current = device.index is not None and torch.cuda.current_device() == device.index
+        self._ctx = None if current else torch.cuda.device(device)
 
     def __enter__(self):
-        self._ctx.__enter__()
+        if self._ctx is not None:
+            self._ctx.__enter__()
         return self
 
     def __exit__(self, *exc):
-        return self._ctx.__exit__(*exc)
+        return self._ctx.__exit__(*exc) if self._ctx is not None else None
