@@ -207,6 +207,31 @@ PhaseConsts phase_consts(float f0, float As, float fs) {
   return pc;
 }
 
+int resident_blocks(const void* fn, int threads, size_t smem) {
+  struct Entry {
+    int dev, threads;
+    const void* fn;
+    size_t smem;
+    int blocks;
+  };
+  // a handful of kernels and shapes; each calling thread keeps its own answers
+  static thread_local Entry entries[16];
+  static thread_local unsigned used = 0;
+  const int dev = current_device();
+  for (unsigned i = 0; i < std::min(used, 16u); ++i) {
+    const Entry& e = entries[i];
+    if (e.dev == dev && e.fn == fn && e.threads == threads && e.smem == smem) return e.blocks;
+  }
+  int n = 0;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, smem) != cudaSuccess || n <= 0) {
+    cudaGetLastError();
+    return 0;
+  }
+  entries[used++ % 16u] = Entry{dev, threads, fn, smem, n};
+  return n;
+}
+
 int pick_splits(int64_t units, int blocks_per_sm, int sm_count, int64_t max_splits) {
   const double slots = static_cast<double>(blocks_per_sm) * sm_count;
   if (units <= 0 || max_splits <= 1) return 1;
@@ -214,6 +239,8 @@ int pick_splits(int64_t units, int blocks_per_sm, int sm_count, int64_t max_spli
   int best = 1;
   double best_score = -1.0;
   const int limit = static_cast<int>(std::min<int64_t>(max_splits, 256));
+  // too little work for one wave: as many blocks as there can be
+  if (static_cast<double>(units) * limit < slots) return limit;
   for (int s = 1; s <= limit; ++s) {
     const double blocks = static_cast<double>(units) * s;
     const double waves = blocks / slots;

@@ -251,6 +251,10 @@ struct PhaseConsts {
 };
 PhaseConsts phase_consts(float f0, float As, float fs);
 
+// Resident blocks per SM of a kernel at this block size and dynamic shared memory (its limit raised
+// to that), remembered per device; 0 when no device answers.
+int resident_blocks(const void* fn, int threads, size_t smem);
+
 // Picks the number of splits of the reduced dimension so that
 // `units * splits` blocks fill the GPU in near-whole waves.
 int pick_splits(int64_t units, int blocks_per_sm, int sm_count, int64_t max_splits);

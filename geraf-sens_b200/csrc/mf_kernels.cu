@@ -385,6 +385,121 @@ __global__ void __launch_bounds__(256) mf_fwd_plain_kernel(const MfFwdP<T> p) {
   }
 }
 
+// Exchange of a PLAIN kernel's terms among the LANES lanes that share an output: each
+// lane stores its two terms, then the even lanes add the 2 LANES real parts in order
+// and the odd lanes the imaginary parts, through shared memory (16-byte loads, rows
+// padded to stay off each other's banks).  Every lane adding both parts took 40% longer
+// over all, and so did shuffles.
+template <int LANES>
+struct TermRows {
+  static constexpr int kTerms = 2 * LANES;
+  float row[2][32 / LANES][kTerms + 4];
+};
+
+// acc: the lane's component.
+template <int LANES>
+__device__ __forceinline__ void add_terms(TermRows<LANES>& x, const float (&term_r)[2], const float (&term_i)[2], int count,
+                                          float& acc) {
+  const int out = (threadIdx.x & 31) / LANES;
+  const int lane = threadIdx.x % LANES;
+  __syncwarp();
+  x.row[0][out][lane] = term_r[0];
+  x.row[1][out][lane] = term_i[0];
+  x.row[0][out][LANES + lane] = term_r[1];
+  x.row[1][out][LANES + lane] = term_i[1];
+  __syncwarp();
+  const float* row = x.row[lane & 1][out];
+  if (count >= 2 * LANES) {
+#pragma unroll
+    for (int k = 0; k < 2 * LANES; k += 4) {
+      const float4 t = *reinterpret_cast<const float4*>(&row[k]);
+      acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, t.x), t.y), t.z), t.w);
+    }
+  } else {
+    for (int k = 0; k < count; ++k) acc = __fadd_rn(acc, row[k]);
+  }
+}
+
+// PLAIN forward with LANES lanes per voxel, for calls of too few voxels to fill the GPU
+// with one thread each (every thread is bound by the latency of its sines and
+// cosines: 13824 voxels x 300 antennas x 128 samples take 3.70 ms at one thread per
+// voxel, 1.26 ms at 8).  Lane j evaluates samples j, j + LANES, ...; every lane then adds
+// the LANES terms in sample order, so the sums are the one-thread kernel's to the bit.
+template <typename T, int LANES>
+__global__ void __launch_bounds__(128) mf_fwd_plain_lanes_kernel(const MfFwdP<T> p) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(16) TermRows<LANES> terms[4];
+  uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
+  float* pos = reinterpret_cast<float*>(smem + p.pos_off);
+  float* kn = reinterpret_cast<float*>(smem + p.kn_off);
+  PairStager<T> stg{reinterpret_cast<T*>(smem + p.buf_off), bar, p.ld, p.rows, p.bulk != 0};
+  const int ntiles = p.A > 0 ? ceil_div(p.A, p.rows) : 0;
+  const int S = static_cast<int>(p.S);
+  if (p.bulk && threadIdx.x == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    fence_barrier_init();
+  }
+  for (int n = threadIdx.x; n < p.ld; n += blockDim.x) {
+    const float sample_time = static_cast<float>(n) / p.fs;
+    kn[n] = 2.0f * kPiF * p.As * sample_time;
+  }
+  __syncthreads();
+  const int lane = threadIdx.x % LANES;
+  const int64_t v = blockIdx.x * static_cast<int64_t>(blockDim.x / LANES) + threadIdx.x / LANES;
+  const bool ok = v < p.N;
+  const float vx = ok ? ld_f(p.voxel, v) : 0.0f;
+  const float vy = ok ? ld_f(p.voxel, p.N + v) : 0.0f;
+  const float vz = ok ? ld_f(p.voxel, 2 * p.N + v) : 0.0f;
+  float acc = 0.0f;
+  auto issue = [&](int tile, int stage) {
+    const int64_t a0 = static_cast<int64_t>(tile) * p.rows;
+    const int rws = static_cast<int>(min(static_cast<int64_t>(p.rows), p.A - a0));
+    stg.issue(stage, p.real, p.imag, a0, rws, S);
+    stage_positions<T, float>(pos, stage, p.rows, p.tx, p.rx, a0, rws);
+  };
+  if (ntiles > 0) issue(0, 0);
+  if (ntiles > 1) issue(1, 1);
+  for (int t = 0; t < ntiles; ++t) {
+    const int s = t & 1;
+    if (!stg.wait(s, (t >> 1) & 1, p.status)) {
+      if (t + 1 < ntiles) stg.drain(s ^ 1, ((t + 1) >> 1) & 1, p.status);
+      return;
+    }
+    const int rws = static_cast<int>(min(static_cast<int64_t>(p.rows), p.A - static_cast<int64_t>(t) * p.rows));
+    for (int r = 0; r < rws; ++r) {
+      const float* ps = pos + (s * p.rows + r) * 6;
+      const float tx_distance = sqrtf(sq(ps[0] - vx) + sq(ps[1] - vy) + sq(ps[2] - vz));
+      const float rx_distance = sqrtf(sq(ps[3] - vx) + sq(ps[4] - vy) + sq(ps[5] - vz));
+      const float distance = tx_distance + rx_distance + kPathBias;
+      const float tau = distance / kSpeedOfLight;
+      const float base_phase = 2.0f * kPiF * kMfStartFrequency * tau;
+      const T* rowr = stg.stage_ptr(s, 0) + r * p.ld;
+      const T* rowi = stg.stage_ptr(s, 1) + r * p.ld;
+      // two groups of LANES samples at a time, whose sines and cosines overlap
+      for (int n0 = 0; n0 < S; n0 += 2 * LANES) {
+        float term_r[2], term_i[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int n = min(n0 + u * LANES + lane, S - 1);
+          const float phase = base_phase + kn[n] * tau;
+          float cos_phase, sin_phase;
+          cos_sin(phase, &cos_phase, &sin_phase);
+          const float neg_sin_phase = -sin_phase;
+          const float sample_real = static_cast<float>(rowr[n]);
+          const float sample_imag = static_cast<float>(rowi[n]);
+          term_r[u] = cos_phase * sample_real - neg_sin_phase * sample_imag;
+          term_i[u] = cos_phase * sample_imag + neg_sin_phase * sample_real;
+        }
+        add_terms<LANES>(terms[threadIdx.x >> 5], term_r, term_i, S - n0, acc);
+      }
+    }
+    __syncthreads();
+    if (t + 2 < ntiles) issue(t + 2, s);
+  }
+  if (ok && lane < 2) (lane == 0 ? p.out_r : p.out_i)[v] = from_f<T>(acc / static_cast<int>(p.A));
+}
+
 // Sums `splits` partial rows of `count` complex values in a fixed order (FP64)
 // and divides by `divisor`.
 template <typename T>
@@ -520,12 +635,18 @@ __global__ void __launch_bounds__(256) mf_bwd_mixed_kernel(const MfBwdP<T> p) {
 // PLAIN adjoint: thread = (antenna, sample), voxels in the reference's order
 // (MatchedFilter_cuda_kernel.cu:186-219).  Per-(a, v) path delays are formed
 // once per voxel tile in shared memory.
-template <typename T>
+// LANES lanes per sample, for calls of few antennas x samples: lane j evaluates voxels j,
+// j + LANES, ... and every lane adds the LANES terms in voxel order, so the sums do
+// not depend on LANES (300 antennas x 128 samples x 13824 voxels: 1.71 ms with one lane,
+// 1.27 ms with 4).
+template <typename T, int LANES>
 __global__ void __launch_bounds__(128) mf_bwd_plain_kernel(const MfBwdP<T> p) {
   constexpr int TILE = 256;
   __shared__ float s_tau[TILE], s_gr[TILE], s_gi[TILE];
+  __shared__ __align__(16) TermRows<LANES> terms[LANES == 1 ? 1 : 4];
   const int64_t a = blockIdx.x;
-  const int64_t n = static_cast<int64_t>(blockIdx.y) * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x % LANES;
+  const int64_t n = static_cast<int64_t>(blockIdx.y) * (blockDim.x / LANES) + threadIdx.x / LANES;
   const bool active = n < p.S;
   const float tx_x = ld_f(p.tx, a * 3 + 0), tx_y = ld_f(p.tx, a * 3 + 1), tx_z = ld_f(p.tx, a * 3 + 2);
   const float rx_x = ld_f(p.rx, a * 3 + 0), rx_y = ld_f(p.rx, a * 3 + 1), rx_z = ld_f(p.rx, a * 3 + 2);
@@ -545,8 +666,13 @@ __global__ void __launch_bounds__(128) mf_bwd_plain_kernel(const MfBwdP<T> p) {
       s_gi[i] = ld_f(p.gi, v);
     }
     __syncthreads();
-    if (active) {
-      for (int i = 0; i < count; ++i) {
+    // Samples past S run along (the lanes of a warp exchange their terms) and are not
+    // stored.  Two groups of LANES voxels at a time, whose sines and cosines overlap.
+    for (int i0 = 0; i0 < count; i0 += 2 * LANES) {
+      float term_r[2], term_i[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int i = min(i0 + u * LANES + lane, count - 1);
         const float tau = s_tau[i];
         const float phase = 2.0f * kPiF * kMfStartFrequency * tau + kn * tau;
         float cos_phase, sin_phase;
@@ -556,16 +682,28 @@ __global__ void __launch_bounds__(128) mf_bwd_plain_kernel(const MfBwdP<T> p) {
         const float grad_imag_out = s_gi[i];
         // The reference's expressions with the FMA contraction its build makes
         // (identified against its outputs): the cos product is fused in both.
-        acc_r = __fadd_rn(acc_r, __fmaf_rn(cos_phase, grad_real_out, __fmul_rn(neg_sin_phase, grad_imag_out)));
-        acc_i = __fadd_rn(acc_i, __fmaf_rn(cos_phase, grad_imag_out, __fmul_rn(sin_phase, grad_real_out)));
+        term_r[u] = __fmaf_rn(cos_phase, grad_real_out, __fmul_rn(neg_sin_phase, grad_imag_out));
+        term_i[u] = __fmaf_rn(cos_phase, grad_imag_out, __fmul_rn(sin_phase, grad_real_out));
+      }
+      if (LANES == 1) {
+        acc_r = __fadd_rn(acc_r, term_r[0]);
+        acc_i = __fadd_rn(acc_i, term_i[0]);
+        if (i0 + 1 < count) {
+          acc_r = __fadd_rn(acc_r, term_r[1]);
+          acc_i = __fadd_rn(acc_i, term_i[1]);
+        }
+      } else {
+        add_terms<LANES>(terms[threadIdx.x >> 5], term_r, term_i, count - i0, acc_r);
       }
     }
     __syncthreads();
   }
-  if (active) {
-    const int total_ant_size = static_cast<int>(p.A);
+  const int total_ant_size = static_cast<int>(p.A);
+  if (LANES == 1 && active) {
     p.out_r[a * p.S + n] = from_f<T>(acc_r / total_ant_size);
     p.out_i[a * p.S + n] = from_f<T>(acc_i / total_ant_size);
+  } else if (active && lane < 2) {  // acc_r is the lane's component
+    (lane == 0 ? p.out_r : p.out_i)[a * p.S + n] = from_f<T>(acc_r / total_ant_size);
   }
 }
 
@@ -743,6 +881,15 @@ FwdShape fwd_shape(const MfArgs& a, const Tuning& t) {
   return s;
 }
 
+// Lanes that share one output of a PLAIN kernel: one where that fills the GPU with 1024
+// threads per SM (about half of what the sines and cosines need to hide their
+// latency), else 4, or 8 where 4 leave less than 768 per SM.
+int plain_lanes(int64_t outputs, int64_t terms) {
+  const int64_t sms = current_device_info().sm_count;
+  if (outputs >= sms * 1024 || terms < 32) return 1;
+  return outputs * 4 >= sms * 768 ? 4 : 8;
+}
+
 template <typename T>
 cudaError_t launch_fwd(const MfArgs& a, const FwdShape& s, void* ws, cudaStream_t st, const int* run_if) {
   MfFwdP<T> p;
@@ -777,9 +924,19 @@ cudaError_t launch_fwd(const MfArgs& a, const FwdShape& s, void* ws, cudaStream_
   p.dup_off = s.layout.dup_off;
 
   const void* fn = fwd_kernel_ptr<T>(a.mode, s.vpt);
+  const int lanes = a.mode == kPlain && s.splits == 1 ? plain_lanes(a.N, a.S) : 1;
+  if (lanes > 1) {
+    fn = lanes == 4 ? reinterpret_cast<const void*>(&mf_fwd_plain_lanes_kernel<T, 4>)
+                    : reinterpret_cast<const void*>(&mf_fwd_plain_lanes_kernel<T, 8>);
+  }
   cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(s.smem));
   if (err != cudaSuccess) return err;
+  if (lanes > 1) {
+    const int per_block = 128 / lanes;
+    void* args[] = {&p};
+    return cudaLaunchKernel(fn, dim3(static_cast<unsigned>((a.N + per_block - 1) / per_block)), dim3(128), args, s.smem, st);
+  }
   const int64_t vtiles = (a.N + static_cast<int64_t>(s.threads) * s.vpt - 1) /
                          (static_cast<int64_t>(s.threads) * s.vpt);
   const int64_t blocks = vtiles * s.splits;
@@ -849,8 +1006,11 @@ cudaError_t launch_bwd(const MfArgs& a, const Tuning& t, void* ws, cudaStream_t 
   p.groups = 1;
   if (a.mode == kPlain) {
     const int threads = 128;
-    dim3 grid(static_cast<unsigned>(a.A), static_cast<unsigned>((a.S + threads - 1) / threads));
-    mf_bwd_plain_kernel<T><<<grid, threads, 0, st>>>(p);
+    const int lanes = plain_lanes(a.A * a.S, a.N);
+    const dim3 grid(static_cast<unsigned>(a.A), static_cast<unsigned>((a.S * lanes + threads - 1) / threads));
+    if (lanes == 1) mf_bwd_plain_kernel<T, 1><<<grid, threads, 0, st>>>(p);
+    else if (lanes == 4) mf_bwd_plain_kernel<T, 4><<<grid, threads, 0, st>>>(p);
+    else mf_bwd_plain_kernel<T, 8><<<grid, threads, 0, st>>>(p);
     return cudaGetLastError();
   }
   const int threads = t.threads;
@@ -938,20 +1098,25 @@ int fwd_blocks_per_sm(const MfArgs& a, const Tuning& t) {
   const void* fn = a.dtype == kF64   ? fwd_kernel_ptr<double>(a.mode, s.vpt)
                    : a.dtype == kF16 ? fwd_kernel_ptr<__half>(a.mode, s.vpt)
                                      : fwd_kernel_ptr<float>(a.mode, s.vpt);
-  int n = 0;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(s.smem)) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, s.threads, s.smem) != cudaSuccess ||
-      n <= 0) {
-    cudaGetLastError();
-    return std::max(1, 1024 / t.threads);
-  }
-  return n;
+  const int n = resident_blocks(fn, s.threads, s.smem);
+  return n > 0 ? n : std::max(1, 1024 / t.threads);
 }
 
 Tuning mf_forward_resolve(const MfArgs& a, const Tuning& req) {
   if (a.mode == kNufft) return mf_nufft_forward_resolve(a, req);
   Tuning t = req;
+  // A call of a few voxels (fewer blocks of the usual shape than SMs, each of which would
+  // walk many antennas one after the other): small blocks, and stages short enough that
+  // the antennas fill the GPU.  343 voxels x 48 antennas x 64 samples: 97 us in one block of
+  // 128 x 4 voxels, 8 us in 144 blocks.
+  if (a.mode == kMixed && t.threads <= 0 && t.items <= 0 && t.stage_rows <= 0 && a.N > 0 && a.A > 0) {
+    const int64_t sms = current_device_info().sm_count;
+    if ((a.N + 511) / 512 * ((a.A + 7) / 8) < sms) {
+      t.threads = 64;
+      t.items = 2;
+      t.stage_rows = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(8, (a.N + 127) / 128 * a.A / sms)));
+    }
+  }
   if (t.threads != 64 && t.threads != 128 && t.threads != 256) t.threads = 128;
   // MIXED keeps 2, 4 or 8 voxels per thread, each with its own recurrence state;
   // four measured fastest on B200 for 49152 x 256 samples x 128^3 voxels
