@@ -764,8 +764,9 @@ __device__ __forceinline__ void red_add4(float4* dst, float2 a, float2 b) {
 // issue slots (ncu, 972 x 50653 pairs): 972 antennas x 201 samples x 50653 voxels
 // take 0.24 ms here, 2.37 ms by the recurrence of the direct kernel.
 constexpr int kMomentTile = 128;
+constexpr int kMomentUnroll = 4;  // voxels whose paths overlap (2: 2% slower; 6 blocks per SM and one: 8%)
 
-template <typename T, bool ACCURATE>
+template <typename T>
 __global__ void __launch_bounds__(128, 4) mf_moment_kernel(const MomentP<T> p) {
   constexpr int Q = MomentCells::Q;
   __shared__ double2 sxy[kMomentTile], szv[kMomentTile];
@@ -833,23 +834,23 @@ __global__ void __launch_bounds__(128, 4) mf_moment_kernel(const MomentP<T> p) {
     }
     __syncthreads();
     const int count = static_cast<int>(min(static_cast<int64_t>(kMomentTile), v_end - v0));
-    for (int i = 0; i < count; i += 2) {
-      float x[2], m[2];
-      float2 w[2];
+    for (int i = 0; i < count; i += kMomentUnroll) {
+      float x[kMomentUnroll], m[kMomentUnroll];
+      float2 w[kMomentUnroll];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
+      for (int u = 0; u < kMomentUnroll; ++u) {
         const double2 xy = sxy[i + u], zv = szv[i + u];
         const float2 g = sg[i + u];
         const Leg lt = leg_length(mt[0], mt[1], mt[2], mt[3], xy.x, xy.y, zv.x, zv.y);
         const Leg lr = leg_length(mr[0], mr[1], mr[2], mr[3], xy.x, xy.y, zv.x, zv.y);
         const float hi = lt.d + lr.d, lo = lt.l + lr.l;
         const CellPos c = pair_cell(p.ph, hi, lo);
-        w[u] = cmul(g, pair_phasor<ACCURATE>(pair_cycles(p.ph, hi, lo)));
+        w[u] = cmul(g, cis_cycles_fast(pair_cycles(p.ph, hi, lo)));
         x[u] = c.x;
         m[u] = c.m;
       }
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
+      for (int u = 0; u < kMomentUnroll; ++u) {
         if (m[u] != cur) {
           flush();
           cur = m[u];
@@ -976,7 +977,7 @@ MomentShape moment_shape(int64_t A, int64_t N) {
   const int64_t tiles = std::max<int64_t>(1, (N + kMomentTile - 1) / kMomentTile);
   int64_t splits = std::max<int64_t>(1, slots / s.groups);
   splits = std::min<int64_t>(std::min<int64_t>(splits, tiles), 2048);
-  s.vox_per_split = (((N + splits - 1) / splits + 1) / 2) * 2;  // whole pairs of voxels
+  s.vox_per_split = (((N + splits - 1) / splits + kMomentUnroll - 1) / kMomentUnroll) * kMomentUnroll;
   s.splits = static_cast<int>((N + s.vox_per_split - 1) / s.vox_per_split);
   return s;
 }
@@ -1016,8 +1017,7 @@ cudaError_t launch_cells_backward(const MfArgs& a, unsigned char* ws, cudaStream
   mp.apad = (a.A + 31) / 32 * 32;
   mp.vox_per_split = sh.vox_per_split;
   mp.ph = pair_phase(pc.k0, pc.b0, pc.k1, pc.b1, a.S, kappa);
-  if (a.mode == kNufft) mf_moment_kernel<T, true><<<dim3(sh.groups, sh.splits), sh.threads, 0, st>>>(mp);
-  else mf_moment_kernel<T, false><<<dim3(sh.groups, sh.splits), sh.threads, 0, st>>>(mp);
+  mf_moment_kernel<T><<<dim3(sh.groups, sh.splits), sh.threads, 0, st>>>(mp);
 
   if (sh.splits > 1) {
     constexpr int pairs = MomentCells::Q / 2;
@@ -1051,7 +1051,8 @@ cudaError_t launch_cells_backward(const MfArgs& a, unsigned char* ws, cudaStream
 // the two kernels (the direct one's error near theta = 0) into 3e-5 of the
 // gradients, more than a training run should move by from one release to the next.
 // The NUFFT form goes the same way from 8 taps on (fewer taps are a coarser form
-// of their own), with the accurate phasor.
+// of their own), its forward with the accurate phasor (64-bit error 1.3e-7 by 8 taps,
+// 1.2e-7 so, 1.7e-7 with the hardware phasor; the adjoint's 1.1e-6 becomes 5e-7 either way).
 bool cells_apply(const MfArgs& a, int taps, int64_t min_antennas) {
   if (a.mode == kPlain || (a.mode == kNufft && taps < 8)) return false;
   return !a.direct_only && a.dtype != kF64 && a.S >= 32 && a.S <= 4096 && a.N >= 512 && a.A >= min_antennas &&
