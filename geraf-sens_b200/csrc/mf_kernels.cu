@@ -883,11 +883,11 @@ FwdShape fwd_shape(const MfArgs& a, const Tuning& t) {
 
 // Lanes that share one output of a PLAIN kernel: one where that fills the GPU with 1024
 // threads per SM (about half of what the sines and cosines need to hide their
-// latency), else 4, or 8 where 4 leave less than 768 per SM.
+// latency), else 4, 8 where 4 leave less than 768 per SM, a warp where 8 leave less than 512.
 int plain_lanes(int64_t outputs, int64_t terms) {
   const int64_t sms = current_device_info().sm_count;
-  if (outputs >= sms * 1024 || terms < 32) return 1;
-  return outputs * 4 >= sms * 768 ? 4 : 8;
+  if (outputs >= sms * 1024 || terms < 16) return 1;
+  return outputs * 4 >= sms * 768 ? 4 : outputs * 8 >= sms * 512 ? 8 : 32;
 }
 
 template <typename T>
@@ -926,8 +926,9 @@ cudaError_t launch_fwd(const MfArgs& a, const FwdShape& s, void* ws, cudaStream_
   const void* fn = fwd_kernel_ptr<T>(a.mode, s.vpt);
   const int lanes = a.mode == kPlain && s.splits == 1 ? plain_lanes(a.N, a.S) : 1;
   if (lanes > 1) {
-    fn = lanes == 4 ? reinterpret_cast<const void*>(&mf_fwd_plain_lanes_kernel<T, 4>)
-                    : reinterpret_cast<const void*>(&mf_fwd_plain_lanes_kernel<T, 8>);
+    fn = lanes == 4   ? reinterpret_cast<const void*>(&mf_fwd_plain_lanes_kernel<T, 4>)
+         : lanes == 8 ? reinterpret_cast<const void*>(&mf_fwd_plain_lanes_kernel<T, 8>)
+                      : reinterpret_cast<const void*>(&mf_fwd_plain_lanes_kernel<T, 32>);
   }
   cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(s.smem));
@@ -1010,7 +1011,8 @@ cudaError_t launch_bwd(const MfArgs& a, const Tuning& t, void* ws, cudaStream_t 
     const dim3 grid(static_cast<unsigned>(a.A), static_cast<unsigned>((a.S * lanes + threads - 1) / threads));
     if (lanes == 1) mf_bwd_plain_kernel<T, 1><<<grid, threads, 0, st>>>(p);
     else if (lanes == 4) mf_bwd_plain_kernel<T, 4><<<grid, threads, 0, st>>>(p);
-    else mf_bwd_plain_kernel<T, 8><<<grid, threads, 0, st>>>(p);
+    else if (lanes == 8) mf_bwd_plain_kernel<T, 8><<<grid, threads, 0, st>>>(p);
+    else mf_bwd_plain_kernel<T, 32><<<grid, threads, 0, st>>>(p);
     return cudaGetLastError();
   }
   const int threads = t.threads;
