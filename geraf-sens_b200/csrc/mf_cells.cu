@@ -13,6 +13,7 @@
 //      kMaxLeg, non-finite positions): its band is only known on the device.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "kernels.h"
 #include "range_cells.cuh"
@@ -760,9 +761,9 @@ __device__ __forceinline__ void red_add4(float4* dst, float2 a, float2 b) {
 // share a cell, and when it changes the moments are added to the antenna's own
 // record in memory (vector reductions without a return value: nothing waits for
 // them, and no other thread touches the record, so the order of its sums, and the
-// result, is the same on every run).  About 100 instructions per 32 pairs at 66% of the
-// issue slots (ncu, 972 x 50653 pairs): 972 antennas x 201 samples x 50653 voxels
-// take 0.24 ms here, 2.37 ms by the recurrence of the direct kernel.
+// result, is the same on every run).  About 88 instructions per 32 pairs (100 where the
+// antennas share no positions) at 68% of the issue slots: 972 antennas x 201 samples x
+// 50653 voxels take 0.19 ms here, 2.37 ms by the recurrence of the direct kernel.
 constexpr int kMomentTile = 128;
 constexpr int kMomentUnroll = 4;  // voxels whose paths overlap (2: 2% slower; 6 blocks per SM and one: 8%)
 
@@ -777,17 +778,43 @@ __global__ void __launch_bounds__(128, 4) mf_moment_kernel(const MomentP<T> p) {
   const int64_t split = blockIdx.y;
   const int64_t v_begin = split * p.vox_per_split;
   const int64_t v_end = min(p.N, v_begin + p.vox_per_split);
+  // The antennas of a warp often share transmitters and receivers (32 channels of a
+  // 3 TX x 4 RX scan have about 20 positions): then each lane forms one position's legs
+  // and takes its own two from the lanes that hold them.
   double mt[4], mr[4];
+  int from_t = 0, from_r = 0;
+  bool shared_legs;
   {
-    double t[3], r[3];
+    float t[3], r[3];
     const int64_t al = min(a, p.A - 1);
+    unsigned same_t = 0xffffffffu, same_r = 0xffffffffu;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       t[c] = ld_f(p.tx, al * 3 + c);
       r[c] = ld_f(p.rx, al * 3 + c);
+      same_t &= __match_any_sync(0xffffffffu, __float_as_uint(t[c]));
+      same_r &= __match_any_sync(0xffffffffu, __float_as_uint(r[c]));
     }
-    leg_antenna(t, p.head->bias, mt);
-    leg_antenna(r, p.head->bias, mr);
+    const int lane = threadIdx.x & 31;
+    const int first_t = __ffs(same_t) - 1, first_r = __ffs(same_r) - 1;
+    const unsigned heads_t = __ballot_sync(0xffffffffu, first_t == lane);
+    const unsigned heads_r = __ballot_sync(0xffffffffu, first_r == lane);
+    const int nt = __popc(heads_t), nr = __popc(heads_r);
+    shared_legs = nt + nr <= 32;
+    from_t = __popc(heads_t & ((1u << first_t) - 1u));
+    from_r = nt + __popc(heads_r & ((1u << first_r) - 1u));
+    // lane i < nt takes the i-th transmitter, lane nt + i the i-th receiver
+    const int want = lane < nt ? static_cast<int>(__fns(heads_t, 0, lane + 1))
+                               : static_cast<int>(__fns(heads_r, 0, min(lane - nt, nr - 1) + 1));
+    double own[3], other[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float ht = __shfl_sync(0xffffffffu, t[c], want), hr = __shfl_sync(0xffffffffu, r[c], want);
+      own[c] = shared_legs ? (lane < nt ? ht : hr) : t[c];
+      other[c] = r[c];
+    }
+    leg_antenna(own, p.head->bias, mt);
+    leg_antenna(other, p.head->bias, mr);
   }
   const bool mine = a < p.apad;
   float4* rec = p.moments + split * kMomentCap * (Q / 2) * p.apad + a;
@@ -834,38 +861,50 @@ __global__ void __launch_bounds__(128, 4) mf_moment_kernel(const MomentP<T> p) {
     }
     __syncthreads();
     const int count = static_cast<int>(min(static_cast<int64_t>(kMomentTile), v_end - v0));
-    for (int i = 0; i < count; i += kMomentUnroll) {
-      float x[kMomentUnroll], m[kMomentUnroll];
-      float2 w[kMomentUnroll];
+    auto sum_tile = [&](auto shared) {
+      constexpr bool SHARED = decltype(shared)::value;
+      for (int i = 0; i < count; i += kMomentUnroll) {
+        float x[kMomentUnroll], m[kMomentUnroll];
+        float2 w[kMomentUnroll];
 #pragma unroll
-      for (int u = 0; u < kMomentUnroll; ++u) {
-        const double2 xy = sxy[i + u], zv = szv[i + u];
-        const float2 g = sg[i + u];
-        const Leg lt = leg_length(mt[0], mt[1], mt[2], mt[3], xy.x, xy.y, zv.x, zv.y);
-        const Leg lr = leg_length(mr[0], mr[1], mr[2], mr[3], xy.x, xy.y, zv.x, zv.y);
-        const float hi = lt.d + lr.d, lo = lt.l + lr.l;
-        const CellPos c = pair_cell(p.ph, hi, lo);
-        w[u] = cmul(g, cis_cycles_fast(pair_cycles(p.ph, hi, lo)));
-        x[u] = c.x;
-        m[u] = c.m;
-      }
-#pragma unroll
-      for (int u = 0; u < kMomentUnroll; ++u) {
-        if (m[u] != cur) {
-          flush();
-          cur = m[u];
-#pragma unroll
-          for (int q = 0; q < Q; ++q) M[q] = make_float2(0.0f, 0.0f);
+        for (int u = 0; u < kMomentUnroll; ++u) {
+          const double2 xy = sxy[i + u], zv = szv[i + u];
+          const float2 g = sg[i + u];
+          Leg lt = leg_length(mt[0], mt[1], mt[2], mt[3], xy.x, xy.y, zv.x, zv.y), lr;
+          if (SHARED) {
+            lr.d = __shfl_sync(0xffffffffu, lt.d, from_r);
+            lr.l = __shfl_sync(0xffffffffu, lt.l, from_r);
+            lt.d = __shfl_sync(0xffffffffu, lt.d, from_t);
+            lt.l = __shfl_sync(0xffffffffu, lt.l, from_t);
+          } else {
+            lr = leg_length(mr[0], mr[1], mr[2], mr[3], xy.x, xy.y, zv.x, zv.y);
+          }
+          const float hi = lt.d + lr.d, lo = lt.l + lr.l;
+          const CellPos c = pair_cell(p.ph, hi, lo);
+          w[u] = cmul(g, cis_cycles_fast(pair_cycles(p.ph, hi, lo)));
+          x[u] = c.x;
+          m[u] = c.m;
         }
-        M[0] = fadd2(M[0], w[u]);
-        float xq = x[u];
 #pragma unroll
-        for (int q = 1; q < Q; ++q) {
-          M[q] = ffma2(make_float2(xq, xq), w[u], M[q]);
-          xq *= x[u];
+        for (int u = 0; u < kMomentUnroll; ++u) {
+          if (m[u] != cur) {
+            flush();
+            cur = m[u];
+#pragma unroll
+            for (int q = 0; q < Q; ++q) M[q] = make_float2(0.0f, 0.0f);
+          }
+          M[0] = fadd2(M[0], w[u]);
+          float xq = x[u];
+#pragma unroll
+          for (int q = 1; q < Q; ++q) {
+            M[q] = ffma2(make_float2(xq, xq), w[u], M[q]);
+            xq *= x[u];
+          }
         }
       }
-    }
+    };
+    if (shared_legs) sum_tile(std::true_type{});
+    else sum_tile(std::false_type{});
   }
   flush();
 }
