@@ -12,8 +12,9 @@
 // Forward: one persistent launch.  A one-block prep pass validates the
 // offsets and lays out work items (antenna, chunk of `chunk` points); resident
 // blocks then take items from an atomic counter until none are left, so
-// antennas with 512 rays and antennas with 8192 rays load-balance; a finish
-// pass sums each antenna's item partials in item order (deterministic).
+// antennas with 512 rays and antennas with 8192 rays load-balance.  An item
+// leaves the moments of its points in range cells (tracer_cells.cuh); a finish
+// pass turns each antenna's moments into samples in item order (deterministic).
 // Adjoint: a point belongs to one antenna, so its gradients need no reduction
 // across antennas; blocks screen runs of points and deal the live ones out
 // over their threads.
@@ -166,10 +167,10 @@ __global__ void __launch_bounds__(kTraceThreads, 6) ragged_fwd_kernel(const RgP<
 template <typename T>
 __global__ void __launch_bounds__(kFinishThreads) ragged_finish_kernel(const RgP<T> p) {
   const int64_t a = blockIdx.x;
-  const int n0 = blockIdx.y * kFinishThreads;
+  const int n0 = blockIdx.y * kFinishSamples;
   const int64_t it = p.item_offsets[a];
   trace_finish<T>(p.c, p.records + it, p.rows + it * p.c.S, p.item_offsets[a + 1] - it,
-                  static_cast<float>(p.offsets[a + 1] - p.offsets[a]), n0, min(p.c.S, n0 + kFinishThreads),
+                  static_cast<float>(p.offsets[a + 1] - p.offsets[a]), n0, min(p.c.S, n0 + kFinishSamples),
                   p.out_r + a * p.c.S, p.out_i + a * p.c.S);
 }
 
@@ -436,7 +437,7 @@ cudaError_t launch_ragged_fwd(const RaggedArgs& a, const Tuning& t, void* ws, cu
   const int64_t blocks = std::max<int64_t>(
       1, std::min<int64_t>(static_cast<int64_t>(per_sm) * current_device_info().sm_count, p.max_items));
   ragged_fwd_kernel<T><<<static_cast<unsigned>(blocks), kTraceThreads, 0, st>>>(p);
-  const dim3 grid(static_cast<unsigned>(a.A), static_cast<unsigned>((a.S + kFinishThreads - 1) / kFinishThreads));
+  const dim3 grid(static_cast<unsigned>(a.A), static_cast<unsigned>((a.S + kFinishSamples - 1) / kFinishSamples));
   ragged_finish_kernel<T><<<grid, kFinishThreads, 0, st>>>(p);
   return cudaGetLastError();
 }

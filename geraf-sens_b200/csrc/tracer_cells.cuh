@@ -10,8 +10,10 @@
 // 128 at a time get the exact geometry, one per thread, so no lane sits out the
 // expensive part (on a typical scene one point in ten is live).  The 128 points'
 // contributions are then sorted by cell in shared memory and added up by groups
-// of eight lanes, one per moment, in list order: no floating-point atomics, the
-// same bits on every run.
+// of eight lanes, one per moment, in list order: no floating-point atomics, and the
+// same bits on every run as long as the run's cells fit the slots below.  (Sums by each
+// warp alone, over the set bits of its match masks and without barriers, took as long for
+// the pre-cull's lists and 40 us longer for 64 antennas x 295000 screened points.)
 //
 // Cells are kept in kTraceSlots slots, cell k in slot k mod kTraceSlots.  Points whose
 // slot another cell of the run holds (2.4 m of path away at 4 GHz swept) are
@@ -397,26 +399,41 @@ __device__ __forceinline__ void trace_store(const TraceSmem& sm, TraceRecord* re
   __syncthreads();
 }
 
-// Samples of one antenna from its runs' records, kFinishThreads threads.  Per slot the cells
-// are taken in ascending order, one per round (one round, unless runs of the
-// antenna lie more than kTraceSlots cells apart); the runs' moments are added in run order.
-constexpr int kFinishThreads = 256;
+// Samples [n_begin, n_begin + kFinishSamples) of one antenna from its runs' records, by
+// kFinishThreads threads.  Per slot the cells are taken in ascending order, one per round
+// (one round, unless runs of the antenna lie more than kTraceSlots cells apart).
+//
+// A call has few such blocks (one per antenna), so each is bound by latency: four
+// groups of threads take every fourth run's moments, then every fourth slot's cells, and
+// add up in a fixed order.  13 antennas x 78 runs: 44 us with one group, 14 us with four;
+// 64 antennas x 23 runs: 19.5 and 10.9 us.
+constexpr int kFinishSamples = 256;
+constexpr int kFinishGroups = 4;
+constexpr int kFinishThreads = kFinishSamples * kFinishGroups;
+
+struct FinishSmem {
+  float4 part[kFinishGroups][kTraceSlots][kTraceQ / 2];
+  float2 mom[kTraceSlots][kTraceQ];
+  float2 acc[kFinishGroups][kFinishSamples];
+  int next[kFinishGroups][kTraceSlots], top[kFinishGroups][kTraceSlots];
+  int tag[kTraceSlots];
+};
 
 template <typename T>
 __device__ __forceinline__ void trace_finish(const TraceConsts& c, const TraceRecord* rec, const float2* rows,
                                              int64_t runs, float divisor, int n_begin, int n_end, T* out_r, T* out_i) {
-  __shared__ float2 mom[kTraceSlots][kTraceQ];
-  __shared__ int tag[kTraceSlots];
-  static_assert(kFinishThreads == kTraceSlots * kTraceQ / 2, "a thread per slot and pair of moments");
-  const int slot = threadIdx.x / (kTraceQ / 2), pair = threadIdx.x % (kTraceQ / 2);
-  const int n = n_begin + threadIdx.x;
+  __shared__ FinishSmem sm;
+  static_assert(kFinishSamples == kTraceSlots * kTraceQ / 2, "a thread of a group per slot and pair of moments");
+  const int group = threadIdx.x / kFinishSamples, in_group = threadIdx.x % kFinishSamples;
+  const int slot = in_group / (kTraceQ / 2), pair = in_group % (kTraceQ / 2);
+  const int n = n_begin + in_group;
   const bool mine = n < n_end;
   float2 acc = make_float2(0.0f, 0.0f);
   float g[kTraceQ];
   bool rowed = false;
   for (int64_t r = threadIdx.x; r < runs; r += kFinishThreads) rowed = rowed || rec[r].has_row != 0;
   if (__syncthreads_or(rowed) && mine) {
-    for (int64_t r = 0; r < runs; ++r) {
+    for (int64_t r = group; r < runs; r += kFinishGroups) {
       if (rec[r].has_row) acc = fadd2(acc, rows[r * c.S + n]);
     }
   }
@@ -426,7 +443,7 @@ __device__ __forceinline__ void trace_finish(const TraceConsts& c, const TraceRe
     // the slot's lowest cell above the one done, and whether higher ones follow
     int next = INT32_MAX, top = INT32_MIN;
 #pragma unroll 4
-    for (int64_t r = pair; r < runs; r += kTraceQ / 2) {
+    for (int64_t r = group + pair * kFinishGroups; r < runs; r += kFinishGroups * kTraceQ / 2) {
       const int t = rec[r].tag[slot];
       if (t != kTraceEmpty && t > done) {
         next = min(next, t);
@@ -438,10 +455,20 @@ __device__ __forceinline__ void trace_finish(const TraceConsts& c, const TraceRe
       next = min(next, __shfl_xor_sync(0xffffffffu, next, o));
       top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
     }
+    if (pair == 0) {
+      sm.next[group][slot] = next;
+      sm.top[group][slot] = top;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kFinishGroups; ++k) {
+      next = min(next, sm.next[k][slot]);
+      top = max(top, sm.top[k][slot]);
+    }
     float4 m = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (next != INT32_MAX) {
 #pragma unroll 8
-      for (int64_t r = 0; r < runs; ++r) {
+      for (int64_t r = group; r < runs; r += kFinishGroups) {
         const int t = rec[r].tag[slot];
         const float4 y = reinterpret_cast<const float4*>(&rec[r].moments[slot][0])[pair];
         const bool take = t == next;  // unused slots hold no moments
@@ -451,20 +478,36 @@ __device__ __forceinline__ void trace_finish(const TraceConsts& c, const TraceRe
         m.w += take ? y.w : 0.0f;
       }
     }
-    reinterpret_cast<float4*>(&mom[slot][0])[pair] = m;
-    if (pair == 0) tag[slot] = next;  // INT32_MAX: none
+    sm.part[group][slot][pair] = m;
     const bool more = next != INT32_MAX && top > next;
     done = next;
     const bool again = __syncthreads_or(more) != 0;
+    if (group == 0) {
+#pragma unroll
+      for (int k = 1; k < kFinishGroups; ++k) {
+        const float4 y = sm.part[k][slot][pair];
+        m.x += y.x;
+        m.y += y.y;
+        m.z += y.z;
+        m.w += y.w;
+      }
+      reinterpret_cast<float4*>(&sm.mom[slot][0])[pair] = m;
+      if (pair == 0) sm.tag[slot] = next;  // INT32_MAX: none
+    }
+    __syncthreads();
     if (mine) {
-      for (int k = 0; k < kTraceSlots; ++k) {
-        if (tag[k] != INT32_MAX) add_cell(c, tag[k], mom[k], g, n, acc);
+      for (int k = group; k < kTraceSlots; k += kFinishGroups) {
+        if (sm.tag[k] != INT32_MAX) add_cell(c, sm.tag[k], sm.mom[k], g, n, acc);
       }
     }
     if (!again) break;
     __syncthreads();
   }
-  if (mine) {
+  sm.acc[group][in_group] = acc;
+  __syncthreads();
+  if (group == 0 && mine) {
+#pragma unroll
+    for (int k = 1; k < kFinishGroups; ++k) acc = fadd2(acc, sm.acc[k][in_group]);
     out_r[n] = from_f<T>(acc.x / divisor);
     out_i[n] = from_f<T>(acc.y / divisor);
   }

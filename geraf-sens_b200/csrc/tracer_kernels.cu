@@ -13,10 +13,12 @@
 // in the reference's FP32 operation order, so amplitudes and culling decisions
 // are bit-identical -- and the sample loop works on (amplitude, delay) only.
 // PLAIN forms then evaluate the reference's per-sample phase with accurate
-// cosf/sinf in its summation order; MIXED forms reduce the carrier phase in
-// FP64 and generate the per-sample phasors with a three-term recurrence
-// (forward) or a Horner recurrence (adjoint), which also yields the position gradient the
-// reference does not provide.
+// cosf/sinf in its summation order.  MIXED forms reduce the carrier phase in FP64
+// and sum the samples through range cells: the forward collects the points'
+// moments per cell of path length (tracer_cells.cuh), the adjoint reads tables of
+// the residual's sum (tracer_adjoint_cells.cu).  The adjoint of this file, a Horner
+// recurrence over the samples, serves the calls that the tables do not; either also
+// yields the position gradient the reference does not provide.
 #include <algorithm>
 
 #include "common.cuh"
@@ -180,9 +182,9 @@ __global__ void __launch_bounds__(kTraceThreads, 5) tracer_fwd_cells_kernel(cons
 template <typename T>
 __global__ void __launch_bounds__(kFinishThreads) tracer_fwd_finish_kernel(const TrCellP<T> p) {
   const int64_t a = blockIdx.x;
-  const int n0 = blockIdx.y * kFinishThreads;
+  const int n0 = blockIdx.y * kFinishSamples;
   trace_finish<T>(p.c, p.records + a * p.splits, p.rows + a * p.splits * p.c.S, p.splits, static_cast<float>(p.P), n0,
-                  min(p.c.S, n0 + kFinishThreads), p.out_r + a * p.c.S, p.out_i + a * p.c.S);
+                  min(p.c.S, n0 + kFinishSamples), p.out_r + a * p.c.S, p.out_i + a * p.c.S);
 }
 
 // ---------------------------------------------------------------------------
@@ -852,7 +854,7 @@ cudaError_t launch_tracer_fwd(const TracerArgs& a, const Tuning& t, void* ws, cu
   }
   if (a.A * t.splits > 0x7fffffff) return cudaErrorInvalidConfiguration;
   tracer_fwd_cells_kernel<T><<<static_cast<unsigned>(a.A * t.splits), kTraceThreads, 0, st>>>(c);
-  const dim3 grid(static_cast<unsigned>(a.A), static_cast<unsigned>((a.S + kFinishThreads - 1) / kFinishThreads));
+  const dim3 grid(static_cast<unsigned>(a.A), static_cast<unsigned>((a.S + kFinishSamples - 1) / kFinishSamples));
   tracer_fwd_finish_kernel<T><<<grid, kFinishThreads, 0, st>>>(c);
   return cudaGetLastError();
 }

@@ -181,7 +181,7 @@ __device__ __forceinline__ bool culled_for_all(const Aperture& ap, const float* 
 // number of listed points of the chunk and boxes[c] (when given) their bounding box.  With a null `aperture` each block
 // bounds the antennas itself.
 template <typename T>
-__global__ void __launch_bounds__(kChunkThreads) point_flags_kernel(const T* normals, const T* points,
+__global__ void __launch_bounds__(kChunkThreads, 4) point_flags_kernel(const T* normals, const T* points,
                                                                     const uint8_t* inb, int64_t P,
                                                                     const Aperture* aperture, const T* tx,
                                                                     const T* rx, int64_t A, uint32_t* words,
@@ -190,23 +190,34 @@ __global__ void __launch_bounds__(kChunkThreads) point_flags_kernel(const T* nor
   __shared__ float box_s[kChunkThreads / 32][6];
   float box[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
   __shared__ Aperture ap_s;
-  if (aperture == nullptr) block_aperture(tx, rx, A, &ap_s);
-  const Aperture ap = aperture != nullptr ? *aperture : ap_s;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int64_t base = static_cast<int64_t>(blockIdx.x) * kChunk;
+  // The points are on their way while the block bounds the antennas (each block is one chain
+  // of latencies: for 9900 points 6 us with the loads here, 10 us with them after the aperture).
+  constexpr int kPer = kChunk / kChunkThreads;
+  float nrm[kPer][3], pos[kPer][3];
+  unsigned in = 0;
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int64_t q = base + k * kChunkThreads + threadIdx.x;
+    const bool there = q < P;
+    if (there && inb[q]) in |= 1u << k;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      nrm[k][j] = there ? ld_f(normals, q * 3 + j) : 0.0f;
+      pos[k][j] = there ? ld_f(points, q * 3 + j) : 0.0f;
+    }
+  }
+  if (aperture == nullptr) block_aperture(tx, rx, A, &ap_s);
+  const Aperture ap = aperture != nullptr ? *aperture : ap_s;
   int c = 0;
 #pragma unroll
-  for (int k = 0; k < kChunk / kChunkThreads; ++k) {
-    const int64_t q = base + k * kChunkThreads + threadIdx.x;
+  for (int k = 0; k < kPer; ++k) {
     bool listed = false;
-    if (q < P && inb[q]) {
-      float n[3], pt[3];
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        n[j] = ld_f(normals, q * 3 + j);
-        pt[j] = ld_f(points, q * 3 + j);
-      }
+    if ((in >> k) & 1u) {
+      const float(&n)[3] = nrm[k];
+      const float(&pt)[3] = pos[k];
       listed = !culled_for_all(ap, n, pt);
       if (listed) {
 #pragma unroll
