@@ -12,7 +12,9 @@
 // from TMA-staged sample tiles, a per-sample constant table and per-(v,a)
 // geometry hoisting.
 //
-// MIXED kernels use that phi is linear in n: with z = exp(-j 2 pi dcyc) the
+// MIXED kernels of this file (the direct form; calls of more antennas, voxels and
+// samples go through the range cells of mf_cells.cu, see mf_cells_forward_applies and
+// mf_cells_backward_applies there) use that phi is linear in n: with z = exp(-j 2 pi dcyc) the
 // forward inner sum is exp(-j phi0) * P_a(z), P_a(z) = sum_n s[a,n] z^n,
 // evaluated by a second-order (Goertzel) recurrence on packed complex samples
 // in 128- or 64-sample blocks; the adjoint generates
@@ -20,6 +22,7 @@
 // re-seeded from exact phasors every K samples.  phi0 is reduced modulo one
 // cycle in FP64 (path_cycles), so only two phasors per (v, a) are evaluated.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -385,50 +388,69 @@ __global__ void __launch_bounds__(256) mf_fwd_plain_kernel(const MfFwdP<T> p) {
   }
 }
 
-// Exchange of a PLAIN kernel's terms among the LANES lanes that share an output: each
-// lane stores its two terms, then the even lanes add the 2 LANES real parts in order
-// and the odd lanes the imaginary parts, through shared memory (16-byte loads, rows
-// padded to stay off each other's banks).  Every lane adding both parts took 40% longer
-// over all, and so did shuffles.
+// Ordered sums of a PLAIN kernel whose outputs are shared by LANES lanes each: in one step
+// every thread of the block leaves kGroups pairs of terms in a shared row per chain (an
+// output's real or imaginary sum); in the next, while new terms are evaluated, the
+// chains of the last step are added up by a lane each, in the reference's order.  The warps
+// take turns at that, so that their schedulers carry the same load.  The adds are then as
+// few as with a thread per output; each lane adding all of its output's terms, from a row
+// of its warp's, took 70 instructions per term instead of about 58 (13824 voxels x 300 antennas x 128
+// samples: forward and adjoint 2.54 ms, so 2.23 ms).
 template <int LANES>
-struct TermRows {
-  static constexpr int kTerms = 2 * LANES;
-  float row[2][32 / LANES][kTerms + 4];
-};
+struct TermSums {
+  static constexpr int kThreads = 128;
+  // groups of LANES terms per output and step: 2, 4 and 8 of 8 lanes 2.90, 2.50 and 2.23 ms
+  // (a barrier per step), 12 or more cost resident blocks; a step of 128 terms of a warp
+  static constexpr int kGroups = LANES < 32 ? 8 : 4;
+  static constexpr int kTerms = kGroups * LANES;
+  static constexpr int kChains = 2 * kThreads / LANES;
+  static constexpr int kAdders = kChains > 32 ? kChains / 32 : 1;  // warps that add in a step
+  alignas(16) float row[2][kChains][kTerms + 4];  // padded off each other's banks
+  float acc[kChains];
 
-// acc: the lane's component.
-template <int LANES>
-__device__ __forceinline__ void add_terms(TermRows<LANES>& x, const float (&term_r)[2], const float (&term_i)[2], int count,
-                                          float& acc) {
-  const int out = (threadIdx.x & 31) / LANES;
-  const int lane = threadIdx.x % LANES;
-  __syncwarp();
-  x.row[0][out][lane] = term_r[0];
-  x.row[1][out][lane] = term_i[0];
-  x.row[0][out][LANES + lane] = term_r[1];
-  x.row[1][out][LANES + lane] = term_i[1];
-  __syncwarp();
-  const float* row = x.row[lane & 1][out];
-  if (count >= 2 * LANES) {
-#pragma unroll
-    for (int k = 0; k < 2 * LANES; k += 4) {
-      const float4 t = *reinterpret_cast<const float4*>(&row[k]);
-      acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, t.x), t.y), t.z), t.w);
-    }
-  } else {
-    for (int k = 0; k < count; ++k) acc = __fadd_rn(acc, row[k]);
+  __device__ __forceinline__ void clear() {
+    if (threadIdx.x < kChains) acc[threadIdx.x] = 0.0f;  // seen after the caller's next barrier
   }
-}
+  __device__ __forceinline__ void put(int step, int group, float re, float im) {
+    const int out = threadIdx.x / LANES, lane = threadIdx.x % LANES;
+    row[step & 1][2 * out][group * LANES + lane] = re;
+    row[step & 1][2 * out + 1][group * LANES + lane] = im;
+  }
+  // Adds the `count` terms per chain that step `step` - 1 left.
+  __device__ __forceinline__ void add(int step, int count) {
+    const int turn = ((static_cast<int>(threadIdx.x) >> 5) - step) & 3;
+    const int chain = turn * 32 + (threadIdx.x & 31);
+    if (turn >= kAdders || chain >= kChains || count == 0) return;
+    const float* x = row[(step - 1) & 1][chain];
+    float s = acc[chain];
+    if (count == kTerms) {
+#pragma unroll
+      for (int k = 0; k < kTerms; k += 4) {
+        const float4 t = *reinterpret_cast<const float4*>(&x[k]);
+        s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, t.x), t.y), t.z), t.w);
+      }
+    } else {
+      int k = 0;
+#pragma unroll 4
+      for (; k + 4 <= count; k += 4) {
+        const float4 t = *reinterpret_cast<const float4*>(&x[k]);
+        s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, t.x), t.y), t.z), t.w);
+      }
+      for (; k < count; ++k) s = __fadd_rn(s, x[k]);
+    }
+    acc[chain] = s;
+  }
+};
 
 // PLAIN forward with LANES lanes per voxel, for calls of too few voxels to fill the GPU
 // with one thread each (every thread is bound by the latency of its sines and
 // cosines: 13824 voxels x 300 antennas x 128 samples take 3.70 ms at one thread per
-// voxel, 1.26 ms at 8).  Lane j evaluates samples j, j + LANES, ...; every lane then adds
-// the LANES terms in sample order, so the sums are the one-thread kernel's to the bit.
+// voxel, 1.13 ms at 8).  Lane j evaluates samples j, j + LANES, ...; the terms are added in
+// sample order, so the sums are the one-thread kernel's to the bit.
 template <typename T, int LANES>
 __global__ void __launch_bounds__(128) mf_fwd_plain_lanes_kernel(const MfFwdP<T> p) {
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(16) TermRows<LANES> terms[4];
+  __shared__ TermSums<LANES> sums;
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
   float* pos = reinterpret_cast<float*>(smem + p.pos_off);
   float* kn = reinterpret_cast<float*>(smem + p.kn_off);
@@ -451,7 +473,9 @@ __global__ void __launch_bounds__(128) mf_fwd_plain_lanes_kernel(const MfFwdP<T>
   const float vx = ok ? ld_f(p.voxel, v) : 0.0f;
   const float vy = ok ? ld_f(p.voxel, p.N + v) : 0.0f;
   const float vz = ok ? ld_f(p.voxel, 2 * p.N + v) : 0.0f;
-  float acc = 0.0f;
+  using Sums = TermSums<LANES>;
+  int step = 0, count = 0;  // of the last step's terms
+  sums.clear();
   auto issue = [&](int tile, int stage) {
     const int64_t a0 = static_cast<int64_t>(tile) * p.rows;
     const int rws = static_cast<int>(min(static_cast<int64_t>(p.rows), p.A - a0));
@@ -476,28 +500,36 @@ __global__ void __launch_bounds__(128) mf_fwd_plain_lanes_kernel(const MfFwdP<T>
       const float base_phase = 2.0f * kPiF * kMfStartFrequency * tau;
       const T* rowr = stg.stage_ptr(s, 0) + r * p.ld;
       const T* rowi = stg.stage_ptr(s, 1) + r * p.ld;
-      // two groups of LANES samples at a time, whose sines and cosines overlap
-      for (int n0 = 0; n0 < S; n0 += 2 * LANES) {
-        float term_r[2], term_i[2];
+      auto term = [&](int n0, int u) {
+        const int n = min(n0 + u * LANES + lane, S - 1);
+        const float phase = base_phase + kn[n] * tau;
+        float cos_phase, sin_phase;
+        cos_sin(phase, &cos_phase, &sin_phase);
+        const float neg_sin_phase = -sin_phase;
+        const float sample_real = static_cast<float>(rowr[n]);
+        const float sample_imag = static_cast<float>(rowi[n]);
+        sums.put(step, u, cos_phase * sample_real - neg_sin_phase * sample_imag,
+                 cos_phase * sample_imag + neg_sin_phase * sample_real);
+      };
+      for (int n0 = 0; n0 < S; n0 += Sums::kTerms) {
+        if (n0 + Sums::kTerms <= S) {
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int n = min(n0 + u * LANES + lane, S - 1);
-          const float phase = base_phase + kn[n] * tau;
-          float cos_phase, sin_phase;
-          cos_sin(phase, &cos_phase, &sin_phase);
-          const float neg_sin_phase = -sin_phase;
-          const float sample_real = static_cast<float>(rowr[n]);
-          const float sample_imag = static_cast<float>(rowi[n]);
-          term_r[u] = cos_phase * sample_real - neg_sin_phase * sample_imag;
-          term_i[u] = cos_phase * sample_imag + neg_sin_phase * sample_real;
+          for (int u = 0; u < Sums::kGroups; ++u) term(n0, u);
+        } else {
+          for (int u = 0; n0 + u * LANES < S; ++u) term(n0, u);
         }
-        add_terms<LANES>(terms[threadIdx.x >> 5], term_r, term_i, S - n0, acc);
+        sums.add(step, count);
+        count = min(Sums::kTerms, S - n0);
+        ++step;
+        __syncthreads();
       }
     }
     __syncthreads();
     if (t + 2 < ntiles) issue(t + 2, s);
   }
-  if (ok && lane < 2) (lane == 0 ? p.out_r : p.out_i)[v] = from_f<T>(acc / static_cast<int>(p.A));
+  sums.add(step, count);
+  __syncthreads();
+  if (ok && lane < 2) (lane == 0 ? p.out_r : p.out_i)[v] = from_f<T>(sums.acc[2 * (threadIdx.x / LANES) + lane] / static_cast<int>(p.A));
 }
 
 // Sums `splits` partial rows of `count` complex values in a fixed order (FP64)
@@ -636,14 +668,14 @@ __global__ void __launch_bounds__(256) mf_bwd_mixed_kernel(const MfBwdP<T> p) {
 // (MatchedFilter_cuda_kernel.cu:186-219).  Per-(a, v) path delays are formed
 // once per voxel tile in shared memory.
 // LANES lanes per sample, for calls of few antennas x samples: lane j evaluates voxels j,
-// j + LANES, ... and every lane adds the LANES terms in voxel order, so the sums do
-// not depend on LANES (300 antennas x 128 samples x 13824 voxels: 1.71 ms with one lane,
-// 1.27 ms with 4).
+// j + LANES, ... and the terms are added in voxel order, so the sums do not depend on
+// LANES (300 antennas x 128 samples x 13824 voxels: 1.71 ms with one lane, 1.10 ms with 4).
 template <typename T, int LANES>
 __global__ void __launch_bounds__(128) mf_bwd_plain_kernel(const MfBwdP<T> p) {
   constexpr int TILE = 256;
   __shared__ float s_tau[TILE], s_gr[TILE], s_gi[TILE];
-  __shared__ __align__(16) TermRows<LANES> terms[LANES == 1 ? 1 : 4];
+  using Sums = TermSums<LANES == 1 ? 4 : LANES>;
+  __shared__ typename std::conditional<LANES == 1, int, Sums>::type sums;
   const int64_t a = blockIdx.x;
   const int lane = threadIdx.x % LANES;
   const int64_t n = static_cast<int64_t>(blockIdx.y) * (blockDim.x / LANES) + threadIdx.x / LANES;
@@ -653,6 +685,8 @@ __global__ void __launch_bounds__(128) mf_bwd_plain_kernel(const MfBwdP<T> p) {
   const float sample_time = static_cast<float>(n) / p.fs;
   const float kn = 2.0f * kPiF * p.As * sample_time;
   float acc_r = 0.0f, acc_i = 0.0f;
+  int step = 0, left = 0;  // terms of the last step, still to be added
+  if constexpr (LANES > 1) sums.clear();
   for (int64_t v0 = 0; v0 < p.N; v0 += TILE) {
     const int count = static_cast<int>(min(static_cast<int64_t>(TILE), p.N - v0));
     for (int i = threadIdx.x; i < count; i += blockDim.x) {
@@ -666,44 +700,66 @@ __global__ void __launch_bounds__(128) mf_bwd_plain_kernel(const MfBwdP<T> p) {
       s_gi[i] = ld_f(p.gi, v);
     }
     __syncthreads();
-    // Samples past S run along (the lanes of a warp exchange their terms) and are not
-    // stored.  Two groups of LANES voxels at a time, whose sines and cosines overlap.
-    for (int i0 = 0; i0 < count; i0 += 2 * LANES) {
-      float term_r[2], term_i[2];
+    auto term = [&](int i, float& term_r, float& term_i) {
+      const float tau = s_tau[i];
+      const float phase = 2.0f * kPiF * kMfStartFrequency * tau + kn * tau;
+      float cos_phase, sin_phase;
+      cos_sin(phase, &cos_phase, &sin_phase);
+      const float neg_sin_phase = -sin_phase;
+      const float grad_real_out = s_gr[i];
+      const float grad_imag_out = s_gi[i];
+      // The reference's expressions with the FMA contraction its build makes
+      // (identified against its outputs): the cos product is fused in both.
+      term_r = __fmaf_rn(cos_phase, grad_real_out, __fmul_rn(neg_sin_phase, grad_imag_out));
+      term_i = __fmaf_rn(cos_phase, grad_imag_out, __fmul_rn(sin_phase, grad_real_out));
+    };
+    if constexpr (LANES == 1) {
+      // two voxels at a time, whose sines and cosines overlap
+      for (int i0 = 0; i0 < count; i0 += 2) {
+        float term_r[2], term_i[2];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int i = min(i0 + u * LANES + lane, count - 1);
-        const float tau = s_tau[i];
-        const float phase = 2.0f * kPiF * kMfStartFrequency * tau + kn * tau;
-        float cos_phase, sin_phase;
-        cos_sin(phase, &cos_phase, &sin_phase);
-        const float neg_sin_phase = -sin_phase;
-        const float grad_real_out = s_gr[i];
-        const float grad_imag_out = s_gi[i];
-        // The reference's expressions with the FMA contraction its build makes
-        // (identified against its outputs): the cos product is fused in both.
-        term_r[u] = __fmaf_rn(cos_phase, grad_real_out, __fmul_rn(neg_sin_phase, grad_imag_out));
-        term_i[u] = __fmaf_rn(cos_phase, grad_imag_out, __fmul_rn(sin_phase, grad_real_out));
-      }
-      if (LANES == 1) {
+        for (int u = 0; u < 2; ++u) term(min(i0 + u, count - 1), term_r[u], term_i[u]);
         acc_r = __fadd_rn(acc_r, term_r[0]);
         acc_i = __fadd_rn(acc_i, term_i[0]);
         if (i0 + 1 < count) {
           acc_r = __fadd_rn(acc_r, term_r[1]);
           acc_i = __fadd_rn(acc_i, term_i[1]);
         }
-      } else {
-        add_terms<LANES>(terms[threadIdx.x >> 5], term_r, term_i, count - i0, acc_r);
+      }
+      __syncthreads();
+    } else {
+      // samples past S run along (the block exchanges its terms) and are not stored
+      auto put = [&](int i0, int u) {
+        float term_r, term_i;
+        term(min(i0 + u * LANES + lane, count - 1), term_r, term_i);
+        sums.put(step, u, term_r, term_i);
+      };
+      for (int i0 = 0; i0 < count; i0 += Sums::kTerms) {
+        if (i0 + Sums::kTerms <= count) {
+#pragma unroll
+          for (int u = 0; u < Sums::kGroups; ++u) put(i0, u);
+        } else {
+          for (int u = 0; i0 + u * LANES < count; ++u) put(i0, u);
+        }
+        sums.add(step, left);
+        left = min(Sums::kTerms, count - i0);
+        ++step;
+        __syncthreads();
       }
     }
-    __syncthreads();
   }
   const int total_ant_size = static_cast<int>(p.A);
   if (LANES == 1 && active) {
     p.out_r[a * p.S + n] = from_f<T>(acc_r / total_ant_size);
     p.out_i[a * p.S + n] = from_f<T>(acc_i / total_ant_size);
-  } else if (active && lane < 2) {  // acc_r is the lane's component
-    (lane == 0 ? p.out_r : p.out_i)[a * p.S + n] = from_f<T>(acc_r / total_ant_size);
+  }
+  if constexpr (LANES > 1) {
+    sums.add(step, left);
+    __syncthreads();
+    if (active && lane < 2) {
+      (lane == 0 ? p.out_r : p.out_i)[a * p.S + n] =
+          from_f<T>(sums.acc[2 * (threadIdx.x / LANES) + lane] / total_ant_size);
+    }
   }
 }
 
@@ -848,6 +904,15 @@ const void* fwd_kernel_ptr(int mode, int vpt) {
   return reinterpret_cast<const void*>(&mf_fwd_plain_kernel<T, 4>);
 }
 
+// Lanes that share one output of a PLAIN kernel: one where that fills the GPU with 1024
+// threads per SM (about half of what the sines and cosines need to hide their
+// latency), else 4, 8 where 4 leave less than 768 per SM, a warp where 8 leave less than 512.
+int plain_lanes(int64_t outputs, int64_t terms) {
+  const int64_t sms = current_device_info().sm_count;
+  if (outputs >= sms * 1024 || terms < 16) return 1;
+  return outputs * 4 >= sms * 768 ? 4 : outputs * 8 >= sms * 512 ? 8 : 32;
+}
+
 FwdShape fwd_shape(const MfArgs& a, const Tuning& t) {
   FwdShape s;
   s.threads = t.threads;
@@ -874,20 +939,18 @@ FwdShape fwd_shape(const MfArgs& a, const Tuning& t) {
     s.rows /= 2;
     s.layout = layout(s.rows);
   }
+  // a PLAIN block that also exchanges terms: stages short enough for six blocks per SM
+  if (a.mode == kPlain && s.splits == 1 && plain_lanes(a.N, a.S) > 1) {
+    while (s.rows > 1 && s.layout.total > 18 * 1024) {
+      s.rows /= 2;
+      s.layout = layout(s.rows);
+    }
+  }
   s.smem = s.layout.total;
   const int64_t rows_total = (a.A + s.rows - 1) / s.rows;
   const int64_t rows_per_split = (rows_total + s.splits - 1) / s.splits;
   s.ant_per_split = std::max<int64_t>(1, rows_per_split) * s.rows;
   return s;
-}
-
-// Lanes that share one output of a PLAIN kernel: one where that fills the GPU with 1024
-// threads per SM (about half of what the sines and cosines need to hide their
-// latency), else 4, 8 where 4 leave less than 768 per SM, a warp where 8 leave less than 512.
-int plain_lanes(int64_t outputs, int64_t terms) {
-  const int64_t sms = current_device_info().sm_count;
-  if (outputs >= sms * 1024 || terms < 16) return 1;
-  return outputs * 4 >= sms * 768 ? 4 : outputs * 8 >= sms * 512 ? 8 : 32;
 }
 
 template <typename T>
@@ -924,7 +987,9 @@ cudaError_t launch_fwd(const MfArgs& a, const FwdShape& s, void* ws, cudaStream_
   p.dup_off = s.layout.dup_off;
 
   const void* fn = fwd_kernel_ptr<T>(a.mode, s.vpt);
-  const int lanes = a.mode == kPlain && s.splits == 1 ? plain_lanes(a.N, a.S) : 1;
+  int lanes = a.mode == kPlain && s.splits == 1 ? plain_lanes(a.N, a.S) : 1;
+  // very long rows leave no room for the exchanged terms
+  if (s.smem + sizeof(TermSums<4>) > static_cast<size_t>(current_device_info().max_smem_optin)) lanes = 1;
   if (lanes > 1) {
     fn = lanes == 4   ? reinterpret_cast<const void*>(&mf_fwd_plain_lanes_kernel<T, 4>)
          : lanes == 8 ? reinterpret_cast<const void*>(&mf_fwd_plain_lanes_kernel<T, 8>)
