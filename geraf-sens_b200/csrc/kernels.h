@@ -209,10 +209,10 @@ struct RaggedArgs {
   float fs, f0, As;
   int dtype;
 };
-// Launch shapes of the batched tracer.  Forward: threads (64, 128, 256),
-// chunk = samples per lane (8, 16, 32), items = points per thread of one work
-// item (0: from the step's size).  Adjoint: stage_rows = residual rows staged
-// per block (1..8; 0: the default of 4, fewer when the rows are long).
+// Launch shapes of the batched tracer.  Forward: items x threads = points of one
+// work item (items 0: from the step's size); the blocks themselves have one shape.
+// Adjoint: stage_rows = residual rows staged per block (1..8; 0: the default of 4,
+// fewer when the rows are long).
 Tuning tracer_ragged_forward_resolve(const RaggedArgs& a, const Tuning& req);
 Tuning tracer_ragged_backward_resolve(const RaggedArgs& a, const Tuning& req);
 size_t tracer_ragged_workspace(int64_t A, int64_t S, int64_t P, const Tuning& t);

@@ -24,6 +24,10 @@
 // the FP64 reduction and the geometry are those of the MIXED form; only the
 // sample sum changes.  Work per (voxel, antenna) is O(W) instead of O(S).
 //
+// Calls of W >= 8 taps that the range cells of the MIXED form take (mf_cells.cu, at
+// least as accurate and faster) run those kernels instead; what is left here are
+// W = 4 and 6, few antennas, float64 arrays, and bands that do not fit the cells.
+//
 // The reference has no such path: its range-bin kernels
 // (MatchedFilter_cuda_kernel.cu:117-169) gather one precomputed bin with no
 // interpolation.  This is an addition of this library.

@@ -20,6 +20,9 @@
 // coefficients weighted by n), and one gather with shared weights evaluates
 // both; the gradient formulas are those of the MIXED adjoint.
 //
+// Calls of W >= 8 taps run the MIXED form's range cells instead (tracer_kernels.cu,
+// resolved_form), which are at least as accurate and faster.
+//
 // No counterpart in the reference.
 #include <algorithm>
 

@@ -54,12 +54,13 @@ extern "C" {
  *        accurate sinf/cosf per (voxel|point, antenna, sample) and the
  *        reference's summation order per output element.  Judged against the
  *        reference kernels (relative L2 <= 1e-5).
- * MIXED: carrier phase f0*tau reduced modulo one cycle in FP64, per-sample
- *        sums by FP32 recurrences (second-order Goertzel, three-term
- *        Chebyshev, packed Horner; a few phasors per (voxel|point, antenna)
- *        instead of one per sample), compensated
- *        (Kahan) accumulation across antennas.  Judged against an FP64 oracle
- *        (relative L2 <= 1e-4).                                              */
+ * MIXED: carrier phase f0*tau reduced modulo one cycle in FP64; the sum over
+ *        the samples through range cells (per antenna, the sum is a smooth
+ *        function of the path length: a polynomial of 6 to 8 terms on each cell
+ *        of 1.9 to 3.7 cm at 4 GHz swept, tables of which are formed in the
+ *        workspace), or by FP32 recurrences over the samples in calls too small
+ *        for tables or with paths beyond them; compensated accumulation across
+ *        antennas.  Judged against an FP64 oracle (relative L2 <= 1e-4).       */
 #define GERAF_MODE_PLAIN 0
 #define GERAF_MODE_MIXED 1
 /* NUFFT (matched filter and signal tracer; no reference counterpart): the
@@ -68,11 +69,16 @@ extern "C" {
  *        interpolation kernel, O(W) instead of O(S) work per
  *        (voxel|point, antenna).  A fast approximate form: relative L2
  *        against the FP64 oracle ~1e-6 at W = 8 (tuning.taps), ~1e-3 at
- *        W = 4.  Needs num_adc_samples <= 4096.  Each adjoint is the exact
- *        adjoint of its forward.  Not available for the ragged tracer.     */
+ *        W = 4.  Needs num_adc_samples <= 4096.  Each adjoint is the
+ *        adjoint of its forward to rounding.  From W = 8 on the range cells of
+ *        the MIXED form, at least as accurate and faster, take its place in the
+ *        tracer and in matched-filter calls large enough for their tables.
+ *        Not available for the ragged tracer.                               */
 #define GERAF_MODE_NUFFT 2
 
-/* Launch shape.  Any field left 0 takes the library default for the call. */
+/* Launch shape.  Any field left 0 takes the library default for the call.  The
+ * fields shape the kernels that they name; calls that go through range cells use
+ * `splits` (tracer) and leave the others to the kernels they fall back to. */
 typedef struct geraf_tuning {
   int32_t threads;          /* threads per block: 64, 128 or 256                       */
   int32_t items_per_thread; /* voxels (MF forward) or points (tracer adjoint): 1, 2, 4 */
@@ -184,7 +190,8 @@ int32_t geraf_mf_forward_noalloc(const void* real, const void* imag, const void*
  * In MIXED and NUFFT mode the forward and the adjoint first list, in their
  * workspace (about 4.3 bytes per point), the in-bounds points that a
  * conservative test cannot cull for every antenna of the call, and visit only
- * those; the workspace is therefore needed even without split partials.
+ * those; the sums over the samples need partials or tables there too, so the
+ * workspace is needed whatever the sizes.
  * Replaces SignalTracer::SignalTracer_forward
  * (geraf/ops/RFSignalTracer/csrc/signal_tracer/SignalTracer_cuda.cu:314-356,
  *  kernel SignalTracer_cuda_kernel.cu:351-450). */
@@ -233,9 +240,9 @@ int32_t geraf_tracer_backward(const void* grad_output_real, const void* grad_out
  * Replaces a loop of SignalTracer::SignalTracer_forward calls, one per antenna
  * (SignalTracer_cuda.cu:314-356): the batched entry point has no single
  * counterpart in the reference. */
-/* Launch shape (`tuning`, may be NULL): threads (64, 128, 256), chunk =
- * samples per lane (8, 16, 32), items_per_thread = points per thread of one
- * work item (0: sized from the step); the workspace size depends on it. */
+/* Launch shape (`tuning`, may be NULL): items_per_thread x threads (64, 128, 256)
+ * = points of one work item (items 0: sized from the step); the workspace size
+ * depends on it.  The blocks' own shape is fixed. */
 int32_t geraf_tracer_ragged_workspace_bytes(int64_t total_ant_size, int64_t num_adc_samples,
                                             int64_t total_point_size, int32_t dtype,
                                             const geraf_tuning_t* tuning, size_t* bytes);
