@@ -38,3 +38,19 @@ def test_backward_bits_do_not_depend_on_the_lanes(cuda, N):
     for a in (1, 64, 128, 512):  # a power of two antennas: dividing by them is exact
         for got, ref in zip(run(a), full):
             np.testing.assert_allclose(got * a, ref[:a] * 2700, rtol=2e-7, atol=0)
+
+
+# rows of several steps of terms, and rows that leave no room in shared memory to exchange terms
+@pytest.mark.parametrize("S", [128, 300, 11500])
+def test_forward_bits_on_long_rows(cuda, S):
+    rng = np.random.default_rng(S)
+    tx, rx = scenes.virtual_array(1)
+    tx, rx = tx[:3], rx[:3]
+    ch = scenes.chirp(S)
+    re, im = rng.standard_normal((2, 3, S)).astype(np.float32)
+    vox = rng.uniform((-0.1, -0.1, 0.3), (0.1, 0.1, 0.5), (160001, 3)).T.astype(np.float32)
+    run = lambda n: mf_forward(re, im, tx, rx, np.ascontiguousarray(vox[:, :n]), ch.adc_sample_rate, ch.As_sci, "plain")
+    full = run(vox.shape[1])
+    for n in (257, 9001, 20003, 40001):
+        for got, ref in zip(run(n), full):
+            np.testing.assert_array_equal(got, ref[:n])
