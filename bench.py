@@ -6,7 +6,8 @@ G (voxel x antenna x sample) per second on the full-size workload -- 49152
 virtual channels (64 x 64 scan x 3TX4RX), 256 ADC samples per chirp, a 128^3
 voxel volume over a cube-shell + torus scene of 30k point scatterers at 20 dB
 SNR (synthetic: the reference's RF data is not released) -- in the MIXED
-arithmetic form (FP64 phase reduction, FP32 Horner phasors, compensated sums).
+arithmetic form (FP64 phase reduction, sample sums through range cells, compensated
+sums).
 
 One step = one backprojection of the whole volume with inputs resident in HBM
 (``value``); ``e2e`` repeats it through the public ``matched_filter_cuda`` call
@@ -14,9 +15,10 @@ from pinned host buffers with the host->device copies and the result read-back
 inside the timed region.  Under torchrun each rank backprojects its own 128^3
 slab of a taller volume (weak scaling, no collective on the data path).
 
-Also reported: the FP32-pipe roofline of the kernel (algorithmic 8 flops per
-voxel-antenna-sample over the measured FP32 FMA rate) with the measured ceiling
-of its Horner loop, and clocks during the timed region.  At N = 1 the line adds
+Also reported: the roofline of the forward's kernel and clocks during the timed
+region.  The MIXED form reads 48 bytes of cell coefficients from shared memory per
+(voxel, antenna) pair, which is what bounds it; the PLAIN form works per sample (8
+flops per voxel-antenna-sample over the measured FP32 FMA rate).  At N = 1 the line adds
 the extras: the PLAIN forward and adjoint, the MIXED MF adjoint, the NUFFT form,
 the tracer forward + adjoint in rays/s, the ragged and stage-1 steps, relative
 L2 errors against the FP64 oracle, and the CPU baseline (the reference-order
@@ -43,6 +45,10 @@ sys.path[:0] = [ROOT, os.path.join(ROOT, "geraf-sens_b200")]
 METRIC = "MF backprojection Gvox·ant·samp/s; tracer fwd+bwd rays/s; rel err vs FP64"
 UNIT = "Gvox·ant·samp/s"
 FLOPS_PER_TRIPLE = 8  # one complex multiply-accumulate of an IF sample by a unit phasor
+# MIXED forward, per (voxel, antenna) pair: six complex coefficients of 8 bytes from shared memory,
+# five steps of a complex-by-real Horner sum and one complex multiply-accumulate
+SMEM_BYTES_PER_PAIR = 48
+FLOPS_PER_PAIR = 5 * 4 + 8
 L2_FLUSH_BYTES = 256 << 20
 
 
@@ -179,15 +185,6 @@ def fp32_peak_tflops(dev) -> float:
     return best
 
 
-def loop_ceiling_tflops(dev) -> float:
-    """Measured rate of the MIXED forward's sample loop alone (geraf_rf_goertzel_probe:
-    the second-order recurrence on packed complex samples, 4 blocks per SM, no
-    per-(voxel, antenna) set-up), the ceiling of that loop's instruction form."""
-    from benchkit import probes
-
-    return probes.measure("goertzel", 4, dev.index or 0)
-
-
 def make_mf_workload(name, rank, world, dev, seed):
     import numpy as np
     import torch
@@ -277,7 +274,40 @@ def launches_per_mf_call(wl, precision) -> int:
     mode = _lib.MODE_MIXED if precision == "mixed" else _lib.MODE_PLAIN
     ws = _lib.workspace_bytes("geraf_mf_forward_workspace_bytes", wl["A"], wl["S"], wl["N"],
                               _lib.DTYPE_F32, mode, None)
+    if precision == "mixed":
+        # the cells' boxes and basis, tables, pairs and sum of the splits; the direct kernel and its
+        # sum are queued behind them and return at once
+        return 6
     return 2 if ws > 0 else 1
+
+
+def mixed_roofline(dev, pairs: float, seconds: float, sm_mhz: float | None) -> dict:
+    """The MIXED forward against the shared-memory bandwidth (128 bytes per SM and clock, at the
+    median SM clock sampled in the timed region): its coefficients are the bytes that a pair
+    cannot do without."""
+    import torch
+
+    achieved = SMEM_BYTES_PER_PAIR * pairs / seconds / 1e12
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    peak = sms * 128 * sm_mhz * 1e6 / 1e12 if sm_mhz else None
+    return {"bound": "shared memory", "achieved": round(achieved, 3), "peak": round(peak, 3) if peak else None,
+            "unit": "TB/s", "frac": round(achieved / peak, 4) if peak else None,
+            "flops_per_launch": FLOPS_PER_PAIR * pairs, "bytes_per_pair": SMEM_BYTES_PER_PAIR,
+            "pairs_per_s_G": round(pairs / seconds / 1e9, 2),
+            "peak_source": "SMs x 128 bytes x the median SM clock sampled in the timed region"}
+
+
+def plain_roofline(dev, triples: float, seconds: float, sm_mhz: float | None, peak: float) -> dict:
+    achieved = FLOPS_PER_TRIPLE * triples / seconds / 1e12
+    roof = {"bound": "fp32", "achieved": round(achieved, 3), "peak": round(peak, 3), "unit": "TFLOP/s",
+            "frac": round(achieved / peak, 4), "flops_per_launch": FLOPS_PER_TRIPLE * triples,
+            "peak_source": "measured FP32 FMA rate (geraf_rf_fma_probe, packed FMA chains) in this process"}
+    spec = spec_fp32_tflops(dev, sm_mhz)
+    if spec is not None:
+        roof["spec_fp32_at_clock"] = {
+            "value": round(spec, 3), "unit": "TFLOP/s", "frac": round(achieved / spec, 4),
+            "source": "SMs x 128 FP32 lanes x 2 flops x the median SM clock sampled in the timed region"}
+    return roof
 
 
 def read_profile_traffic(workload: str):
@@ -381,9 +411,11 @@ def run_ours(args):
     e2e_value = world * triples / (e2e_ms * 1e-3) / 1e9
 
     peak = fp32_peak_tflops(dev)
-    ceiling = loop_ceiling_tflops(dev) if args.precision == "mixed" else None
-    achieved = FLOPS_PER_TRIPLE * triples / (kms * 1e-3) / 1e12
-    traffic = read_profile_traffic(args.workload)
+    sm_mhz = (clock_info or {}).get("sm_mhz")
+    roofline = (mixed_roofline(dev, float(A) * N, kms * 1e-3, sm_mhz) if args.precision == "mixed"
+                else plain_roofline(dev, triples, kms * 1e-3, sm_mhz, peak))
+    roofline["traffic"] = read_profile_traffic(args.workload)
+    roofline["kernel_ms"] = round(kms, 3)
     launches = launches_per_mf_call(wl, args.precision) * args.steps
 
     line = {
@@ -401,27 +433,10 @@ def run_ours(args):
         "parallelism": f"voxel slabs x{world}, no collective",
         "e2e": {"value": round(e2e_value, 3), "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h), "steps": e2e_steps},
-        "roofline": {"bound": "fp32", "achieved": round(achieved, 3), "peak": round(peak, 3),
-                     "unit": "TFLOP/s", "frac": round(achieved / peak, 4), "traffic": traffic,
-                     "flops_per_launch": FLOPS_PER_TRIPLE * triples,
-                     "peak_source": "measured FP32 FMA rate (geraf_rf_fma_probe, packed FMA chains) in this process",
-                     "kernel_ms": round(kms, 3)},
+        "roofline": roofline,
         "gpu_launches": launches,
         "clocks": clock_info,
     }
-    spec = spec_fp32_tflops(dev, (clock_info or {}).get("sm_mhz"))
-    if spec is not None:
-        line["roofline"]["spec_fp32_at_clock"] = {
-            "value": round(spec, 3), "unit": "TFLOP/s", "frac": round(achieved / spec, 4),
-            "source": "SMs x 128 FP32 lanes x 2 flops x the median SM clock sampled in the timed region"}
-    if ceiling is not None:
-        # The sample loop alone, without the per-(voxel, antenna) set-up: the ceiling of
-        # the kernel's instruction form, below the FMA-rate peak (operand fetch).
-        line["roofline"]["loop_ceiling"] = {
-            "value": round(ceiling, 3), "unit": "TFLOP/s", "frac_of_peak": round(ceiling / peak, 4),
-            "kernel_frac_of_ceiling": round(achieved / ceiling, 4),
-            "source": "geraf_rf_goertzel_probe (the forward's second-order recurrence loop alone, "
-                      "4 blocks per SM) in this process"}
 
     # The extras are single-GPU measurements: under torchrun (N > 1) they would only hold
     # every GPU while rank 0 repeats them, so they run at N = 1 alone.
@@ -677,7 +692,8 @@ def _adjoint_extra(args, wl, dev, art) -> dict:
 
 def _nufft_extra(wl, dev, out_r, out_i, art) -> dict:
     """The matched filter's fast approximate form (oversampled range FFT + 8-point
-    ES interpolation) on the full workload: forward and adjoint times, in the
+    ES interpolation; at this size and width the library runs the MIXED form's range cells
+    in its place) on the full workload: forward and adjoint times, in the
     headline's unit (the same voxel x antenna x sample sums, evaluated in O(W)
     per voxel-antenna pair), and their relative L2 against the MIXED form over
     every output element (the MIXED form is itself ~2e-7 from FP64)."""
@@ -742,7 +758,7 @@ def tracer_live_pairs(tw, chunk: int = 8) -> int:
 def tracer_listed_points(tw) -> int:
     """Points that the MIXED tracer's per-point pre-cull keeps (the in-bounds
     points it cannot cull for every antenna; csrc/tracer_precull.cu), restated in
-    torch FP64 on the device."""
+    torch on the device: the kernel's FP32 test with its margin of 2e-4, in FP64."""
     import torch
 
     d = torch.float64
@@ -758,11 +774,11 @@ def tracer_listed_points(tw) -> int:
     nrm, m = nn.sqrt(), 1.0 + 2.0 * nn
     icn = (ic * n).sum(1)
     ni, no = ic.norm(dim=1), oc.norm(dim=1)
-    back = icn - rt * nrm > 1e-4 * (ni + rt) * nrm
+    back = icn - rt * nrm > 2e-4 * (ni + rt) * nrm
     hi = ic - 2.0 * icn[:, None] * n
     ho = oc - 2.0 * (oc * n).sum(1)[:, None] * n
     bound = (oc * hi).sum(1) + rr * hi.norm(dim=1) + rt * ho.norm(dim=1) + m * rr * rt
-    away = bound < -1e-4 * (no + rr) * (ni + rt) * m
+    away = bound < -2e-4 * (no + rr) * (ni + rt) * m
     return int((tw["inbounds"] & ~(back | away)).sum())
 
 
@@ -829,7 +845,8 @@ def _tracer_extra(args, dev, art) -> dict:
     tr["nufft"]["rel_l2_vs_mixed"] = {k: rel(outs["nufft"][i], outs["mixed"][i])
                                       for i, k in enumerate(("signal", "grad_sigmas", "grad_normals",
                                                              "grad_points"))}
-    # roofline of the MIXED forward + adjoint: 12 flops per (point, antenna, sample)
+    # the direct sums' 12 flops per (point, antenna, sample) as an equivalent rate: the range cells
+    # do not work per sample, so it may exceed the FMA rate
     live = tracer_live_pairs(tw)
     peak = art.get("fp32_peak")
     flops_all = 12.0 * At * P * St
@@ -843,10 +860,11 @@ def _tracer_extra(args, dev, art) -> dict:
         roof["peak"] = round(peak, 3)
         roof["frac_all"] = round(flops_all / (ms_m * 1e-3) / 1e12 / peak, 4)
         roof["frac_live"] = round(flops_live / (ms_m * 1e-3) / 1e12 / peak, 4)
-        roof["note"] = ("frac_live is the roofline: culled pairs carry no samples to sum; frac_all "
-                        "counts every triple as the reference's kernels visit them.  The kernels form "
-                        "the geometry of every pair of the points the per-point pre-cull keeps "
-                        "(listed_point_fraction) and sum the samples of live pairs only")
+        roof["note"] = ("equivalent rates of the direct per-sample sums: frac_live over the samples of live "
+                        "pairs, frac_all over every triple as the reference's kernels visit them.  The "
+                        "kernels test every pair of the points the per-point pre-cull keeps "
+                        "(listed_point_fraction) and sum the live pairs through range cells, a fixed "
+                        "number of operations per pair instead of one per sample")
     res["tracer"] = {"workload": f"{At} antennas x {tw['rays']} rays x {P // tw['rays']} samples, S={St}",
                      "unit": "rays/s (ray = ray x antenna pair)", "mixed_with_point_grads": tr["mixed"],
                      "nufft_with_point_grads": tr["nufft"], "plain": tr["plain"], "roofline": roof,
