@@ -394,13 +394,14 @@ __global__ void __launch_bounds__(256) mf_fwd_plain_kernel(const MfFwdP<T> p) {
 // chains of the last step are added up by a lane each, in the reference's order.  The warps
 // take turns at that, so that their schedulers carry the same load.  The adds are then as
 // few as with a thread per output; each lane adding all of its output's terms, from a row
-// of its warp's, took 70 instructions per term instead of about 58 (13824 voxels x 300 antennas x 128
-// samples: forward and adjoint 2.54 ms, so 2.23 ms).
+// of its warp's, took 70 instructions per term (13824 voxels x 300 antennas x 128 samples: forward
+// and adjoint 2.54 ms, so 2.06 ms).
 template <int LANES>
 struct TermSums {
   static constexpr int kThreads = 128;
-  // groups of LANES terms per output and step: 2, 4 and 8 of 8 lanes 2.90, 2.50 and 2.23 ms
-  // (a barrier per step), 12 or more cost resident blocks; a step of 128 terms of a warp
+  // groups of LANES terms per output and step: 2, 4 and 8 of 8 lanes took 2.90, 2.50 and 2.23 ms (a
+  // barrier per step; 2.06 ms with the registers of six blocks per SM and no clamped indexes in
+  // full steps), 12 or more cost resident blocks
   static constexpr int kGroups = LANES < 32 ? 8 : 4;
   static constexpr int kTerms = kGroups * LANES;
   static constexpr int kChains = 2 * kThreads / LANES;
@@ -445,10 +446,10 @@ struct TermSums {
 // PLAIN forward with LANES lanes per voxel, for calls of too few voxels to fill the GPU
 // with one thread each (every thread is bound by the latency of its sines and
 // cosines: 13824 voxels x 300 antennas x 128 samples take 3.70 ms at one thread per
-// voxel, 1.13 ms at 8).  Lane j evaluates samples j, j + LANES, ...; the terms are added in
+// voxel, 1.06 ms at 8).  Lane j evaluates samples j, j + LANES, ...; the terms are added in
 // sample order, so the sums are the one-thread kernel's to the bit.
 template <typename T, int LANES>
-__global__ void __launch_bounds__(128) mf_fwd_plain_lanes_kernel(const MfFwdP<T> p) {
+__global__ void __launch_bounds__(128, 6) mf_fwd_plain_lanes_kernel(const MfFwdP<T> p) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ TermSums<LANES> sums;
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
@@ -500,8 +501,7 @@ __global__ void __launch_bounds__(128) mf_fwd_plain_lanes_kernel(const MfFwdP<T>
       const float base_phase = 2.0f * kPiF * kMfStartFrequency * tau;
       const T* rowr = stg.stage_ptr(s, 0) + r * p.ld;
       const T* rowi = stg.stage_ptr(s, 1) + r * p.ld;
-      auto term = [&](int n0, int u) {
-        const int n = min(n0 + u * LANES + lane, S - 1);
+      auto term = [&](int n, int u) {
         const float phase = base_phase + kn[n] * tau;
         float cos_phase, sin_phase;
         cos_sin(phase, &cos_phase, &sin_phase);
@@ -514,9 +514,9 @@ __global__ void __launch_bounds__(128) mf_fwd_plain_lanes_kernel(const MfFwdP<T>
       for (int n0 = 0; n0 < S; n0 += Sums::kTerms) {
         if (n0 + Sums::kTerms <= S) {
 #pragma unroll
-          for (int u = 0; u < Sums::kGroups; ++u) term(n0, u);
+          for (int u = 0; u < Sums::kGroups; ++u) term(n0 + lane + u * LANES, u);
         } else {
-          for (int u = 0; n0 + u * LANES < S; ++u) term(n0, u);
+          for (int u = 0; n0 + u * LANES < S; ++u) term(min(n0 + lane + u * LANES, S - 1), u);
         }
         sums.add(step, count);
         count = min(Sums::kTerms, S - n0);
@@ -669,9 +669,9 @@ __global__ void __launch_bounds__(256) mf_bwd_mixed_kernel(const MfBwdP<T> p) {
 // once per voxel tile in shared memory.
 // LANES lanes per sample, for calls of few antennas x samples: lane j evaluates voxels j,
 // j + LANES, ... and the terms are added in voxel order, so the sums do not depend on
-// LANES (300 antennas x 128 samples x 13824 voxels: 1.71 ms with one lane, 1.10 ms with 4).
+// LANES (300 antennas x 128 samples x 13824 voxels: 1.71 ms with one lane, 1.06 ms with 4).
 template <typename T, int LANES>
-__global__ void __launch_bounds__(128) mf_bwd_plain_kernel(const MfBwdP<T> p) {
+__global__ void __launch_bounds__(128, 6) mf_bwd_plain_kernel(const MfBwdP<T> p) {
   constexpr int TILE = 256;
   __shared__ float s_tau[TILE], s_gr[TILE], s_gi[TILE];
   using Sums = TermSums<LANES == 1 ? 4 : LANES>;
@@ -729,17 +729,17 @@ __global__ void __launch_bounds__(128) mf_bwd_plain_kernel(const MfBwdP<T> p) {
       __syncthreads();
     } else {
       // samples past S run along (the block exchanges its terms) and are not stored
-      auto put = [&](int i0, int u) {
+      auto put = [&](int i, int u) {
         float term_r, term_i;
-        term(min(i0 + u * LANES + lane, count - 1), term_r, term_i);
+        term(i, term_r, term_i);
         sums.put(step, u, term_r, term_i);
       };
       for (int i0 = 0; i0 < count; i0 += Sums::kTerms) {
         if (i0 + Sums::kTerms <= count) {
 #pragma unroll
-          for (int u = 0; u < Sums::kGroups; ++u) put(i0, u);
+          for (int u = 0; u < Sums::kGroups; ++u) put(i0 + lane + u * LANES, u);
         } else {
-          for (int u = 0; i0 + u * LANES < count; ++u) put(i0, u);
+          for (int u = 0; i0 + u * LANES < count; ++u) put(min(i0 + lane + u * LANES, count - 1), u);
         }
         sums.add(step, left);
         left = min(Sums::kTerms, count - i0);
