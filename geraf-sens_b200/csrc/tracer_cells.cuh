@@ -11,7 +11,7 @@
 // expensive part (on a typical scene one point in ten is live).  The 128 points'
 // contributions are then sorted by cell in shared memory and added up by groups
 // of eight lanes, one per moment, in list order: no floating-point atomics, and the
-// same bits on every run as long as the run's cells fit the slots below.  (Sums by each
+// same bits on every run.  (Sums by each
 // warp alone, over the set bits of its match masks and without barriers, took as long for
 // the pre-cull's lists and 40 us longer for 64 antennas x 295000 screened points.)
 //
@@ -78,6 +78,7 @@ struct TraceSmem {
   int4 hist[kTraceSlots];  // per warp
   int start[kTraceSlots + 1];
   int tag[kTraceSlots];
+  int claim[kTraceSlots];  // lowest cell that wants an empty slot
   int list[kTraceThreads * (kTracePer + 1)];
   alignas(16) int counts[kTracePer * kTraceWarps];
   uint32_t defer[kTraceRun / 32];
@@ -104,6 +105,7 @@ __device__ __forceinline__ void trace_begin(TraceSmem& sm) {
   }
   for (int i = threadIdx.x; i < kTraceSlots; i += kTraceThreads) {
     sm.tag[i] = kTraceEmpty;
+    sm.claim[i] = INT32_MAX;
     sm.hist[i] = make_int4(0, 0, 0, 0);
   }
   for (int i = threadIdx.x; i < kTraceRun / 32; i += kTraceThreads) sm.defer[i] = 0u;
@@ -128,7 +130,10 @@ static __device__ __noinline__ void trace_evict(TraceSmem& sm, const TraceConsts
   for (int i = threadIdx.x; i < kTraceSlots * kTraceQ; i += kTraceThreads) {
     (&sm.moments[0][0])[i] = make_float2(0.0f, 0.0f);
   }
-  for (int s = threadIdx.x; s < kTraceSlots; s += kTraceThreads) sm.tag[s] = kTraceEmpty;
+  for (int s = threadIdx.x; s < kTraceSlots; s += kTraceThreads) {
+    sm.tag[s] = kTraceEmpty;
+    sm.claim[s] = INT32_MAX;
+  }
   if (threadIdx.x == 0) sm.has_row = 1;
   __syncthreads();
 }
@@ -138,12 +143,13 @@ static __device__ __noinline__ void trace_evict(TraceSmem& sm, const TraceConsts
 __device__ __forceinline__ bool trace_batch(TraceSmem& sm, bool live, float2 w, int k, float x, int pos) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int slot = k & (kTraceSlots - 1);
-  bool in = false;
-  if (live) {
-    const int old = sm.tag[slot] == k ? k : atomicCAS(&sm.tag[slot], kTraceEmpty, k);
-    in = old == kTraceEmpty || old == k;
-    if (!in) atomicOr(&sm.defer[pos >> 5], 1u << (pos & 31));
-  }
+  // An empty slot goes to the lowest cell of the batch that wants it, whatever the order of
+  // the threads; it is settled below, and those that lose it leave rows of zeros.
+  int held = k;
+  if (live) held = sm.tag[slot];
+  const bool want = held == kTraceEmpty;
+  if (want) atomicMin(&sm.claim[slot], k);
+  const bool in = live && (want || held == k);
   const unsigned same = __match_any_sync(0xffffffffu, in ? slot : kTraceSlots);
   const int rank = __popc(same & ((1u << lane) - 1u));
   if (in && rank == 0) reinterpret_cast<int*>(&sm.hist[slot])[warp] = __popc(same);
@@ -164,12 +170,25 @@ __device__ __forceinline__ bool trace_batch(TraceSmem& sm, bool live, float2 w, 
     const int f = e + sa;
     sm.hist[2 * lane + 1] = make_int4(f, f + b.x, f + b.x + b.y, f + b.x + b.y + b.z);
     if (lane == 31) sm.start[kTraceSlots] = run;
+  } else if (warp == 1) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int c = sm.claim[lane + 32 * j];
+      if (c != INT32_MAX && sm.tag[lane + 32 * j] == kTraceEmpty) sm.tag[lane + 32 * j] = c;
+    }
   }
   __syncthreads();
+  bool out = held != k;
+  if (want) out = sm.tag[slot] != k;
+  if (out) atomicOr(&sm.defer[pos >> 5], 1u << (pos & 31));
   if (in) {  // the contribution row w x^q, at its place in cell order
     const int place = reinterpret_cast<const int*>(&sm.hist[slot])[warp] + rank;
     float4* dst = reinterpret_cast<float4*>(&sm.rows[place][0]);
     float2 v = w;
+    if (out) {
+      v = make_float2(0.0f, 0.0f);
+      x = 0.0f;
+    }
 #pragma unroll
     for (int q = 0; q < kTraceQ; q += 2) {
       const float2 u = make_float2(v.x * x, v.y * x);
@@ -188,7 +207,7 @@ __device__ __forceinline__ bool trace_batch(TraceSmem& sm, bool live, float2 w, 
     for (int i = i0; i < i1; ++i) acc = fadd2(acc, sm.rows[i][q]);
     sm.moments[s][q] = acc;
   }
-  return __syncthreads_or(live && !in) != 0;
+  return __syncthreads_or(out) != 0;
 }
 
 // A point and its contribution.

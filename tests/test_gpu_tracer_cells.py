@@ -96,3 +96,13 @@ def test_ragged_runs(cuda, depth):
             pairs[k].append((counts[a] * got[e].double().cpu().numpy(), counts[a] * ref))
     for p in pairs:
         assert rel_l2(np.concatenate([g for g, _ in p]), np.concatenate([r for _, r in p])) < TOL
+
+
+@pytest.mark.parametrize("depth", [(0.3, 0.5), (0.3, 3.3)], ids=["near", "deep"])
+def test_forward_bits_repeat(cuda, depth):
+    """Which cell takes a slot does not depend on the order of the threads."""
+    c = case(7, 7, 20000, 128, depth)
+    first = tracer_forward(c, c["S"], "mixed", tuning={"splits": 2})
+    for _ in range(5):
+        for got, ref in zip(tracer_forward(c, c["S"], "mixed", tuning={"splits": 2}), first):
+            np.testing.assert_array_equal(got, ref)
