@@ -29,10 +29,11 @@ constexpr int kTableTile = 256;  // samples staged at a time by the table kernel
 struct CellHead {
   int bad;  // set when some antenna's cells do not fit: the direct kernel runs instead
   int pad[3];
+  double center[3];  // of the voxels' box: the origin of AntMeta and of the pairs' legs
 };
 
 struct AntMeta {
-  double t[4];  // -2 t, |t|^2 in units of 2^-20 m (biased, see leg_length)
+  double t[4];  // -2 t, |t|^2 from the centre, in units of 2^-20 m (biased, see leg_length)
   double r[4];
   int c0, cells;  // first cell (absolute) and number of cells
   int same_tx;    // the transmitter equals the preceding antenna's
@@ -171,12 +172,16 @@ __global__ void __launch_bounds__(kTableThreads) mf_cell_table_kernel(const Tabl
     double vv = 0.0;
     bool same = a > 0;
 #pragma unroll
-    for (int c = 0; c < 6; ++c) box[c] = box_s[c];
-#pragma unroll
     for (int c = 0; c < 3; ++c) {
       t[c] = ld_f(p.tx, a * 3 + c);
       r[c] = ld_f(p.rx, a * 3 + c);
       if (a > 0) same = same && t[c] == static_cast<double>(ld_f(p.tx, (a - 1) * 3 + c));
+      const double center = box_center(box_s[c], box_s[3 + c]);
+      if (a == 0) p.head->center[c] = center;
+      box[c] = box_s[c] - center;
+      box[3 + c] = box_s[3 + c] - center;
+      t[c] -= center;
+      r[c] -= center;
       const double e = fmax(fabs(box[c]), fabs(box[3 + c]));
       vv = fma(e, e, vv);
     }
@@ -371,7 +376,8 @@ __global__ void __launch_bounds__(kGatherThreads + 32, kGatherBlocks) mf_cell_ga
       for (int w = 1; w < kGatherThreads / 32; ++w) {
         r = threadIdx.x < 3 ? fminf(r, sm.red[w][threadIdx.x]) : fmaxf(r, sm.red[w][threadIdx.x]);
       }
-      sm.box[threadIdx.x] = r;
+      // from the centre, as the antennas' positions are; all NaN voxels leave an empty box
+      sm.box[threadIdx.x] = static_cast<float>(static_cast<double>(r) - p.head->center[threadIdx.x % 3]);
     }
     if (threadIdx.x == 32) {
       for (int s = 0; s < kGatherStages; ++s) {
@@ -402,7 +408,10 @@ __global__ void __launch_bounds__(kGatherThreads + 32, kGatherBlocks) mf_cell_ga
         c0 = m.c0;
         leg_range(tp, sm.box, tn, tf);
         leg_range(rp, sm.box, rn, rf);
-        // one cell of margin on either side covers the FP32 rounding (~1e-4 cells)
+        // One cell of margin on either side covers the FP32 rounding: positions from the centre
+        // are below 8 m and paths below 16 m (kMaxLeg), good to 3e-6 m in all, a third of a
+        // cell at the narrowest cells taken (1e5 per metre, mf_cells_scale_ok).  The pairs'
+        // cells therefore stay in the row without a check per pair.
         lo = static_cast<int>(floorf((sqrtf(tn) + sqrtf(rn)) * p.kappa)) - 1 - c0;
         int hi = static_cast<int>(ceilf((sqrtf(tf) + sqrtf(rf)) * p.kappa)) + 1 - c0;
         lo = min(max(lo, 0), m.cells - 1);
@@ -448,9 +457,9 @@ __global__ void __launch_bounds__(kGatherThreads + 32, kGatherBlocks) mf_cell_ga
 #pragma unroll
   for (int j = 0; j < VPT; ++j) {
     const bool nan = (nan_voxel >> j) & 1u;
-    vx[j] = static_cast<double>(nan ? sm.box[0] : fx[j]) * kUnit;
-    vy[j] = static_cast<double>(nan ? sm.box[1] : fy[j]) * kUnit;
-    vz[j] = static_cast<double>(nan ? sm.box[2] : fz[j]) * kUnit;
+    vx[j] = (nan ? sm.box[0] : fx[j] - p.head->center[0]) * kUnit;
+    vy[j] = (nan ? sm.box[1] : fy[j] - p.head->center[1]) * kUnit;
+    vz[j] = (nan ? sm.box[2] : fz[j] - p.head->center[2]) * kUnit;
     vv[j] = fma(vx[j], vx[j], fma(vy[j], vy[j], vz[j] * vz[j]));
   }
   float yr[VPT], yi[VPT], cr[VPT], ci[VPT];
@@ -614,7 +623,8 @@ struct MomentHead {
   int bad;
   int k0, cells;
   int pad;
-  double bias;  // |v|^2 bound for leg_antenna
+  double bias;       // |v|^2 bound for leg_antenna
+  double center[3];  // of the voxels' box: the origin of the pairs' legs
 };
 
 struct MomentLayout {
@@ -724,8 +734,10 @@ __global__ void __launch_bounds__(32 * 19) moment_band_kernel(const float* parti
       near[e] += gap * gap;
       far[e] += reach * reach;
     }
-    const double m = fmax(fabs(lo), fabs(hi));
+    const double center = box_center(s[k], s[3 + k]);
+    const double m = fmax(fabs(lo - center), fabs(hi - center));
     vv += m * m;
+    head->center[k] = center;
   }
   const double ft = sqrt(far[0]), fr = sqrt(far[1]);
   const double lo = floor((sqrt(near[0]) + sqrt(near[1])) * kappa) - 1.0, hi = ceil((ft + fr) * kappa) + 1.0;
@@ -810,8 +822,8 @@ __global__ void __launch_bounds__(128, 4) mf_moment_kernel(const MomentP<T> p) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const float ht = __shfl_sync(0xffffffffu, t[c], want), hr = __shfl_sync(0xffffffffu, r[c], want);
-      own[c] = shared_legs ? (lane < nt ? ht : hr) : t[c];
-      other[c] = r[c];
+      own[c] = static_cast<double>(shared_legs ? (lane < nt ? ht : hr) : t[c]) - p.head->center[c];
+      other[c] = static_cast<double>(r[c]) - p.head->center[c];
     }
     leg_antenna(own, p.head->bias, mt);
     leg_antenna(other, p.head->bias, mr);
@@ -842,18 +854,18 @@ __global__ void __launch_bounds__(128, 4) mf_moment_kernel(const MomentP<T> p) {
       if (v < v_end) {
         const float fx = ld_f(p.voxel, v), fy = ld_f(p.voxel, p.N + v), fz = ld_f(p.voxel, 2 * p.N + v);
         g = make_float2(ld_f(p.gr, v), ld_f(p.gi, v));
-        x = fx * kUnit;
-        y = fy * kUnit;
-        z = fz * kUnit;
+        x = (fx - p.head->center[0]) * kUnit;
+        y = (fy - p.head->center[1]) * kUnit;
+        z = (fz - p.head->center[2]) * kUnit;
         if (fx != fx || fy != fy || fz != fz) g = make_float2(NAN, NAN);  // its every sample is NaN
       }
       if (v >= v_end || g.x != g.x) {
-        // somewhere in the box: the split's first voxel, or antenna 0's cell k0 when that is NaN too
+        // somewhere in the box: the split's first voxel, or the box's centre when that is NaN too
         const float fx = ld_f(p.voxel, v_begin), fy = ld_f(p.voxel, p.N + v_begin), fz = ld_f(p.voxel, 2 * p.N + v_begin);
         const bool ok = fx == fx && fy == fy && fz == fz;
-        x = ok ? fx * kUnit : 0.0;
-        y = ok ? fy * kUnit : 0.0;
-        z = ok ? fz * kUnit : 0.0;
+        x = ok ? (fx - p.head->center[0]) * kUnit : 0.0;
+        y = ok ? (fy - p.head->center[1]) * kUnit : 0.0;
+        z = ok ? (fz - p.head->center[2]) * kUnit : 0.0;
       }
       sxy[i] = make_double2(x, y);
       szv[i] = make_double2(z, fma(x, x, fma(y, y, z * z)));

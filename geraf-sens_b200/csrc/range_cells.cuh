@@ -65,6 +65,11 @@ __device__ __forceinline__ float rsqrt_fast(float x) {
 // s = |t - v|^2 = |t|^2 + |v|^2 - 2 t.v in FP64: 4 operations instead of 6, its
 // cancellation (~1e-16 of the squared coordinates) far below what the phase
 // needs (~1e-10 m^2).  tt carries a bias of that size so that s stays positive.
+// Both hold only for coordinates that are small themselves, so t and v are taken from
+// the centre of the scene's box (box_center), differences that FP64 forms exactly or
+// nearly so: the centre is no further from an antenna than the box's far corner, so with legs
+// below 8 m both stay below 8 m wherever the scene lies (about an origin 3 km away the
+// phase would be off by 5e-4 rad, about one 1000 km away by cells).
 // No conversion between FP32 and FP64 is issued: they share the 16-lane unit of the
 // rsqrt, sine and cosine, which bounded the kernel with them (115 issue cycles
 // per 32 pairs of the forward at 3072 x 110592 pairs); the words are shifted or
@@ -140,7 +145,12 @@ __device__ __forceinline__ CellPos pair_cell(const PairPhase& p, float hi, float
   return c;
 }
 
-// A point's or an antenna's coordinates for leg_length.
+// Middle of one side of the scene's box.
+__device__ __forceinline__ double box_center(float lo, float hi) {
+  return 0.5 * (static_cast<double>(lo) + static_cast<double>(hi));
+}
+
+// An antenna's coordinates for leg_length; bias bounds the voxels' |v|^2.
 __device__ __forceinline__ void leg_antenna(const double* t, double bias, double* m) {
 #pragma unroll
   for (int c = 0; c < 3; ++c) m[c] = -2.0 * kUnit * t[c];

@@ -169,3 +169,25 @@ def test_forward_non_finite_inputs(cuda):
     y = forward(c)
     keep = np.setdiff1d(np.arange(y.size), [77, 600])
     assert rel_l2(y[keep], ref[keep]) < 1e-5 and not np.isfinite(y[77])
+
+
+# The result does not depend on where the scene lies: only differences of positions enter it.  The
+# oracle takes the same FP32 positions, whose grid at the largest offset is 6 cm.
+@pytest.mark.parametrize("offset", [(0.0, 0.0, 100.0), (-1e3, 300.0, 0.0), (3e3, 3e3, -3e3), (1e4, 0.0, 0.0), (0.0, 1e6, 0.0)])
+@pytest.mark.parametrize("precision", ["mixed", "nufft"])
+def test_scenes_far_from_the_origin(cuda, offset, precision):
+    A, S, N = 140, 128, 6001
+    c = case(11, A, S, N)
+    for k in ("tx", "rx"):
+        c[k] = np.ascontiguousarray((c[k] + np.array(offset)).astype(np.float32))
+    c["vox"] = np.ascontiguousarray((c["vox"] + np.array(offset)[:, None]).astype(np.float32))
+    ch = c["ch"]
+    args = c["tx"], c["rx"], c["vox"]
+    pos = c["vox"][:, c["rng"].integers(0, N, 6)].T
+    c["re"], c["im"] = scenes.synthesize_if_numpy(*args[:2], pos, np.ones(6) + 0.5j, ch, snr_db=20.0, rng=c["rng"])
+    y = mf_forward(c["re"], c["im"], *args, ch.adc_sample_rate, ch.As_sci, precision)
+    assert rel_l2(y[0] + 1j * y[1], oracle(c)) < TOL
+    gr, gi = c["rng"].standard_normal((2, N)).astype(np.float32)
+    h = mf_backward(gr, gi, *args, A, S, ch.adc_sample_rate, ch.As_sci, precision)
+    r = orc.mf_backward(gr, gi, *args, A, S, ch.adc_sample_rate, ch.As_sci)
+    assert rel_l2(h[0] + 1j * h[1], r[0] + 1j * r[1]) < TOL
