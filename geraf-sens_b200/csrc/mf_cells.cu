@@ -770,7 +770,9 @@ __device__ __forceinline__ void red_add4(float4* dst, float2 a, float2 b) {
 // One thread per antenna; the voxels of the block's split pass through shared
 // memory in tiles and every thread reads the same one (broadcast).  The moments
 // of the thread's current cell stay in registers; consecutive voxels mostly
-// share a cell, and when it changes the moments are added to the antenna's own
+// share a cell, and when it changes, and after each tile (so that a cell that holds
+// hundreds of thousands of voxels is summed in two levels: one chain of 200000 terms of one
+// sign erred by 2e-5), the moments are added to the antenna's own
 // record in memory (vector reductions without a return value: nothing waits for
 // them, and no other thread touches the record, so the order of its sums, and the
 // result, is the same on every run).  About 88 instructions per 32 pairs (100 where the
@@ -840,9 +842,10 @@ __global__ void __launch_bounds__(128, 4) mf_moment_kernel(const MomentP<T> p) {
   auto flush = [&]() {
     const int k = static_cast<int>(__float_as_uint(cur) - kRoundMagicBits) - k0;
     float4* dst = rec + static_cast<int64_t>(min(max(k, 0), cells - 1)) * (Q / 2) * p.apad;
-    if (mine) {
 #pragma unroll
-      for (int q = 0; q < Q; q += 2) red_add4(dst + (q / 2) * p.apad, M[q], M[q + 1]);
+    for (int q = 0; q < Q; q += 2) {
+      if (mine) red_add4(dst + (q / 2) * p.apad, M[q], M[q + 1]);
+      M[q] = M[q + 1] = make_float2(0.0f, 0.0f);
     }
   };
   for (int64_t v0 = v_begin; v0 < v_end; v0 += kMomentTile) {
@@ -902,8 +905,6 @@ __global__ void __launch_bounds__(128, 4) mf_moment_kernel(const MomentP<T> p) {
           if (m[u] != cur) {
             flush();
             cur = m[u];
-#pragma unroll
-            for (int q = 0; q < Q; ++q) M[q] = make_float2(0.0f, 0.0f);
           }
           // even moments from w, odd ones from w x, both times powers of x^2 (a chain of
           // three products, not seven: 5.03 -> 4.98 ms of the 3072 x 256 x 64^3 step)
@@ -923,41 +924,38 @@ __global__ void __launch_bounds__(128, 4) mf_moment_kernel(const MomentP<T> p) {
     };
     if (shared_legs) sum_tile(std::true_type{});
     else sum_tile(std::false_type{});
+    flush();  // no chain of sums in registers is longer than a tile
   }
-  flush();
 }
 
 // Sums the splits' records into the first one's: block (x: 32 antennas, y: a pair
-// of moments of one cell), 16 warps over the splits, in a fixed order.
+// of moments of one cell), 16 warps over the splits, in a fixed order and in FP64, as the
+// partial sums of the other forms are.
 constexpr int kSumWarps = 16;
 
 __global__ void __launch_bounds__(32 * kSumWarps) mf_moment_sum_kernel(float4* moments, const MomentHead* head,
                                                                        int64_t apad, int splits, int pairs) {
-  __shared__ float4 part[kSumWarps][32];
+  __shared__ double part[kSumWarps][4][32];
   if (head->bad || static_cast<int>(blockIdx.y) >= head->cells * pairs) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t stride = static_cast<int64_t>(kMomentCap) * pairs * apad;
   float4* src = moments + static_cast<int64_t>(blockIdx.y) * apad + blockIdx.x * 32 + lane;
-  float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 4
   for (int k = warp; k < splits; k += kSumWarps) {
     const float4 y = src[k * stride];
-    s.x += y.x;
-    s.y += y.y;
-    s.z += y.z;
-    s.w += y.w;
+    s[0] += y.x;
+    s[1] += y.y;
+    s[2] += y.z;
+    s[3] += y.w;
   }
-  part[warp][lane] = s;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) part[warp][c][lane] = s[c];
   __syncthreads();
-  if (warp != 0) return;
-  for (int w = 1; w < kSumWarps; ++w) {
-    const float4 y = part[w][lane];
-    s.x += y.x;
-    s.y += y.y;
-    s.z += y.z;
-    s.w += y.w;
-  }
-  *src = s;
+  if (warp >= 4) return;
+  double t = 0.0;  // warp c: component c
+  for (int w = 0; w < kSumWarps; ++w) t += part[w][warp][lane];
+  (&src->x)[warp] = static_cast<float>(t);
 }
 
 template <typename T>
