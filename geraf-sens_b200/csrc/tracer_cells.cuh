@@ -85,8 +85,8 @@ struct TraceSmem {
   int has_row;
 };
 
-// Adds a cell's moments, seen by sample n, to acc.
-__device__ __forceinline__ void add_cell(const TraceConsts& c, int k, const float2* m, const float* g, int n, float2& acc) {
+// A cell's moments as sample n sees them.
+__device__ __forceinline__ float2 cell_sample(const TraceConsts& c, int k, const float2* m, const float* g, int n) {
   const double ph = (n - 0.5 * (c.S - 1)) * fma(c.k1, k * c.inv_kappa, c.b1);
   const float2 e = cis_cycles(static_cast<float>(ph - rint(ph)));
   float2 ev = make_float2(0.0f, 0.0f), od = make_float2(0.0f, 0.0f);
@@ -95,8 +95,7 @@ __device__ __forceinline__ void add_cell(const TraceConsts& c, int k, const floa
     ev = ffma2(make_float2(g[q], g[q]), m[q], ev);
     od = ffma2(make_float2(g[q + 1], g[q + 1]), m[q + 1], od);
   }
-  const float2 z = cmul(e, make_float2(ev.x - od.y, ev.y + od.x));
-  acc = fadd2(acc, z);
+  return cmul(e, make_float2(ev.x - od.y, ev.y + od.x));
 }
 
 __device__ __forceinline__ void trace_begin(TraceSmem& sm) {
@@ -122,7 +121,7 @@ static __device__ __noinline__ void trace_evict(TraceSmem& sm, const TraceConsts
     cell_basis<kTraceQ>(c.theta_step * (n - 0.5 * (c.S - 1)), g);
     float2 acc = first ? make_float2(0.0f, 0.0f) : row[n];
     for (int s = 0; s < kTraceSlots; ++s) {
-      if (sm.tag[s] != kTraceEmpty) add_cell(c, sm.tag[s], sm.moments[s], g, n, acc);
+      if (sm.tag[s] != kTraceEmpty) acc = fadd2(acc, cell_sample(c, sm.tag[s], sm.moments[s], g, n));
     }
     row[n] = acc;
   }
@@ -202,10 +201,12 @@ __device__ __forceinline__ bool trace_batch(TraceSmem& sm, bool live, float2 w, 
   for (int s = threadIdx.x / kTraceQ; s < kTraceSlots; s += kTraceThreads / kTraceQ) {
     const int i0 = sm.start[s], i1 = sm.start[s + 1];
     if (i0 == i1) continue;
-    float2 acc = sm.moments[s][q];
+    // the batch's sum first, then onto the cell's: two levels, so that a cell of hundreds of
+    // thousands of points errs by the square root of its batches, not of its points
+    float2 acc = sm.rows[i0][q];
 #pragma unroll 4
-    for (int i = i0; i < i1; ++i) acc = fadd2(acc, sm.rows[i][q]);
-    sm.moments[s][q] = acc;
+    for (int i = i0 + 1; i < i1; ++i) acc = fadd2(acc, sm.rows[i][q]);
+    sm.moments[s][q] = fadd2(sm.moments[s][q], acc);
   }
   return __syncthreads_or(out) != 0;
 }
@@ -424,16 +425,18 @@ __device__ __forceinline__ void trace_store(const TraceSmem& sm, TraceRecord* re
 //
 // A call has few such blocks (one per antenna), so each is bound by latency: four
 // groups of threads take every fourth run's moments, then every fourth slot's cells, and
-// add up in a fixed order.  13 antennas x 78 runs: 44 us with one group, 14 us with four;
+// add up in a fixed order, in FP64 as the partial sums of the other forms are.  13 antennas x 78 runs: 44 us with one group, 14 us with four;
 // 64 antennas x 23 runs: 19.5 and 10.9 us.
 constexpr int kFinishSamples = 256;
 constexpr int kFinishGroups = 4;
 constexpr int kFinishThreads = kFinishSamples * kFinishGroups;
 
 struct FinishSmem {
-  float4 part[kFinishGroups][kTraceSlots][kTraceQ / 2];
+  union {
+    double4 part[kFinishGroups][kTraceSlots][kTraceQ / 2];
+    double2 acc[kFinishGroups][kFinishSamples];
+  };
   float2 mom[kTraceSlots][kTraceQ];
-  float2 acc[kFinishGroups][kFinishSamples];
   int next[kFinishGroups][kTraceSlots], top[kFinishGroups][kTraceSlots];
   int tag[kTraceSlots];
 };
@@ -447,13 +450,17 @@ __device__ __forceinline__ void trace_finish(const TraceConsts& c, const TraceRe
   const int slot = in_group / (kTraceQ / 2), pair = in_group % (kTraceQ / 2);
   const int n = n_begin + in_group;
   const bool mine = n < n_end;
-  float2 acc = make_float2(0.0f, 0.0f);
+  double2 acc = make_double2(0.0, 0.0);
+  auto add = [](double2& s, float2 x) {
+    s.x += x.x;
+    s.y += x.y;
+  };
   float g[kTraceQ];
   bool rowed = false;
   for (int64_t r = threadIdx.x; r < runs; r += kFinishThreads) rowed = rowed || rec[r].has_row != 0;
   if (__syncthreads_or(rowed) && mine) {
     for (int64_t r = group; r < runs; r += kFinishGroups) {
-      if (rec[r].has_row) acc = fadd2(acc, rows[r * c.S + n]);
+      if (rec[r].has_row) add(acc, rows[r * c.S + n]);
     }
   }
   if (mine) cell_basis<kTraceQ>(c.theta_step * (n - 0.5 * (c.S - 1)), g);
@@ -484,7 +491,7 @@ __device__ __forceinline__ void trace_finish(const TraceConsts& c, const TraceRe
       next = min(next, sm.next[k][slot]);
       top = max(top, sm.top[k][slot]);
     }
-    float4 m = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    double4 m = make_double4(0.0, 0.0, 0.0, 0.0);
     if (next != INT32_MAX) {
 #pragma unroll 8
       for (int64_t r = group; r < runs; r += kFinishGroups) {
@@ -504,31 +511,35 @@ __device__ __forceinline__ void trace_finish(const TraceConsts& c, const TraceRe
     if (group == 0) {
 #pragma unroll
       for (int k = 1; k < kFinishGroups; ++k) {
-        const float4 y = sm.part[k][slot][pair];
+        const double4 y = sm.part[k][slot][pair];
         m.x += y.x;
         m.y += y.y;
         m.z += y.z;
         m.w += y.w;
       }
-      reinterpret_cast<float4*>(&sm.mom[slot][0])[pair] = m;
+      reinterpret_cast<float4*>(&sm.mom[slot][0])[pair] =
+          make_float4(static_cast<float>(m.x), static_cast<float>(m.y), static_cast<float>(m.z), static_cast<float>(m.w));
       if (pair == 0) sm.tag[slot] = next;  // INT32_MAX: none
     }
     __syncthreads();
     if (mine) {
       for (int k = group; k < kTraceSlots; k += kFinishGroups) {
-        if (sm.tag[k] != INT32_MAX) add_cell(c, sm.tag[k], sm.mom[k], g, n, acc);
+        if (sm.tag[k] != INT32_MAX) add(acc, cell_sample(c, sm.tag[k], sm.mom[k], g, n));
       }
     }
     if (!again) break;
     __syncthreads();
   }
-  sm.acc[group][in_group] = acc;
+  sm.acc[group][in_group] = acc;  // over part, last read before the last barrier
   __syncthreads();
   if (group == 0 && mine) {
 #pragma unroll
-    for (int k = 1; k < kFinishGroups; ++k) acc = fadd2(acc, sm.acc[k][in_group]);
-    out_r[n] = from_f<T>(acc.x / divisor);
-    out_i[n] = from_f<T>(acc.y / divisor);
+    for (int k = 1; k < kFinishGroups; ++k) {
+      acc.x += sm.acc[k][in_group].x;
+      acc.y += sm.acc[k][in_group].y;
+    }
+    out_r[n] = from_f<T>(static_cast<float>(acc.x) / divisor);
+    out_i[n] = from_f<T>(static_cast<float>(acc.y) / divisor);
   }
 }
 
