@@ -148,8 +148,12 @@ __device__ __forceinline__ float dot3f(const float* a, const float* b) {
 // True when every pair of the point is culled with the margin above.  The offsets
 // from the centres are formed in FP64 (exact to ~1e-16 of the coordinates), the rest in
 // FP32 with the margin doubled: its rounding, below 3e-6 of the terms compared, leaves
-// every culled point well inside the 1e-4 that the argument needs.  (In FP64 throughout,
-// the four square roots and ~60 operations took 12 us for 524288 points.)
+// every culled point well inside the 1e-4 that the argument needs.  That holds for squares
+// that FP32 carries to full precision only: normals or offsets shorter than 1e-15, whose
+// squares near or pass its smallest normal number (and vanish in sqrt_rough, and the margin
+// with them), are left to the exact form.  Overflowing terms end in infinities or NaN on the
+// side that lists the point.  (In FP64 throughout, the four square roots and ~60 operations
+// took 12 us for 524288 points.)
 __device__ __forceinline__ bool culled_for_all(const Aperture& ap, const float* n, const float* pf) {
   constexpr float kMargin = 2e-4f;
   float ic[3], oc[3];
@@ -159,13 +163,14 @@ __device__ __forceinline__ bool culled_for_all(const Aperture& ap, const float* 
     oc[k] = static_cast<float>(ap.cr[k] - static_cast<double>(pf[k]));
   }
   const float rt = static_cast<float>(ap.rt), rr = static_cast<float>(ap.rr);
-  const float nn = dot3f(n, n);
+  const float nn = dot3f(n, n), ii = dot3f(ic, ic), oo = dot3f(oc, oc);
+  if (!(fminf(nn, fminf(ii, oo)) > 1e-30f)) return false;
   const float nrm = sqrt_rough(nn);
   const float m = 1.0f + 2.0f * nn;
   const float icn = dot3f(ic, n);
-  const float ni = sqrt_rough(dot3f(ic, ic)) + rt;
+  const float ni = sqrt_rough(ii) + rt;
   if (icn - rt * nrm > kMargin * ni * nrm) return true;
-  const float no = sqrt_rough(dot3f(oc, oc)) + rr;
+  const float no = sqrt_rough(oo) + rr;
   const float ocn = dot3f(oc, n);
   float hi[3], ho[3];
 #pragma unroll

@@ -8,7 +8,9 @@ import numpy as np
 import pytest
 import torch
 
+from conftest import rel_l2
 from gpu_helpers import tracer_backward, tracer_forward
+from oracle import rf_oracle as orc
 from oracle import workload_parity as wp
 
 pytestmark = pytest.mark.gpu
@@ -194,3 +196,26 @@ def test_precull_one_block_kernels(cuda, A, P, S):
     rows = np.arange(0, A, max(1, A // 4))
     err = wp.tracer_forward_error(_c(tracer_forward(w, S, "mixed")), w, rows)
     assert err < MIXED_TOL
+
+
+@pytest.mark.parametrize("length", [1e-22, 1e-20, 1e-12, 1.0])
+def test_short_normals_keep_their_aperture_margin(cuda, length):
+    """Receivers behind the points, transmitters on both sides of them: each point faces the
+    transmitter of one side, whatever the length of its normal (the signs of the products
+    decide, and hardly any reflection bends a path that short normals leave straight)."""
+    rng = np.random.default_rng(4)
+    P, S, A = 2000, 64, 8
+    f = np.float32
+    side = np.where(np.arange(A) % 2 == 0, 1.0, -1.0)
+    tx = np.stack([0.1 * side, np.zeros(A), np.zeros(A)], 1).astype(f)
+    rx = np.stack([0.02 * side, np.zeros(A), np.full(A, 0.8)], 1).astype(f)
+    pts = rng.uniform((0.01, -0.05, 0.35), (0.05, 0.05, 0.45), (P, 3)).astype(f)
+    # along x, the aperture's wide side: i.n > 0 for the left transmitters and the centre, < 0 for the right
+    nrm = np.broadcast_to(np.array([length, 0, 0]), (P, 3)).astype(f)
+    fs, f0, As, inb = 5.0e6, 770.0, 4e9 * 5e6 / S / 1e8, np.ones(P, bool)
+    sig = rng.uniform(0, 1, (A, P)).astype(f)
+    w = dict(normals=nrm, sigmas=sig, points=pts, tx=tx, rx=rx, inbounds=inb, fs=fs, f0=f0, As=As)
+    got = _c(tracer_forward(w, S, "mixed"))
+    ref = _c(orc.tracer_forward(nrm, sig, pts, tx, rx, inb, S, fs, f0, As, "f64"))
+    assert np.abs(ref[side > 0]).max() > 0 and np.abs(ref[side < 0]).max() == 0
+    assert rel_l2(got, ref) < MIXED_TOL

@@ -352,3 +352,65 @@ def test_point_precull_is_conservative():
         skipped += int(skip.sum())
         total += M
     assert skipped > total // 4  # most points facing away are left out
+
+
+def _culled_for_all_f32(ap, n, p):
+    """numpy restatement of culled_for_all() in csrc/tracer_precull.cu as the kernel evaluates it:
+    offsets from FP64 differences, the rest in FP32, a square root that flushes denormal
+    numbers, a margin of 2e-4, and normals or offsets below 1e-15 left to the exact form."""
+    f = np.float32
+    ct, rt, cr, rr = ap
+    rt, rr = f(rt), f(rr)
+
+    def dot(a, b):
+        return (a * b).sum(1, dtype=f)
+
+    def root(x):
+        return np.sqrt(np.where(x < f(1.17549435e-38), f(0), x))
+
+    ic = (p.astype(np.float64) - ct).astype(f)
+    oc = (cr - p.astype(np.float64)).astype(f)
+    nn, ii, oo = dot(n, n), dot(ic, ic), dot(oc, oc)
+    nrm, m = root(nn), f(1) + f(2) * nn
+    icn, ocn = dot(ic, n), dot(oc, n)
+    ni, no = root(ii) + rt, root(oo) + rr
+    hi = ic - f(2) * icn[:, None] * n
+    ho = oc - f(2) * ocn[:, None] * n
+    bound = dot(oc, hi) + rr * root(dot(hi, hi)) + rt * root(dot(ho, ho)) + m * rr * rt
+    culled = (icn - rt * nrm > f(2e-4) * ni * nrm) | (bound < f(-2e-4) * no * ni * m)
+    return culled & (np.minimum(nn, np.minimum(ii, oo)) > f(1e-30))
+
+
+def test_point_precull_rounds_on_the_safe_side():
+    """The pre-cull as the kernel rounds it, on points pushed onto its own boundary (normals found
+    by bisection between one it culls and one it lists), with normals from 1e-25 to 1e3 long and
+    compact, wide and distant apertures: what it leaves out is culled for every antenna."""
+    rng = np.random.default_rng(2)
+    f = np.float32
+    skipped = 0
+    with np.errstate(over="ignore", under="ignore", invalid="ignore"):
+        for trial in range(10):
+            A, M = 16, 30_000
+            spread = (0.0, 0.002, 0.02, 0.1, 0.3)[trial % 5]
+            at = np.array([0.0, 0.0, 0.0]) if trial < 5 else np.array([40.0, -3.0, 7.0])
+            tx = (at + rng.normal(0, spread, (A, 3))).astype(f)
+            rx = (at + rng.normal(0, max(spread / 2, 1e-3), (A, 3)) + (trial % 3 == 2) * np.array([0.3, 0.0, 0.9])).astype(f)
+            p = (at + np.array([0, 0, 0.4]) + rng.normal(0, 0.15, (M, 3))).astype(f)
+            ap = _aperture_f64(tx, rx)
+            scale = 10.0 ** rng.uniform(*((-25.0, 3.0) if trial % 2 else (-0.5, 0.5)), (M, 1))
+            n0, n1 = rng.normal(0, 1, (2, M, 3))
+            n0, n1 = (x / np.linalg.norm(x, axis=1, keepdims=True) * scale for x in (n0, n1))
+            at_0 = _culled_for_all_f32(ap, n0.astype(f), p)
+            lo, hi = np.zeros((M, 1)), np.ones((M, 1))
+            for _ in range(40):  # the side of n0 stays at lo
+                mid = 0.5 * (lo + hi)
+                same = _culled_for_all_f32(ap, (n0 + mid * (n1 - n0)).astype(f), p) == at_0
+                lo, hi = np.where(same[:, None], mid, lo), np.where(same[:, None], hi, mid)
+            for t in (lo, hi):
+                n = (n0 + t * (n1 - n0)).astype(f)
+                skip = _culled_for_all_f32(ap, n, p)
+                for a in range(A):
+                    exact = _culled_reference_f32(np.broadcast_to(tx[a], p.shape), np.broadcast_to(rx[a], p.shape), n, p)
+                    assert not np.any(skip & ~exact), (trial, a)
+                skipped += int(skip.sum())
+    assert skipped > 50_000
