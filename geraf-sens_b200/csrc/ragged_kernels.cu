@@ -134,6 +134,14 @@ __device__ __forceinline__ int64_t item_antenna(const int64_t* item_offsets, int
   return lo;
 }
 
+// Points [first, first + count) of antenna a.
+template <typename T>
+__device__ __forceinline__ void item_range(const RgP<T>& p, int64_t item, int64_t& a, int64_t& first, int64_t& count) {
+  a = item_antenna(p.item_offsets, p.A, item);
+  first = p.offsets[a] + (item - p.item_offsets[a]) * p.chunk;
+  count = min(p.offsets[a + 1] - first, static_cast<int64_t>(p.chunk));
+}
+
 // Each work item's points go into the moments of their cells (tracer_cells.cuh).
 // 64 antennas x 295000 points each (10% live) x 256 samples: 173 us against 590 us with
 // a recurrence over the samples of every live point and a compaction per 128 points.
@@ -147,19 +155,38 @@ __global__ void __launch_bounds__(kTraceThreads, 6) ragged_fwd_kernel(const RgP<
     __syncthreads();
     const int64_t item = s_item;
     if (item >= total) break;
-    const int64_t a = item_antenna(p.item_offsets, p.A, item);
-    const int64_t first = p.offsets[a] + (item - p.item_offsets[a]) * p.chunk;
-    const int64_t count = min(p.offsets[a + 1] - first, static_cast<int64_t>(p.chunk));
+    int64_t a, first, count;
+    item_range(p, item, a, first, count);
     float txp[3], rxp[3];
     ld3(p.tx, a, txp);
     ld3(p.rx, a, rxp);
     trace_begin(sm);
-    for (int64_t at = first; at < first + count; at += kTraceRun) {
-      trace_screened<T>(sm, p.c, p.rows + item * p.c.S, p.normals + at * 3, p.points + at * 3, p.sigmas + at,
-                        p.inb != nullptr ? p.inb + at : nullptr, txp, rxp,
-                        static_cast<int>(min(first + count - at, static_cast<int64_t>(kTraceRun))));
+    const bool fits = trace_screened<T>(sm, p.c, p.normals + first * 3, p.points + first * 3, p.sigmas + first,
+                                        p.inb != nullptr ? p.inb + first : nullptr, txp, rxp, static_cast<int>(count));
+    if (!fits) {  // no cells: the record is a row, from ragged_fwd_direct_kernel
+      for (int i = threadIdx.x; i < kTraceSlots; i += kTraceThreads) sm.tag[i] = kTraceEmpty;
     }
-    trace_store(sm, p.records + item);
+    trace_store(sm, p.records + item, !fits);
+  }
+}
+
+// The items whose cells do not fit their slots; a launch without any reads their records'
+// flags alone.  (Within the kernel above it would take registers from the cells: 3 to 35%.)
+template <typename T>
+__global__ void __launch_bounds__(kTraceThreads) ragged_fwd_direct_kernel(const RgP<T> p) {
+  __shared__ DirectSmem sm;
+  const int64_t total = p.item_offsets[p.A];
+  for (int64_t item = blockIdx.x; item < total; item += gridDim.x) {
+    if (p.records[item].has_row == 0) continue;
+    int64_t a, first, count;
+    item_range(p, item, a, first, count);
+    float txp[3], rxp[3];
+    ld3(p.tx, a, txp);
+    ld3(p.rx, a, rxp);
+    trace_direct<T>(
+        sm, p.c, p.normals, p.points, txp, rxp, count,
+        [&](int64_t pos) -> int64_t { return p.inb == nullptr || p.inb[first + pos] ? first + pos : -1; },
+        [&](int64_t q) { return ld_f(p.sigmas, q); }, [&](int n, float2 y) { p.rows[item * p.c.S + n] = y; });
   }
 }
 
@@ -437,6 +464,7 @@ cudaError_t launch_ragged_fwd(const RaggedArgs& a, const Tuning& t, void* ws, cu
   const int64_t blocks = std::max<int64_t>(
       1, std::min<int64_t>(static_cast<int64_t>(per_sm) * current_device_info().sm_count, p.max_items));
   ragged_fwd_kernel<T><<<static_cast<unsigned>(blocks), kTraceThreads, 0, st>>>(p);
+  ragged_fwd_direct_kernel<T><<<static_cast<unsigned>(blocks), kTraceThreads, 0, st>>>(p);
   const dim3 grid(static_cast<unsigned>(a.A), static_cast<unsigned>((a.S + kFinishSamples - 1) / kFinishSamples));
   ragged_finish_kernel<T><<<grid, kFinishThreads, 0, st>>>(p);
   return cudaGetLastError();

@@ -15,13 +15,14 @@
 // warp alone, over the set bits of its match masks and without barriers, took as long for
 // the pre-cull's lists and 40 us longer for 64 antennas x 295000 screened points.)
 //
-// Cells are kept in kTraceSlots slots, cell k in slot k mod kTraceSlots.  Points whose
-// slot another cell of the run holds (2.4 m of path away at 4 GHz swept) are
-// deferred: when the run's other points are done, the moments so far are turned into
-// samples, added to the run's row of samples, and the deferred points have the slots
-// to themselves.  A wide scene thus takes a few passes over its live points, not one
-// conversion per conflict.  (128 slots took 10 to 13% longer on scenes that need a
-// dozen cells.)
+// Cells are kept in kTraceSlots slots, cell k in slot k mod kTraceSlots.  (128 slots took 10
+// to 13% longer on scenes that need a dozen cells.)  Points whose cells share a slot are
+// 2.4 m of path or more apart (at 4 GHz swept): the block then leaves the rest of its share
+// (of a list; a screened share as a whole) to trace_direct, at the cost of a recurrence over
+// the samples but whatever the scene's depth.  Measured on 64 antennas x 262144 points, 10% live,
+// x 128 samples: 68 us through the cells in a scene 0.2 m deep, 106 us in one 3 m deep
+// (several passes over the points, each with its own cells, took 197 us there and 851 us in
+// one 30 m deep).
 #pragma once
 
 #include "range_cells.cuh"
@@ -36,7 +37,6 @@ constexpr int kTracePer = 4;  // points per thread and screening pass
 constexpr int kTraceQ = MomentCells::Q;
 constexpr int kTraceSlots = 64;
 constexpr int kTraceEmpty = INT32_MIN + 1;  // no finite path has this cell
-constexpr int kTraceRun = 16384;            // positions per run, at most (the deferral mask's size)
 constexpr int kTraceRow = kTraceQ + 2;      // float2 per contribution row: 80 bytes, conflict-free
 
 struct TraceConsts {
@@ -63,8 +63,8 @@ inline TraceConsts trace_consts(double k0, double b0, double k1, double b1, int6
   return t;
 }
 
-// A run's result: moments of the cells in its slots (tag kTraceEmpty: unused), and a
-// row of S samples when `rows` says that cells were evicted.
+// A share's result: moments of the cells in its slots (tag kTraceEmpty: unused), and a
+// row of S samples when has_row says so.
 struct TraceRecord {
   float2 moments[kTraceSlots][kTraceQ];
   int tag[kTraceSlots];
@@ -78,11 +78,8 @@ struct TraceSmem {
   int4 hist[kTraceSlots];  // per warp
   int start[kTraceSlots + 1];
   int tag[kTraceSlots];
-  int claim[kTraceSlots];  // lowest cell that wants an empty slot
   int list[kTraceThreads * (kTracePer + 1)];
   alignas(16) int counts[kTracePer * kTraceWarps];
-  uint32_t defer[kTraceRun / 32];
-  int has_row;
 };
 
 // A cell's moments as sample n sees them.
@@ -104,54 +101,24 @@ __device__ __forceinline__ void trace_begin(TraceSmem& sm) {
   }
   for (int i = threadIdx.x; i < kTraceSlots; i += kTraceThreads) {
     sm.tag[i] = kTraceEmpty;
-    sm.claim[i] = INT32_MAX;
     sm.hist[i] = make_int4(0, 0, 0, 0);
   }
-  for (int i = threadIdx.x; i < kTraceRun / 32; i += kTraceThreads) sm.defer[i] = 0u;
-  if (threadIdx.x == 0) sm.has_row = 0;
   __syncthreads();
 }
 
-// The moments of all slots go to the run's row of samples (in device memory, touched
-// by this block only) and the slots are emptied.
-static __device__ __noinline__ void trace_evict(TraceSmem& sm, const TraceConsts c, float2* row) {
-  const bool first = sm.has_row == 0;
-  for (int n = threadIdx.x; n < c.S; n += kTraceThreads) {
-    float g[kTraceQ];
-    cell_basis<kTraceQ>(c.theta_step * (n - 0.5 * (c.S - 1)), g);
-    float2 acc = first ? make_float2(0.0f, 0.0f) : row[n];
-    for (int s = 0; s < kTraceSlots; ++s) {
-      if (sm.tag[s] != kTraceEmpty) acc = fadd2(acc, cell_sample(c, sm.tag[s], sm.moments[s], g, n));
-    }
-    row[n] = acc;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < kTraceSlots * kTraceQ; i += kTraceThreads) {
-    (&sm.moments[0][0])[i] = make_float2(0.0f, 0.0f);
-  }
-  for (int s = threadIdx.x; s < kTraceSlots; s += kTraceThreads) {
-    sm.tag[s] = kTraceEmpty;
-    sm.claim[s] = INT32_MAX;
-  }
-  if (threadIdx.x == 0) sm.has_row = 1;
-  __syncthreads();
-}
-
-// One batch: thread t holds a live contribution w at cell k, offset x, of the run's
-// position `pos` (or none).  Returns, on every thread, whether any was deferred.
-__device__ __forceinline__ bool trace_batch(TraceSmem& sm, bool live, float2 w, int k, float x, int pos) {
+// One batch: thread t holds a live contribution w at cell k, offset x (or none).  False, on
+// every thread, when two cells want one slot, whatever the order of the threads: nothing of
+// the batch is then added, and with KEEP the slots are as they were.
+template <bool KEEP>
+__device__ __forceinline__ bool trace_batch(TraceSmem& sm, bool live, float2 w, int k, float x) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int slot = k & (kTraceSlots - 1);
-  // An empty slot goes to the lowest cell of the batch that wants it, whatever the order of
-  // the threads; it is settled below, and those that lose it leave rows of zeros.
   int held = k;
   if (live) held = sm.tag[slot];
-  const bool want = held == kTraceEmpty;
-  if (want) atomicMin(&sm.claim[slot], k);
-  const bool in = live && (want || held == k);
-  const unsigned same = __match_any_sync(0xffffffffu, in ? slot : kTraceSlots);
+  if (held == kTraceEmpty) sm.tag[slot] = k;  // one of them stays
+  const unsigned same = __match_any_sync(0xffffffffu, live ? slot : kTraceSlots);
   const int rank = __popc(same & ((1u << lane) - 1u));
-  if (in && rank == 0) reinterpret_cast<int*>(&sm.hist[slot])[warp] = __popc(same);
+  if (live && rank == 0) reinterpret_cast<int*>(&sm.hist[slot])[warp] = __popc(same);
   __syncthreads();
   if (warp == 0) {  // exclusive prefix over (slot, warp), two slots per lane
     const int4 a = sm.hist[2 * lane], b = sm.hist[2 * lane + 1];
@@ -169,25 +136,13 @@ __device__ __forceinline__ bool trace_batch(TraceSmem& sm, bool live, float2 w, 
     const int f = e + sa;
     sm.hist[2 * lane + 1] = make_int4(f, f + b.x, f + b.x + b.y, f + b.x + b.y + b.z);
     if (lane == 31) sm.start[kTraceSlots] = run;
-  } else if (warp == 1) {
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int c = sm.claim[lane + 32 * j];
-      if (c != INT32_MAX && sm.tag[lane + 32 * j] == kTraceEmpty) sm.tag[lane + 32 * j] = c;
-    }
   }
   __syncthreads();
-  bool out = held != k;
-  if (want) out = sm.tag[slot] != k;
-  if (out) atomicOr(&sm.defer[pos >> 5], 1u << (pos & 31));
-  if (in) {  // the contribution row w x^q, at its place in cell order
+  const bool other = live && sm.tag[slot] != k;
+  if (live) {  // the contribution row w x^q, at its place in cell order
     const int place = reinterpret_cast<const int*>(&sm.hist[slot])[warp] + rank;
     float4* dst = reinterpret_cast<float4*>(&sm.rows[place][0]);
     float2 v = w;
-    if (out) {
-      v = make_float2(0.0f, 0.0f);
-      x = 0.0f;
-    }
 #pragma unroll
     for (int q = 0; q < kTraceQ; q += 2) {
       const float2 u = make_float2(v.x * x, v.y * x);
@@ -195,7 +150,10 @@ __device__ __forceinline__ bool trace_batch(TraceSmem& sm, bool live, float2 w, 
       v = make_float2(u.x * x, u.y * x);
     }
   }
-  __syncthreads();
+  if (__syncthreads_or(other)) {
+    if (KEEP && held == kTraceEmpty) sm.tag[slot] = kTraceEmpty;  // the slots that this batch took
+    return false;
+  }
   for (int i = threadIdx.x; i < kTraceSlots; i += kTraceThreads) sm.hist[i] = make_int4(0, 0, 0, 0);
   const int q = threadIdx.x & (kTraceQ - 1);
   for (int s = threadIdx.x / kTraceQ; s < kTraceSlots; s += kTraceThreads / kTraceQ) {
@@ -208,7 +166,8 @@ __device__ __forceinline__ bool trace_batch(TraceSmem& sm, bool live, float2 w, 
     for (int i = i0 + 1; i < i1; ++i) acc = fadd2(acc, sm.rows[i][q]);
     sm.moments[s][q] = fadd2(sm.moments[s][q], acc);
   }
-  return __syncthreads_or(out) != 0;
+  __syncthreads();
+  return true;
 }
 
 // A point and its contribution.
@@ -225,11 +184,11 @@ __device__ __forceinline__ void load_point(const T* normals, const T* points, in
   }
 }
 
-__device__ __forceinline__ bool trace_point(const TraceConsts& c, const float* txp, const float* rxp, const TracePoint& t,
-                                            float2& w, int& cell, float& x) {
+// Amplitude and path length of a live point.
+__device__ __forceinline__ bool trace_path(const float* txp, const float* rxp, const TracePoint& t, float& amp, double& d) {
   PairGeom g;
   if (!pair_geometry(txp, rxp, t.nrm, t.pt, g)) return false;
-  const float amp = t.sigma * g.align / sq(g.dist);
+  amp = t.sigma * g.align / sq(g.dist);
   double st = 0.0, sr = 0.0;
 #pragma unroll
   for (int a = 2; a >= 0; --a) {
@@ -238,7 +197,15 @@ __device__ __forceinline__ bool trace_point(const TraceConsts& c, const float* t
     st = fma(dt, dt, st);
     sr = fma(dr, dr, sr);
   }
-  const double d = sqrt_f64_fast(st) + sqrt_f64_fast(sr);
+  d = sqrt_f64_fast(st) + sqrt_f64_fast(sr);
+  return true;
+}
+
+__device__ __forceinline__ bool trace_point(const TraceConsts& c, const float* txp, const float* rxp, const TracePoint& t,
+                                            float2& w, int& cell, float& x) {
+  float amp;
+  double d;
+  if (!trace_path(txp, rxp, t, amp, d)) return false;
   const double ph = fma(d, c.K, c.b);
   const double u = d * c.kappa, ku = rint(u);
   cell = fabs(ku) < 1073741824.0 ? static_cast<int>(ku) : 0;  // a non-finite path: w is NaN
@@ -248,25 +215,69 @@ __device__ __forceinline__ bool trace_point(const TraceConsts& c, const float* t
   return true;
 }
 
-// A run's list of positions, filled 512 positions at a time and served in batches of 128.
+// `count` positions in batches of consecutive ones: for points of
+// which most are live (the pre-cull's list).  index_of gives the point at a position, or -1 when
+// it is out of bounds.  The next batch's points are loaded while one is summed.  Returns how
+// many positions are in the moments: all, or those before the first batch that is not.
 template <typename T, typename IndexOf, typename SigmaOf>
-struct TraceList {
-  TraceSmem& sm;
-  const TraceConsts& c;
-  const T* normals;
-  const T* points;
-  const float* txp;
-  const float* rxp;
-  IndexOf index_of;  // the point at a position, or -1 when it is out of bounds
-  SigmaOf sigma_of;
-  int listed = 0;
-  bool deferred = false;
+__device__ __forceinline__ int trace_all(TraceSmem& sm, const TraceConsts& c, const T* normals, const T* points,
+                                          const float* txp, const float* rxp, int count, IndexOf index_of,
+                                          SigmaOf sigma_of) {
+  TracePoint next;
+  int64_t next_q = -1;
+  auto load = [&](int pos) {
+    next_q = pos < count ? index_of(pos) : -1;
+    if (next_q >= 0) {
+      load_point(normals, points, next_q, next.nrm, next.pt);
+      next.sigma = sigma_of(next_q);
+    }
+  };
+  load(threadIdx.x);
+  for (int p0 = 0; p0 < count; p0 += kTraceThreads) {
+    float2 w = make_float2(0.0f, 0.0f);
+    float x = 0.0f;
+    int cell = 0;
+    const bool live = next_q >= 0 && trace_point(c, txp, rxp, next, w, cell, x);
+    load(p0 + kTraceThreads + threadIdx.x);
+    if (!trace_batch<true>(sm, live, w, cell, x)) return p0;
+  }
+  return count;
+}
 
-  // Lane l of warp w keeps position p0 + 128 j + 32 w + l where bit l of its mask[j] is set.
-  // The list's order is that of (warp, j, lane): the same on every run.
-  __device__ __forceinline__ void append(int p0, const unsigned (&mask)[kTracePer]) {
-    static_assert(kTracePer == 4, "one 16-byte load per warp's counts");
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// `count` consecutive points (their arrays from the first one on; inb may be null), screened first: those that the early test cannot cull are listed, 512
+// positions at a time, and served in batches of 128.  False when a batch was not added.
+template <typename T>
+__device__ __forceinline__ bool trace_screened(TraceSmem& sm, const TraceConsts& c, const T* normals, const T* points,
+                                               const T* sigmas, const uint8_t* inb, const float* txp, const float* rxp,
+                                               int count) {
+  static_assert(kTracePer == 4, "one 16-byte load per warp's counts");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int listed = 0;
+  float nrm[kTracePer][3], pt[kTracePer][3];
+  unsigned in = 0;  // bit j: point j of the thread is in bounds
+  auto load = [&](int p0) {  // of the next pass, in flight while batches are summed
+    in = 0;
+    const int rest = count - p0 - static_cast<int>(threadIdx.x);
+    const T* pn = normals + (static_cast<int64_t>(p0) + threadIdx.x) * 3;
+    const T* pp = points + (static_cast<int64_t>(p0) + threadIdx.x) * 3;
+    const uint8_t* pb = inb != nullptr ? inb + p0 + threadIdx.x : nullptr;
+#pragma unroll
+    for (int j = 0; j < kTracePer; ++j) {
+      if (j * kTraceThreads < rest && (pb == nullptr || pb[j * kTraceThreads])) {
+        in |= 1u << j;
+        load_point(pn, pp, j * kTraceThreads, nrm[j], pt[j]);
+      }
+    }
+  };
+  load(0);
+  for (int p0 = 0; p0 < count; p0 += kTraceThreads * kTracePer) {
+    // Lane l of warp w keeps position p0 + 128 j + 32 w + l where bit l of its mask[j] is set.
+    // The list's order is that of (warp, j, lane): the same on every run.
+    unsigned mask[kTracePer];
+#pragma unroll
+    for (int j = 0; j < kTracePer; ++j) {
+      mask[j] = __ballot_sync(0xffffffffu, ((in >> j) & 1u) && !surely_culled(txp, rxp, nrm[j], pt[j]));
+    }
     if (lane == 0) {
       *reinterpret_cast<int4*>(&sm.counts[warp * kTracePer]) =
           make_int4(__popc(mask[0]), __popc(mask[1]), __popc(mask[2]), __popc(mask[3]));
@@ -288,134 +299,125 @@ struct TraceList {
       before += n.x + n.y + n.z + n.w;
     }
     listed = before;
-  }
-
-  // The full batches, or all of the list (after a barrier that follows append).
-  __device__ __forceinline__ void serve(bool drain) {
+    load(p0 + kTraceThreads * kTracePer);
+    __syncthreads();
+    const bool drain = p0 + kTraceThreads * kTracePer >= count;
     while (listed >= kTraceThreads || (drain && listed > 0)) {
       const int cnt = min(listed, kTraceThreads);
       listed -= cnt;
       bool live = false;
       float2 w = make_float2(0.0f, 0.0f);
       float x = 0.0f;
-      int cell = 0, pos = 0;
+      int cell = 0;
       if (threadIdx.x < cnt) {
-        pos = sm.list[listed + threadIdx.x];
-        const int64_t q = index_of(pos);
+        const int q = sm.list[listed + threadIdx.x];
         TracePoint t;
         load_point(normals, points, q, t.nrm, t.pt);
-        t.sigma = sigma_of(q);
+        t.sigma = ld_f(sigmas, q);
         live = trace_point(c, txp, rxp, t, w, cell, x);
       }
-      if (trace_batch(sm, live, w, cell, x, pos)) deferred = true;
+      if (!trace_batch<false>(sm, live, w, cell, x)) return false;
     }
   }
+  return true;
+}
 
-  // Passes over the deferred positions until none is left.
-  __device__ __forceinline__ void serve_deferred(int count, float2* row) {
-    while (deferred) {
-      deferred = false;
-      trace_evict(sm, c, row);
-      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-      for (int p0 = 0; p0 < count; p0 += kTraceThreads * kTracePer) {
-        unsigned mask[kTracePer];
-#pragma unroll
-        for (int j = 0; j < kTracePer; ++j) {
-          const int word = (p0 >> 5) + j * kTraceWarps + warp;
-          mask[j] = word < kTraceRun / 32 ? sm.defer[word] : 0u;
-          __syncwarp();
-          if (lane == 0 && mask[j] != 0u) sm.defer[word] = 0u;
-        }
-        append(p0, mask);
-        __syncthreads();
-        serve(p0 + kTraceThreads * kTracePer >= count);
-      }
-    }
-  }
+// trace_direct: samples of a thread, and groups of them that one sweep over the points covers.
+constexpr int kDirectK = 16;
+constexpr int kDirectGroups = 16;
+
+struct DirectSmem {
+  float2 seeds[kDirectGroups][kTraceThreads];
+  float2 zeta[kTraceThreads];
+  int counts[kTraceWarps];
 };
 
-template <typename T, typename IndexOf, typename SigmaOf>
-__device__ __forceinline__ TraceList<T, IndexOf, SigmaOf> trace_list(TraceSmem& sm, const TraceConsts& c, const T* normals,
-                                                                     const T* points, const float* txp, const float* rxp,
-                                                                     IndexOf index_of, SigmaOf sigma_of) {
-  return TraceList<T, IndexOf, SigmaOf>{sm, c, normals, points, txp, rxp, index_of, sigma_of};
-}
 
-// `count` positions, at most kTraceRun, in batches of consecutive ones: for points of
-// which most are live (the pre-cull's list).  The next batch's points are loaded
-// while one is summed.
-template <typename T, typename IndexOf, typename SigmaOf>
-__device__ __forceinline__ void trace_all(TraceSmem& sm, const TraceConsts& c, float2* row, const T* normals,
-                                          const T* points, const float* txp, const float* rxp, int count,
-                                          IndexOf index_of, SigmaOf sigma_of) {
-  auto list = trace_list<T>(sm, c, normals, points, txp, rxp, index_of, sigma_of);
-  TracePoint next;
-  int64_t next_q = -1;
-  auto load = [&](int pos) {
-    next_q = pos < count ? index_of(pos) : -1;
-    if (next_q >= 0) {
-      load_point(normals, points, next_q, next.nrm, next.pt);
-      next.sigma = sigma_of(next_q);
-    }
-  };
-  load(threadIdx.x);
-  for (int p0 = 0; p0 < count; p0 += kTraceThreads) {
-    float2 w = make_float2(0.0f, 0.0f);
-    float x = 0.0f;
-    int cell = 0;
-    const bool live = next_q >= 0 && trace_point(c, txp, rxp, next, w, cell, x);
-    load(p0 + kTraceThreads + threadIdx.x);
-    if (trace_batch(sm, live, w, cell, x, p0 + threadIdx.x)) list.deferred = true;
-  }
-  list.serve_deferred(count, row);
-}
-
-// `count` consecutive points, at most kTraceRun (their arrays from the first one on;
-// inb may be null), screened first.
-template <typename T>
-__device__ __forceinline__ void trace_screened(TraceSmem& sm, const TraceConsts& c, float2* row, const T* normals,
-                                               const T* points, const T* sigmas, const uint8_t* inb, const float* txp,
-                                               const float* rxp, int count) {
-  auto list = trace_list<T>(sm, c, normals, points, txp, rxp, [](int pos) { return pos; },
-                            [=](int64_t q) { return ld_f(sigmas, q); });
-  float nrm[kTracePer][3], pt[kTracePer][3];
-  unsigned in = 0;  // bit j: point j of the thread is in bounds
-  auto load = [&](int p0) {  // of the next pass, in flight while batches are summed
-    in = 0;
-    const int rest = count - p0 - static_cast<int>(threadIdx.x);
-    const T* pn = normals + (static_cast<int64_t>(p0) + threadIdx.x) * 3;
-    const T* pp = points + (static_cast<int64_t>(p0) + threadIdx.x) * 3;
-    const uint8_t* pb = inb != nullptr ? inb + p0 + threadIdx.x : nullptr;
+// Samples without cells: store(n, sum over the live points of positions [0, count)).  A tile of
+// 128 points leaves each group of 16 samples its start phasors, and thread (group, lane) runs its
+// lane's points through its samples by the recurrence of rotate_accumulate, in two levels of
+// sums (a tile's, the share's).  A sweep over the points covers 256 samples.  About 2 issue slots
+// per live (point, sample): 64 antennas x 262144 live points x 128 samples take 634 us,
+// whatever their paths.
+template <typename T, typename IndexOf, typename SigmaOf, typename Store>
+__device__ __forceinline__ void trace_direct(DirectSmem& sm, const TraceConsts& c, const T* normals, const T* points,
+                                             const float* txp, const float* rxp, int64_t count, IndexOf index_of,
+                                             SigmaOf sigma_of, Store store) {
+  constexpr int K = kDirectK;
+  int G = 1;
+  while (G < kDirectGroups && G * K < c.S) G *= 2;
+  const int L = kTraceThreads / G;
+  const int group = threadIdx.x / L, in_group = threadIdx.x % L;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double mid = 0.5 * (c.S - 1);
+  for (int n0 = 0; n0 < c.S; n0 += G * K) {
+    float2 acc[K], sum[K];
 #pragma unroll
-    for (int j = 0; j < kTracePer; ++j) {
-      if (j * kTraceThreads < rest && (pb == nullptr || pb[j * kTraceThreads])) {
-        in |= 1u << j;
-        load_point(pn, pp, j * kTraceThreads, nrm[j], pt[j]);
+    for (int m = 0; m < K; ++m) acc[m] = sum[m] = make_float2(0.0f, 0.0f);
+    for (int64_t p0 = 0; p0 < count; p0 += kTraceThreads) {
+      TracePoint t;
+      const int64_t q = p0 + threadIdx.x < count ? index_of(p0 + threadIdx.x) : -1;
+      if (q >= 0) {
+        load_point(normals, points, q, t.nrm, t.pt);
+        t.sigma = sigma_of(q);
       }
-    }
-  };
-  load(0);
-  for (int p0 = 0; p0 < count; p0 += kTraceThreads * kTracePer) {
-    unsigned mask[kTracePer];
+      float2 w = make_float2(0.0f, 0.0f), zt = w, zk = w;
+      float amp;
+      double d;
+      const bool live = q >= 0 && !surely_culled(txp, rxp, t.nrm, t.pt) && trace_path(txp, rxp, t, amp, d);
+      if (live) {
+        const double step = fma(d, c.k1, c.b1), kc = step * K;
+        const double start = fma(d, c.K, c.b) + (n0 - mid) * step;
+        const float2 e = cis_cycles_fast(static_cast<float>(start - rint(start)));
+        w = make_float2(amp * e.x, amp * e.y);
+        zt = cis_cycles(static_cast<float>(step - rint(step)));
+        zk = cis_cycles(static_cast<float>(kc - rint(kc)));
+      }
+      const unsigned ballot = __ballot_sync(0xffffffffu, live);
+      if (lane == 0) sm.counts[warp] = __popc(ballot);
+      __syncthreads();
+      int slot = __popc(ballot & ((1u << lane) - 1u)), total = 0;
 #pragma unroll
-    for (int j = 0; j < kTracePer; ++j) {
-      mask[j] = __ballot_sync(0xffffffffu, ((in >> j) & 1u) && !surely_culled(txp, rxp, nrm[j], pt[j]));
+      for (int k = 0; k < kTraceWarps; ++k) {
+        if (k < warp) slot += sm.counts[k];
+        total += sm.counts[k];
+      }
+      if (live) {
+        sm.zeta[slot] = zt;
+        for (int k = 0; k < G; ++k) {
+          sm.seeds[k][slot] = w;
+          w = cmul(w, zk);
+        }
+      }
+      __syncthreads();
+      rotate_tile<K>(sm.seeds[group], sm.zeta, in_group, L, total, acc);
+#pragma unroll
+      for (int m = 0; m < K; ++m) sum[m] = fadd2(sum[m], acc[m]);
+      __syncthreads();
     }
-    list.append(p0, mask);
-    load(p0 + kTraceThreads * kTracePer);
+    float2* red = &sm.seeds[0][0];  // [G K][L]
+#pragma unroll
+    for (int m = 0; m < K; ++m) red[(group * K + m) * L + in_group] = sum[m];
     __syncthreads();
-    list.serve(p0 + kTraceThreads * kTracePer >= count);
+    for (int i = threadIdx.x; i < G * K && n0 + i < c.S; i += kTraceThreads) {
+      double2 x = make_double2(0.0, 0.0);
+      for (int k = 0; k < L; ++k) {
+        x.x += red[i * L + k].x;
+        x.y += red[i * L + k].y;
+      }
+      store(n0 + i, make_float2(static_cast<float>(x.x), static_cast<float>(x.y)));
+    }
+    __syncthreads();
   }
-  list.serve_deferred(count, row);
 }
 
-__device__ __forceinline__ void trace_store(const TraceSmem& sm, TraceRecord* rec) {
+__device__ __forceinline__ void trace_store(const TraceSmem& sm, TraceRecord* rec, bool has_row) {
   __syncthreads();
   for (int i = threadIdx.x; i < kTraceSlots * kTraceQ; i += kTraceThreads) {
     if (sm.tag[i / kTraceQ] != kTraceEmpty) (&rec->moments[0][0])[i] = (&sm.moments[0][0])[i];
   }
   for (int i = threadIdx.x; i < kTraceSlots; i += kTraceThreads) rec->tag[i] = sm.tag[i];
-  if (threadIdx.x == 0) rec->has_row = sm.has_row;
+  if (threadIdx.x == 0) rec->has_row = has_row ? 1 : 0;
   __syncthreads();
 }
 

@@ -157,26 +157,54 @@ struct TrCellP {
   TraceConsts c;
 };
 
+// Positions [begin, end) of share b.
 template <typename T>
-__global__ void __launch_bounds__(kTraceThreads, 5) tracer_fwd_cells_kernel(const TrCellP<T> p) {
-  __shared__ TraceSmem sm;
-  const int64_t a = blockIdx.x / p.splits;
-  const int split = blockIdx.x % p.splits;
+__device__ __forceinline__ void share_range(const TrCellP<T>& p, int64_t b, int64_t& begin, int64_t& end) {
   const int64_t npts = p.plist != nullptr ? static_cast<int64_t>(*p.plist_count) : p.P;
   const int64_t per_split = (npts + p.splits - 1) / p.splits;
-  const int64_t begin = split * per_split, end = min(npts, begin + per_split);
+  begin = b % p.splits * per_split;
+  end = min(npts, begin + per_split);
+}
+
+// Positions [begin, end) of share b (not inlined: it would take registers from the cells).
+template <typename T>
+static __device__ __noinline__ void share_direct(DirectSmem& sm, const TrCellP<T>& p, int64_t b, int64_t begin, int64_t end) {
+  const int64_t a = b / p.splits;
+  float txp[3], rxp[3];
+  load3(p.tx, a, txp);
+  load3(p.rx, a, rxp);
+  const T* sigmas = p.sigmas + a * p.P;
+  const int* plist = p.plist;
+  const uint8_t* inb = p.inb;
+  float2* row = p.rows + b * p.c.S;
+  trace_direct<T>(
+      sm, p.c, p.normals, p.points, txp, rxp, end - begin,
+      [&](int64_t pos) -> int64_t { return plist != nullptr ? plist[begin + pos] : inb[begin + pos] ? begin + pos : -1; },
+      [&](int64_t q) { return ld_f(sigmas, q); }, [&](int n, float2 y) { row[n] = y; });
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kTraceThreads, 5) tracer_fwd_cells_kernel(const __grid_constant__ TrCellP<T> p) {
+  __shared__ union {
+    TraceSmem cells;
+    DirectSmem direct;
+  } smem;
+  TraceSmem& sm = smem.cells;
+  const int64_t a = blockIdx.x / p.splits;
+  int64_t begin, end;
+  share_range(p, blockIdx.x, begin, end);
   float txp[3], rxp[3];
   load3(p.tx, a, txp);
   load3(p.rx, a, rxp);
   trace_begin(sm);
-  for (int64_t at = begin; at < end; at += kTraceRun) {
-    trace_all<T>(
-        sm, p.c, p.rows + blockIdx.x * static_cast<int64_t>(p.c.S), p.normals, p.points, txp, rxp,
-        static_cast<int>(min(end - at, static_cast<int64_t>(kTraceRun))),
-        [&](int pos) { return p.plist != nullptr ? p.plist[at + pos] : p.inb[at + pos] ? static_cast<int>(at + pos) : -1; },
-        [&](int64_t q) { return ld_f(p.sigmas, a * p.P + q); });
-  }
-  trace_store(sm, p.records + blockIdx.x);
+  const int64_t from = begin + trace_all<T>(
+      sm, p.c, p.normals, p.points, txp, rxp, static_cast<int>(max(int64_t{0}, end - begin)),
+      [&](int64_t pos) -> int64_t {
+        return p.plist != nullptr ? p.plist[begin + pos] : p.inb[begin + pos] ? begin + pos : -1;
+      },
+      [&](int64_t q) { return ld_f(p.sigmas, a * p.P + q); });
+  trace_store(sm, p.records + blockIdx.x, from < end);
+  if (from < end) share_direct(smem.direct, p, blockIdx.x, from, end);
 }
 
 template <typename T>
@@ -809,12 +837,16 @@ TrP<T> make_params(const TracerArgs& a) {
 // pre-cull applies) the point list region.
 size_t list_region_offset(size_t partial_bytes) { return (partial_bytes + 255) & ~static_cast<size_t>(255); }
 
-// Workspace of the MIXED forward: the runs' records, their rows of samples, the point list.
-size_t fwd_records_bytes(const TracerArgs& a, int splits) {
-  return list_region_offset(static_cast<size_t>(splits) * a.A * sizeof(TraceRecord));
-}
-size_t fwd_partial_bytes(const TracerArgs& a, int splits) {
-  return fwd_records_bytes(a, splits) + list_region_offset(static_cast<size_t>(splits) * a.A * a.S * sizeof(float2));
+// Workspace of the MIXED forward: the shares' records, their rows of samples, the point list.
+struct FwdLayout {
+  size_t rows, list;
+};
+FwdLayout fwd_layout(const TracerArgs& a, int splits) {
+  const size_t shares = static_cast<size_t>(splits) * a.A;
+  FwdLayout l;
+  l.rows = list_region_offset(shares * sizeof(TraceRecord));
+  l.list = l.rows + list_region_offset(shares * a.S * sizeof(float2));
+  return l;
 }
 
 template <typename T>
@@ -841,11 +873,12 @@ cudaError_t launch_tracer_fwd(const TracerArgs& a, const Tuning& t, void* ws, cu
   c.c = trace_consts(p.k0, p.b0, p.k1, p.b1, a.S);
   unsigned char* base = static_cast<unsigned char*>(ws);
   c.records = reinterpret_cast<TraceRecord*>(base);
-  c.rows = reinterpret_cast<float2*>(base + fwd_records_bytes(a, t.splits));
+  const FwdLayout l = fwd_layout(a, t.splits);
+  c.rows = reinterpret_cast<float2*>(base + l.rows);
   c.plist = nullptr;
   c.plist_count = nullptr;
   if (tracer_point_list_applies(a)) {
-    void* lws = base + fwd_partial_bytes(a, t.splits);
+    void* lws = base + l.list;
     const cudaError_t err = tracer_point_list(a, lws, false, st);
     if (err != cudaSuccess) return err;
     const PointList pl = tracer_point_list_view(lws, a.P);
@@ -1011,8 +1044,8 @@ size_t tracer_forward_workspace(const TracerArgs& call, const Tuning& t) {
   const TracerArgs a = resolved_form(call, t);
   if (a.mode == kNufft) return tracer_nufft_forward_workspace(a, t);
   if (a.mode == kPlain) return 0;
-  const size_t partial_bytes = fwd_partial_bytes(a, t.splits);
-  return tracer_point_list_applies(a) ? partial_bytes + tracer_point_list_bytes(a.P) : partial_bytes;
+  const size_t before_list = fwd_layout(a, t.splits).list;
+  return tracer_point_list_applies(a) ? before_list + tracer_point_list_bytes(a.P) : before_list;
 }
 
 cudaError_t tracer_forward(const TracerArgs& call, const Tuning& t, void* ws, cudaStream_t st) {

@@ -121,3 +121,16 @@ def test_many_points_of_one_cell(cuda, splits):
     r = orc.tracer_forward(c["normals"], c["sigmas"], c["points"], c["tx"], c["rx"], c["inbounds"], S, float(c["fs"]),
                            float(c["f0"]), float(c["As"]), "f64")
     assert rel_l2(x[0] + 1j * x[1], r[0] + 1j * r[1]) < 2e-6 + 3 * 1.1e-6
+
+
+@pytest.mark.parametrize("S", [33, 300])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_scene_that_leaves_its_slots_midway(cuda, S, splits):
+    """Points sorted by their distance, 150 cells of them: a share's first batches go through the
+    cells, the rest does not (300 samples: two sweeps over it)."""
+    c = case(14, 5, 3000, S, (0.3, 3.3))
+    order = np.argsort(np.linalg.norm(c["points"], axis=1))
+    for k in ("normals", "points", "inbounds"):
+        c[k] = np.ascontiguousarray(c[k][order])
+    c["sigmas"] = np.ascontiguousarray(c["sigmas"][:, order])
+    check(c, "mixed", {"splits": splits})
