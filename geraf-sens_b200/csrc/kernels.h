@@ -255,6 +255,10 @@ PhaseConsts phase_consts(float f0, float As, float fs);
 // to that), remembered per device; 0 when no device answers.
 int resident_blocks(const void* fn, int threads, size_t smem);
 
+// Whether the tracer forwards' moments become samples by warps (tracer_cells.cuh, trace_finish_few):
+// antennas for several times the blocks that would otherwise take one each (two per SM).
+bool finish_by_warps(int64_t A, int64_t S, double kappa);
+
 // Picks the number of splits of the reduced dimension so that
 // `units * splits` blocks fill the GPU in near-whole waves.
 int pick_splits(int64_t units, int blocks_per_sm, int sm_count, int64_t max_splits);

@@ -192,13 +192,51 @@ __global__ void __launch_bounds__(kTraceThreads) ragged_fwd_direct_kernel(const 
 
 // x[a, n] = (sum of antenna a's items, in item order) / P_a.
 template <typename T>
-__global__ void __launch_bounds__(kFinishThreads) ragged_finish_kernel(const RgP<T> p) {
-  const int64_t a = blockIdx.x;
+__device__ __forceinline__ void finish_antenna(const RgP<T>& p, int64_t a) {
   const int n0 = blockIdx.y * kFinishSamples;
   const int64_t it = p.item_offsets[a];
   trace_finish<T>(p.c, p.records + it, p.rows + it * p.c.S, p.item_offsets[a + 1] - it,
                   static_cast<float>(p.offsets[a + 1] - p.offsets[a]), n0, min(p.c.S, n0 + kFinishSamples),
                   p.out_r + a * p.c.S, p.out_i + a * p.c.S);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kFinishThreads) ragged_finish_kernel(const RgP<T> p) {
+  finish_antenna(p, blockIdx.x);
+}
+
+// Of many antennas, those of more than kFewShares items: a block looks at antennas a =
+// blockIdx.x, + gridDim.x, ...
+template <typename T>
+__global__ void __launch_bounds__(kFinishThreads) ragged_finish_long_kernel(const RgP<T> p) {
+  __shared__ int64_t todo[kFinishThreads];
+  __shared__ int count;
+  for (int64_t a0 = blockIdx.x; a0 < p.A; a0 += static_cast<int64_t>(gridDim.x) * kFinishThreads) {
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    const int64_t a = a0 + static_cast<int64_t>(threadIdx.x) * gridDim.x;
+    if (a < p.A && p.item_offsets[a + 1] - p.item_offsets[a] > kFewShares) todo[atomicAdd(&count, 1)] = a;
+    __syncthreads();
+    for (int i = 0; i < count; ++i) {
+      finish_antenna(p, todo[i]);
+      __syncthreads();
+    }
+    __syncthreads();
+  }
+}
+
+// The others.
+template <typename T>
+__global__ void __launch_bounds__(kFewThreads) ragged_finish_few_kernel(const RgP<T> p) {
+  extern __shared__ __align__(16) unsigned char few_smem[];
+  const FewTable f = few_table(p.c, few_smem);
+  const int64_t warps = static_cast<int64_t>(gridDim.x) * (kFewThreads / 32);
+  for (int64_t a = blockIdx.x * static_cast<int64_t>(kFewThreads / 32) + (threadIdx.x >> 5); a < p.A; a += warps) {
+    const int64_t it = p.item_offsets[a], items = p.item_offsets[a + 1] - it;
+    if (items > kFewShares) continue;
+    trace_finish_few<T>(p.c, f, p.records + it, p.rows + it * p.c.S, static_cast<int>(items),
+                        static_cast<float>(p.offsets[a + 1] - p.offsets[a]), p.out_r + a * p.c.S, p.out_i + a * p.c.S);
+  }
 }
 
 // Antenna owning point pi: the last a with offsets[a] <= pi.  *owned is false
@@ -465,8 +503,15 @@ cudaError_t launch_ragged_fwd(const RaggedArgs& a, const Tuning& t, void* ws, cu
       1, std::min<int64_t>(static_cast<int64_t>(per_sm) * current_device_info().sm_count, p.max_items));
   ragged_fwd_kernel<T><<<static_cast<unsigned>(blocks), kTraceThreads, 0, st>>>(p);
   ragged_fwd_direct_kernel<T><<<static_cast<unsigned>(blocks), kTraceThreads, 0, st>>>(p);
-  const dim3 grid(static_cast<unsigned>(a.A), static_cast<unsigned>((a.S + kFinishSamples - 1) / kFinishSamples));
-  ragged_finish_kernel<T><<<grid, kFinishThreads, 0, st>>>(p);
+  const int64_t sms = current_device_info().sm_count;
+  const unsigned parts = static_cast<unsigned>((a.S + kFinishSamples - 1) / kFinishSamples);
+  if (!finish_by_warps(a.A, a.S, p.c.kappa)) {
+    ragged_finish_kernel<T><<<dim3(static_cast<unsigned>(a.A), parts), kFinishThreads, 0, st>>>(p);
+  } else {
+    ragged_finish_long_kernel<T><<<dim3(static_cast<unsigned>(std::min<int64_t>(a.A, 2 * sms)), parts), kFinishThreads, 0, st>>>(p);
+    const int64_t by_warps = std::min<int64_t>((a.A + kFewThreads / 32 - 1) / (kFewThreads / 32), sms * 8);
+    ragged_finish_few_kernel<T><<<static_cast<unsigned>(by_warps), kFewThreads, few_smem_bytes(a.S), st>>>(p);
+  }
   return cudaGetLastError();
 }
 

@@ -215,6 +215,17 @@ __global__ void __launch_bounds__(kFinishThreads) tracer_fwd_finish_kernel(const
                   min(p.c.S, n0 + kFinishSamples), p.out_r + a * p.c.S, p.out_i + a * p.c.S);
 }
 
+template <typename T>
+__global__ void __launch_bounds__(kFewThreads) tracer_fwd_finish_few_kernel(const TrCellP<T> p) {
+  extern __shared__ __align__(16) unsigned char few_smem[];
+  const FewTable f = few_table(p.c, few_smem);
+  const int64_t warps = static_cast<int64_t>(gridDim.x) * (kFewThreads / 32);
+  for (int64_t a = blockIdx.x * static_cast<int64_t>(kFewThreads / 32) + (threadIdx.x >> 5); a < p.A; a += warps) {
+    trace_finish_few<T>(p.c, f, p.records + a * p.splits, p.rows + a * p.splits * p.c.S, p.splits,
+                        static_cast<float>(p.P), p.out_r + a * p.c.S, p.out_i + a * p.c.S);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Adjoint (point-major).  Block = point tile x antenna split; the residual
 // rows g[a, :] stream through a double-buffered TMA ring.
@@ -849,6 +860,14 @@ FwdLayout fwd_layout(const TracerArgs& a, int splits) {
   return l;
 }
 
+}  // namespace
+
+bool finish_by_warps(int64_t A, int64_t S, double kappa) {
+  return A >= 2 * static_cast<int64_t>(current_device_info().sm_count) && S <= kFewSamples && kappa > kTraceMinKappa;
+}
+
+namespace {
+
 template <typename T>
 cudaError_t launch_tracer_fwd(const TracerArgs& a, const Tuning& t, void* ws, cudaStream_t st) {
   TrP<T> p = make_params<T>(a);
@@ -887,6 +906,12 @@ cudaError_t launch_tracer_fwd(const TracerArgs& a, const Tuning& t, void* ws, cu
   }
   if (a.A * t.splits > 0x7fffffff) return cudaErrorInvalidConfiguration;
   tracer_fwd_cells_kernel<T><<<static_cast<unsigned>(a.A * t.splits), kTraceThreads, 0, st>>>(c);
+  const int sms = current_device_info().sm_count;
+  if (finish_by_warps(a.A, a.S, c.c.kappa) && t.splits <= kFewShares) {
+    const int64_t blocks = std::min<int64_t>((a.A + kFewThreads / 32 - 1) / (kFewThreads / 32), sms * 8);
+    tracer_fwd_finish_few_kernel<T><<<static_cast<unsigned>(blocks), kFewThreads, few_smem_bytes(a.S), st>>>(c);
+    return cudaGetLastError();
+  }
   const dim3 grid(static_cast<unsigned>(a.A), static_cast<unsigned>((a.S + kFinishSamples - 1) / kFinishSamples));
   tracer_fwd_finish_kernel<T><<<grid, kFinishThreads, 0, st>>>(c);
   return cudaGetLastError();
@@ -1031,10 +1056,14 @@ Tuning tracer_forward_resolve(const TracerArgs& call, const Tuning& req) {
     t.splits = 1;
     return t;
   }
-  // MIXED: one block per (antenna, split of the points), at most a block per batch of points
+  // MIXED: one block per (antenna, split of the points), at most a block per batch of points, or
+  // per 16384 points where the antennas fill the GPU by themselves (each share costs a
+  // record of its cells: 3072 antennas x 3000 points x 32 samples, 207 us with 6 splits, 78 us with one)
   const int64_t batches = std::max<int64_t>(1, (a.P + kTraceThreads - 1) / kTraceThreads);
   if (t.splits <= 0) {
-    t.splits = pick_splits(std::max<int64_t>(1, a.A), 5, current_device_info().sm_count, batches);
+    const int sms = current_device_info().sm_count;
+    const int64_t most = a.A >= 5 * static_cast<int64_t>(sms) ? std::max<int64_t>(1, a.P / 16384) : batches;
+    t.splits = pick_splits(std::max<int64_t>(1, a.A), 5, sms, most);
   }
   t.splits = static_cast<int>(std::min<int64_t>(std::max(t.splits, 1), batches));
   return t;

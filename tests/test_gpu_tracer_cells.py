@@ -134,3 +134,47 @@ def test_scene_that_leaves_its_slots_midway(cuda, S, splits):
         c[k] = np.ascontiguousarray(c[k][order])
     c["sigmas"] = np.ascontiguousarray(c["sigmas"][:, order])
     check(c, "mixed", {"splits": splits})
+
+
+# many antennas of few points (their moments become samples by warps): one share each and several,
+# remainders of the 32 samples, the longest rows that go this way and longer ones, a falling sweep
+@pytest.mark.parametrize("A,P,S,splits", [(300, 700, 33, 0), (300, 1500, 64, 3), (301, 130, 384, 1), (301, 130, 512, 1),
+                                          (1200, 60, 100, 0)])
+@pytest.mark.parametrize("fall", [1.0, -1.0])
+def test_many_antennas_of_few_points(cuda, A, P, S, splits, fall):
+    c = case(15, A, P, S)
+    tx, rx = scenes.virtual_array(10)
+    c["tx"], c["rx"] = tx[:A].astype(np.float32), rx[:A].astype(np.float32)
+    c["As"] = np.float32(fall * c["As"])
+    check(c, "mixed", {"splits": splits})
+
+
+@pytest.mark.parametrize("depth", [(0.3, 0.5), (0.3, 3.3)], ids=["near", "deep"])
+def test_ragged_many_antennas(cuda, depth):
+    """Antennas of 0 to 40 points and one of 30000 in one call, against FP64."""
+    from geraf_b200.ops.RFSignalTracer.ragged import signal_tracer_ragged
+
+    A, S = 310, 96
+    rng = np.random.default_rng(16)
+    counts = rng.integers(0, 41, A)
+    counts[[0, A - 1]] = 0
+    counts[200] = 30000
+    off = np.concatenate([[0], np.cumsum(counts)])
+    c = case(16, 1, int(off[-1]), S, depth)
+    tx, rx = (x[:A].astype(np.float32) for x in scenes.virtual_array(6))
+    scal = float(c["fs"]), float(c["f0"]), float(c["As"])
+    x = signal_tracer_ragged(cu(c["normals"]), cu(c["sigmas"][0]), cu(c["points"]), torch.tensor(off, device="cuda"), cu(tx),
+                             cu(rx), S, *scal, inbounds=torch.tensor(c["inbounds"], device="cuda"),
+                             tuning={"items_per_thread": 8})
+    x = x[0].cpu().numpy() + 1j * x[1].cpu().numpy()
+    got, ref = [], []
+    for a in range(A):
+        if counts[a] == 0:
+            assert np.isnan(x[a]).all()
+            continue
+        e = slice(off[a], off[a + 1])
+        r = orc.tracer_forward(c["normals"][e], c["sigmas"][:, e], c["points"][e], tx[a:a + 1], rx[a:a + 1],
+                               c["inbounds"][e], S, *scal, "f64")
+        got.append(counts[a] * x[a])
+        ref.append(counts[a] * (r[0] + 1j * r[1])[0])
+    assert rel_l2(np.array(got), np.array(ref)) < TOL
