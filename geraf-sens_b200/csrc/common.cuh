@@ -352,7 +352,7 @@ __device__ __forceinline__ void rotate_tile(const float2* seeds, const float2* z
 
 // Residual sums of the tracer adjoints for one (point, antenna) pair, from a
 // residual row g (real and imaginary parts, ld samples, ld a multiple of 4,
-// samples past S zero) in shared memory:
+// samples past S zero), four samples n .. n + 3 at a time by load4(n, re, im):
 //   Q  = sum_n conj(g_n) zeta^n,   Q1 = zeta Q'(zeta) = sum_n n conj(g_n) zeta^n.
 // Horner in w = zeta^2 on the even and odd samples at once, one chain per lane
 // of packed f32x2 operands.  The lanes carry the conjugates
@@ -362,9 +362,8 @@ __device__ __forceinline__ void rotate_tile(const float2* seeds, const float2* z
 //   conj(Q1) = 2 conj(w) E' + conj(zeta) (2 conj(w) O' + O).
 // Per two samples: 4 fma.rn.f32x2 for (E, O), 4 more for (E', O') when Q1 is
 // wanted.
-template <bool WITH_Q1, typename R>
-__device__ __forceinline__ void residual_sums(const R* rowr, const R* rowi, int ld, float2 zt, float2& q,
-                                              float2& q1) {
+template <bool WITH_Q1, typename Load4>
+__device__ __forceinline__ void residual_sums(Load4 load4, int ld, float2 zt, float2& q, float2& q1) {
   const float2 wz = cmul(zt, zt);
   const float2 wr2 = make_float2(wz.x, wz.x), wi2 = make_float2(wz.y, wz.y);
   const float2 nwi2 = make_float2(-wz.y, -wz.y);
@@ -372,8 +371,8 @@ __device__ __forceinline__ void residual_sums(const R* rowr, const R* rowi, int 
   float2 dr2 = make_float2(0.0f, 0.0f), di2 = make_float2(0.0f, 0.0f);  // (E', O')
 #pragma unroll 2
   for (int n = ld - 4; n >= 0; n -= 4) {
-    const float4 a4 = lds4(rowr + n);
-    const float4 b4 = lds4(rowi + n);
+    float4 a4, b4;
+    load4(n, a4, b4);
     const float2 gre[2] = {make_float2(a4.z, a4.w), make_float2(a4.x, a4.y)};
     const float2 gim[2] = {make_float2(b4.z, b4.w), make_float2(b4.x, b4.y)};
 #pragma unroll
@@ -403,6 +402,18 @@ __device__ __forceinline__ void residual_sums(const R* rowr, const R* rowi, int 
   } else {
     q1 = make_float2(0.0f, 0.0f);
   }
+}
+
+// The same from a row in shared memory.
+template <bool WITH_Q1, typename R>
+__device__ __forceinline__ void residual_sums(const R* rowr, const R* rowi, int ld, float2 zt, float2& q,
+                                              float2& q1) {
+  residual_sums<WITH_Q1>(
+      [=](int n, float4& re, float4& im) {
+        re = lds4(rowr + n);
+        im = lds4(rowi + n);
+      },
+      ld, zt, q, q1);
 }
 
 // Stages the tx and rx positions of `rws` antennas from a0 into slot `stage`

@@ -253,6 +253,38 @@ __device__ __forceinline__ int64_t point_antenna(const int64_t* offsets, int64_t
   return lo;
 }
 
+// Gradients of one point that the early test cannot cull; a point that the exact geometry culls
+// keeps what it has.  sums(zeta, q, q1) is residual_sums over the antenna's row.
+template <typename T, bool WITH_POINTS, typename Sums>
+__device__ __forceinline__ void point_gradients(const RgP<T>& p, int64_t pi, const float* txp, const float* rxp,
+                                                float inv_pa, Sums sums) {
+  float nrm[3], pt[3];
+  ld3(p.normals, pi, nrm);
+  ld3(p.points, pi, pt);
+  const float sigma = ld_f(p.sigmas, pi);
+  PairGeom g;
+  if (!pair_geometry(txp, rxp, nrm, pt, g)) return;
+  const PhaseCycles pc =
+      path_cycles(static_cast<double>(txp[0]) - pt[0], static_cast<double>(txp[1]) - pt[1],
+                  static_cast<double>(txp[2]) - pt[2], static_cast<double>(rxp[0]) - pt[0],
+                  static_cast<double>(rxp[1]) - pt[1], static_cast<double>(rxp[2]) - pt[2], p.k0, p.b0, p.k1, p.b1);
+  float2 q, q1;
+  sums(cis_cycles(pc.dcyc), q, q1);
+  float gs, gn[3] = {0.0f, 0.0f, 0.0f}, gp[3] = {0.0f, 0.0f, 0.0f};
+  const float2 e0 = cis_cycles_fast(pc.frac0);
+  // sum_n w_n (g_i cos - g_r sin) = -Im(exp(j phi0) (w0 Q + w1 Q1))
+  const float w0 = static_cast<float>(2.0 * static_cast<double>(kPiF) * p.f0);
+  const float w1s = static_cast<float>(2.0 * static_cast<double>(kPiF) * p.As / p.fs);
+  const float f = cmul(e0, make_float2(w0 * q.x + w1s * q1.x, w0 * q.y + w1s * q1.y)).y;
+  pair_gradients<WITH_POINTS>(g, cmul(e0, q).x, f, sigma, nrm, &gs, gn, gp);
+  p.g_sigmas[pi] = from_f<T>(gs * inv_pa);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    p.g_normals[pi * 3 + c] = from_f<T>(gn[c] * inv_pa);
+    if (WITH_POINTS) p.g_points[pi * 3 + c] = from_f<T>(gp[c] * inv_pa);
+  }
+}
+
 // Adjoint.  A point belongs to one antenna, so its gradients depend on nothing else.  A
 // block takes a run of consecutive points, kBwdTile at a time: it writes zeros for
 // all of them (whole lines), screens them with the early test while the next tile's
@@ -296,32 +328,10 @@ __global__ void __launch_bounds__(kBwdThreads, 6) ragged_bwd_kernel(const RgP<T>
   // Gradients of listed points [from, from + cnt) of the current antenna.
   auto batch = [&](int cnt, int from) {
     if (threadIdx.x >= cnt) return;
-    const int64_t pi = begin + list[from + threadIdx.x];
-    float nrm[3], pt[3];
-    ld3(p.normals, pi, nrm);
-    ld3(p.points, pi, pt);
-    const float sigma = ld_f(p.sigmas, pi);
-    PairGeom g;
-    if (!pair_geometry(txp, rxp, nrm, pt, g)) return;  // keeps its zeros
-    const PhaseCycles pc =
-        path_cycles(static_cast<double>(txp[0]) - pt[0], static_cast<double>(txp[1]) - pt[1],
-                    static_cast<double>(txp[2]) - pt[2], static_cast<double>(rxp[0]) - pt[0],
-                    static_cast<double>(rxp[1]) - pt[1], static_cast<double>(rxp[2]) - pt[2], p.k0, p.b0, p.k1, p.b1);
-    float2 q, q1;
-    residual_sums<WITH_POINTS>(rowr, rowi, ld, cis_cycles(pc.dcyc), q, q1);
-    float gs, gn[3] = {0.0f, 0.0f, 0.0f}, gp[3] = {0.0f, 0.0f, 0.0f};
-    const float2 e0 = cis_cycles_fast(pc.frac0);
-    // sum_n w_n (g_i cos - g_r sin) = -Im(exp(j phi0) (w0 Q + w1 Q1))
-    const float w0 = static_cast<float>(2.0 * static_cast<double>(kPiF) * p.f0);
-    const float w1s = static_cast<float>(2.0 * static_cast<double>(kPiF) * p.As / p.fs);
-    const float f = cmul(e0, make_float2(w0 * q.x + w1s * q1.x, w0 * q.y + w1s * q1.y)).y;
-    pair_gradients<WITH_POINTS>(g, cmul(e0, q).x, f, sigma, nrm, &gs, gn, gp);
-    p.g_sigmas[pi] = from_f<T>(gs * inv_pa);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      p.g_normals[pi * 3 + c] = from_f<T>(gn[c] * inv_pa);
-      if (WITH_POINTS) p.g_points[pi * 3 + c] = from_f<T>(gp[c] * inv_pa);
-    }
+    point_gradients<T, WITH_POINTS>(p, begin + list[from + threadIdx.x], txp, rxp, inv_pa,
+                                    [&](float2 zeta, float2& q, float2& q1) {
+                                      residual_sums<WITH_POINTS>(rowr, rowi, ld, zeta, q, q1);
+                                    });
   };
   // The full batches that the list holds; all of it when `drain`.  Between two barriers.
   auto serve = [&](bool drain) {
@@ -412,6 +422,80 @@ __global__ void __launch_bounds__(kBwdThreads, 6) ragged_bwd_kernel(const RgP<T>
     __syncthreads();
   }
   serve(true);
+}
+
+// The adjoint where antennas have few points each, which would have the kernel above change
+// antennas (a row to stage, three barriers) every few points: a block screens 512 points,
+// each with its own antenna, lists those that the early test cannot cull, and its threads
+// read their antennas' rows from device memory.  Bound by those reads.  64 samples, 1000
+// antennas of one point: 1.40 ms above, 30 us here; 256 samples, 49152 x 4: 779 and 86 us, 16384
+// x 32: 199 and 130 us; above 48 points the rows in shared memory win (2000 x 64: 50 us above,
+// 106 us by this form's forerunner).
+constexpr int kShortPoints = 48;  // per antenna, on average
+
+template <typename T, bool WITH_POINTS>
+__global__ void __launch_bounds__(kBwdThreads, 6) ragged_bwd_short_kernel(const RgP<T> p, int ld, int vector_rows) {
+  __shared__ int list[kBwdTile];
+  __shared__ int s_listed;
+  const int64_t begin = blockIdx.x * static_cast<int64_t>(kBwdTile);
+  const int64_t end = min(p.P, begin + kBwdTile);
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) s_listed = 0;
+  zero_range(p.g_sigmas, begin, end);
+  zero_range(p.g_normals, begin * 3, end * 3);
+  if (WITH_POINTS) zero_range(p.g_points, begin * 3, end * 3);
+  __syncthreads();
+#pragma unroll 1
+  for (int j = 0; j < kBwdPer; ++j) {
+    const int64_t pi = begin + j * kBwdThreads + threadIdx.x;
+    bool keep = false;
+    if (pi < end) {
+      bool owned;
+      const int64_t a = point_antenna(p.offsets, p.A, pi, &owned);
+      if (!owned && p.status != nullptr) atomicExch(p.status, kStatusBadOffsets);
+      if (owned && (p.inb == nullptr || p.inb[pi])) {
+        float nrm[3], pt[3], txp[3], rxp[3];
+        ld3(p.normals, pi, nrm);
+        ld3(p.points, pi, pt);
+        ld3(p.tx, a, txp);
+        ld3(p.rx, a, rxp);
+        keep = !surely_culled(txp, rxp, nrm, pt);
+      }
+    }
+    const unsigned mask = __ballot_sync(0xffffffffu, keep);
+    int at = 0;
+    if (lane == 0 && mask != 0u) at = atomicAdd(&s_listed, __popc(mask));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (keep) list[at + __popc(mask & ((1u << lane) - 1u))] = j * kBwdThreads + static_cast<int>(threadIdx.x);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < s_listed; i += kBwdThreads) {
+    const int64_t pi = begin + list[i];
+    bool owned;
+    const int64_t a = point_antenna(p.offsets, p.A, pi, &owned);
+    float txp[3], rxp[3];
+    ld3(p.tx, a, txp);
+    ld3(p.rx, a, rxp);
+    const float inv_pa = 1.0f / static_cast<float>(p.offsets[a + 1] - p.offsets[a]);
+    const T* gr = p.gr + a * p.S;
+    const T* gi = p.gi + a * p.S;
+    const int S = static_cast<int>(p.S);
+    point_gradients<T, WITH_POINTS>(p, pi, txp, rxp, inv_pa, [&](float2 zeta, float2& q, float2& q1) {
+      residual_sums<WITH_POINTS>(
+          [=](int n, float4& re, float4& im) {
+            if (vector_rows) {
+              re = lds4(gr + n);
+              im = lds4(gi + n);
+            } else {
+              re = make_float4(ld_f(gr, n), n + 1 < S ? ld_f(gr, n + 1) : 0.0f, n + 2 < S ? ld_f(gr, n + 2) : 0.0f,
+                               n + 3 < S ? ld_f(gr, n + 3) : 0.0f);
+              im = make_float4(ld_f(gi, n), n + 1 < S ? ld_f(gi, n + 1) : 0.0f, n + 2 < S ? ld_f(gi, n + 2) : 0.0f,
+                               n + 3 < S ? ld_f(gi, n + 3) : 0.0f);
+            }
+          },
+          S > 0 ? ld : 0, zeta, q, q1);
+    });
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -524,6 +608,14 @@ cudaError_t launch_ragged_bwd(const RaggedArgs& a, const Tuning& t, cudaStream_t
   const void* fn = with_points ? reinterpret_cast<const void*>(&ragged_bwd_kernel<T, true>)
                                : reinterpret_cast<const void*>(&ragged_bwd_kernel<T, false>);
   auto aligned16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
+  if (a.P < kShortPoints * a.A) {
+    int vector_rows = a.S % 4 == 0 && aligned16(a.grad_real_out) && aligned16(a.grad_imag_out) ? 1 : 0;
+    const int64_t tiles = (a.P + kBwdTile - 1) / kBwdTile;
+    if (tiles > 0x7fffffff) return cudaErrorInvalidConfiguration;
+    if (with_points) ragged_bwd_short_kernel<T, true><<<static_cast<unsigned>(tiles), kBwdThreads, 0, st>>>(p, ld, vector_rows);
+    else ragged_bwd_short_kernel<T, false><<<static_cast<unsigned>(tiles), kBwdThreads, 0, st>>>(p, ld, vector_rows);
+    return cudaGetLastError();
+  }
   int aligned = aligned16(a.grad_sigmas) && aligned16(a.grad_normals) && aligned16(a.grad_points) ? 1 : 0;
   // Runs of consecutive points: a few per resident block, so that the last ones end together.
   const int64_t slots = static_cast<int64_t>(current_device_info().sm_count) * 6;

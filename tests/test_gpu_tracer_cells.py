@@ -178,3 +178,37 @@ def test_ragged_many_antennas(cuda, depth):
         got.append(counts[a] * x[a])
         ref.append(counts[a] * (r[0] + 1j * r[1])[0])
     assert rel_l2(np.array(got), np.array(ref)) < TOL
+
+
+# fewer than 48 points per antenna on average (rows read from device memory, 16 bytes at a time where
+# the samples allow it), and the most that is not
+@pytest.mark.parametrize("most,S", [(1, 64), (40, 33), (40, 36), (94, 64), (97, 64)])
+@pytest.mark.parametrize("dtype,with_points", [(torch.float32, True), (torch.float32, False), (torch.float64, True)])
+def test_ragged_adjoint_of_short_antennas(cuda, most, S, dtype, with_points):
+    from geraf_b200.ops.RFSignalTracer.ragged import signal_tracer_ragged
+
+    A = 210
+    rng = np.random.default_rng(most)
+    counts = np.full(A, 1) if most == 1 else rng.permutation(np.arange(A) * (most + 1) // A)  # 0 .. most
+    off = np.concatenate([[0], np.cumsum(counts)])
+    c = case(most, 1, int(off[-1]), S)
+    tx, rx = (x[:A].astype(np.float32) for x in scenes.virtual_array(5))
+    scal = float(c["fs"]), float(c["f0"]), float(c["As"])
+    t = [cu(c["normals"], dtype).requires_grad_(True), cu(c["sigmas"][0], dtype).requires_grad_(True),
+         cu(c["points"], dtype).requires_grad_(with_points)]
+    x = signal_tracer_ragged(*t, torch.tensor(off, device="cuda"), cu(tx, dtype), cu(rx, dtype), S, *scal,
+                             inbounds=torch.tensor(c["inbounds"], device="cuda"))
+    gr, gi = rng.standard_normal((2, A, S)).astype(np.float32)
+    got = torch.autograd.grad(x, t[:2 + with_points], (cu(gr, dtype), cu(gi, dtype)))
+    refs = [], [], []
+    scale = np.repeat(counts, counts)  # without its antenna's 1 / points, as above
+    for a in range(A):
+        e = slice(off[a], off[a + 1])
+        if counts[a]:
+            r = orc.tracer_backward(gr[a:a + 1], gi[a:a + 1], c["normals"][e], c["sigmas"][:, e], c["points"][e],
+                                    tx[a:a + 1], rx[a:a + 1], c["inbounds"][e], *scal)
+            for k, w in enumerate((r[0], r[1][0], r[2])):
+                refs[k].append(counts[a] * w)
+    for g, w in zip(got, refs):
+        g = g.double().cpu().numpy()
+        assert rel_l2(g * scale.reshape(-1, *[1] * (g.ndim - 1)), np.concatenate(w)) < TOL
