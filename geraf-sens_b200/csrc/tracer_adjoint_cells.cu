@@ -5,8 +5,9 @@
 //
 // Launches: the band of cells from the boxes of the listed points and of the
 // antennas, with the interpolation basis; the antennas' tables; the pairs.  Where the
-// band does not fit adj_cells() cells the pairs are left to the general kernel
-// (tracer_kernels.cu), which returns at once otherwise.
+// band does not fit adj_cells() cells, or has more than kFreeCells and too few points for
+// them, the pairs are left to the general kernel (tracer_kernels.cu), which returns at once
+// otherwise.
 #include <algorithm>
 #include <cmath>
 
@@ -19,12 +20,21 @@ namespace {
 using namespace tracer;
 
 constexpr int kQ = GatherCells::Q;
-// Cells per antenna: 9.6 m of path at 4 GHz swept; 2.4 m for large arrays, whose tables
-// would outgrow the rest of the call's memory.
-int64_t adj_cells(int64_t A) { return A <= 2048 ? 512 : 128; }
 constexpr int kBandThreads = 1024;
 constexpr int kTableThreads = 128;
 constexpr int kTableCells = 16;  // cells per block of the table kernel
+// Cells per antenna: 50 MB of tables, between 4096 (77 m of path at 4 GHz swept, several times
+// the unambiguous path of 1000 samples) and 128 (2.4 m, for large arrays).
+int64_t adj_cells(int64_t A) {
+  if (A > 2048) return 128;
+  return std::min<int64_t>(4096, (int64_t{1} << 20) / std::max<int64_t>(A, 1) / kTableCells * kTableCells);
+}
+// Up to this many cells cost little whatever the points; more are worth their tables from
+// kCellPoints listed points per cell on (64 antennas, 3200 cells, 26000 and 262144 points of 128
+// samples: 183 and 411 us, 186 and 1187 us by the general kernel; 5 points per cell: 97 us
+// against 86 us).
+constexpr int kFreeCells = 512;
+constexpr int kCellPoints = 8;
 constexpr int kPairThreads = 128;
 constexpr int kPairAnts = 32;    // antennas staged at a time
 
@@ -56,6 +66,7 @@ struct BandP {
   int64_t chunks, A;
   const T* tx;
   const T* rx;
+  const int* listed;
   AdjHead* head;
   float* basis;
   int max_cells;
@@ -126,7 +137,9 @@ __global__ void __launch_bounds__(kBandThreads) adj_band_kernel(const BandP<T> p
   const double lo = floor((sqrt(near[0]) + sqrt(near[1])) * p.c.kappa) - 1.0;
   const double hi = ceil((sqrt(far[0]) + sqrt(far[1])) * p.c.kappa) + 1.0;
   const bool none = box[0] > box[3];  // no listed point: no pairs either
-  const bool fits = none || (hi - lo + 1.0 <= p.max_cells && hi < 1073741824.0);  // false for NaN
+  const double cells = hi - lo + 1.0;
+  const bool fits = none || (cells <= p.max_cells && hi < 1073741824.0 &&  // false for NaN
+                             (cells <= kFreeCells || cells * kCellPoints <= *p.listed));
   p.head->bad = fits ? 0 : 1;
   p.head->k0 = fits && !none ? static_cast<int>(lo) : 0;
   p.head->cells = fits && !none ? static_cast<int>(hi - lo) + 1 : 0;
@@ -143,42 +156,45 @@ struct AdjTableP {
   AdjConsts c;
 };
 
-// Block (antenna, 16 cells): thread (cell, slice of 8) as in the matched filter's table.
+// Block (antenna, groups of 16 cells y, y + gridDim.y, ...): thread (cell, slice of 8) as in the
+// matched filter's table.
 template <typename T>
 __global__ void __launch_bounds__(kTableThreads) adj_table_kernel(const AdjTableP<T> p) {
   constexpr int kSlices = kTableThreads / kTableCells;
   __shared__ float2 red[kSlices][kTableCells][kQ];
-  const int cell = static_cast<int>(blockIdx.y) * kTableCells + threadIdx.x % kTableCells;
   const int cells = p.head->cells;
-  if (static_cast<int>(blockIdx.y) * kTableCells >= cells) return;
   const int64_t a = blockIdx.x;
   const int slice = threadIdx.x / kTableCells;
-  const double dk = fma(p.c.k1, static_cast<double>(p.head->k0 + cell) / p.c.kappa, p.c.b1);
   const double mid = 0.5 * (p.c.S - 1);
-  float2 acc[kQ];
+  for (int first = static_cast<int>(blockIdx.y) * kTableCells; first < cells; first += gridDim.y * kTableCells) {
+    const int cell = first + threadIdx.x % kTableCells;
+    const double dk = fma(p.c.k1, static_cast<double>(p.head->k0 + cell) / p.c.kappa, p.c.b1);
+    float2 acc[kQ];
 #pragma unroll
-  for (int q = 0; q < kQ; ++q) acc[q] = make_float2(0.0f, 0.0f);
-  for (int n = slice; n < p.c.S; n += kSlices) {
-    const double ph = (n - mid) * dk;
-    const float2 e = cis_cycles(static_cast<float>(ph - rint(ph)));
-    const float xr = ld_f(p.gr, a * p.c.S + n), xi = ld_f(p.gi, a * p.c.S + n);
-    const float2 v = make_float2(fmaf(xr, e.x, xi * e.y), fmaf(xi, e.x, -xr * e.y));
-    const float2 w = make_float2(v.y, -v.x);
+    for (int q = 0; q < kQ; ++q) acc[q] = make_float2(0.0f, 0.0f);
+    for (int n = slice; n < p.c.S; n += kSlices) {
+      const double ph = (n - mid) * dk;
+      const float2 e = cis_cycles(static_cast<float>(ph - rint(ph)));
+      const float xr = ld_f(p.gr, a * p.c.S + n), xi = ld_f(p.gi, a * p.c.S + n);
+      const float2 v = make_float2(fmaf(xr, e.x, xi * e.y), fmaf(xi, e.x, -xr * e.y));
+      const float2 w = make_float2(v.y, -v.x);
 #pragma unroll
-    for (int q = 0; q < kQ; ++q) {
-      const float g = p.basis[static_cast<int64_t>(n) * kQ + q];
-      acc[q] = ffma2(make_float2(g, g), (q & 1) ? w : v, acc[q]);
+      for (int q = 0; q < kQ; ++q) {
+        const float g = p.basis[static_cast<int64_t>(n) * kQ + q];
+        acc[q] = ffma2(make_float2(g, g), (q & 1) ? w : v, acc[q]);
+      }
     }
-  }
 #pragma unroll
-  for (int q = 0; q < kQ; ++q) red[slice][threadIdx.x % kTableCells][q] = acc[q];
-  __syncthreads();
-  float2* out = p.table + (a * p.max_cells + blockIdx.y * kTableCells) * kQ;
-  const int live = min(kTableCells, cells - static_cast<int>(blockIdx.y) * kTableCells);
-  for (int i = threadIdx.x; i < live * kQ; i += kTableThreads) {
-    float2 s = (&red[0][0][0])[i];
-    for (int k = 1; k < kSlices; ++k) s = fadd2(s, (&red[k][0][0])[i]);
-    out[i] = s;
+    for (int q = 0; q < kQ; ++q) red[slice][threadIdx.x % kTableCells][q] = acc[q];
+    __syncthreads();
+    float2* out = p.table + (a * p.max_cells + first) * kQ;
+    const int live = min(kTableCells, cells - first);
+    for (int i = threadIdx.x; i < live * kQ; i += kTableThreads) {
+      float2 s = (&red[0][0][0])[i];
+      for (int k = 1; k < kSlices; ++k) s = fadd2(s, (&red[k][0][0])[i]);
+      out[i] = s;
+    }
+    __syncthreads();
   }
 }
 
@@ -294,6 +310,7 @@ cudaError_t launch_adjoint(const TracerArgs& a, unsigned char* ws, PointList lis
   bp.A = a.A;
   bp.tx = static_cast<const T*>(a.tx);
   bp.rx = static_cast<const T*>(a.rx);
+  bp.listed = list.count;
   bp.head = head;
   bp.basis = reinterpret_cast<float*>(ws + l.basis);
   bp.max_cells = static_cast<int>(adj_cells(a.A));
@@ -308,7 +325,8 @@ cudaError_t launch_adjoint(const TracerArgs& a, unsigned char* ws, PointList lis
   tp.table = reinterpret_cast<float2*>(ws + l.table);
   tp.max_cells = bp.max_cells;
   tp.c = c;
-  adj_table_kernel<T><<<dim3(static_cast<unsigned>(a.A), static_cast<unsigned>(bp.max_cells / kTableCells)), kTableThreads, 0, st>>>(tp);
+  const unsigned groups = std::min(bp.max_cells, kFreeCells) / kTableCells;
+  adj_table_kernel<T><<<dim3(static_cast<unsigned>(a.A), groups), kTableThreads, 0, st>>>(tp);
 
   AdjPairP<T> pp;
   pp.normals = static_cast<const T*>(a.normals);

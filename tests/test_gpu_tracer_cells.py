@@ -212,3 +212,9 @@ def test_ragged_adjoint_of_short_antennas(cuda, most, S, dtype, with_points):
     for g, w in zip(got, refs):
         g = g.double().cpu().numpy()
         assert rel_l2(g * scale.reshape(-1, *[1] * (g.ndim - 1)), np.concatenate(w)) < TOL
+
+
+@pytest.mark.parametrize("precision", ["mixed", "nufft"])
+def test_adjoint_tables_of_more_cells(cuda, precision):
+    """640 cells with points enough for their tables (the general kernel takes them otherwise)."""
+    check(case(17, 5, 9000, 128, (0.3, 6.0)), precision)
