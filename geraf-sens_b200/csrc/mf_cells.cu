@@ -617,7 +617,7 @@ cudaError_t launch_cells_forward(const MfArgs& a, unsigned char* ws, const CellL
 // band of cells; the moments; the samples from the moments; the direct kernel,
 // which returns at once unless the band did not fit.
 constexpr int kMomentCap = 24 * MomentCells::kOver;  // cells: 1.8 m of path at 4 GHz swept
-constexpr int kBoxFloats = 20;                       // voxels, tx, rx: lo xyz, hi xyz; a NaN count; pad
+constexpr int kBoxFloats = 20;                       // voxels, tx, rx: lo xyz, hi xyz; not for the cells; pad
 
 struct MomentHead {
   int bad;
@@ -646,6 +646,8 @@ MomentLayout moment_layout(int64_t A, int64_t S, int splits, size_t partial_byte
 template <typename T>
 struct BoxP {
   const T* voxel;  // [3, N]
+  const T* gr;     // [N]
+  const T* gi;
   const T* tx;     // [A, 3]
   const T* rx;
   int64_t N, A;
@@ -666,7 +668,8 @@ __global__ void __launch_bounds__(256) moment_prep_kernel(const BoxP<T> p) {
 #pragma unroll
     for (int q = 0; q < Q; ++q) p.basis[n * Q + q] = g[q];
   }
-  float b[18], nan_antennas = 0.0f;
+  float b[18];
+  float out = 0.0f;  // 1: a NaN antenna, or an infinite gradient, of which the moments' sums would make a NaN
 #pragma unroll
   for (int c = 0; c < 18; ++c) b[c] = (c % 6) < 3 ? INFINITY : -INFINITY;
   auto add = [&](float* box, float x, int c) {
@@ -676,19 +679,20 @@ __global__ void __launch_bounds__(256) moment_prep_kernel(const BoxP<T> p) {
   for (int64_t v = gid; v < p.N; v += step) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) add(b, ld_f(p.voxel, c * p.N + v), c);
+    if (fabsf(ld_f(p.gr, v)) == INFINITY || fabsf(ld_f(p.gi, v)) == INFINITY) out = 1.0f;
   }
   for (int64_t a = gid; a < p.A; a += step) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const float t = ld_f(p.tx, a * 3 + c), r = ld_f(p.rx, a * 3 + c);
-      if (t != t || r != r) nan_antennas = 1.0f;
+      if (t != t || r != r) out = 1.0f;
       add(b + 6, t, c);
       add(b + 12, r, c);
     }
   }
 #pragma unroll
   for (int c = 0; c < 19; ++c) {
-    float x = c < 18 ? b[c < 18 ? c : 0] : nan_antennas;
+    float x = c < 18 ? b[c < 18 ? c : 0] : out;
     const bool low = c < 18 && (c % 6) < 3;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -1048,6 +1052,8 @@ cudaError_t launch_cells_backward(const MfArgs& a, unsigned char* ws, cudaStream
 
   BoxP<T> bp;
   bp.voxel = static_cast<const T*>(a.voxel);
+  bp.gr = static_cast<const T*>(a.grad_real_out);
+  bp.gi = static_cast<const T*>(a.grad_imag_out);
   bp.tx = static_cast<const T*>(a.tx);
   bp.rx = static_cast<const T*>(a.rx);
   bp.N = a.N;
@@ -1061,8 +1067,8 @@ cudaError_t launch_cells_backward(const MfArgs& a, unsigned char* ws, cudaStream
 
   MomentP<T> mp;
   mp.voxel = bp.voxel;
-  mp.gr = static_cast<const T*>(a.grad_real_out);
-  mp.gi = static_cast<const T*>(a.grad_imag_out);
+  mp.gr = bp.gr;
+  mp.gi = bp.gi;
   mp.tx = bp.tx;
   mp.rx = bp.rx;
   mp.moments = reinterpret_cast<float4*>(ws + l.moments);

@@ -150,7 +150,7 @@ struct AdjTableP {
   const T* gr;
   const T* gi;
   const float* basis;
-  const AdjHead* head;
+  AdjHead* head;
   float2* table;  // [A][max_cells][kQ]
   int max_cells;
   AdjConsts c;
@@ -176,6 +176,8 @@ __global__ void __launch_bounds__(kTableThreads) adj_table_kernel(const AdjTable
       const double ph = (n - mid) * dk;
       const float2 e = cis_cycles(static_cast<float>(ph - rint(ph)));
       const float xr = ld_f(p.gr, a * p.c.S + n), xi = ld_f(p.gi, a * p.c.S + n);
+      // an infinite residual is the general kernel's (the polynomial would make a NaN of it)
+      if (fabsf(xr) == INFINITY || fabsf(xi) == INFINITY) p.head->bad = 1;
       const float2 v = make_float2(fmaf(xr, e.x, xi * e.y), fmaf(xi, e.x, -xr * e.y));
       const float2 w = make_float2(v.y, -v.x);
 #pragma unroll

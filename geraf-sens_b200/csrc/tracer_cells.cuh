@@ -36,7 +36,10 @@ constexpr int kTraceWarps = kTraceThreads / 32;
 constexpr int kTracePer = 4;  // points per thread and screening pass
 constexpr int kTraceQ = MomentCells::Q;
 constexpr int kTraceSlots = 64;
-constexpr int kTraceEmpty = INT32_MIN + 1;  // no finite path has this cell
+constexpr int kTraceEmpty = INT32_MIN + 1;  // no path has this cell
+// Not for the cells, whose sums of powers would make a NaN of it: an infinite amplitude; or a
+// path whose cell's number no int holds (4e7 m at 4 GHz swept).
+constexpr int kTraceOut = INT32_MIN + 2;
 constexpr int kTraceRow = kTraceQ + 2;      // float2 per contribution row: 80 bytes, conflict-free
 
 constexpr double kTraceMinKappa = 1e-6;     // cells per metre
@@ -109,8 +112,8 @@ __device__ __forceinline__ void trace_begin(TraceSmem& sm) {
 }
 
 // One batch: thread t holds a live contribution w at cell k, offset x (or none).  False, on
-// every thread, when two cells want one slot, whatever the order of the threads: nothing of
-// the batch is then added, and with KEEP the slots are as they were.
+// every thread, when two cells want one slot, whatever the order of the threads, or one is
+// kTraceOut: nothing of the batch is then added, and with KEEP the slots are as they were.
 template <bool KEEP>
 __device__ __forceinline__ bool trace_batch(TraceSmem& sm, bool live, float2 w, int k, float x) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -140,7 +143,7 @@ __device__ __forceinline__ bool trace_batch(TraceSmem& sm, bool live, float2 w, 
     if (lane == 31) sm.start[kTraceSlots] = run;
   }
   __syncthreads();
-  const bool other = live && sm.tag[slot] != k;
+  const bool other = live && (sm.tag[slot] != k || k == kTraceOut);
   if (live) {  // the contribution row w x^q, at its place in cell order
     const int place = reinterpret_cast<const int*>(&sm.hist[slot])[warp] + rank;
     float4* dst = reinterpret_cast<float4*>(&sm.rows[place][0]);
@@ -210,7 +213,8 @@ __device__ __forceinline__ bool trace_point(const TraceConsts& c, const float* t
   if (!trace_path(txp, rxp, t, amp, d)) return false;
   const double ph = fma(d, c.K, c.b);
   const double u = d * c.kappa, ku = rint(u);
-  cell = fabs(ku) < 1073741824.0 ? static_cast<int>(ku) : 0;  // a non-finite path: w is NaN
+  if (fabs(ku) < 1073741824.0 && fabsf(amp) < INFINITY) cell = static_cast<int>(ku);
+  else cell = ku != ku || amp != amp ? 0 : kTraceOut;  // a NaN may go anywhere
   x = static_cast<float>(u - ku);
   const float2 e = cis_cycles_fast(static_cast<float>(ph - rint(ph)));
   w = make_float2(amp * e.x, amp * e.y);

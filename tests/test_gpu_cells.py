@@ -209,3 +209,23 @@ def test_backward_many_voxels_of_one_cell(cuda):
     r = orc.mf_backward(gr, gi, np.ascontiguousarray(tx[some]), np.ascontiguousarray(rx[some]), vox, some.size, S,
                         ch.adc_sample_rate, ch.As_sci)
     assert rel_l2((h[0] + 1j * h[1])[some] * A, (r[0] + 1j * r[1]) * some.size) < TOL + 3 * 8e-7
+
+
+@pytest.mark.parametrize("value,part", [(np.inf, 0), (-np.inf, 1)])
+def test_infinite_gradient(cuda, value, part):
+    """One infinite gradient leaves no finite sample, and the first one of every antenna (no
+    recurrence yet) infinite with the sign of the phase."""
+    c = case(41, 200, 64, 10000)
+    g = c["rng"].standard_normal((2, 10000)).astype(np.float32)
+    g[part, 100] = value
+    ch = c["ch"]
+    got = mf_backward(*g, c["tx"], c["rx"], c["vox"], 200, 64, ch.adc_sample_rate, ch.As_sci, "mixed")
+    assert not np.isfinite(got).any()
+    one = np.zeros((2, 1))
+    one[part] = np.sign(value)
+    ref = orc.mf_backward(*one, c["tx"], c["rx"], np.ascontiguousarray(c["vox"][:, 100:101]), 200, 64,
+                          ch.adc_sample_rate, ch.As_sci)
+    for x, r in zip(got, ref):
+        clear = np.abs(r[:, 0]) > 1e-3 / 200
+        assert clear.sum() > 150
+        np.testing.assert_array_equal(x[clear, 0], np.copysign(np.inf, r[clear, 0]))

@@ -218,3 +218,32 @@ def test_ragged_adjoint_of_short_antennas(cuda, most, S, dtype, with_points):
 def test_adjoint_tables_of_more_cells(cuda, precision):
     """640 cells with points enough for their tables (the general kernel takes them otherwise)."""
     check(case(17, 5, 9000, 128, (0.3, 6.0)), precision)
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf])
+@pytest.mark.parametrize("splits", [0, 1])
+def test_infinite_values(cuda, value, splits):
+    """An infinite sigma leaves no finite sample, and the first of every antenna (no recurrence yet)
+    infinite with the sign of the phase; so does an infinite residual at sample 0 with the gradients."""
+    A, P, S, q = 5, 3000, 64, 77
+    c = case(19, A, P, S)
+    c["inbounds"][q] = True
+    c["normals"][q] = -c["points"][q] / np.linalg.norm(c["points"][q])
+    geo = lambda e, sig: (c["normals"][e], sig, c["points"][e], c["tx"], c["rx"], c["inbounds"][e])
+    scal = float(c["fs"]), float(c["f0"]), float(c["As"])
+    d = dict(c, sigmas=c["sigmas"].copy())
+    d["sigmas"][:, q] = value
+    got = tracer_forward(d, S, "mixed", tuning={"splits": splits})
+    assert not np.isfinite(got).any()
+    e = slice(q, q + 1)
+    ref = orc.tracer_forward(*geo(e, np.full((A, 1), np.sign(value), np.float32)), S, *scal, "f64")
+    for x, r in zip(got, ref):
+        np.testing.assert_array_equal(x[:, 0], np.copysign(np.inf, r[:, 0]))
+    g = np.zeros((2, A, S), np.float32)
+    g[0, 2, 0] = value
+    got = tracer_backward(c, *g, "mixed", tuning={"splits": splits})[1]
+    unit = np.where(np.isinf(g), np.sign(g), 0).astype(np.float32)
+    ref = orc.tracer_backward(*unit, *geo(slice(None), c["sigmas"]), *scal)[1]
+    clear = np.abs(ref[2]) > 1e-3 * np.abs(ref[2]).max()
+    np.testing.assert_array_equal(got[2][clear], np.copysign(np.inf, ref[2][clear]))
+    np.testing.assert_array_equal(np.delete(got, 2, 0), 0)
