@@ -400,30 +400,21 @@ __global__ void __launch_bounds__(128) nufft_tracer_gather_kernel(const TrGather
   }
 }
 
+// W is 4 or 6: more taps go through the range cells (resolved_form).
 template <typename T, bool WP>
 const void* gather_ptr(int W) {
-  switch (W) {
-    case 4: return reinterpret_cast<const void*>(&nufft_tracer_gather_kernel<T, 4, WP>);
-    case 6: return reinterpret_cast<const void*>(&nufft_tracer_gather_kernel<T, 6, WP>);
-    case 10: return reinterpret_cast<const void*>(&nufft_tracer_gather_kernel<T, 10, WP>);
-    case 12: return reinterpret_cast<const void*>(&nufft_tracer_gather_kernel<T, 12, WP>);
-    default: return reinterpret_cast<const void*>(&nufft_tracer_gather_kernel<T, 8, WP>);
-  }
+  return W == 4 ? reinterpret_cast<const void*>(&nufft_tracer_gather_kernel<T, 4, WP>)
+                : reinterpret_cast<const void*>(&nufft_tracer_gather_kernel<T, 6, WP>);
 }
 
 template <typename T>
 const void* spread_ptr(int W) {
-  switch (W) {
-    case 4: return reinterpret_cast<const void*>(&nufft_tracer_spread_kernel<T, 4>);
-    case 6: return reinterpret_cast<const void*>(&nufft_tracer_spread_kernel<T, 6>);
-    case 10: return reinterpret_cast<const void*>(&nufft_tracer_spread_kernel<T, 10>);
-    case 12: return reinterpret_cast<const void*>(&nufft_tracer_spread_kernel<T, 12>);
-    default: return reinterpret_cast<const void*>(&nufft_tracer_spread_kernel<T, 8>);
-  }
+  return W == 4 ? reinterpret_cast<const void*>(&nufft_tracer_spread_kernel<T, 4>)
+                : reinterpret_cast<const void*>(&nufft_tracer_spread_kernel<T, 6>);
 }
 
 struct TrNufftShape {
-  int M = 16, Mp = 32, log2M = 4, h = 0, W = 8;
+  int M = 16, Mp = 32, log2M = 4, h = 0, W = 6;
   double beta = 0.0;
   // forward
   int vsplits = 1;
@@ -666,7 +657,6 @@ cudaError_t launch_tracer_nufft_backward(const TracerArgs& a, const Tuning& t, v
 Tuning tracer_nufft_forward_resolve(const TracerArgs& a, const Tuning& req) {
   Tuning t = req;
   t.threads = kSpreadThreads;
-  if (t.taps != 4 && t.taps != 6 && t.taps != 8 && t.taps != 10 && t.taps != 12) t.taps = 8;
   t.items = 1;
   t.stage_rows = 1;
   // point splits: at most kVoxelsPerThread points per thread and block, and
@@ -696,7 +686,6 @@ cudaError_t tracer_nufft_forward(const TracerArgs& a, const Tuning& t, void* ws,
 Tuning tracer_nufft_backward_resolve(const TracerArgs& a, const Tuning& req) {
   Tuning t = req;
   if (t.threads != 64 && t.threads != 128) t.threads = 128;
-  if (t.taps != 4 && t.taps != 6 && t.taps != 8 && t.taps != 10 && t.taps != 12) t.taps = 8;
   t.items = 1;
   // two antennas per grid stage: half the shared memory of four, so twice the
   // blocks fit each SM (measured: 128 antennas x 262144 points x 256 samples,
