@@ -821,7 +821,7 @@ def _tracer_extra(args, dev, art) -> dict:
 
     tuned = {}
     if not args.no_tune:
-        for op, run, cands in (("tracer_forward", fwd, autotune.sample_major_candidates()),
+        for op, run, cands in (("tracer_forward", fwd, autotune.tracer_forward_candidates()),
                                ("tracer_backward", bwd, autotune.tracer_backward_candidates())):
             default_ms = autotune.time_call(lambda run=run: run("mixed"), iters=5, warmup=2)
             best, results = autotune.tune(op, (At, St, P), _lib.MODE_MIXED,

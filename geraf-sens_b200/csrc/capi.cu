@@ -641,8 +641,8 @@ GERAF_EXPORT int32_t geraf_tracer_backward_ragged(
   a.f0 = start_frequency;
   a.As = chirp_slope_scaled;
   a.dtype = dtype;
-  return finish_launch(tracer_backward_ragged(a, tracer_ragged_backward_resolve(a, to_tuning(tuning)),
-                                              static_cast<cudaStream_t>(stream)),
+  (void)tuning;  // the blocks have one shape
+  return finish_launch(tracer_backward_ragged(a, static_cast<cudaStream_t>(stream)),
                        "signal_tracer_backward_ragged launch");
 }
 

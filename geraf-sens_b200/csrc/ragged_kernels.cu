@@ -600,8 +600,8 @@ cudaError_t launch_ragged_fwd(const RaggedArgs& a, const Tuning& t, void* ws, cu
 }
 
 template <typename T>
-cudaError_t launch_ragged_bwd(const RaggedArgs& a, const Tuning& t, cudaStream_t st) {
-  RgP<T> p = make_rg<T>(a, t, nullptr);
+cudaError_t launch_ragged_bwd(const RaggedArgs& a, cudaStream_t st) {
+  RgP<T> p = make_rg<T>(a, Tuning{}, nullptr);
   const int ld = static_cast<int>(((std::max<int64_t>(a.S, 1) + 3) / 4) * 4);
   const size_t smem = static_cast<size_t>(2 * ld) * sizeof(float);
   const bool with_points = a.grad_points != nullptr;
@@ -637,16 +637,6 @@ Tuning tracer_ragged_forward_resolve(const RaggedArgs& a, const Tuning& req) {
   return t;
 }
 
-Tuning tracer_ragged_backward_resolve(const RaggedArgs& a, const Tuning& req) {
-  Tuning t = req;
-  const int64_t ld = ((std::max<int64_t>(a.S, 1) + 3) / 4) * 4;
-  // staged rows within 48 KB of shared memory
-  const int cap = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(8, (48 * 1024) / (8 * ld))));
-  if (t.stage_rows <= 0) t.stage_rows = 4;
-  t.stage_rows = std::max(1, std::min(t.stage_rows, cap));
-  return t;
-}
-
 size_t tracer_ragged_workspace(int64_t A, int64_t S, int64_t P, const Tuning& t) {
   return ragged_layout(A, S, P, t).total;
 }
@@ -657,10 +647,10 @@ cudaError_t tracer_forward_ragged(const RaggedArgs& a, const Tuning& t, void* ws
   return launch_ragged_fwd<float>(a, t, ws, st);
 }
 
-cudaError_t tracer_backward_ragged(const RaggedArgs& a, const Tuning& t, cudaStream_t st) {
+cudaError_t tracer_backward_ragged(const RaggedArgs& a, cudaStream_t st) {
   if (a.P == 0) return cudaSuccess;
-  if (a.dtype == kF64) return launch_ragged_bwd<double>(a, t, st);
-  return launch_ragged_bwd<float>(a, t, st);
+  if (a.dtype == kF64) return launch_ragged_bwd<double>(a, st);
+  return launch_ragged_bwd<float>(a, st);
 }
 
 }  // namespace geraf

@@ -115,21 +115,27 @@ def mf_forward_candidates(mode: int) -> list[dict]:
 
 
 def sample_major_candidates() -> list[dict]:
-    """MF adjoint / tracer forward: threads x samples-per-lane."""
+    """MF adjoint: threads x samples-per-lane."""
     return [{"threads": t, "chunk": c} for t in (64, 128, 256) for c in (8, 16, 32)]
 
 
+def tracer_forward_candidates() -> list[dict]:
+    """Tracer forward: shares of an antenna's points (0: the library's choice)."""
+    return [{"splits": s} for s in (0, 1, 2, 4, 8, 16, 32, 64)]
+
+
 def tracer_backward_candidates() -> list[dict]:
-    return [{"threads": t, "stage_rows": r} for t in (64, 128) for r in (4, 8, 16)]
+    """Tracer adjoint: splits of the antennas (0: the library's choice); the threads shape the
+    kernel that takes the scenes without cell tables."""
+    return [{"threads": t, "splits": s} for t in (64, 128) for s in (0, 1, 2, 4, 8)]
 
 
 def ragged_forward_candidates() -> list[dict]:
-    """Batched tracer forward: threads x samples-per-lane x points per thread of a work item."""
-    return [{"threads": t, "chunk": c, "items_per_thread": i}
-            for t in (64, 128, 256) for c in (8, 16) for i in (16, 32)]
+    """Batched tracer forward: points of a work item, as threads x points per thread (0: the
+    library's choice)."""
+    return [{"threads": 128, "items_per_thread": i} for i in (0, 4, 8, 16, 32, 64)]
 
 
 def ragged_backward_candidates() -> list[dict]:
-    """Batched tracer adjoint: residual rows staged per block."""
-    return [{"stage_rows": r} for r in (1, 2, 4, 8)]
-
+    """Batched tracer adjoint: its blocks have one shape."""
+    return [{}]

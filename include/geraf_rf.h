@@ -257,7 +257,7 @@ int32_t geraf_tracer_forward_ragged(const void* normals, const void* sigmas, con
                                     size_t workspace_bytes, void* stream);
 /* Adjoint of geraf_tracer_forward_ragged: grad_sigmas [P], grad_normals [P,3]
  * and, when non-NULL, grad_points [P,3]; out-of-bounds points get zeros.
- * `tuning` (may be NULL): stage_rows = residual rows staged per block (1..8). 
+ * `tuning` (may be NULL) is accepted and changes nothing: the blocks have one shape.
  * Replaces the per-antenna SignalTracer::SignalTracer_backward_normal_sigma
  * calls (SignalTracer_cuda.cu:358-406). */
 int32_t geraf_tracer_backward_ragged(const void* grad_output_real, const void* grad_output_imag,

@@ -66,6 +66,17 @@ def test_autotune_cache_roundtrip(tmp_path, monkeypatch):
         assert c["threads"] in (64, 128, 256)
 
 
+def test_autotune_candidates_differ_in_what_the_kernels_read():
+    """The tracer forward reads `splits`, the batched forward the points of a work item, the batched
+    adjoint nothing: no list times one launch twice."""
+    splits = [c["splits"] for c in autotune.tracer_forward_candidates()]
+    assert len(set(splits)) == len(splits) > 1
+    items = [c["threads"] * c["items_per_thread"] for c in autotune.ragged_forward_candidates()]
+    assert len(set(items)) == len(items) > 1
+    assert len(autotune.ragged_backward_candidates()) == 1
+    assert {"threads", "splits"} <= set(autotune.tracer_backward_candidates()[0])
+
+
 def test_virtual_arrays_and_grids():
     tx, rx = scenes.virtual_array(16)
     assert tx.shape == (3072, 3) and rx.shape == (3072, 3) and tx.dtype == np.float32
