@@ -3,6 +3,7 @@ how many lanes share one, to the bit.  A call of many outputs takes one lane eac
 first rows or columns alone take 4, 8 or 32."""
 import numpy as np
 import pytest
+import torch
 
 from benchkit import scenes
 from gpu_helpers import mf_backward, mf_forward
@@ -54,3 +55,19 @@ def test_forward_bits_on_long_rows(cuda, S):
     for n in (257, 9001, 20003, 40001):
         for got, ref in zip(run(n), full):
             np.testing.assert_array_equal(got, ref[:n])
+
+
+# outputs in the middle of the range that takes 8 lanes (64 to 192 per SM), voxels in whole steps and not
+@pytest.mark.parametrize("N", [16, 33, 64, 300])
+def test_backward_bits_with_eight_lanes(cuda, N):
+    sms = torch.cuda.get_device_properties(cuda).multi_processor_count
+    A, S = 256, sms // 2
+    rng = np.random.default_rng(N)
+    tx, rx = scenes.virtual_array(18)
+    ch = scenes.chirp(S)
+    vox = rng.uniform((-0.1, -0.1, 0.3), (0.1, 0.1, 0.5), (N, 3)).T.astype(np.float32).copy()
+    gr, gi = rng.standard_normal((2, N)).astype(np.float32)
+    run = lambda a: mf_backward(gr, gi, tx[:a], rx[:a], vox, a, S, ch.adc_sample_rate, ch.As_sci, "plain")
+    full = run(2048 + A)  # one lane each
+    for got, ref in zip(run(A), full):
+        np.testing.assert_allclose(got * A, ref[:A] * (2048 + A), rtol=2e-7, atol=0)
