@@ -256,6 +256,8 @@ int resident_blocks(const void* fn, int threads, size_t smem);
 // Whether the tracer forwards' moments become samples by warps (tracer_cells.cuh, trace_finish_few):
 // antennas for several times the blocks that would otherwise take one each (two per SM).
 bool finish_by_warps(int64_t A, int64_t S, double kappa);
+// Launches such a kernel (one argument, tracer_cells.cuh's shared memory) as blocks that stay resident.
+cudaError_t launch_few(const void* fn, void* params, int64_t A, int64_t S, cudaStream_t st);
 
 // Picks the number of splits of the reduced dimension so that
 // `units * splits` blocks fill the GPU in near-whole waves.

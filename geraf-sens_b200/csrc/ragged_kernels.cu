@@ -593,8 +593,8 @@ cudaError_t launch_ragged_fwd(const RaggedArgs& a, const Tuning& t, void* ws, cu
     ragged_finish_kernel<T><<<dim3(static_cast<unsigned>(a.A), parts), kFinishThreads, 0, st>>>(p);
   } else {
     ragged_finish_long_kernel<T><<<dim3(static_cast<unsigned>(std::min<int64_t>(a.A, 2 * sms)), parts), kFinishThreads, 0, st>>>(p);
-    const int64_t by_warps = std::min<int64_t>((a.A + kFewThreads / 32 - 1) / (kFewThreads / 32), sms * 8);
-    ragged_finish_few_kernel<T><<<static_cast<unsigned>(by_warps), kFewThreads, few_smem_bytes(a.S), st>>>(p);
+    err = launch_few(reinterpret_cast<const void*>(&ragged_finish_few_kernel<T>), &p, a.A, a.S, st);
+    if (err != cudaSuccess) return err;
   }
   return cudaGetLastError();
 }

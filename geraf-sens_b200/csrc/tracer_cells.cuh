@@ -556,9 +556,10 @@ __device__ __forceinline__ void trace_finish(const TraceConsts& c, const TraceRe
 // for 32 samples at a time.  What depends on the sample alone is in shared memory too: its
 // basis, its phasor e^{j 2 pi n' b1}, and the cells' phasors, which are roots of unity: with
 // kappa = 2 S |k1|, cell k turns sample n by (2 n - S + 1) k / (4 S) cycles.  49152 antennas x 300
-// points x 64 samples: 1755 us by blocks of 1024 threads, 104 us so.
+// points x 64 samples: 1755 us by blocks of 1024 threads, 104 us so; 5739 x 1396 x 512, forward: 485 and
+// 137 us, 13347 x 9 x 512 in one batch: 1032 and 310 us.
 constexpr int kFewThreads = 128;
-constexpr int kFewSamples = 384;  // 46 KB of shared memory
+constexpr int kFewSamples = 1024;  // 94 KB of shared memory; the product of a turn and a cell stays below 2^24
 constexpr int kFewShares = 8;
 static_assert(MomentCells::kOver == 2, "cells of 1 / (2 S k1)");
 

@@ -866,6 +866,20 @@ bool finish_by_warps(int64_t A, int64_t S, double kappa) {
   return A >= 2 * static_cast<int64_t>(current_device_info().sm_count) && S <= kFewSamples && kappa > kTraceMinKappa;
 }
 
+cudaError_t launch_few(const void* fn, void* params, int64_t A, int64_t S, cudaStream_t st) {
+  const size_t smem = few_smem_bytes(S);
+  const DeviceInfo dev = current_device_info();
+  // blocks that shared memory lets stay, up to 8 per SM: each forms the table once
+  const int64_t resident = std::min<int64_t>(8, std::max<int64_t>(1, (dev.max_smem_optin + 1024) / (smem + 1024)));
+  const int64_t blocks = std::min<int64_t>((A + kFewThreads / 32 - 1) / (kFewThreads / 32), resident * dev.sm_count);
+  // one limit for all sizes: other threads may be launching the kernel at theirs
+  const cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(few_smem_bytes(kFewSamples)));
+  if (err != cudaSuccess) return err;
+  void* args[] = {params};
+  return cudaLaunchKernel(fn, dim3(static_cast<unsigned>(blocks)), dim3(kFewThreads), args, smem, st);
+}
+
 namespace {
 
 template <typename T>
@@ -906,11 +920,8 @@ cudaError_t launch_tracer_fwd(const TracerArgs& a, const Tuning& t, void* ws, cu
   }
   if (a.A * t.splits > 0x7fffffff) return cudaErrorInvalidConfiguration;
   tracer_fwd_cells_kernel<T><<<static_cast<unsigned>(a.A * t.splits), kTraceThreads, 0, st>>>(c);
-  const int sms = current_device_info().sm_count;
   if (finish_by_warps(a.A, a.S, c.c.kappa) && t.splits <= kFewShares) {
-    const int64_t blocks = std::min<int64_t>((a.A + kFewThreads / 32 - 1) / (kFewThreads / 32), sms * 8);
-    tracer_fwd_finish_few_kernel<T><<<static_cast<unsigned>(blocks), kFewThreads, few_smem_bytes(a.S), st>>>(c);
-    return cudaGetLastError();
+    return launch_few(reinterpret_cast<const void*>(&tracer_fwd_finish_few_kernel<T>), &c, a.A, a.S, st);
   }
   const dim3 grid(static_cast<unsigned>(a.A), static_cast<unsigned>((a.S + kFinishSamples - 1) / kFinishSamples));
   tracer_fwd_finish_kernel<T><<<grid, kFinishThreads, 0, st>>>(c);

@@ -247,3 +247,12 @@ def test_infinite_values(cuda, value, splits):
     clear = np.abs(ref[2]) > 1e-3 * np.abs(ref[2]).max()
     np.testing.assert_array_equal(got[2][clear], np.copysign(np.inf, ref[2][clear]))
     np.testing.assert_array_equal(np.delete(got, 2, 0), 0)
+
+
+@pytest.mark.parametrize("S", [700, 1024, 1025])
+def test_many_antennas_of_long_rows(cuda, S):
+    """The longest rows whose moments become samples by warps, and one longer."""
+    c = case(20, 300, 90, S)
+    tx, rx = scenes.virtual_array(6)
+    c["tx"], c["rx"] = tx[:300].astype(np.float32), rx[:300].astype(np.float32)
+    check(c, "mixed")
