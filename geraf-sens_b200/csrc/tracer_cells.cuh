@@ -560,7 +560,7 @@ __device__ __forceinline__ void trace_finish(const TraceConsts& c, const TraceRe
 // 137 us, 13347 x 9 x 512 in one batch: 1032 and 310 us.
 constexpr int kFewThreads = 128;
 constexpr int kFewSamples = 1024;  // 94 KB of shared memory; the product of a turn and a cell stays below 2^24
-constexpr int kFewShares = 8;
+constexpr int kFewShares = 16;
 static_assert(MomentCells::kOver == 2, "cells of 1 / (2 S k1)");
 
 struct FewWarp {
@@ -604,19 +604,33 @@ __device__ __forceinline__ FewTable few_table(const TraceConsts& c, unsigned cha
   return f;
 }
 
-// Used slots of a share into w; returns their number.
-__device__ __forceinline__ int few_slots(const TraceRecord& x, int M, FewWarp& w) {
+// Used slots of `shares` shares into w, their moments added up; returns their number, or -1
+// where two shares have other cells in a slot.
+__device__ __forceinline__ int few_slots(const TraceRecord* rec, int shares, int M, FewWarp& w) {
   const int lane = threadIdx.x & 31;
-  int used = 0;
+  int tag[kTraceSlots / 32], used = 0;
+  bool clash = false;
   __syncwarp();
 #pragma unroll
+  for (int h = 0; h < kTraceSlots / 32; ++h) tag[h] = rec[0].tag[h * 32 + lane];
+#pragma unroll 2
+  for (int r = 1; r < shares; ++r) {
+#pragma unroll
+    for (int h = 0; h < kTraceSlots / 32; ++h) {
+      const int t = rec[r].tag[h * 32 + lane];
+      if (t == kTraceEmpty) continue;
+      clash = clash || (tag[h] != kTraceEmpty && tag[h] != t);
+      tag[h] = t;
+    }
+  }
+  if (__any_sync(0xffffffffu, clash)) return -1;
+#pragma unroll
   for (int h = 0; h < kTraceSlots / 32; ++h) {
-    const int tag = x.tag[h * 32 + lane];
-    const unsigned set = __ballot_sync(0xffffffffu, tag != kTraceEmpty);
-    if (tag != kTraceEmpty) {
+    const unsigned set = __ballot_sync(0xffffffffu, tag[h] != kTraceEmpty);
+    if (tag[h] != kTraceEmpty) {
       const int e = used + __popc(set & ((1u << lane) - 1u));
       w.slot[e] = h * 32 + lane;
-      w.cell[e] = (tag % M + M) % M;
+      w.cell[e] = (tag[h] % M + M) % M;
     }
     used += __popc(set);
   }
@@ -624,7 +638,24 @@ __device__ __forceinline__ int few_slots(const TraceRecord& x, int M, FewWarp& w
   constexpr int kParts = kTraceQ / 2;
 #pragma unroll 2
   for (int i = lane; i < used * kParts; i += 32) {
-    w.moments[i / kParts][i % kParts] = reinterpret_cast<const float4*>(&x.moments[w.slot[i / kParts]][0])[i % kParts];
+    const int slot = w.slot[i / kParts];
+    const float4 first = reinterpret_cast<const float4*>(&rec[0].moments[slot][0])[i % kParts];
+    if (shares == 1) {
+      w.moments[i / kParts][i % kParts] = first;
+      continue;
+    }
+    double4 m = make_double4(0.0, 0.0, 0.0, 0.0);
+#pragma unroll 4
+    for (int r = 0; r < shares; ++r) {
+      const float4 y = reinterpret_cast<const float4*>(&rec[r].moments[slot][0])[i % kParts];
+      const bool take = rec[r].tag[slot] != kTraceEmpty;  // unused slots hold no moments
+      m.x += take ? y.x : 0.0f;
+      m.y += take ? y.y : 0.0f;
+      m.z += take ? y.z : 0.0f;
+      m.w += take ? y.w : 0.0f;
+    }
+    w.moments[i / kParts][i % kParts] =
+        make_float4(static_cast<float>(m.x), static_cast<float>(m.y), static_cast<float>(m.z), static_cast<float>(m.w));
   }
   __syncwarp();
   return used;
@@ -637,7 +668,9 @@ __device__ __forceinline__ void trace_finish_few(const TraceConsts& c, const Few
   const int M = 4 * c.S;
   const float inv_m = 1.0f / static_cast<float>(M);
   FewWarp& w = *f.warp;
-  int used = 0;
+  // the shares as one where their cells agree, as in all but deep scenes they do, else one by one
+  int used = shares > 0 ? few_slots(rec, shares, M, w) : 0;
+  const bool together = used >= 0;
   for (int n0 = 0; n0 < c.S; n0 += 32) {
     const int n = min(n0 + lane, c.S - 1);
     const int turn = 2 * n - c.S + 1 + (2 * n < c.S - 1 ? M : 0);
@@ -651,8 +684,8 @@ __device__ __forceinline__ void trace_finish_few(const TraceConsts& c, const Few
       g[q + 3] = y.w;
     }
     double2 acc = make_double2(0.0, 0.0);
-    for (int r = 0; r < shares; ++r) {
-      if (n0 == 0 || shares > 1) used = few_slots(rec[r], M, w);
+    for (int r = 0; r < (together ? 1 : shares); ++r) {
+      if (!together) used = few_slots(rec + r, 1, M, w);
       float2 sum = make_float2(0.0f, 0.0f);
 #pragma unroll 2
       for (int e = 0; e < used; ++e) {
@@ -671,9 +704,14 @@ __device__ __forceinline__ void trace_finish_few(const TraceConsts& c, const Few
         sum = fadd2(sum, cmul(f.root[root_at(i)], make_float2(ev.x - od.y, ev.y + od.x)));
       }
       sum = cmul(sum, f.offset[n]);
-      if (rec[r].has_row) sum = fadd2(sum, rows[static_cast<int64_t>(r) * c.S + n]);
       acc.x += sum.x;
       acc.y += sum.y;
+    }
+    for (int r = 0; r < shares; ++r) {
+      if (rec[r].has_row == 0) continue;
+      const float2 y = rows[static_cast<int64_t>(r) * c.S + n];
+      acc.x += y.x;
+      acc.y += y.y;
     }
     if (n0 + lane < c.S) {
       out_r[n] = from_f<T>(static_cast<float>(acc.x) / divisor);

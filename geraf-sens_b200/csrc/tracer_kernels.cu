@@ -1067,14 +1067,17 @@ Tuning tracer_forward_resolve(const TracerArgs& call, const Tuning& req) {
     t.splits = 1;
     return t;
   }
-  // MIXED: one block per (antenna, split of the points), at most a block per batch of points, or
-  // per 16384 points where the antennas fill the GPU by themselves (each share costs a
-  // record of its cells: 3072 antennas x 3000 points x 32 samples, 207 us with 6 splits, 78 us with one)
+  // MIXED: one block per (antenna, split of the points).  Each share costs a record of its cells, so
+  // one wave of blocks, or shares of 2048 points where those are more (632 antennas x 1774 points
+  // x 200 samples: 87 us with one, 322 us with a share per batch of 128; 1000 x 20000 x 128: 711 us with one,
+  // 493 us with 5); where the antennas fill the GPU, no more than the finish by warps adds up.
   const int64_t batches = std::max<int64_t>(1, (a.P + kTraceThreads - 1) / kTraceThreads);
   if (t.splits <= 0) {
     const int sms = current_device_info().sm_count;
-    const int64_t most = a.A >= 5 * static_cast<int64_t>(sms) ? std::max<int64_t>(1, a.P / 16384) : batches;
-    t.splits = pick_splits(std::max<int64_t>(1, a.A), 5, sms, most);
+    const int64_t antennas = std::max<int64_t>(1, a.A), wave = 5 * static_cast<int64_t>(sms);
+    int64_t most = std::max(wave / antennas, (a.P + 2047) / 2048);
+    if (antennas >= wave) most = std::min<int64_t>(most, kFewShares);
+    t.splits = pick_splits(antennas, 5, sms, std::min(most, batches));
   }
   t.splits = static_cast<int>(std::min<int64_t>(std::max(t.splits, 1), batches));
   return t;

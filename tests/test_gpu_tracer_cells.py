@@ -256,3 +256,17 @@ def test_many_antennas_of_long_rows(cuda, S):
     tx, rx = scenes.virtual_array(6)
     c["tx"], c["rx"] = tx[:300].astype(np.float32), rx[:300].astype(np.float32)
     check(c, "mixed")
+
+
+@pytest.mark.parametrize("depth,splits", [((0.3, 0.5), 16), ((0.3, 0.5), 17), ((0.3, 0.5), 0), ((0.3, 1.9), 5), ((0.3, 3.3), 5)],
+                         ids=["most", "more", "default", "cells_of_two_rounds", "deep"])
+def test_shares_of_many_antennas(cuda, depth, splits):
+    """The shares of an antenna are added up before they become samples, where their cells agree (up to 16
+    shares); in the deeper scenes they hold other cells in a slot, or rows beside cells."""
+    c = case(21, 300, 3000, 70, depth)
+    tx, rx = scenes.virtual_array(6)
+    c["tx"], c["rx"] = tx[:300].astype(np.float32), rx[:300].astype(np.float32)
+    order = np.argsort(np.linalg.norm(c["points"], axis=1))
+    for k in ("normals", "points", "inbounds"):
+        c[k] = np.ascontiguousarray(c[k][order])
+    check(c, "mixed", {"splits": splits})
