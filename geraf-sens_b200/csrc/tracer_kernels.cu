@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(128) tracer_bwd_plain_kernel(const TrP<T> p) {
 // registers allowed, measured on 64 antennas x 524288 points x 128 samples and
 // 128 antennas x 262144 points x 256 samples.
 template <typename T, bool WITH_POINTS>
-__global__ void __launch_bounds__(128, 6) tracer_bwd_mixed_kernel(const TrP<T> p) {
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : 6) tracer_bwd_mixed_kernel(const TrP<T> p) {
   constexpr int NC = WITH_POINTS ? 6 : 3;
   extern __shared__ __align__(128) unsigned char smem[];
   if (p.run_if != nullptr && *p.run_if == 0) return;
