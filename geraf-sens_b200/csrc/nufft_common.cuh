@@ -431,6 +431,7 @@ __global__ void __launch_bounds__(512) nufft_adjoint_fft_kernel(const AdjFftP<T>
   for (int64_t a = blockIdx.x; a < p.A; a += gridDim.x) {
     for (int l = threadIdx.x; l < M; l += blockDim.x) {
       float2 acc = make_float2(0.0f, 0.0f);
+#pragma unroll 8
       for (int vs = 0; vs < p.vsplits; ++vs) {
         const float2 v = p.grid[(static_cast<int64_t>(vs) * p.A + a) * M + l];
         acc.x += v.x;
