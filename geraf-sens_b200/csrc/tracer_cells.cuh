@@ -552,14 +552,14 @@ __device__ __forceinline__ void trace_finish(const TraceConsts& c, const TraceRe
 }
 
 // The same for many antennas of few shares each, where a block per antenna mostly waits: a warp
-// per antenna brings the used slots of a share together in shared memory and walks them
-// for 32 samples at a time.  What depends on the sample alone is in shared memory too: its
+// per antenna brings the used slots of its shares together in shared memory and walks them
+// for 64 samples at a time.  What depends on the sample alone is in shared memory too: its
 // basis, its phasor e^{j 2 pi n' b1}, and the cells' phasors, which are roots of unity: with
 // kappa = 2 S |k1|, cell k turns sample n by (2 n - S + 1) k / (4 S) cycles.  49152 antennas x 300
 // points x 64 samples: 1755 us by blocks of 1024 threads, 104 us so; 5739 x 1396 x 512, forward: 485 and
-// 137 us, 13347 x 9 x 512 in one batch: 1032 and 310 us.
-constexpr int kFewThreads = 128;
-constexpr int kFewSamples = 1024;  // 94 KB of shared memory; the product of a turn and a cell stays below 2^24
+// 125 us, 13347 x 9 x 512 in one batch: 1032 and 216 us (137 and 310 us with one sample per lane and 128 threads).
+constexpr int kFewThreads = 256;  // (128: 12 warps per SM at 512 samples, twice that so)
+constexpr int kFewSamples = 1024;  // 112 KB of shared memory; the product of a turn and a cell stays below 2^24
 constexpr int kFewShares = 16;
 static_assert(MomentCells::kOver == 2, "cells of 1 / (2 S k1)");
 
@@ -661,8 +661,9 @@ __device__ __forceinline__ int few_slots(const TraceRecord* rec, int shares, int
   return used;
 }
 
-template <typename T>
-__device__ __forceinline__ void trace_finish_few(const TraceConsts& c, const FewTable& f, const TraceRecord* rec,
+// kPer samples per lane share the reads of the moments.
+template <int kPer, typename T>
+__device__ __forceinline__ void finish_few_samples(const TraceConsts& c, const FewTable& f, const TraceRecord* rec,
                                                  const float2* rows, int shares, float divisor, T* out_r, T* out_i) {
   const int lane = threadIdx.x & 31;
   const int M = 4 * c.S;
@@ -671,53 +672,80 @@ __device__ __forceinline__ void trace_finish_few(const TraceConsts& c, const Few
   // the shares as one where their cells agree, as in all but deep scenes they do, else one by one
   int used = shares > 0 ? few_slots(rec, shares, M, w) : 0;
   const bool together = used >= 0;
-  for (int n0 = 0; n0 < c.S; n0 += 32) {
-    const int n = min(n0 + lane, c.S - 1);
-    const int turn = 2 * n - c.S + 1 + (2 * n < c.S - 1 ? M : 0);
-    float g[kTraceQ];
+  for (int n0 = 0; n0 < c.S; n0 += 32 * kPer) {
+    int n[kPer], turn[kPer];
+    float g[kPer][kTraceQ];
+    double2 acc[kPer];
 #pragma unroll
-    for (int q = 0; q < kTraceQ; q += 4) {
-      const float4 y = *reinterpret_cast<const float4*>(&f.basis[n * kTraceQ + q]);
-      g[q] = y.x;
-      g[q + 1] = y.y;
-      g[q + 2] = y.z;
-      g[q + 3] = y.w;
+    for (int u = 0; u < kPer; ++u) {
+      n[u] = min(n0 + 32 * u + lane, c.S - 1);
+      turn[u] = 2 * n[u] - c.S + 1 + (2 * n[u] < c.S - 1 ? M : 0);
+      acc[u] = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int q = 0; q < kTraceQ; q += 4) {
+        const float4 y = *reinterpret_cast<const float4*>(&f.basis[n[u] * kTraceQ + q]);
+        g[u][q] = y.x;
+        g[u][q + 1] = y.y;
+        g[u][q + 2] = y.z;
+        g[u][q + 3] = y.w;
+      }
     }
-    double2 acc = make_double2(0.0, 0.0);
     for (int r = 0; r < (together ? 1 : shares); ++r) {
       if (!together) used = few_slots(rec + r, 1, M, w);
-      float2 sum = make_float2(0.0f, 0.0f);
-#pragma unroll 2
-      for (int e = 0; e < used; ++e) {
-        // turn * cell mod M: a product below 2^24, its quotient off by one at most
-        const int product = turn * w.cell[e];
-        int i = product - static_cast<int>(static_cast<float>(product) * inv_m) * M;
-        i += i < 0 ? M : 0;
-        i -= i >= M ? M : 0;
-        float2 ev = make_float2(0.0f, 0.0f), od = make_float2(0.0f, 0.0f);
+      float2 sum[kPer];
 #pragma unroll
-        for (int q = 0; q < kTraceQ; q += 2) {
-          const float4 y = w.moments[e][q / 2];
-          ev = ffma2(make_float2(g[q], g[q]), make_float2(y.x, y.y), ev);
-          od = ffma2(make_float2(g[q + 1], g[q + 1]), make_float2(y.z, y.w), od);
+      for (int u = 0; u < kPer; ++u) sum[u] = make_float2(0.0f, 0.0f);
+      for (int e = 0; e < used; ++e) {
+        float4 y[kTraceQ / 2];
+#pragma unroll
+        for (int q = 0; q < kTraceQ / 2; ++q) y[q] = w.moments[e][q];
+        const int cell = w.cell[e];
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+          // turn * cell mod M: a product below 2^24, its quotient off by one at most
+          const int product = turn[u] * cell;
+          int i = product - static_cast<int>(static_cast<float>(product) * inv_m) * M;
+          i += i < 0 ? M : 0;
+          i -= i >= M ? M : 0;
+          float2 ev = make_float2(0.0f, 0.0f), od = make_float2(0.0f, 0.0f);
+#pragma unroll
+          for (int q = 0; q < kTraceQ; q += 2) {
+            ev = ffma2(make_float2(g[u][q], g[u][q]), make_float2(y[q / 2].x, y[q / 2].y), ev);
+            od = ffma2(make_float2(g[u][q + 1], g[u][q + 1]), make_float2(y[q / 2].z, y[q / 2].w), od);
+          }
+          sum[u] = fadd2(sum[u], cmul(f.root[root_at(i)], make_float2(ev.x - od.y, ev.y + od.x)));
         }
-        sum = fadd2(sum, cmul(f.root[root_at(i)], make_float2(ev.x - od.y, ev.y + od.x)));
       }
-      sum = cmul(sum, f.offset[n]);
-      acc.x += sum.x;
-      acc.y += sum.y;
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        sum[u] = cmul(sum[u], f.offset[n[u]]);
+        acc[u].x += sum[u].x;
+        acc[u].y += sum[u].y;
+      }
     }
     for (int r = 0; r < shares; ++r) {
       if (rec[r].has_row == 0) continue;
-      const float2 y = rows[static_cast<int64_t>(r) * c.S + n];
-      acc.x += y.x;
-      acc.y += y.y;
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        const float2 y = rows[static_cast<int64_t>(r) * c.S + n[u]];
+        acc[u].x += y.x;
+        acc[u].y += y.y;
+      }
     }
-    if (n0 + lane < c.S) {
-      out_r[n] = from_f<T>(static_cast<float>(acc.x) / divisor);
-      out_i[n] = from_f<T>(static_cast<float>(acc.y) / divisor);
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      if (n0 + 32 * u + lane >= c.S) continue;
+      out_r[n[u]] = from_f<T>(static_cast<float>(acc[u].x) / divisor);
+      out_i[n[u]] = from_f<T>(static_cast<float>(acc[u].y) / divisor);
     }
   }
+}
+
+template <typename T>
+__device__ __forceinline__ void trace_finish_few(const TraceConsts& c, const FewTable& f, const TraceRecord* rec,
+                                                 const float2* rows, int shares, float divisor, T* out_r, T* out_i) {
+  if (c.S > 32) finish_few_samples<2>(c, f, rec, rows, shares, divisor, out_r, out_i);
+  else finish_few_samples<1>(c, f, rec, rows, shares, divisor, out_r, out_i);
 }
 
 }  // namespace tracer

@@ -869,8 +869,8 @@ bool finish_by_warps(int64_t A, int64_t S, double kappa) {
 cudaError_t launch_few(const void* fn, void* params, int64_t A, int64_t S, cudaStream_t st) {
   const size_t smem = few_smem_bytes(S);
   const DeviceInfo dev = current_device_info();
-  // blocks that shared memory lets stay, up to 8 per SM: each forms the table once
-  const int64_t resident = std::min<int64_t>(8, std::max<int64_t>(1, (dev.max_smem_optin + 1024) / (smem + 1024)));
+  // blocks that registers (3) and shared memory let stay: each forms the table once
+  const int64_t resident = std::min<int64_t>(3, std::max<int64_t>(1, (dev.max_smem_optin + 1024) / (smem + 1024)));
   const int64_t blocks = std::min<int64_t>((A + kFewThreads / 32 - 1) / (kFewThreads / 32), resident * dev.sm_count);
   // one limit for all sizes: other threads may be launching the kernel at theirs
   const cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
