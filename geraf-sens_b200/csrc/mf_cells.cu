@@ -156,7 +156,7 @@ template <typename T>
 __global__ void __launch_bounds__(kTableThreads) mf_cell_table_kernel(const TableP<T> p) {
   constexpr int Q = GatherCells::Q;
   __shared__ float box_s[6];
-  __shared__ int band_s[2];
+  __shared__ int band_s[2], skip_s;
   __shared__ float2 smp[kTableTile];
   __shared__ float bas[kTableTile * Q];
   __shared__ float2 red[kTableThreads * Q];
@@ -164,8 +164,11 @@ __global__ void __launch_bounds__(kTableThreads) mf_cell_table_kernel(const Tabl
   if (threadIdx.x < 32) {
     const float b = warp_bbox(p.bbox, p.blocks, threadIdx.x);
     if (threadIdx.x < 6) box_s[threadIdx.x] = b;
+  } else if (threadIdx.x == 32) {
+    skip_s = *reinterpret_cast<const volatile int*>(&p.head->bad);  // one answer for the whole block
   }
   __syncthreads();
+  if (skip_s) return;  // an earlier antenna's cells did not fit
   if (threadIdx.x == 0) {
     double t[3], r[3], box[6];
     AntMeta m;
