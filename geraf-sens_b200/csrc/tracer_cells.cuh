@@ -332,9 +332,22 @@ __device__ __forceinline__ bool trace_screened(TraceSmem& sm, const TraceConsts&
 constexpr int kDirectK = 16;
 constexpr int kDirectGroups = 16;
 
+// Antennas of so few points take it as a whole where there are many of them: a point costs at most 2 S
+// slots there, a cell about 35 S when the moments become samples, and the record between the two
+// kernels goes.  Forward of 8853 antennas x 39 points x 128 samples, 10 m deep, 128 us through
+// the cells and 60 so, 3072 x 384 x 128 64 and 58 us; past that the cells win (3072 x 384 x 512, all live: 100 and 143 us,
+// but 68 and 45 with a tenth of 256 points live).  The batched tracer keeps its short antennas in the cells (13347 of 9
+// points x 512: 219 us, 310 so).
+constexpr int kDirectPoints = 384;
+
 struct DirectSmem {
-  float2 seeds[kDirectGroups][kTraceThreads];
-  float2 zeta[kTraceThreads];
+  union {
+    struct {
+      float2 seeds[kDirectGroups][kTraceThreads];
+      float2 zeta[kTraceThreads];
+    };
+    float2 red[kDirectK * (kTraceThreads + kDirectGroups)];  // [G K][L + 1], off each other's banks
+  };
   int counts[kTraceWarps];
 };
 
@@ -401,17 +414,25 @@ __device__ __forceinline__ void trace_direct(DirectSmem& sm, const TraceConsts& 
       for (int m = 0; m < K; ++m) sum[m] = fadd2(sum[m], acc[m]);
       __syncthreads();
     }
-    float2* red = &sm.seeds[0][0];  // [G K][L]
 #pragma unroll
-    for (int m = 0; m < K; ++m) red[(group * K + m) * L + in_group] = sum[m];
+    for (int m = 0; m < K; ++m) sm.red[(group * K + m) * (L + 1) + in_group] = sum[m];
     __syncthreads();
-    for (int i = threadIdx.x; i < G * K && n0 + i < c.S; i += kTraceThreads) {
+    // few samples: several lanes of a warp to a sum (one pass over the sums then)
+    const int per = max(1, kTraceThreads / (G * K));
+    for (int i = threadIdx.x / per; i < G * K; i += kTraceThreads / per) {
       double2 x = make_double2(0.0, 0.0);
-      for (int k = 0; k < L; ++k) {
-        x.x += red[i * L + k].x;
-        x.y += red[i * L + k].y;
+      for (int k = threadIdx.x % per; k < L; k += per) {
+        const float2 y = sm.red[i * (L + 1) + k];
+        x.x += y.x;
+        x.y += y.y;
       }
-      store(n0 + i, make_float2(static_cast<float>(x.x), static_cast<float>(x.y)));
+      for (int o = per / 2; o > 0; o >>= 1) {
+        x.x += __shfl_xor_sync(0xffffffffu, x.x, o);
+        x.y += __shfl_xor_sync(0xffffffffu, x.y, o);
+      }
+      if (n0 + i < c.S && threadIdx.x % per == 0) {
+        store(n0 + i, make_float2(static_cast<float>(x.x), static_cast<float>(x.y)));
+      }
     }
     __syncthreads();
   }

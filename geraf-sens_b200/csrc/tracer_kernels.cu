@@ -207,6 +207,26 @@ __global__ void __launch_bounds__(kTraceThreads, 5) tracer_fwd_cells_kernel(cons
   if (from < end) share_direct(smem.direct, p, blockIdx.x, from, end);
 }
 
+// Many antennas of up to kDirectPoints points: a block per antenna, without cells.
+template <typename T>
+__global__ void __launch_bounds__(kTraceThreads) tracer_fwd_short_kernel(const __grid_constant__ TrCellP<T> p) {
+  __shared__ DirectSmem sm;
+  const int64_t a = blockIdx.x;
+  const int64_t count = p.plist != nullptr ? static_cast<int64_t>(*p.plist_count) : p.P;
+  float txp[3], rxp[3];
+  load3(p.tx, a, txp);
+  load3(p.rx, a, rxp);
+  const float divisor = static_cast<float>(p.P);
+  trace_direct<T>(
+      sm, p.c, p.normals, p.points, txp, rxp, count,
+      [&](int64_t pos) -> int64_t { return p.plist != nullptr ? p.plist[pos] : p.inb[pos] ? pos : -1; },
+      [&](int64_t q) { return ld_f(p.sigmas, a * p.P + q); },
+      [&](int n, float2 y) {
+        p.out_r[a * p.c.S + n] = from_f<T>(y.x / divisor);
+        p.out_i[a * p.c.S + n] = from_f<T>(y.y / divisor);
+      });
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kFinishThreads) tracer_fwd_finish_kernel(const TrCellP<T> p) {
   const int64_t a = blockIdx.x;
@@ -882,6 +902,11 @@ cudaError_t launch_few(const void* fn, void* params, int64_t A, int64_t S, cudaS
 
 namespace {
 
+// Forward calls that tracer_fwd_short_kernel takes: two blocks per SM or more.
+bool short_antennas(const TracerArgs& a) {
+  return a.P <= kDirectPoints && a.A >= 2 * static_cast<int64_t>(current_device_info().sm_count);
+}
+
 template <typename T>
 cudaError_t launch_tracer_fwd(const TracerArgs& a, const Tuning& t, void* ws, cudaStream_t st) {
   TrP<T> p = make_params<T>(a);
@@ -919,6 +944,10 @@ cudaError_t launch_tracer_fwd(const TracerArgs& a, const Tuning& t, void* ws, cu
     c.plist_count = pl.count;
   }
   if (a.A * t.splits > 0x7fffffff) return cudaErrorInvalidConfiguration;
+  if (t.splits == 1 && short_antennas(a)) {
+    tracer_fwd_short_kernel<T><<<static_cast<unsigned>(a.A), kTraceThreads, 0, st>>>(c);
+    return cudaGetLastError();
+  }
   tracer_fwd_cells_kernel<T><<<static_cast<unsigned>(a.A * t.splits), kTraceThreads, 0, st>>>(c);
   if (finish_by_warps(a.A, a.S, c.c.kappa) && t.splits <= kFewShares) {
     return launch_few(reinterpret_cast<const void*>(&tracer_fwd_finish_few_kernel<T>), &c, a.A, a.S, st);
@@ -1077,6 +1106,7 @@ Tuning tracer_forward_resolve(const TracerArgs& call, const Tuning& req) {
     const int64_t antennas = std::max<int64_t>(1, a.A), wave = 5 * static_cast<int64_t>(sms);
     int64_t most = std::max(wave / antennas, (a.P + 2047) / 2048);
     if (antennas >= wave) most = std::min<int64_t>(most, kFewShares);
+    if (short_antennas(a)) most = 1;
     t.splits = pick_splits(antennas, 5, sms, std::min(most, batches));
   }
   t.splits = static_cast<int>(std::min<int64_t>(std::max(t.splits, 1), batches));

@@ -270,3 +270,21 @@ def test_shares_of_many_antennas(cuda, depth, splits):
     for k in ("normals", "points", "inbounds"):
         c[k] = np.ascontiguousarray(c[k][order])
     check(c, "mixed", {"splits": splits})
+
+
+# many antennas of so few points that the cells are left out: no point in bounds, one point, the most
+# (384) and one more; samples that leave several lanes to a sum (16, 32, 64), remainders, two sweeps
+@pytest.mark.parametrize("P,S", [(1, 16), (7, 1), (384, 33), (385, 33), (200, 70), (130, 300), (384, 1030)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_many_antennas_of_so_few_points(cuda, P, S, dtype):
+    c = case(22, 300, P, S)
+    tx, rx = scenes.virtual_array(6)
+    c["tx"], c["rx"] = tx[:300].astype(np.float32), rx[:300].astype(np.float32)
+    c["inbounds"][0] = True
+    geo = (c["normals"], c["sigmas"], c["points"], c["tx"], c["rx"], c["inbounds"])
+    x = tracer_forward(c, S, "mixed", dtype=dtype)
+    r = orc.tracer_forward(*geo, S, float(c["fs"]), float(c["f0"]), float(c["As"]), "f64")
+    assert rel_l2(x[0] + 1j * x[1], r[0] + 1j * r[1]) < TOL
+    c["inbounds"][:] = False
+    for got in tracer_forward(c, S, "mixed", dtype=dtype):
+        np.testing.assert_array_equal(got, 0)
