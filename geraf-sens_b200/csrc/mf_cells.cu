@@ -783,7 +783,8 @@ __device__ __forceinline__ void red_add4(float4* dst, float2 a, float2 b) {
 // record in memory (vector reductions without a return value: nothing waits for
 // them, and no other thread touches the record, so the order of its sums, and the
 // result, is the same on every run).  About 88 instructions per 32 pairs (100 where the
-// antennas share no positions) at 68% of the issue slots: 972 antennas x 201 samples x
+// antennas share no positions) at 68% of the issue slots (FMA pipe 40%, XU 20%, FP64 11%;
+// 14 warps per SM): 972 antennas x 201 samples x
 // 50653 voxels take 0.19 ms here, 2.37 ms by the recurrence of the direct kernel.
 constexpr int kMomentTile = 128;
 constexpr int kMomentUnroll = 4;  // voxels whose paths overlap (2: 2% slower; 6 blocks per SM and one: 8%)
@@ -1110,10 +1111,11 @@ cudaError_t launch_cells_backward(const MfArgs& a, unsigned char* ws, cudaStream
 
 // The cells take over where the pairs outweigh the tables and the extra
 // launches: enough voxels per table row, and a direct call of more than ~20 us.
-// Calls of up to 128 antennas, the size of a training step's chunk, keep the
-// direct kernel: the gradient of |y| divides by |y|, which turns the ~2e-6 between
-// the two kernels (the direct one's error near theta = 0) into 3e-5 of the
-// gradients, more than a training run should move by from one release to the next.
+// MIXED forwards of up to 128 antennas keep the direct kernel although the cells are the faster and the
+// more exact form there too (128 antennas x 256 samples, points along 2048 rays: 1.33 ms against about a
+// fifth): the gradient of |y| divides by |y|, which turns the direct kernel's ~2e-6 near theta = 0 into 3e-5
+// of a training step's gradients.  The line is drawn for the sake of those values; nothing in the
+// kernels asks for it.
 // The NUFFT form goes the same way from 8 taps on (fewer taps are a coarser form
 // of their own), its forward with the accurate phasor (64-bit error 1.3e-7 by 8 taps,
 // 1.2e-7 so, 1.7e-7 with the hardware phasor; the adjoint's 1.1e-6 becomes 5e-7 either way).

@@ -291,11 +291,10 @@ __device__ __forceinline__ void point_gradients(const RgP<T>& p, int64_t pi, con
 // points are on their way, lists those the test cannot cull and, a full block of
 // them at a time, gives them the exact geometry and the residual sums (packed
 // even/odd Horner over the antenna's row in shared memory).
-// The sums stay a recurrence over the samples here: the cell polynomials of
-// tracer_gradients.cuh would need tables, for which a call has no workspace (formed per
-// block in shared memory they took 309 us against 365 us here, on 64 antennas x 295000
-// points, 10% live, x 256 samples, and moved the largest gradients by up to 1e-3 of
-// their norm, the recurrence's own error).  404 us with 1024-point blocks that each
+// The sums stay a recurrence over the samples here, the less exact form: the cell polynomials
+// of tracer_gradients.cuh err by up to 3.7e-5 in single gradients, the recurrence by up to 4.8e-4.  They
+// need tables, for which this entry point has no workspace; formed per block in shared memory they took
+// 309 us against 365 us here (64 antennas x 295000 points, 10% live, x 256 samples).  404 us with 1024-point blocks that each
 // looked their antenna up first and stored zeros point by point.
 constexpr int kBwdThreads = 128;
 constexpr int kBwdPer = 4;

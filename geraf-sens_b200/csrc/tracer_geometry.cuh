@@ -1,7 +1,9 @@
 // Specular geometry of the lensless signal tracer, shared by the tracer
 // kernels (reference: geraf/ops/RFSignalTracer/csrc/signal_tracer/SignalTracer_cuda_kernel.cu:19-197).
-// Everything is evaluated in the reference's FP32 operation order, so
-// amplitudes and culling decisions match the reference bit for bit.
+// specular_geometry and path_distance keep the reference's FP32 order of operations: the PLAIN
+// form's amplitudes and culling decisions match the reference bit for bit.  The MIXED and
+// NUFFT forms' culling does too; their amplitudes (pair_geometry, without divisions and square
+// roots) agree to a few ulp.
 #pragma once
 
 #include "common.cuh"

@@ -9,11 +9,11 @@
 // (reference: geraf/ops/RFSignalTracer/csrc/signal_tracer/SignalTracer_cuda_kernel.cu:19-197, 351-587).
 //
 // The reference recomputes the specular geometry for every (point, antenna,
-// sample) triple.  Here the geometry is formed once per (point, antenna) --
-// in the reference's FP32 operation order, so amplitudes and culling decisions
-// are bit-identical -- and the sample loop works on (amplitude, delay) only.
-// PLAIN forms then evaluate the reference's per-sample phase with accurate
-// cosf/sinf in its summation order.  MIXED forms reduce the carrier phase in FP64
+// sample) triple.  Here the geometry is formed once per (point, antenna) and the
+// sample loop works on (amplitude, delay) only.  PLAIN forms keep the reference's
+// FP32 order of operations, so that amplitudes and culling decisions are bit-identical, and
+// evaluate its per-sample phase with accurate cosf/sinf in its summation order.  MIXED forms
+// decide culling to the same bit (pair_geometry), reduce the carrier phase in FP64
 // and sum the samples through range cells: the forward collects the points'
 // moments per cell of path length (tracer_cells.cuh), the adjoint reads tables of
 // the residual's sum (tracer_adjoint_cells.cu).  The adjoint of this file, a Horner
