@@ -23,18 +23,21 @@ constexpr int kQ = GatherCells::Q;
 constexpr int kBandThreads = 1024;
 constexpr int kTableThreads = 256;  // (128: 4 us more for few antennas)
 constexpr int kTableCells = 16;  // cells per block of the table kernel
-// Cells per antenna: 50 MB of tables, between 4096 (77 m of path at 4 GHz swept, several times
-// the unambiguous path of 1000 samples) and 128 (2.4 m, for large arrays).
-int64_t adj_cells(int64_t A) {
-  if (A > 2048) return 128;
-  return std::min<int64_t>(4096, (int64_t{1} << 20) / std::max<int64_t>(A, 1) / kTableCells * kTableCells);
-}
 // Up to this many cells cost little whatever the points; more are worth their tables from
 // kCellPoints listed points per cell on (64 antennas, 3200 cells, 26000 and 262144 points of 128
 // samples: 183 and 411 us, 186 and 1187 us by the general kernel; 5 points per cell: 97 us
 // against 86 us).
 constexpr int kFreeCells = 512;
 constexpr int kCellPoints = 8;
+// Cells that a call has room for, per antenna: those that its points can be worth (the tables of 169
+// antennas and 4 points would take 50 MB otherwise, not 4), up to 4096 (77 m of path at 4 GHz swept, several
+// times the unambiguous path of 1000 samples) and 100 MB of tables; 128 (2.4 m) for large arrays.
+int64_t adj_cells(int64_t A, int64_t P) {
+  if (A > 2048) return 128;
+  const int64_t room = (int64_t{1} << 21) / std::max<int64_t>(A, 1);
+  const int64_t worth = std::max<int64_t>(kFreeCells, (P + kCellPoints - 1) / kCellPoints);
+  return std::min(std::min<int64_t>(4096, room), worth + kTableCells - 1) / kTableCells * kTableCells;
+}
 constexpr int kPairThreads = 128;
 constexpr int kPairAnts = 32;    // antennas staged at a time
 
@@ -56,7 +59,7 @@ AdjLayout adj_layout(const TracerArgs& a) {
   l.boxes = 256;
   l.basis = up256(l.boxes + static_cast<size_t>(tracer_point_chunks(a.P)) * 6 * sizeof(float));
   l.table = up256(l.basis + static_cast<size_t>(a.S) * kQ * sizeof(float));
-  l.total = up256(l.table + static_cast<size_t>(a.A) * adj_cells(a.A) * kQ * sizeof(float2));
+  l.total = up256(l.table + static_cast<size_t>(a.A) * adj_cells(a.A, a.P) * kQ * sizeof(float2));
   return l;
 }
 
@@ -321,7 +324,7 @@ cudaError_t launch_adjoint(const TracerArgs& a, unsigned char* ws, PointList lis
   bp.listed = list.count;
   bp.head = head;
   bp.basis = reinterpret_cast<float*>(ws + l.basis);
-  bp.max_cells = static_cast<int>(adj_cells(a.A));
+  bp.max_cells = static_cast<int>(adj_cells(a.A, a.P));
   bp.c = c;
   adj_band_kernel<T><<<1, kBandThreads, 0, st>>>(bp);
 

@@ -194,3 +194,17 @@ def test_public_signatures_match_reference():
                                               "nomralization"]
     assert positional(bilinear_raysample_cuda) == ["normals", "sigmas", "z_vals", "tgt_z_vals",
                                                    "N_ant", "N_ray", "Nz", "Nz_tgt"]
+
+
+def test_tracer_adjoint_workspace_follows_the_points():
+    """Tables of cells only as far as the points are worth them: 512 cells of 48 bytes per antenna for few
+    points, 4096 for many, 100 MB at most, 128 cells for large arrays; the point list and partials beside them."""
+    from geraf_b200 import _lib
+
+    query = lambda A, P: _lib.workspace_bytes("geraf_tracer_backward_workspace_bytes", A, 101, P, 0, _lib.MODE_MIXED, 1, None)
+    few, many = query(169, 4), query(169, 400_000)
+    assert 169 * 512 * 48 <= few < 169 * 512 * 48 + (1 << 20)
+    assert many > 169 * 4096 * 48
+    for A in (1, 64, 512, 513, 2048):
+        assert query(A, 4) < 100_700_000 + (1 << 20)
+    assert query(2049, 4) < 2049 * 128 * 48 + (1 << 20)
