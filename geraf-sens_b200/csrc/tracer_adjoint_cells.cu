@@ -22,7 +22,7 @@ using namespace tracer;
 constexpr int kQ = GatherCells::Q;
 constexpr int kBandThreads = 1024;
 constexpr int kTableThreads = 256;  // (128: 4 us more for few antennas)
-constexpr int kTableCells = 16;  // cells per block of the table kernel
+constexpr int kTableCells = 16;  // cells per block of the table kernel, at most
 // Up to this many cells cost little whatever the points; more are worth their tables from
 // kCellPoints listed points per cell on (64 antennas, 3200 cells, 26000 and 262144 points of 128
 // samples: 183 and 411 us, 186 and 1187 us by the general kernel; 5 points per cell: 97 us
@@ -38,6 +38,7 @@ int64_t adj_cells(int64_t A, int64_t P) {
   const int64_t worth = std::max<int64_t>(kFreeCells, (P + kCellPoints - 1) / kCellPoints);
   return std::min(std::min<int64_t>(4096, room), worth + kTableCells - 1) / kTableCells * kTableCells;
 }
+constexpr int kFewAntennas = 64;  // for tables of 4 cells a block
 constexpr int kPairThreads = 128;
 constexpr int kPairAnts = 32;    // antennas staged at a time
 
@@ -76,17 +77,22 @@ struct BandP {
   AdjConsts c;
 };
 
-// One block.  Lane groups of 32 x 18 box components would leave most of a block idle on
-// long chunk lists, so every thread reduces all components over its share.
+// The first block bounds the band; lane groups of 32 x 18 box components would leave most of it idle on
+// long chunk lists, so every thread reduces all components over its share.  The others form the
+// basis, kBasisSamples each (all of it in the one block took 20 us for 1000 samples).
+constexpr int kBasisSamples = 64;
 template <typename T>
 __global__ void __launch_bounds__(kBandThreads) adj_band_kernel(const BandP<T> p) {
   __shared__ float red[kBandThreads / 32][18];
   __shared__ float box[18];
-  for (int n = threadIdx.x; n < p.c.S; n += kBandThreads) {
+  if (blockIdx.x > 0) {
+    const int n = (blockIdx.x - 1) * kBasisSamples + threadIdx.x;
+    if (threadIdx.x >= kBasisSamples || n >= p.c.S) return;
     float g[kQ];
     cell_basis<kQ>(p.c.theta_step * (n - 0.5 * (p.c.S - 1)), g);
 #pragma unroll
     for (int q = 0; q < kQ; ++q) p.basis[static_cast<int64_t>(n) * kQ + q] = g[q];
+    return;
   }
   float b[18];
 #pragma unroll
@@ -159,18 +165,20 @@ struct AdjTableP {
   AdjConsts c;
 };
 
-// Block (antenna, groups of 16 cells y, y + gridDim.y, ...): thread (cell, slice of 16) as in the
-// matched filter's table.
-template <typename T>
+// Block (antenna, groups of CELLS cells y, y + gridDim.y, ...): thread (cell, slice of the samples) as in the
+// matched filter's table.  A thread is one chain of its slice's samples, so few antennas take 4
+// cells and 64 slices: the adjoint of 1 antenna x 4096 points x 1000 samples 43 us with 16 cells, 27 us so, 48 x
+// 100000 x 1000 72 and 55 us, but 64 x 524288 x 128 151 and 152, 250 x 100000 x 128 123 and 135.
+template <typename T, int CELLS>
 __global__ void __launch_bounds__(kTableThreads) adj_table_kernel(const AdjTableP<T> p) {
-  constexpr int kSlices = kTableThreads / kTableCells;
-  __shared__ float2 red[kSlices][kTableCells][kQ];
+  constexpr int kSlices = kTableThreads / CELLS;
+  __shared__ float2 red[kSlices][CELLS][kQ];
   const int cells = p.head->cells;
   const int64_t a = blockIdx.x;
-  const int slice = threadIdx.x / kTableCells;
+  const int slice = threadIdx.x / CELLS;
   const double mid = 0.5 * (p.c.S - 1);
-  for (int first = static_cast<int>(blockIdx.y) * kTableCells; first < cells; first += gridDim.y * kTableCells) {
-    const int cell = first + threadIdx.x % kTableCells;
+  for (int first = static_cast<int>(blockIdx.y) * CELLS; first < cells; first += gridDim.y * CELLS) {
+    const int cell = first + threadIdx.x % CELLS;
     const double dk = fma(p.c.k1, static_cast<double>(p.head->k0 + cell) / p.c.kappa, p.c.b1);
     float2 acc[kQ];
 #pragma unroll
@@ -190,10 +198,10 @@ __global__ void __launch_bounds__(kTableThreads) adj_table_kernel(const AdjTable
       }
     }
 #pragma unroll
-    for (int q = 0; q < kQ; ++q) red[slice][threadIdx.x % kTableCells][q] = acc[q];
+    for (int q = 0; q < kQ; ++q) red[slice][threadIdx.x % CELLS][q] = acc[q];
     __syncthreads();
     float2* out = p.table + (a * p.max_cells + first) * kQ;
-    const int live = min(kTableCells, cells - first);
+    const int live = min(CELLS, cells - first);
     for (int i = threadIdx.x; i < live * kQ; i += kTableThreads) {
       // slices in fours, then the fours
       float2 s = make_float2(0.0f, 0.0f);
@@ -326,7 +334,7 @@ cudaError_t launch_adjoint(const TracerArgs& a, unsigned char* ws, PointList lis
   bp.basis = reinterpret_cast<float*>(ws + l.basis);
   bp.max_cells = static_cast<int>(adj_cells(a.A, a.P));
   bp.c = c;
-  adj_band_kernel<T><<<1, kBandThreads, 0, st>>>(bp);
+  adj_band_kernel<T><<<1 + (c.S + kBasisSamples - 1) / kBasisSamples, kBandThreads, 0, st>>>(bp);
 
   AdjTableP<T> tp;
   tp.gr = static_cast<const T*>(a.grad_real_out);
@@ -336,8 +344,9 @@ cudaError_t launch_adjoint(const TracerArgs& a, unsigned char* ws, PointList lis
   tp.table = reinterpret_cast<float2*>(ws + l.table);
   tp.max_cells = bp.max_cells;
   tp.c = c;
-  const unsigned groups = std::min(bp.max_cells, kFreeCells) / kTableCells;
-  adj_table_kernel<T><<<dim3(static_cast<unsigned>(a.A), groups), kTableThreads, 0, st>>>(tp);
+  const unsigned antennas = static_cast<unsigned>(a.A), cells = std::min(bp.max_cells, kFreeCells);
+  if (a.A < kFewAntennas) adj_table_kernel<T, 4><<<dim3(antennas, cells / 4), kTableThreads, 0, st>>>(tp);
+  else adj_table_kernel<T, kTableCells><<<dim3(antennas, cells / kTableCells), kTableThreads, 0, st>>>(tp);
 
   AdjPairP<T> pp;
   pp.normals = static_cast<const T*>(a.normals);

@@ -288,3 +288,10 @@ def test_many_antennas_of_so_few_points(cuda, P, S, dtype):
     c["inbounds"][:] = False
     for got in tracer_forward(c, S, "mixed", dtype=dtype):
         np.testing.assert_array_equal(got, 0)
+
+
+# the adjoint's tables by 4 cells a block (fewer than 64 antennas) and by 16: samples that leave slices
+# without one, and remainders of the basis's blocks of 64
+@pytest.mark.parametrize("A,S", [(1, 32), (1, 1000), (2, 65), (63, 129), (64, 129)])
+def test_adjoint_tables_of_few_antennas(cuda, A, S):
+    check(case(23, A, 2000, S), "mixed")
