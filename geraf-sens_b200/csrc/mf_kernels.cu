@@ -716,16 +716,22 @@ __global__ void __launch_bounds__(128, 6) mf_bwd_plain_kernel(const MfBwdP<T> p)
     if constexpr (LANES == 1) {
       // two voxels at a time, whose sines and cosines overlap; none for the threads past the samples (they
       // ran along before: 2865 antennas x 64 samples x 616 voxels 351 us, 5267 x 30 x 611 613 us)
-      for (int i0 = 0; active && i0 < count; i0 += 2) {
+      int i0 = 0;
+      for (; active && i0 + 1 < count; i0 += 2) {
         float term_r[2], term_i[2];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) term(min(i0 + u, count - 1), term_r[u], term_i[u]);
-        acc_r = __fadd_rn(acc_r, term_r[0]);
-        acc_i = __fadd_rn(acc_i, term_i[0]);
-        if (i0 + 1 < count) {
-          acc_r = __fadd_rn(acc_r, term_r[1]);
-          acc_i = __fadd_rn(acc_i, term_i[1]);
+        for (int u = 0; u < 2; ++u) term(i0 + u, term_r[u], term_i[u]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          acc_r = __fadd_rn(acc_r, term_r[u]);
+          acc_i = __fadd_rn(acc_i, term_i[u]);
         }
+      }
+      if (active && i0 < count) {  // the last of an odd number
+        float term_r, term_i;
+        term(i0, term_r, term_i);
+        acc_r = __fadd_rn(acc_r, term_r);
+        acc_i = __fadd_rn(acc_i, term_i);
       }
       __syncthreads();
     } else {
