@@ -579,9 +579,7 @@ template <typename T>
 cudaError_t launch_ragged_fwd(const RaggedArgs& a, const Tuning& t, void* ws, cudaStream_t st) {
   RgP<T> p = make_rg<T>(a, t, ws);
   ragged_prep_kernel<T><<<1, 1024, 0, st>>>(p);
-  int per_sm = 0;
-  cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, &ragged_fwd_kernel<T>, kTraceThreads, 0);
-  if (err != cudaSuccess) return err;
+  const int per_sm = resident_blocks(reinterpret_cast<const void*>(&ragged_fwd_kernel<T>), kTraceThreads, 0);
   const int64_t blocks = std::max<int64_t>(
       1, std::min<int64_t>(static_cast<int64_t>(per_sm) * current_device_info().sm_count, p.max_items));
   ragged_fwd_kernel<T><<<static_cast<unsigned>(blocks), kTraceThreads, 0, st>>>(p);
@@ -592,7 +590,7 @@ cudaError_t launch_ragged_fwd(const RaggedArgs& a, const Tuning& t, void* ws, cu
     ragged_finish_kernel<T><<<dim3(static_cast<unsigned>(a.A), parts), kFinishThreads, 0, st>>>(p);
   } else {
     ragged_finish_long_kernel<T><<<dim3(static_cast<unsigned>(std::min<int64_t>(a.A, 2 * sms)), parts), kFinishThreads, 0, st>>>(p);
-    err = launch_few(reinterpret_cast<const void*>(&ragged_finish_few_kernel<T>), &p, a.A, a.S, st);
+    const cudaError_t err = launch_few(reinterpret_cast<const void*>(&ragged_finish_few_kernel<T>), &p, a.A, a.S, st);
     if (err != cudaSuccess) return err;
   }
   return cudaGetLastError();
