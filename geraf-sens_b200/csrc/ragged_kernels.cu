@@ -142,13 +142,38 @@ __device__ __forceinline__ void item_range(const RgP<T>& p, int64_t item, int64_
   count = min(p.offsets[a + 1] - first, static_cast<int64_t>(p.chunk));
 }
 
+// Row of an item whose cells do not fit their slots.
+template <typename T>
+__device__ __forceinline__ void item_direct(DirectSmem& sm, const RgP<T>& p, int64_t item) {
+  int64_t a, first, count;
+  item_range(p, item, a, first, count);
+  float txp[3], rxp[3];
+  ld3(p.tx, a, txp);
+  ld3(p.rx, a, rxp);
+  trace_direct<T>(
+      sm, p.c, p.normals, p.points, txp, rxp, count,
+      [&](int64_t pos) -> int64_t { return p.inb == nullptr || p.inb[first + pos] ? first + pos : -1; },
+      [&](int64_t q) { return ld_f(p.sigmas, q); }, [&](int n, float2 y) { p.rows[item * p.c.S + n] = y; });
+}
+// (Not inlined: it would take registers from the cells.)
+template <typename T>
+static __device__ __noinline__ void item_direct_call(DirectSmem& sm, const RgP<T>& p, int64_t item) {
+  item_direct(sm, p, item);
+}
+
 // Each work item's points go into the moments of their cells (tracer_cells.cuh).
 // 64 antennas x 295000 points each (10% live) x 256 samples: 173 us against 590 us with
 // a recurrence over the samples of every live point and a compaction per 128 points.
-template <typename T>
-__global__ void __launch_bounds__(kTraceThreads, 6) ragged_fwd_kernel(const RgP<T> p) {
-  __shared__ TraceSmem sm;
+// An item whose cells do not fit their slots leaves a row instead: by ROWS from here, else from
+// ragged_fwd_direct_kernel.
+template <typename T, bool ROWS>
+__global__ void __launch_bounds__(kTraceThreads, 6) ragged_fwd_kernel(const __grid_constant__ RgP<T> p) {
+  __shared__ union {
+    TraceSmem cells;
+    DirectSmem direct;
+  } smem;
   __shared__ long long s_item;
+  TraceSmem& sm = smem.cells;
   const int64_t total = p.item_offsets[p.A];
   for (;;) {
     if (threadIdx.x == 0) s_item = static_cast<long long>(atomicAdd(p.counter, 1ull));
@@ -163,30 +188,24 @@ __global__ void __launch_bounds__(kTraceThreads, 6) ragged_fwd_kernel(const RgP<
     trace_begin(sm);
     const bool fits = trace_screened<T>(sm, p.c, p.normals + first * 3, p.points + first * 3, p.sigmas + first,
                                         p.inb != nullptr ? p.inb + first : nullptr, txp, rxp, static_cast<int>(count));
-    if (!fits) {  // no cells: the record is a row, from ragged_fwd_direct_kernel
+    if (!fits) {  // no cells
       for (int i = threadIdx.x; i < kTraceSlots; i += kTraceThreads) sm.tag[i] = kTraceEmpty;
     }
     trace_store(sm, p.records + item, !fits);
+    if (ROWS && !fits) item_direct_call(smem.direct, p, item);
   }
 }
 
-// The items whose cells do not fit their slots; a launch without any reads their records'
-// flags alone.  (Within the kernel above it would take registers from the cells: 3 to 35%.)
+// The rows of calls of many items; a launch without any reads their records' flags alone.  (Within the
+// kernel above it takes registers from the cells: 64 antennas x 100000 points x 256 samples, forward and
+// adjoint, 235 -> 272 us.  Calls of an item per block are bound by their launches, so one fewer counts for
+// more there: 8 to 32 antennas x 19000 to 63000 points 157 -> 155 us.)
 template <typename T>
 __global__ void __launch_bounds__(kTraceThreads) ragged_fwd_direct_kernel(const RgP<T> p) {
   __shared__ DirectSmem sm;
   const int64_t total = p.item_offsets[p.A];
   for (int64_t item = blockIdx.x; item < total; item += gridDim.x) {
-    if (p.records[item].has_row == 0) continue;
-    int64_t a, first, count;
-    item_range(p, item, a, first, count);
-    float txp[3], rxp[3];
-    ld3(p.tx, a, txp);
-    ld3(p.rx, a, rxp);
-    trace_direct<T>(
-        sm, p.c, p.normals, p.points, txp, rxp, count,
-        [&](int64_t pos) -> int64_t { return p.inb == nullptr || p.inb[first + pos] ? first + pos : -1; },
-        [&](int64_t q) { return ld_f(p.sigmas, q); }, [&](int n, float2 y) { p.rows[item * p.c.S + n] = y; });
+    if (p.records[item].has_row != 0) item_direct(sm, p, item);
   }
 }
 
@@ -579,11 +598,14 @@ template <typename T>
 cudaError_t launch_ragged_fwd(const RaggedArgs& a, const Tuning& t, void* ws, cudaStream_t st) {
   RgP<T> p = make_rg<T>(a, t, ws);
   ragged_prep_kernel<T><<<1, 1024, 0, st>>>(p);
-  const int per_sm = resident_blocks(reinterpret_cast<const void*>(&ragged_fwd_kernel<T>), kTraceThreads, 0);
-  const int64_t blocks = std::max<int64_t>(
-      1, std::min<int64_t>(static_cast<int64_t>(per_sm) * current_device_info().sm_count, p.max_items));
-  ragged_fwd_kernel<T><<<static_cast<unsigned>(blocks), kTraceThreads, 0, st>>>(p);
-  ragged_fwd_direct_kernel<T><<<static_cast<unsigned>(blocks), kTraceThreads, 0, st>>>(p);
+  const int per_sm = resident_blocks(reinterpret_cast<const void*>(&ragged_fwd_kernel<T, false>), kTraceThreads, 0);
+  const int64_t resident = std::max<int64_t>(1, static_cast<int64_t>(per_sm) * current_device_info().sm_count);
+  if (p.max_items <= resident) {
+    ragged_fwd_kernel<T, true><<<static_cast<unsigned>(p.max_items), kTraceThreads, 0, st>>>(p);
+  } else {
+    ragged_fwd_kernel<T, false><<<static_cast<unsigned>(resident), kTraceThreads, 0, st>>>(p);
+    ragged_fwd_direct_kernel<T><<<static_cast<unsigned>(resident), kTraceThreads, 0, st>>>(p);
+  }
   const int64_t sms = current_device_info().sm_count;
   const unsigned parts = static_cast<unsigned>((a.S + kFinishSamples - 1) / kFinishSamples);
   if (!finish_by_warps(a.A, a.S, p.c.kappa)) {

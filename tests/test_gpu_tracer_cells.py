@@ -295,3 +295,24 @@ def test_many_antennas_of_so_few_points(cuda, P, S, dtype):
 @pytest.mark.parametrize("A,S", [(1, 32), (1, 1000), (2, 65), (63, 129), (64, 129)])
 def test_adjoint_tables_of_few_antennas(cuda, A, S):
     check(case(23, A, 2000, S), "mixed")
+
+
+# more work items than the GPU holds blocks: rows of items past their cells from a kernel of their own
+@pytest.mark.parametrize("depth", [(0.3, 0.5), (0.3, 3.3)], ids=["near", "deep"])
+def test_ragged_items_past_the_resident_blocks(cuda, depth):
+    from geraf_b200.ops.RFSignalTracer.ragged import signal_tracer_ragged
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    P = 256 * 6 * sms + 129  # items of 256 points
+    c = case(24, 2, P, 33, depth)
+    off = [0, P - 700, P]
+    scal = float(c["fs"]), float(c["f0"]), float(c["As"])
+    x = signal_tracer_ragged(cu(c["normals"]), cu(c["sigmas"][0]), cu(c["points"]), torch.tensor(off, device="cuda"),
+                             cu(c["tx"]), cu(c["rx"]), c["S"], *scal, inbounds=torch.tensor(c["inbounds"], device="cuda"),
+                             tuning={"items_per_thread": 2})
+    x = x[0].cpu().numpy() + 1j * x[1].cpu().numpy()
+    for a in range(2):
+        e = slice(off[a], off[a + 1])
+        r = orc.tracer_forward(c["normals"][e], c["sigmas"][:1, e], c["points"][e], c["tx"][a:a + 1], c["rx"][a:a + 1],
+                               c["inbounds"][e], c["S"], *scal, "f64")
+        assert rel_l2(x[a], (r[0] + 1j * r[1])[0]) < TOL
